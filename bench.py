@@ -54,7 +54,7 @@ def parse():
                    help="time the headline modes only (no block widths, workloads or comparison): for profiling")
     p.add_argument("--rhs", type=int, default=0, help="solve only the first RHS (a smaller case for profiling)")
     p.add_argument("--lane-warps", type=int, default=0,
-                   help="jacobian: the lane solve at this many warps per block instead of the autotuner's pick "
+                   help="jacobian: the lane solve at this many warps per block instead of the automatic choice "
                         "(a fixed kernel for profiling)")
     p.add_argument("--workload", default="ptdf", choices=["ptdf", "n1", "adjoint", "complex", "jacobian"],
                    help="ptdf: the headline PTDF block with the other workloads as extra keys; n1, adjoint, complex, jacobian: "
@@ -354,8 +354,8 @@ def workload_complex(gpu, steps: int, warm: int, rank: int, world: int, device: 
 def workload_jacobian(gpu, steps: int, warm: int, rank: int, world: int, device: int, lane_warps: int = 0) -> dict:
     """The Newton-Raphson Jacobian of the 10,000-bus complex network (order 17,998, AMD LU on the
     host; the reference's other matrix for its GPU survey): 4,096 right-hand sides, device arrays,
-    FP64, split over the ranks by columns; the autotuner picks the solve, or `lane_warps` fixes the
-    lane solve's blocks."""
+    FP64, split over the ranks by columns; the automatic choice, or the lane solve with `lane_warps`
+    warps a block."""
     import torch
 
     from ybus_b200 import FP64, GpuFactor, configs, replicas
@@ -368,7 +368,7 @@ def workload_jacobian(gpu, steps: int, warm: int, rank: int, world: int, device:
         factor.set_lane(FP64, lane_warps)
         tuned = {"kind": 5, "tile": 0, "warps": lane_warps, "fixed": True}
     else:
-        tuned = factor.autotune(FP64, rhs.shape[0])  # as a caller would, once per factor
+        tuned = {"kind": 0, **factor.spread_info(FP64, rhs.shape[0])}
     b = torch.from_numpy(rhs).cuda()
     x = torch.empty_like(b)
     # a stream of our own: the legacy default stream's handle is 0, which the C ABI reads as the
@@ -394,7 +394,7 @@ def workload_jacobian(gpu, steps: int, warm: int, rank: int, world: int, device:
             "unit": "RHS/s", "higher_is_better": True, "ms_per_step": ms,
             "config": {"n_bus": sysj.n_bus, "order": int(sysj.lu.n), "lu_entries": int(sysj.lu.l.idx.size + sysj.lu.u.idx.size),
                        "rhs": int(sysj.rhs.shape[0]), "split": f"columns over {world} GPU(s)",
-                       "autotuned": {k: v for k, v in tuned.items() if k != "ms"}}}
+                       "solve": tuned}}
 
 
 WORKLOADS = {"n1": workload_n1, "adjoint": workload_adjoint, "complex": workload_complex, "jacobian": workload_jacobian}
@@ -514,23 +514,18 @@ def main():
         return replicas.max_over_ranks(elapsed_ms), launch_ms, kernels
 
     # which solve each mode runs (the library's automatic choice, read back from its settings)
-    lane = lane32 = None
-    try:
-        lane = factor.lane_info(FP64)
-    except Exception:
-        pass
+    lane32 = None
     try:
         lane32 = factor.lane_info(FP32)
     except Exception:
         pass
-    lane_min, refine_min = factor.lane_min_count(FP64), factor.refine_lane_min_count()
-    use_lane = lane is not None and count >= lane_min and lane["slots"] <= 64
+    refine_min = factor.refine_lane_min_count()
     use_lane32 = lane32 is not None and count >= max(refine_min, factor.lane_min_count(FP32)) and lane32["slots"] <= 64
 
     def solver_of(mode):
-        if mode == "fp64" and use_lane:
-            return {"solver": "lane", "kernel": "lane_solve_kernel<double>", "launches_per_step": 3,
-                    "lane": {k: lane[k] for k in ("warps", "slots", "domains", "top", "pages", "smem")}}
+        if mode == "fp64":  # gather, forward sweep, the top's sums and product, backward sweep, scatter
+            return {"solver": "spread", "kernel": "spread_sweep_kernel<double>", "launches_per_step": 6,
+                    "spread": factor.spread_info(FP64, count)}
         if mode == "fp32_ir" and use_lane32:
             # an initialisation and the gather, per pass a solve, a residual (the update folded
             # in), a decision and the restore of columns a pass made no better, and between passes
@@ -538,9 +533,8 @@ def main():
             return {"solver": "lane", "kernel": "lane_solve_kernel<float>",
                     "launches_per_step": 2 + 4 * (IR_MAX_STEPS + 1) + max(0, IR_MAX_STEPS - 1),
                     "lane": {k: lane32[k] for k in ("warps", "slots", "domains", "top", "pages", "smem")}}
-        prec = FP64 if mode == "fp64" else FP32
         return {"solver": "domain", "kernel": "domain_tile_kernel", "launches_per_step": 1,
-                "tile": factor.domain_info(prec)["tile"]}
+                "tile": factor.domain_info(FP32)["tile"]}
 
     from oracle import oracle as orc  # the checker, outside the timed regions
     p, i, v = bp.arrays()
@@ -562,15 +556,14 @@ def main():
     time.sleep(0.3)
     results = {}
     for mode in modes:
-        on_lane = mode == "fp64" and use_lane
-        elapsed_ms, launch_ms, kernels = timed(lambda: solve(mode), lane_timing=on_lane)
+        elapsed_ms, launch_ms, kernels = timed(lambda: solve(mode), lane_timing=mode == "fp64")
         r = check(mode, {"rhs_s": total * a.steps / (elapsed_ms / 1e3), "ms_per_step": elapsed_ms / a.steps,
                          "launch_ms": launch_ms})
         steps_mean = r.get("mean_corrections", 0.0)
         r["algorithmic_bytes_per_launch"] = algorithmic_bytes(n, count, info, mode, steps_mean, len(i))
         r.update(solver_of(mode))
-        # the dominant kernel's own launch time where the library records it (the lane solve), else
-        # the step's launches
+        # the solve's own time between gather and scatter where the library records it (its sweeps and
+        # the top), else the step's launches
         r["kernel_ms"] = launch_ms
         if kernels:
             r["kernels"] = kernels
@@ -595,9 +588,8 @@ def main():
                 steps_w = max(3, min(a.steps, 10))
                 elapsed_ms, launch_ms, _ = timed(lambda: blocks(mode, width), steps=steps_w)
                 r = check(mode, {"rhs_s": total * steps_w / (elapsed_ms / 1e3), "ms_per_step": elapsed_ms / steps_w,
-                                 "launches_per_step": -(-count // width)})
-                r["solver"] = solver_of(mode)["solver"] if width >= (lane_min if mode == "fp64" else refine_min) \
-                    else "domain"
+                                 "launches_per_step": -(-count // width) * (6 if mode == "fp64" else 1)})
+                r["solver"] = solver_of(mode)["solver"] if mode == "fp64" or width >= refine_min else "domain"
                 by_width[str(width)][mode] = r
     clock_info = clocks.stop()
 

@@ -88,8 +88,9 @@ int32_t yb_factor_plan_info(const yb_factor *f, int32_t *fwd_levels, int32_t *bw
  * of two; threads a multiple of 32 up to 512; resident blocks per SM 1..8). */
 int32_t yb_factor_set_tile(yb_factor *f, int32_t precision, int32_t tile_width, int32_t threads,
                            int32_t blocks_per_sm);
-/* No ybus counterpart: which tile solve runs for a precision: 0 automatic (the lane solve for
- * solves of at least the lane threshold's right-hand sides when the factor admits it; else the
+/* No ybus counterpart: which tile solve runs for a precision: 0 automatic (the spread solve when the
+ * factor admits it and no shape or threshold of the solves below was set for the precision; else the
+ * lane solve for solves of at least the lane threshold's right-hand sides when the factor admits it; else the
  * domain solve at the widest tile that fits in shared memory; else the streamed solve likewise;
  * else the global-scratch solve), 1 the level-sliced shared-memory solve, 2 the global-scratch
  * solve, 3 the streamed solve, 4 the domain solve, 5 the lane solve (1, 3, 4 and 5 give
@@ -97,6 +98,12 @@ int32_t yb_factor_set_tile(yb_factor *f, int32_t precision, int32_t tile_width, 
  * admits no domain or lane layout). The lane solve serves yb_solve_many_device and yb_solve_many;
  * the pair, refined and batched solves take the automatic choice among the others. */
 int32_t yb_factor_set_tile_kind(yb_factor *f, int32_t precision, int32_t kind);
+/* No ybus counterpart: the spread solve (one right-hand side per lane, one warp per bundle of subtree
+ * domains and 32 right-hand sides, the top of the elimination forest as a dense map between the two
+ * sweeps), which the automatic choice takes for plain solves. info receives 6 values for a solve of
+ * `count` right-hand sides: {tasks (bundles), domains, top rows, live values per lane, partial values
+ * per group of 32, bytes of its records}; YB_ERROR_INVALID_ARGUMENT if the solve takes another kind. */
+int32_t yb_factor_spread_info(yb_factor *f, int32_t precision, int64_t count, int64_t *info);
 /* No ybus counterpart: the lane solve (one right-hand side per lane, a block of warps per 32; the
  * factor's rows in an elimination-tree postorder cut into subtree domains the warps take in
  * parallel under a top warp 0 takes, a few tens of live values per lane in shared memory; b, the
@@ -129,8 +136,8 @@ int32_t yb_factor_set_refine_lane_min_count(yb_factor *f, int64_t min_count);
  * (either output may be NULL). */
 int32_t yb_factor_lane_min_counts(const yb_factor *f, int32_t precision, int64_t *lane_min_count,
                                   int64_t *refine_lane_min_count);
-/* No ybus counterpart: with on = 1, every lane-solve launch from now on records CUDA events around
- * its three kernels (gather, solve, scatter) on the caller's stream, for up to 4096 launches;
+/* No ybus counterpart: with on = 1, every lane or spread solve from now on records CUDA events around
+ * its gather, its solve and its scatter on the caller's stream, for up to 4096 launches;
  * on = 0 stops. Either way the record so far is cleared. */
 int32_t yb_factor_time_lane(yb_factor *f, int32_t on);
 /* No ybus counterpart: waits for the recorded lane-solve launches and returns the total device

@@ -13,6 +13,7 @@
 #include "lane_solve.cuh"
 #include "lane_refine.cuh"
 #include "smem_solve.cuh"
+#include "spread_launch.hpp"
 #include "stream_solve.cuh"
 #include "solve.cuh"
 
@@ -349,6 +350,7 @@ extern "C" int32_t yb_factor_set_tile(yb_factor *f, int32_t precision, int32_t t
     t.width = tile_width;
     t.threads = threads;
     t.blocks_per_sm = blocks_per_sm;
+    t.shaped = true;
     return YB_OK;
   });
 }
@@ -375,6 +377,7 @@ extern "C" int32_t yb_factor_set_stream(yb_factor *f, int32_t precision, int32_t
     require(narrow_rows >= 0, "narrow rows must not be negative");
     TileConfig &t = precision == YB_FP64 ? f->tile64 : f->tile32;
     t.stream_warps = warps, t.ring = ring, t.page_bytes = page_bytes, t.narrow_rows = narrow_rows;
+    t.shaped = true;
     return YB_OK;
   });
 }
@@ -384,7 +387,8 @@ extern "C" int32_t yb_factor_set_tail_level(yb_factor *f, int32_t precision, int
     require(f != nullptr, "null factor");
     require(precision == YB_FP64 || precision == YB_FP32, "unknown precision");
     require(tail_level >= -1, "the tail level is -1 (chosen), 0 (none) or a forward level");
-    (precision == YB_FP64 ? f->tile64 : f->tile32).tail_level = tail_level;
+    TileConfig &t = precision == YB_FP64 ? f->tile64 : f->tile32;
+    t.tail_level = tail_level, t.shaped = true;
     return YB_OK;
   });
 }
@@ -945,6 +949,7 @@ void solve_device(yb_factor *f, const double *b, int64_t ldb, double *x, int64_t
   if (count <= 0 || f->n == 0) return;
   auto run = [&](auto zero, const TileConfig &configured, auto &fwd, auto &bwd, auto &scratch, auto &cache) {
     using T = decltype(zero);
+    if (configured.kind == kTileAuto && !configured.shaped && spread_solve<T>(f, b, ldb, x, ldx, count, stream)) return;
     if (configured.kind == kTileLane || (configured.kind == kTileAuto && count >= lane_threshold<T>(f, configured))) {
       DeviceLane *d = lane_pick<T>(f, lane_shape(f, configured, count), configured.lane_rpl, stream);
       if (d && (configured.kind == kTileLane || d->slots <= kLaneAutoSlots)) {
@@ -1278,6 +1283,7 @@ extern "C" int32_t yb_factor_set_domain(yb_factor *f, int32_t precision, int32_t
     require(cut >= -1, "the cut is -1 (chosen) or a forward level");
     TileConfig &t = precision == YB_FP64 ? f->tile64 : f->tile32;
     t.domain_warps = warps, t.domain_ring = ring, t.domain_page = page_bytes, t.domain_cut = cut;
+    t.shaped = true;
     return YB_OK;
   });
 }
@@ -1323,6 +1329,24 @@ extern "C" int32_t yb_factor_lane_info(yb_factor *f, int32_t precision, int64_t 
   });
 }
 
+extern "C" int32_t yb_factor_spread_info(yb_factor *f, int32_t precision, int64_t count, int64_t *info) {
+  return guard([&] {
+    require(f != nullptr && info != nullptr, "null argument");
+    require(precision == YB_FP64 || precision == YB_FP32, "unknown precision");
+    require(!f->is_complex, "a real factor only");
+    require(count >= 1, "at least one right-hand side");
+    cuda_check(cudaSetDevice(f->gpu->device), "cudaSetDevice");
+    const TileConfig &t = precision == YB_FP64 ? f->tile64 : f->tile32;
+    DeviceSpread *d = nullptr;
+    if (t.kind == kTileAuto && !t.shaped && !f->single && f->n > 0)
+      d = spread_for(f, precision == YB_FP64 ? 8 : 4, (count + 31) / 32, f->gpu->stream);
+    if (!d) throw host::Error(host::kInvalidArgument, "the solve this precision runs is not the spread solve");
+    const int64_t v[6] = {d->tasks, d->domains, d->top, d->slots, d->partials, d->blob_bytes};
+    std::copy(v, v + 6, info);
+    return YB_OK;
+  });
+}
+
 extern "C" int32_t yb_factor_set_lane(yb_factor *f, int32_t precision, int32_t warps, int32_t page_bytes) {
   return guard([&] {
     require(f != nullptr, "null factor");
@@ -1331,7 +1355,7 @@ extern "C" int32_t yb_factor_set_lane(yb_factor *f, int32_t precision, int32_t w
     require(page_bytes == 0 || (page_bytes >= 256 && page_bytes <= 16384 && page_bytes % 16 == 0),
             "pages of 256 to 16384 bytes, a multiple of 16, or 0 for the automatic choice");
     TileConfig &t = precision == YB_FP64 ? f->tile64 : f->tile32;
-    t.lane_warps = warps, t.lane_page = page_bytes, t.lane_warps_auto = false;
+    t.lane_warps = warps, t.lane_page = page_bytes, t.lane_warps_auto = false, t.shaped = true;
     return YB_OK;
   });
 }
@@ -1341,7 +1365,8 @@ extern "C" int32_t yb_factor_set_lane_rhs_per_lane(yb_factor *f, int32_t precisi
     require(f != nullptr, "null factor");
     require(precision == YB_FP64 || precision == YB_FP32, "unknown precision");
     require(rhs_per_lane == 1 || rhs_per_lane == 2, "1 or 2 right-hand sides per lane");
-    (precision == YB_FP64 ? f->tile64 : f->tile32).lane_rpl = rhs_per_lane;
+    TileConfig &t = precision == YB_FP64 ? f->tile64 : f->tile32;
+    t.lane_rpl = rhs_per_lane, t.shaped = true;
     return YB_OK;
   });
 }
@@ -1351,7 +1376,8 @@ extern "C" int32_t yb_factor_set_lane_min_count(yb_factor *f, int32_t precision,
     require(f != nullptr, "null factor");
     require(precision == YB_FP64 || precision == YB_FP32, "unknown precision");
     require(min_count >= -1, "a count, or -1 for the automatic threshold");
-    (precision == YB_FP64 ? f->tile64 : f->tile32).lane_min_count = min_count;
+    TileConfig &t = precision == YB_FP64 ? f->tile64 : f->tile32;
+    t.lane_min_count = min_count, t.shaped = true;
     return YB_OK;
   });
 }

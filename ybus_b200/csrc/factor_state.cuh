@@ -6,6 +6,7 @@
 #include <array>
 #include <map>
 #include <memory>
+#include <mutex>
 #include <string>
 #include <tuple>
 
@@ -100,6 +101,9 @@ struct TileConfig {
   int threads = 512;      // threads per block
   int blocks_per_sm = 1;  // resident blocks per SM the grid is sized for
   int kind = kTileAuto;
+  // a caller set a shape or a threshold of the solves below: the automatic choice is then among them,
+  // as it is for a factor that admits no spread layout
+  bool shaped = false;
   // the streamed solve's shape: warps per block, pages in flight per warp, page bytes, and the
   // row count under which a level goes to warp 0 (0: twice the rows of a slice)
   int stream_warps = 8, ring = 4, page_bytes = 2048, narrow_rows = 0;
@@ -135,6 +139,38 @@ struct DeviceLane {
   int64_t res_matrix = -1;  // the attach count it was built for
   DeviceArray<int32_t> res_ptr, res_len, res_col;
   DeviceArray<double> res_val;
+};
+
+// A spread layout on the device (SpreadLayout in plan.hpp), with the top's dense map.
+struct DeviceSpread {
+  int32_t n = 0, tasks = 0, domains = 0, top = 0, slots = 0, partials = 0;
+  int64_t blob_bytes = 0;
+  bool split = false;  // the top as two maps (an LU factor), m and m2, instead of one, m
+  double top_condition = 0;
+  DeviceArray<uint8_t> blob, m, m2;
+  DeviceArray<int32_t> task_row, fwd_page, bwd_page, in_pos, out_pos, part_ptr;
+  std::vector<int32_t> host_out_pos;
+};
+
+// A workspace of the plain spread solve, for one stream at a time: the event marks its last use, so a
+// stream that takes it over (or one that got a destroyed stream's handle) waits for that.
+struct SpreadWork {
+  static constexpr size_t kMost = 4;  // workspaces a factor keeps; a further stream waits for the oldest
+  cudaStream_t stream = nullptr;
+  cudaEvent_t done = nullptr;
+  uint64_t used = 0;  // the solve that used it last
+  DeviceArray<uint8_t> work, partial;
+  SpreadWork() = default;
+  SpreadWork(const SpreadWork &) = delete;
+  SpreadWork &operator=(const SpreadWork &) = delete;
+  ~SpreadWork() {
+    if (done) cudaEventDestroy(done);
+  }
+};
+
+// The complex batch's workspace for the spread solve.
+struct SpreadBatchWork {
+  DeviceArray<uint8_t> work, partial, args;
 };
 
 // A domain layout on the device (DomainLayout in plan.hpp).
@@ -187,6 +223,12 @@ struct yb_factor {
   std::map<std::tuple<int, int, int, int>, std::unique_ptr<yb::DeviceDomain>> domains;
   // lane layouts by (value bytes, warps, page bytes); a null entry: the factor admits none
   std::map<std::tuple<int, int, int, int>, std::unique_ptr<yb::DeviceLane>> lanes;
+  // spread layouts by (value bytes, groups up to; a null entry: the factor admits none) and the plain
+  // solve's workspaces, one per stream in use; the mutex guards both
+  std::map<std::pair<int, int64_t>, std::unique_ptr<yb::DeviceSpread>> spreads;
+  std::vector<std::unique_ptr<yb::SpreadWork>> spread_work;
+  uint64_t spread_solves = 0;
+  std::mutex spread_mutex;
   yb::DeviceArray<uint8_t> lane_work, lane_partial;  // the lane solve's work and partial arrays
   yb::LaneTiming lane_timing;
   yb::DeviceArray<int32_t> error;  // the device error word (a bounded wait that ran out)
@@ -238,6 +280,7 @@ namespace yb {
 void solve_pairs_device(yb_factor *f, int64_t count, const int32_t *plus, const int32_t *minus, const double *base,
                         const double *alpha, const double *inverse_weight, int32_t *singular, double *out, int64_t ldo,
                         cudaStream_t stream);
+cudaEvent_t *lane_timing_slot(yb_factor *f);  // the events of the next timed lane or spread solve, or null
 void solve_single_row_device(yb_factor *f, const double *b, int64_t ldb, double *x, int64_t ldx, int64_t count,
                              cudaStream_t stream);
 }

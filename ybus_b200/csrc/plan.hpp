@@ -261,4 +261,80 @@ template <class T>
 LaneLayout lane_layout(const Plan<T> &plan, int32_t value_bytes, int32_t page_bytes, int32_t max_slots, int32_t warps,
                        int32_t rpl = 1);
 
+// The factor for the spread solve (spread_solve.cuh: one right-hand side per lane, like the lane
+// solve, but every warp on its own): the rows in a postorder of the elimination forest, cut into
+// subtree domains under a top, the domains bundled into tasks (LPT by work). A task's rows are
+// consecutive positions, so its warp reads and writes the work array [group][position][32 lanes]
+// front to back in the forward sweep and back to front in the backward one. Each sweep of a task is
+// a stream of packets in pages of kSpreadPage bytes, read by every warp that solves the task (one
+// per group of 32 right-hand sides). The top is solved between the two sweeps as a dense map
+// x_T = M r_T in the factor's full precision, whatever the packets' values are.
+//
+// A packet is 16-byte aligned: a head {uint32 kind, bytes, count, 0}, then by kind
+//   kSpreadRows4 / kSpreadRows1: four (one) rows' records {value 0, value 1, 1/diagonal, uint32 slots,
+//     uint32 flags | pairs << 8}, then each row's `pairs` further pairs of entries {value a, value b,
+//     uint32 slot a | slot b << 8 | flags << 16}. `slots` holds the row's own slot, its first entry's
+//     and its second's, a byte each. Forward: z = (b + acc) / diagonal into the row's place, acc the own
+//     slot (kSpreadSelf), else what the row before left, else nothing; then per entry the slot's value
+//     (kSpreadLoad0, 1; without it nothing yet) less value z goes into the slot (kSpreadStore0, 1) or,
+//     the first entry's, is left to the next row (kSpreadCarry). Backward: x = (z - sum of value times
+//     slot (kSpreadLoad0, 1) or, the first entry's, times the row before's x (kSpreadCarry)) /
+//     diagonal into the row's place and with kSpreadSelf into its slot. A further pair: kSpreadLoad0, 1
+//     and kSpreadStore1 (or, backward, kSpreadLoad1) alike; its first entry is always there.
+//   kSpreadMore: `count` further pairs for a row whose entries do not fit its packet (forward: after
+//     it, with the same z; backward: before it, into the sum it starts from).
+//   kSpreadMove: `count` {uint32 index, uint32 slot}: forward, a domain's updates of top rows: the
+//     partial array's row `index` takes the slot; backward, the top solutions a domain reads: the
+//     slot takes top row `index`.
+//   kSpreadPageEnd: the page ends; kSpreadEnd: the task's sweep ends.
+enum SpreadKind : uint32_t {
+  kSpreadRows4 = 0,
+  kSpreadRows1 = 1,
+  kSpreadMore = 2,
+  kSpreadMove = 3,
+  kSpreadPageEnd = 4,
+  kSpreadEnd = 5
+};
+enum SpreadFlag : uint32_t {
+  kSpreadSelf = 1,
+  kSpreadLoad0 = 2,
+  kSpreadStore0 = 4,
+  kSpreadCarry = 8,
+  kSpreadLoad1 = 16,
+  kSpreadStore1 = 32
+};
+constexpr int kSpreadPage = 2048;       // bytes of a page (two in flight per block)
+constexpr int kSpreadMostSlots = 254;   // live values per lane at most (a byte each)
+constexpr int kSpreadMostTop = 1536;    // rows of the dense top at most
+constexpr int kSpreadPad = 32;          // rows before and after the work array that prefetches may read
+
+// Bytes of a row's record and of a further pair for values of `value_bytes`.
+inline YB_HOST_DEVICE constexpr uint32_t spread_row_bytes(int value_bytes) { return value_bytes == 16 ? 64 : 32; }
+inline YB_HOST_DEVICE constexpr uint32_t spread_pair_bytes(int value_bytes) {
+  return value_bytes == 16 ? 48 : value_bytes == 8 ? 32 : 16;
+}
+
+template <class V> struct SpreadLayout {  // V: double or complex<double>, the plan's values
+  int32_t n = 0, tasks = 0, domains = 0, top = 0, slots = 0, partials = 0;
+  double cost = 0;                                // the cut's estimate in cycles
+  std::vector<int32_t> task_row;                  // [tasks + 1] first position of each task; the top after them
+  std::vector<uint8_t> blob;                      // pages: every task's forward, then its backward stream
+  std::vector<int32_t> fwd_page, bwd_page;        // [2 tasks] first page and page count of each stream
+  std::vector<int32_t> in_pos, out_pos;           // [n] rows of b and of x -> positions
+  std::vector<int32_t> part_ptr;                  // [top + 1] the partial rows of each top row
+  // the top's own triangles by rows (columns as top indices) for its dense map
+  std::vector<int32_t> l_ptr, l_col, u_ptr, u_col;
+  std::vector<V> l_val, u_val, l_dinv, u_dinv;
+  double s_norm = 0;                              // a bound of the infinity norm of the top's Schur complement
+  double l_norm = 0, u_norm = 0;                  // the infinity norms of L_TT and U_TT
+};
+
+// Builds the spread layout of `plan` for packets of `value_bytes` (half of the plan's value's bytes, or all
+// of them) and `groups` groups of 32 right-hand sides on `sms` SMs of `blocks` blocks each, for which the
+// cut is chosen.
+// Throws host::Error (kInvalidArgument) when no postorder serves both sweeps, (kTooLarge) when the
+// slots or the top would be too large.
+template <class V>
+SpreadLayout<V> spread_layout(const Plan<V> &plan, int32_t value_bytes, int64_t groups, int32_t sms, int32_t blocks = 6);
+
 }  // namespace yb

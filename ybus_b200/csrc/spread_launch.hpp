@@ -1,0 +1,45 @@
+// The spread solve's entry points for the C ABI's translation units (spread_launch.cu).
+#pragma once
+
+#include <cstdint>
+#include <vector>
+
+#include "factor_state.cuh"
+
+namespace yb {
+
+// The automatic choice takes the spread solve up to this many live values per lane: with more, too
+// few warps fit an SM to cover their shared-memory latency.
+constexpr int32_t kSpreadAutoSlots = 64, kSpreadAutoSlotsComplex = 400;
+
+// The spread layout for `groups` groups of 32 right-hand sides with values of `value_bytes`, made and
+// uploaded at its first use; null if the factor admits none.
+DeviceSpread *spread_for(yb_factor *f, int value_bytes, int64_t groups, cudaStream_t stream);
+
+// Solves `count` right-hand sides (device arrays, column-major) in T (double or float); false, with
+// nothing done, where the factor admits no spread layout, or under stream capture where it has none
+// or too small a workspace yet.
+template <class T>
+bool spread_solve(yb_factor *f, const double *b, int64_t ldb, double *x, int64_t ldx, int64_t count, cudaStream_t stream);
+
+// The sweeps and the top of `groups` groups whose right-hand sides are in `work` (at positions, with
+// kSpreadPad rows before and after), the solutions into `xout` (work itself, or another array of its layout);
+// groups with a zero in `group_active` (null: none) are skipped.
+template <class T>
+void spread_sweeps(yb_factor *f, DeviceSpread *d, T *work, T *xout, int64_t groups, const uint8_t *group_active,
+                   cudaStream_t stream);
+
+// One factor's part of a complex batch: right-hand sides and solutions complex128, column-major.
+struct SpreadSystem {
+  yb_factor *factor;
+  DeviceSpread *layout;
+  const cplx<double> *b;
+  cplx<double> *x;
+  int64_t count;
+};
+
+// Solves every system's right-hand sides in complex values of R (double or float) in one run of
+// launches, into x or (add) onto it.
+template <class R> void spread_batch(const std::vector<SpreadSystem> &systems, bool add, SpreadBatchWork &work, cudaStream_t stream);
+
+}  // namespace yb

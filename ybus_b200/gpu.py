@@ -237,6 +237,13 @@ class GpuFactor:
         return {"tile": w.value, "cut": cut.value, "top": top.value, "records": rec.value, "bytes": by.value,
                 "smem": sm.value, "model_cycles": cyc.value}
 
+    def spread_info(self, precision: int = FP64, count: int = 1) -> dict:
+        """The spread solve's layout for a solve of `count` right-hand sides, which the automatic choice
+        takes for plain solves (an error if it takes another)."""
+        v = np.zeros(6, np.int64)
+        _check(lib().yb_factor_spread_info(self._h, precision, int(count), ptr(v)))
+        return dict(zip(("tasks", "domains", "top", "slots", "partials", "bytes"), (int(a) for a in v)))
+
     def set_lane_rhs_per_lane(self, precision: int, rhs_per_lane: int) -> None:
         """How many right-hand sides each lane of the plain lane solve carries (1 or 2)."""
         _check(lib().yb_factor_set_lane_rhs_per_lane(self._h, precision, rhs_per_lane))
