@@ -145,10 +145,16 @@ struct DeviceLane {
 struct DeviceSpread {
   int32_t n = 0, tasks = 0, domains = 0, top = 0, slots = 0, partials = 0;
   int64_t blob_bytes = 0;
-  bool split = false;  // the top as two maps (an LU factor), m and m2, instead of one, m
+  int64_t serial = 0;  // no two layouts of a process share one
+  bool split = false;  // the top as two maps (a real LU factor), m and m2, instead of one, m
+  bool refine = false;  // ... as one with a correction by S (a complex factor)
   double top_condition = 0;
-  DeviceArray<uint8_t> blob, m, m2;
-  DeviceArray<int32_t> task_row, fwd_page, bwd_page, in_pos, out_pos, part_ptr;
+  DeviceArray<uint8_t> store;  // what the pointers below point into
+  const uint8_t *blob = nullptr;
+  const int32_t *task_row = nullptr, *fwd_page = nullptr, *bwd_page = nullptr, *in_pos = nullptr, *out_pos = nullptr;
+  const int32_t *part_ptr = nullptr, *s_ptr = nullptr, *s_col = nullptr;
+  const void *s_val = nullptr;
+  void *m = nullptr, *m2 = nullptr;
   std::vector<int32_t> host_out_pos;
 };
 
@@ -168,9 +174,12 @@ struct SpreadWork {
   }
 };
 
-// The complex batch's workspace for the spread solve.
+// The complex batch's workspace for the spread solve, and the lists of its launches' blocks, which
+// depend on the layouts (by their serial numbers) and the counts alone.
 struct SpreadBatchWork {
-  DeviceArray<uint8_t> work, partial, args;
+  DeviceArray<uint8_t> work, partial, nets, items;
+  std::vector<int64_t> key;
+  size_t n_io = 0, n_sweep = 0, n_sum = 0, n_top = 0;
 };
 
 // A domain layout on the device (DomainLayout in plan.hpp).

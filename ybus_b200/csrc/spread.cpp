@@ -12,10 +12,16 @@
 // cost a larger top, whose dense map grows with its square. The cap is the one whose estimate is
 // least (cost_of below).
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <complex>
 #include <cstring>
+#include <exception>
+#include <functional>
+#include <mutex>
 #include <numeric>
+#include <system_error>
+#include <thread>
 #include <vector>
 
 #include "plan.hpp"
@@ -84,7 +90,8 @@ template <class V> struct PacketWriter {
   const uint32_t vb, rb, pb;
   int32_t pages = 0;
   size_t pos = 0;
-  std::vector<Row> held;  // rows waiting to make a packet of four
+  Row held[4];  // rows waiting to make a packet of four; their storage is used again
+  int n_held = 0;
   Moves waiting;          // forward: moves that follow the held rows
   PacketWriter(std::vector<uint8_t> &b, int32_t value_bytes, bool back)
       : blob(b), full(value_bytes == (int32_t)sizeof(V)), backward(back), vb((uint32_t)value_bytes),
@@ -153,12 +160,12 @@ template <class V> struct PacketWriter {
     for (uint32_t i = 0; i < pairs; ++i, p += pb) pair(p, e[2 * i], 2 * i + 1 < count ? e + 2 * i + 1 : nullptr);
   }
   void flush_rows() {  // held rows that make no packet of four: one by one
-    for (const Row &r : held) rows(&r, 1);
-    held.clear();
+    for (int k = 0; k < n_held; ++k) rows(&held[k], 1);
+    n_held = 0;
     put_moves(waiting);
     waiting.clear();
   }
-  void row(Row r) {
+  void row(Row &r) {  // r's storage is taken, another's left
     const size_t most = 2 + 2 * (size_t)most_pairs();
     if (r.entries.size() > most) {  // a row longer than a packet: in runs of pairs (forward after it, backward before)
       flush_rows();
@@ -173,13 +180,13 @@ template <class V> struct PacketWriter {
       if (!backward) runs();
       return;
     }
-    held.push_back(std::move(r));
-    if (held.size() == 4) {
+    std::swap(held[n_held++], r);
+    if (n_held == 4) {
       uint32_t bytes = 16;
       for (const Row &h : held) bytes += row_bytes(h);
       if (bytes + 16 <= (uint32_t)kSpreadPage) {
-        rows(held.data(), 4);
-        held.clear();
+        rows(held, 4);
+        n_held = 0;
       }
       flush_rows();
     }
@@ -187,7 +194,7 @@ template <class V> struct PacketWriter {
   // Forward: after the rows so far; backward: before the rows to come (and so, when rows are held,
   // before their packet: the moved slots are free until then).
   void moves(const Moves &m) {
-    if (backward || held.empty())
+    if (backward || n_held == 0)
       put_moves(m);
     else
       waiting.insert(waiting.end(), m.begin(), m.end());
@@ -214,12 +221,11 @@ template <class V> double magnitude_of(const V &v) { return std::abs(v); }
 }  // namespace
 
 template <class V>
-SpreadLayout<V> spread_layout(const Plan<V> &plan, int32_t value_bytes, int64_t groups, int32_t sms, int32_t blocks) {
+SpreadLayout<V> spread_layout(const Plan<V> &plan, int32_t value_bytes, int64_t groups, int32_t sms, int32_t blocks,
+                              const std::function<int32_t(int32_t)> &fit) {
   if (value_bytes != (int32_t)sizeof(V) && value_bytes * 2 != (int32_t)sizeof(V))
     throw host::Error(host::kInvalidArgument, "packet values are the plan's, or half as wide");
   const int32_t n = plan.n;
-  SpreadLayout<V> lay;
-  lay.n = n;
   // each row's entries in both sweeps
   std::vector<int32_t> fat(n), bat(n);  // the row's index in each sweep's order
   for (int32_t p = 0; p < n; ++p) fat[plan.fwd.row[p]] = p, bat[plan.bwd.row[p]] = p;
@@ -269,8 +275,9 @@ SpreadLayout<V> spread_layout(const Plan<V> &plan, int32_t value_bytes, int64_t 
     for (int32_t c = 0; c < n; ++c) child[fill[parent[c] < 0 ? n : parent[c]]++] = c;
   }
   for (int32_t v = 0; v <= n; ++v)
-    std::stable_sort(child.begin() + child_ptr[v], child.begin() + child_ptr[v + 1],
-                     [&](int32_t a, int32_t b) { return size[a] > size[b]; });
+    if (child_ptr[v + 1] - child_ptr[v] > 1)
+      std::sort(child.begin() + child_ptr[v], child.begin() + child_ptr[v + 1],
+                [&](int32_t a, int32_t b) { return size[a] != size[b] ? size[a] > size[b] : a < b; });
   order.reserve(n);
   {
     std::vector<std::pair<int32_t, int32_t>> stack{{n, child_ptr[n]}};
@@ -326,18 +333,26 @@ SpreadLayout<V> spread_layout(const Plan<V> &plan, int32_t value_bytes, int64_t 
   // scheduler; the top's map: a tile's chain of steps, its values from L2, half the FP64 rate; and, with
   // a top, two launches more.
   const double G = (double)std::max<int64_t>(1, groups);
+  // A complex top is four products of reals for one. That its map is applied twice is not charged: with 8
+  // in place of 4 a batch of 16 networks of 500 to 3,000 buses took 873 us for 912, and refined 5,778 for 5,650.
+  constexpr double kTop = sizeof(V) == 16 ? 4 : 1;
   auto cost_of = [&](const Cut &c) {
     const double all = c.tasks * std::ceil(G / 4), wave = (double)blocks * sms, full = std::floor(all / wave);
     const double left = std::ceil((all - full * wave) / sms);
     const double sweeps = c.longest * (full * std::max<double>(kAlone, blocks) + (left > 0 ? std::max(kAlone, left) : 0.0));
     const double t = c.top;
-    return sweeps + (c.top ? 20 * t + t * t / 100 + G * t * t / sms + 8000 : 0);
+    return sweeps + (c.top ? 20 * t + t * t / 100 + kTop * G * t * t / sms + 8000 : 0);
   };
+  constexpr int kCaps = 45;  // caps a quarter octave apart
+  auto cap_of = [&](int k) { return total / std::pow(2.0, 1 + k / 4.0); };
+  std::vector<int32_t> near;  // the rows that some cap has at its top or roots a domain at
+  for (int32_t v = 0; v < n; ++v)
+    if (parent[v] < 0 || sub[parent[v]] > cap_of(kCaps - 1)) near.push_back(v);
   auto cut_at = [&](double cap) {
     Cut c;
     c.cap = cap;
     double domain_work = 0, largest = 0;
-    for (int32_t v = 0; v < n; ++v) {
+    for (int32_t v : near) {
       if (sub[v] > cap)
         ++c.top;
       else if (parent[v] < 0 || sub[parent[v]] > cap)
@@ -350,218 +365,297 @@ SpreadLayout<V> spread_layout(const Plan<V> &plan, int32_t value_bytes, int64_t 
     c.cost = c.top > kSpreadMostTop ? INFINITY : cost_of(c);
     return c;
   };
-  Cut best = cut_at(total + 1);  // one domain per tree, no top
-  for (int k = 0; k <= 44; ++k) {  // caps a quarter octave apart
-    Cut c = cut_at(total / std::pow(2.0, 1 + k / 4.0));
-    if (c.cost < best.cost) best = std::move(c);
-  }
-  lay.cost = best.cost;
-  lay.domains = (int32_t)best.roots.size();
-  lay.tasks = best.tasks;
-  // LPT: the domains to the tasks by work, each task's domains in postorder, the longest task first
-  std::vector<std::vector<int32_t>> task_domains(lay.tasks);
-  {
-    std::vector<int32_t> by_work(best.roots);
-    std::stable_sort(by_work.begin(), by_work.end(), [&](int32_t a, int32_t b) { return sub[a] > sub[b]; });
-    std::vector<double> load(lay.tasks, 0.0);
-    for (int32_t r : by_work) {
-      const size_t w = (size_t)(std::min_element(load.begin(), load.end()) - load.begin());
-      load[w] += sub[r];
-      task_domains[w].push_back(r);
+  auto choose = [&] {
+    Cut best = cut_at(total + 1);  // one domain per tree, no top
+    for (int k = 0; k < kCaps; ++k) {
+      Cut c = cut_at(cap_of(k));
+      if (c.cost < best.cost) best = std::move(c);
     }
-    std::vector<size_t> by_load(lay.tasks);
-    std::iota(by_load.begin(), by_load.end(), 0);
-    std::stable_sort(by_load.begin(), by_load.end(), [&](size_t a, size_t b) { return load[a] > load[b]; });
-    std::vector<std::vector<int32_t>> sorted;
-    for (size_t w : by_load) sorted.push_back(std::move(task_domains[w]));
-    task_domains = std::move(sorted);
-    for (auto &d : task_domains) std::sort(d.begin(), d.end(), [&](int32_t a, int32_t b) { return pos[a] < pos[b]; });
-  }
-  // positions: task by task, each domain in postorder, then the top in postorder
-  std::vector<int32_t> newpos(n, -1), at(n), domain_of(n, -1);
-  std::vector<std::vector<std::pair<int32_t, int32_t>>> ranges(lay.tasks);  // each domain's positions, first and last
-  int32_t next = 0, domain_count = 0;
-  for (int32_t w = 0; w < lay.tasks; ++w) {
+    return best;
+  };
+  auto lay_out = [&](const Cut &best) {
+    SpreadLayout<V> lay;
+    lay.n = n;
+    lay.cost = best.cost;
+    lay.domains = (int32_t)best.roots.size();
+    lay.tasks = best.tasks;
+    // LPT: the domains to the tasks by work, each task's domains in postorder, the longest task first
+    std::vector<std::vector<int32_t>> task_domains(lay.tasks);
+    {
+      std::vector<int32_t> by_work(best.roots);
+      std::stable_sort(by_work.begin(), by_work.end(), [&](int32_t a, int32_t b) { return sub[a] > sub[b]; });
+      std::vector<double> load(lay.tasks, 0.0);
+      for (int32_t r : by_work) {
+        const size_t w = (size_t)(std::min_element(load.begin(), load.end()) - load.begin());
+        load[w] += sub[r];
+        task_domains[w].push_back(r);
+      }
+      std::vector<size_t> by_load(lay.tasks);
+      std::iota(by_load.begin(), by_load.end(), 0);
+      std::stable_sort(by_load.begin(), by_load.end(), [&](size_t a, size_t b) { return load[a] > load[b]; });
+      std::vector<std::vector<int32_t>> sorted;
+      for (size_t w : by_load) sorted.push_back(std::move(task_domains[w]));
+      task_domains = std::move(sorted);
+      for (auto &d : task_domains) std::sort(d.begin(), d.end(), [&](int32_t a, int32_t b) { return pos[a] < pos[b]; });
+    }
+    // positions: task by task, each domain in postorder, then the top in postorder
+    std::vector<int32_t> newpos(n, -1), at(n), domain_of(n, -1);
+    std::vector<std::vector<std::pair<int32_t, int32_t>>> ranges(lay.tasks);  // each domain's positions, first and last
+    int32_t next = 0, domain_count = 0;
+    for (int32_t w = 0; w < lay.tasks; ++w) {
+      lay.task_row.push_back(next);
+      for (int32_t r : task_domains[w]) {
+        const int32_t d0 = next;
+        for (int32_t t = pos[r] - size[r] + 1; t <= pos[r]; ++t) newpos[order[t]] = next++, domain_of[order[t]] = domain_count;
+        ranges[w].push_back({d0, next - 1});
+        ++domain_count;
+      }
+    }
     lay.task_row.push_back(next);
-    for (int32_t r : task_domains[w]) {
-      const int32_t d0 = next;
-      for (int32_t t = pos[r] - size[r] + 1; t <= pos[r]; ++t) newpos[order[t]] = next++, domain_of[order[t]] = domain_count;
-      ranges[w].push_back({d0, next - 1});
-      ++domain_count;
+    const int32_t top0 = next;
+    for (int32_t t = 0; t < n; ++t)
+      if (newpos[order[t]] < 0) newpos[order[t]] = next++;
+    lay.top = n - top0;
+    for (int32_t v = 0; v < n; ++v) at[newpos[v]] = v;
+    // the top rows each domain updates, and those it reads, by position; the partial rows: one per
+    // (domain, top row it updates), each top row's together, by domain
+    std::vector<std::vector<int32_t>> updates(domain_count), reads(domain_count);
+    for (int32_t p = 0; p < top0; ++p) {
+      const int32_t d = domain_of[at[p]];
+      for (int32_t q = col_ptr[at[p]]; q < col_ptr[at[p] + 1]; ++q)
+        if (newpos[col_row[q]] >= top0) updates[d].push_back(newpos[col_row[q]]);
+      for (int32_t q = b0(at[p]); q < b1(at[p]); ++q)
+        if (newpos[plan.bwd.col[q]] >= top0) reads[d].push_back(newpos[plan.bwd.col[q]]);
     }
-  }
-  lay.task_row.push_back(next);
-  const int32_t top0 = next;
-  for (int32_t t = 0; t < n; ++t)
-    if (newpos[order[t]] < 0) newpos[order[t]] = next++;
-  lay.top = n - top0;
-  for (int32_t v = 0; v < n; ++v) at[newpos[v]] = v;
-  // the top rows each domain updates, and those it reads, by position; the partial rows: one per
-  // (domain, top row it updates), each top row's together, by domain
-  std::vector<std::vector<int32_t>> updates(domain_count), reads(domain_count);
-  for (int32_t p = 0; p < top0; ++p) {
-    const int32_t d = domain_of[at[p]];
-    for (int32_t q = col_ptr[at[p]]; q < col_ptr[at[p] + 1]; ++q)
-      if (newpos[col_row[q]] >= top0) updates[d].push_back(newpos[col_row[q]]);
-    for (int32_t q = b0(at[p]); q < b1(at[p]); ++q)
-      if (newpos[plan.bwd.col[q]] >= top0) reads[d].push_back(newpos[plan.bwd.col[q]]);
-  }
-  std::vector<int32_t> part_next(lay.top + 1, 0);
-  for (auto *sets : {&updates, &reads})
-    for (auto &v : *sets) {
-      std::sort(v.begin(), v.end());
-      v.erase(std::unique(v.begin(), v.end()), v.end());
-    }
-  for (const auto &v : updates)
-    for (int32_t p : v) ++part_next[p - top0 + 1];
-  for (int32_t i = 0; i < lay.top; ++i) part_next[i + 1] += part_next[i];
-  lay.part_ptr = part_next;
-  lay.partials = part_next[lay.top];
-  // the packets. A domain's last row leaves nothing to the next domain's first (their trees differ),
-  // and the slots a domain's moves use are given back only after the packet they may wait for.
-  std::vector<int32_t> slot(n, -1), readers(n, 0);
-  std::vector<std::pair<uint32_t, uint32_t>> moves;
-  int32_t peak = 0, d = 0;
-  lay.fwd_page.resize(2 * (size_t)lay.tasks), lay.bwd_page.resize(2 * (size_t)lay.tasks);
-  for (int32_t w = 0; w < lay.tasks; ++w) {
-    const int32_t first_domain = d;
-    lay.fwd_page[2 * w] = (int32_t)(lay.blob.size() / kSpreadPage);
-    {
-      PacketWriter<V> pw(lay.blob, value_bytes, false);
-      SpreadSlots slots;
-      std::vector<int32_t> late;  // slots whose moves wait for the held rows
-      auto settle = [&] {
-        if (!pw.held.empty()) return;
-        for (int32_t s : late) slots.give(s);
-        late.clear();
-      };
-      for (auto [d0, d1] : ranges[w]) {
-        for (int32_t p = d0; p <= d1; ++p) {
-          const int32_t j = at[p], after = p < d1 ? at[p + 1] : -1;
-          typename PacketWriter<V>::Row row{plan.fwd.dinv[fat[j]], -1, {}};
-          // the targets' slots before the row's own is given back: the kernel reads them together
-          int32_t given = -1;
-          for (int32_t q = col_ptr[j]; q < col_ptr[j + 1]; ++q) {
-            const int32_t r = col_row[q];
-            const bool load = slot[r] >= 0;
-            if (r == after) {  // to the next row, which alone reads it
-              const uint8_t was = load ? (uint8_t)slot[r] : 0;
-              if (load) given = slot[r], slot[r] = -1;
-              row.entries.insert(row.entries.begin(), {col_val[q], was, load, false, true});
-            } else {
-              if (!load) slot[r] = slots.take();
-              row.entries.push_back({col_val[q], (uint8_t)slot[r], load, true, false});
-            }
-          }
-          if (slot[j] >= 0) row.self = slot[j], slots.give(slot[j]), slot[j] = -1;
-          if (given >= 0) slots.give(given);
-          pw.row(std::move(row));
-          settle();
-        }
-        moves.clear();
-        for (int32_t p : updates[d]) {
-          const int32_t r = at[p];
-          moves.push_back({(uint32_t)part_next[p - top0]++, (uint32_t)slot[r]});
-          late.push_back(slot[r]);
-          slot[r] = -1;
-        }
-        pw.moves(moves);
-        settle();
-        ++d;
+    std::vector<int32_t> part_next(lay.top + 1, 0);
+    for (auto *sets : {&updates, &reads})
+      for (auto &v : *sets) {
+        std::sort(v.begin(), v.end());
+        v.erase(std::unique(v.begin(), v.end()), v.end());
       }
-      pw.end();
-      lay.fwd_page[2 * w + 1] = pw.pages;
-      peak = std::max(peak, slots.peak);
-    }
-    lay.bwd_page[2 * w] = (int32_t)(lay.blob.size() / kSpreadPage);
-    {
-      PacketWriter<V> pw(lay.blob, value_bytes, true);
-      SpreadSlots slots;
-      std::vector<int32_t> late;  // slots given up while rows are held: a move may run before them
-      auto settle = [&] {
-        if (!pw.held.empty()) return;
-        for (int32_t s : late) slots.give(s);
-        late.clear();
+    for (const auto &v : updates)
+      for (int32_t p : v) ++part_next[p - top0 + 1];
+    for (int32_t i = 0; i < lay.top; ++i) part_next[i + 1] += part_next[i];
+    lay.part_ptr = part_next;
+    lay.partials = part_next[lay.top];
+    // the packets. A domain's last row leaves nothing to the next domain's first (their trees differ),
+    // and the slots a domain's moves use are given back only after the packet they may wait for.
+    // Tasks share nothing here, so threads write them, each with its own marks.
+    std::vector<int32_t> task_domain(lay.tasks + 1, 0);  // each task's first domain
+    for (int32_t w = 0; w < lay.tasks; ++w) task_domain[w + 1] = task_domain[w] + (int32_t)ranges[w].size();
+    std::vector<std::vector<uint32_t>> part_of(domain_count);  // the partial rows of each domain's updates
+    for (int32_t d = 0; d < domain_count; ++d)
+      for (int32_t p : updates[d]) part_of[d].push_back((uint32_t)part_next[p - top0]++);
+    lay.fwd_page.resize(2 * (size_t)lay.tasks), lay.bwd_page.resize(2 * (size_t)lay.tasks);
+    std::vector<std::vector<uint8_t>> blobs(lay.tasks);
+    std::exception_ptr error;
+    std::mutex error_mutex;
+    std::atomic<int32_t> next_task{0}, peak{0};
+    auto write_task = [&](int32_t w, std::vector<int32_t> &slot, std::vector<int32_t> &readers) {
+      std::vector<uint8_t> &blob = blobs[w];
+      std::vector<std::pair<uint32_t, uint32_t>> moves;
+      typename PacketWriter<V>::Row row;
+      const int32_t first_domain = task_domain[w];
+      int32_t d = first_domain;
+      auto note = [&](int32_t slots) {
+        for (int32_t was = peak; was < slots && !peak.compare_exchange_weak(was, slots);) {}
       };
-      for (size_t i = ranges[w].size(); i-- > 0;) {
-        const auto [p0, p1] = ranges[w][i];
-        const int32_t dom = first_domain + (int32_t)i;
-        for (int32_t p = p0; p <= p1; ++p)
-          for (int32_t q = b0(at[p]); q < b1(at[p]); ++q) ++readers[plan.bwd.col[q]];
-        moves.clear();
-        for (int32_t p : reads[dom]) {
-          slot[at[p]] = slots.take();
-          moves.push_back({(uint32_t)(p - top0), (uint32_t)slot[at[p]]});
-        }
-        pw.moves(moves);
-        for (int32_t p = p1; p >= p0; --p) {
-          const int32_t j = at[p], before = p < p1 ? at[p + 1] : -1, after = p > p0 ? at[p - 1] : -1;
-          typename PacketWriter<V>::Row row{plan.bwd.dinv[bat[j]], -1, {}};
-          for (int32_t q = b0(j); q < b1(j); ++q) {
-            const int32_t c = plan.bwd.col[q];
-            if (c == before) {  // the row just solved: its x is still in a register (readers does not count this)
-              row.entries.insert(row.entries.begin(), {plan.bwd.val[q], 0, false, false, true});
-              continue;
+      {
+        PacketWriter<V> pw(blob, value_bytes, false);
+        SpreadSlots slots;
+        std::vector<int32_t> late;  // slots whose moves wait for the held rows
+        auto settle = [&] {
+          if (pw.n_held > 0) return;
+          for (int32_t s : late) slots.give(s);
+          late.clear();
+        };
+        for (auto [d0, d1] : ranges[w]) {
+          for (int32_t p = d0; p <= d1; ++p) {
+            const int32_t j = at[p], after = p < d1 ? at[p + 1] : -1;
+            row.dinv = plan.fwd.dinv[fat[j]], row.self = -1, row.entries.clear();
+            // the targets' slots before the row's own is given back: the kernel reads them together
+            int32_t given = -1;
+            for (int32_t q = col_ptr[j]; q < col_ptr[j + 1]; ++q) {
+              const int32_t r = col_row[q];
+              const bool load = slot[r] >= 0;
+              if (r == after) {  // to the next row, which alone reads it
+                const uint8_t was = load ? (uint8_t)slot[r] : 0;
+                if (load) given = slot[r], slot[r] = -1;
+                row.entries.insert(row.entries.begin(), {col_val[q], was, load, false, true});
+              } else {
+                if (!load) slot[r] = slots.take();
+                row.entries.push_back({col_val[q], (uint8_t)slot[r], load, true, false});
+              }
             }
-            row.entries.push_back({plan.bwd.val[q], (uint8_t)slot[c], true, false, false});
+            if (slot[j] >= 0) row.self = slot[j], slots.give(slot[j]), slot[j] = -1;
+            if (given >= 0) slots.give(given);
+            pw.row(row);
+            settle();
           }
-          for (int32_t q = b0(j); q < b1(j); ++q) {
-            const int32_t c = plan.bwd.col[q];
-            if (c != before && --readers[c] == 0) {
-              // in the last rows of a domain a slot may be taken next by the moves of another
-              if (newpos[c] >= top0 || p - p0 < 4) late.push_back(slot[c]);
-              else slots.give(slot[c]);
-              slot[c] = -1;
-            }
+          moves.clear();
+          for (size_t i = 0; i < updates[d].size(); ++i) {
+            const int32_t r = at[updates[d][i]];
+            moves.push_back({part_of[d][i], (uint32_t)slot[r]});
+            late.push_back(slot[r]);
+            slot[r] = -1;
           }
-          if (after >= 0)
-            for (int32_t q = b0(after); q < b1(after); ++q)
-              if (plan.bwd.col[q] == j) --readers[j];
-          if (readers[j] > 0) slot[j] = slots.take(), row.self = slot[j];
-          pw.row(std::move(row));
+          pw.moves(moves);
           settle();
+          ++d;
         }
+        pw.end();
+        lay.fwd_page[2 * w + 1] = pw.pages;
+        note(slots.peak);
       }
-      pw.end();
-      lay.bwd_page[2 * w + 1] = pw.pages;
-      peak = std::max(peak, slots.peak);
+      lay.bwd_page[2 * w] = (int32_t)(blob.size() / kSpreadPage);
+      {
+        PacketWriter<V> pw(blob, value_bytes, true);
+        SpreadSlots slots;
+        std::vector<int32_t> late;  // slots given up while rows are held: a move may run before them
+        auto settle = [&] {
+          if (pw.n_held > 0) return;
+          for (int32_t s : late) slots.give(s);
+          late.clear();
+        };
+        for (size_t i = ranges[w].size(); i-- > 0;) {
+          const auto [p0, p1] = ranges[w][i];
+          const int32_t dom = first_domain + (int32_t)i;
+          for (int32_t p = p0; p <= p1; ++p)
+            for (int32_t q = b0(at[p]); q < b1(at[p]); ++q) ++readers[plan.bwd.col[q]];
+          moves.clear();
+          for (int32_t p : reads[dom]) {
+            slot[at[p]] = slots.take();
+            moves.push_back({(uint32_t)(p - top0), (uint32_t)slot[at[p]]});
+          }
+          pw.moves(moves);
+          for (int32_t p = p1; p >= p0; --p) {
+            const int32_t j = at[p], before = p < p1 ? at[p + 1] : -1, after = p > p0 ? at[p - 1] : -1;
+            row.dinv = plan.bwd.dinv[bat[j]], row.self = -1, row.entries.clear();
+            for (int32_t q = b0(j); q < b1(j); ++q) {
+              const int32_t c = plan.bwd.col[q];
+              if (c == before) {  // the row just solved: its x is still in a register (readers does not count this)
+                row.entries.insert(row.entries.begin(), {plan.bwd.val[q], 0, false, false, true});
+                continue;
+              }
+              row.entries.push_back({plan.bwd.val[q], (uint8_t)slot[c], true, false, false});
+            }
+            for (int32_t q = b0(j); q < b1(j); ++q) {
+              const int32_t c = plan.bwd.col[q];
+              if (c != before && --readers[c] == 0) {
+                // in the last rows of a domain a slot may be taken next by the moves of another
+                if (newpos[c] >= top0 || p - p0 < 4) late.push_back(slot[c]);
+                else slots.give(slot[c]);
+                slot[c] = -1;
+              }
+            }
+            if (after >= 0)
+              for (int32_t q = b0(after); q < b1(after); ++q)
+                if (plan.bwd.col[q] == j) --readers[j];
+            if (readers[j] > 0) slot[j] = slots.take(), row.self = slot[j];
+            pw.row(row);
+            settle();
+          }
+        }
+        pw.end();
+        lay.bwd_page[2 * w + 1] = pw.pages;
+        note(slots.peak);
+      }
+    };
+    auto write_tasks = [&] {
+      try {
+        std::vector<int32_t> slot(n, -1), readers(n, 0);
+        for (int32_t w = next_task++; w < lay.tasks; w = next_task++) write_task(w, slot, readers);
+      } catch (...) {
+        const std::lock_guard<std::mutex> lock(error_mutex);
+        error = std::current_exception();
+      }
+    };
+    {
+      // a thread for 4,096 rows, at most eight: 46,293 rows' packets took 28 ms with one
+      const int32_t most = std::min<int32_t>({8, n / 4096, lay.tasks, (int32_t)std::thread::hardware_concurrency()});
+      std::vector<std::thread> threads;
+      try {
+        for (int32_t i = 1; i < most; ++i) threads.emplace_back(write_tasks);
+      } catch (const std::system_error &) {  // no more threads: those there are do
+      }
+      write_tasks();
+      for (auto &t : threads) t.join();
     }
-  }
-  lay.slots = std::max(peak, 1);
-  // the top's triangles by rows
-  lay.l_ptr.assign(1, 0), lay.u_ptr.assign(1, 0);
-  for (int32_t i = 0; i < lay.top; ++i) {
-    const int32_t j = at[top0 + i];
-    for (int32_t q = f0(j); q < f1(j); ++q)
-      if (newpos[plan.fwd.col[q]] >= top0) lay.l_col.push_back(newpos[plan.fwd.col[q]] - top0), lay.l_val.push_back(plan.fwd.val[q]);
-    for (int32_t q = b0(j); q < b1(j); ++q) {  // a top row's backward entries are top rows: its ancestors
-      if (newpos[plan.bwd.col[q]] < top0) throw host::Error(host::kInternal, "a top row reads a row below the top");
-      lay.u_col.push_back(newpos[plan.bwd.col[q]] - top0), lay.u_val.push_back(plan.bwd.val[q]);
+    if (error) std::rethrow_exception(error);
+    size_t blob_bytes = 0;
+    for (int32_t w = 0; w < lay.tasks; ++w) {
+      lay.fwd_page[2 * w] = (int32_t)(blob_bytes / kSpreadPage), lay.bwd_page[2 * w] += lay.fwd_page[2 * w];
+      blob_bytes += blobs[w].size();
     }
-    lay.l_ptr.push_back((int32_t)lay.l_col.size()), lay.u_ptr.push_back((int32_t)lay.u_col.size());
-    lay.l_dinv.push_back(plan.fwd.dinv[fat[j]]), lay.u_dinv.push_back(plan.bwd.dinv[bat[j]]);
-  }
-  // the norms; || |L_TT| |U_TT| e ||inf bounds the Schur complement's
-  {
-    std::vector<double> u(lay.top);
+    lay.blob.reserve(blob_bytes);
+    for (const auto &b : blobs) lay.blob.insert(lay.blob.end(), b.begin(), b.end());
+    lay.slots = std::max<int32_t>(peak, 1);
+    // the top's triangles by rows
+    lay.l_ptr.assign(1, 0), lay.u_ptr.assign(1, 0);
     for (int32_t i = 0; i < lay.top; ++i) {
-      u[i] = 1.0 / magnitude_of(lay.u_dinv[i]);
-      for (int32_t q = lay.u_ptr[i]; q < lay.u_ptr[i + 1]; ++q) u[i] += magnitude_of(lay.u_val[q]);
-      lay.u_norm = std::max(lay.u_norm, u[i]);
+      const int32_t j = at[top0 + i];
+      for (int32_t q = f0(j); q < f1(j); ++q)
+        if (newpos[plan.fwd.col[q]] >= top0) lay.l_col.push_back(newpos[plan.fwd.col[q]] - top0), lay.l_val.push_back(plan.fwd.val[q]);
+      for (int32_t q = b0(j); q < b1(j); ++q) {  // a top row's backward entries are top rows: its ancestors
+        if (newpos[plan.bwd.col[q]] < top0) throw host::Error(host::kInternal, "a top row reads a row below the top");
+        lay.u_col.push_back(newpos[plan.bwd.col[q]] - top0), lay.u_val.push_back(plan.bwd.val[q]);
+      }
+      lay.l_ptr.push_back((int32_t)lay.l_col.size()), lay.u_ptr.push_back((int32_t)lay.u_col.size());
+      lay.l_dinv.push_back(plan.fwd.dinv[fat[j]]), lay.u_dinv.push_back(plan.bwd.dinv[bat[j]]);
     }
-    for (int32_t i = 0; i < lay.top; ++i) {
-      double l = 1.0 / magnitude_of(lay.l_dinv[i]), s = l * u[i];
-      for (int32_t q = lay.l_ptr[i]; q < lay.l_ptr[i + 1]; ++q)
-        l += magnitude_of(lay.l_val[q]), s += magnitude_of(lay.l_val[q]) * u[lay.l_col[q]];
-      lay.l_norm = std::max(lay.l_norm, l), lay.s_norm = std::max(lay.s_norm, s);
+    // the norms; || |L_TT| |U_TT| e ||inf bounds the Schur complement's
+    {
+      std::vector<double> u(lay.top);
+      for (int32_t i = 0; i < lay.top; ++i) {
+        u[i] = 1.0 / magnitude_of(lay.u_dinv[i]);
+        for (int32_t q = lay.u_ptr[i]; q < lay.u_ptr[i + 1]; ++q) u[i] += magnitude_of(lay.u_val[q]);
+        lay.u_norm = std::max(lay.u_norm, u[i]);
+      }
+      for (int32_t i = 0; i < lay.top; ++i) {
+        double l = 1.0 / magnitude_of(lay.l_dinv[i]), s = l * u[i];
+        for (int32_t q = lay.l_ptr[i]; q < lay.l_ptr[i + 1]; ++q)
+          l += magnitude_of(lay.l_val[q]), s += magnitude_of(lay.l_val[q]) * u[lay.l_col[q]];
+        lay.l_norm = std::max(lay.l_norm, l), lay.s_norm = std::max(lay.s_norm, s);
+      }
     }
+    if (std::is_same_v<V, std::complex<double>>) {
+      lay.s_ptr.assign(1, 0);
+      std::vector<V> sum(lay.top, V(0));
+      std::vector<int32_t> seen(lay.top, -1), cols;
+      for (int32_t i = 0; i < lay.top; ++i) {
+        cols.clear();
+        auto add = [&](V l, int32_t k) {  // l times U's row k
+          auto entry = [&](int32_t c, V u) {
+            if (seen[c] != i) seen[c] = i, sum[c] = V(0), cols.push_back(c);
+            sum[c] += l * u;
+          };
+          entry(k, V(1) / lay.u_dinv[k]);
+          for (int32_t q = lay.u_ptr[k]; q < lay.u_ptr[k + 1]; ++q) entry(lay.u_col[q], lay.u_val[q]);
+        };
+        for (int32_t q = lay.l_ptr[i]; q < lay.l_ptr[i + 1]; ++q) add(lay.l_val[q], lay.l_col[q]);
+        add(V(1) / lay.l_dinv[i], i);
+        std::sort(cols.begin(), cols.end());
+        for (int32_t c : cols) lay.s_col.push_back(c), lay.s_val.push_back(sum[c]);
+        lay.s_ptr.push_back((int32_t)lay.s_col.size());
+      }
+    }
+    lay.in_pos.resize(n), lay.out_pos.resize(n);
+    for (int32_t i = 0; i < n; ++i) lay.in_pos[i] = newpos[plan.in_slot[i]], lay.out_pos[i] = newpos[plan.out_slot[i]];
+    return lay;
+  };
+  const Cut cut = choose();
+  SpreadLayout<V> lay = lay_out(cut);
+  const int32_t fitting = fit ? fit(lay.slots) : blocks;
+  if (fitting < blocks) {  // the slots let an SM hold fewer: for those, where the cut is then another
+    blocks = fitting;
+    const Cut again = choose();
+    if (again.cap != cut.cap) return lay_out(again);
+    lay.cost = again.cost;
   }
-  lay.in_pos.resize(n), lay.out_pos.resize(n);
-  for (int32_t i = 0; i < n; ++i) lay.in_pos[i] = newpos[plan.in_slot[i]], lay.out_pos[i] = newpos[plan.out_slot[i]];
   return lay;
 }
 
-template SpreadLayout<double> spread_layout(const Plan<double> &, int32_t, int64_t, int32_t, int32_t);
-template SpreadLayout<host::c128> spread_layout(const Plan<host::c128> &, int32_t, int64_t, int32_t, int32_t);
+template SpreadLayout<double> spread_layout(const Plan<double> &, int32_t, int64_t, int32_t, int32_t, const std::function<int32_t(int32_t)> &);
+template SpreadLayout<host::c128> spread_layout(const Plan<host::c128> &, int32_t, int64_t, int32_t, int32_t, const std::function<int32_t(int32_t)> &);
 
 }  // namespace yb

@@ -1,8 +1,13 @@
 // Launches of the spread solve (spread_solve.cuh): layouts made and uploaded at first use, one
 // factor's solves, and the complex batch over many factors.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
+#include <functional>
+#include <set>
+#include <system_error>
+#include <thread>
 
 #include "capi_common.hpp"
 #include "spread_launch.hpp"
@@ -34,79 +39,168 @@ template <class V> std::vector<typename DeviceValue<V>::type> device_values(cons
   for (size_t i = 0; i < v.size(); ++i) out[i] = DeviceValue<V>::from(v[i]);
   return out;
 }
-std::vector<int32_t> some(const std::vector<int32_t> &v) { return v.empty() ? std::vector<int32_t>{0} : v; }
 
 template <class T, bool BATCH> void allow_smem(const yb_gpu *gpu);
-template <class V>
-std::unique_ptr<DeviceSpread> make_spread(const Plan<V> &plan, int kind, int value_bytes, int64_t groups, const yb_gpu *gpu,
-                                          cudaStream_t s) {
-  using M = typename DeviceValue<V>::type;
-  // the blocks an SM holds by the kernel's registers; where a layout's slots let it hold fewer, the cut
-  // is chosen again for those
+
+// The layout on the host: for the blocks an SM holds by the kernel's registers, and where its slots let
+// an SM hold fewer, with the cut chosen again for those.
+template <class V> SpreadLayout<V> host_spread(const Plan<V> &plan, int value_bytes, int64_t groups, const yb_gpu *gpu) {
   const int most = value_bytes == 16 ? spread_blocks<cplx<double>>() : value_bytes == 8 ? spread_blocks<double>() : spread_blocks<float>();
-  SpreadLayout<V> lay = spread_layout(plan, value_bytes, groups, gpu->sm_count, most);
-  const size_t smem = (value_bytes == 16 ? spread_smem<cplx<double>>(lay.slots, kSpreadWarps)
-                       : value_bytes == 8 ? spread_smem<double>(lay.slots, kSpreadWarps)
-                                          : spread_smem<float>(lay.slots, kSpreadWarps)) + 1024;
-  const int fit = std::max<int>(1, (int)((size_t)gpu->smem_per_sm / smem));
-  if (fit < most) lay = spread_layout(plan, value_bytes, groups, gpu->sm_count, fit);
+  return spread_layout<V>(plan, value_bytes, groups, gpu->sm_count, most, [&](int32_t slots) {
+    const size_t smem = (value_bytes == 16 ? spread_smem<cplx<double>>(slots, kSpreadWarps)
+                         : value_bytes == 8 ? spread_smem<double>(slots, kSpreadWarps)
+                                            : spread_smem<float>(slots, kSpreadWarps)) + 1024;
+    return (int32_t)std::max<size_t>(1, (size_t)gpu->smem_per_sm / smem);
+  });
+}
+
+// Arrays put one after the other, 256-byte aligned, into one allocation, their places told when it is made.
+struct Packer {
+  std::vector<uint8_t> bytes;
+  size_t size = 0;  // what is uploaded and what is only reserved
+  std::vector<std::pair<size_t, std::function<void(uint8_t *)>>> places;
+  template <class P> void place(size_t n, P *&to) {
+    size = (size + 255) / 256 * 256;
+    places.emplace_back(size, [&to](uint8_t *p) { to = reinterpret_cast<P *>(p); });
+    size += std::max<size_t>(n, 1) * sizeof(P);
+  }
+  template <class P, class T> void put(const std::vector<T> &v, P *&to) {  // all puts before the first reserve
+    place(v.size(), to);
+    bytes.resize(size);
+    if (!v.empty()) std::memcpy(bytes.data() + places.back().first, v.data(), v.size() * sizeof(T));
+  }
+  void upload(DeviceArray<uint8_t> &to, cudaStream_t s) {
+    to.resize(size);
+    if (!bytes.empty()) cuda_check(cudaMemcpyAsync(to.get(), bytes.data(), bytes.size(), cudaMemcpyHostToDevice, s), "spread layout upload");
+    for (auto &[at, tell] : places) tell(to.get() + at);
+  }
+};
+
+// Layouts on the device, with their tops' maps; null where a map's condition is too large (or no layout
+// came). A layout is one allocation, all that making the maps needs another, and all maps are made by one
+// launch: an allocation for every array, and a launch and a wait for every map, took 105 ms for the first
+// pass over 16 complex networks.
+template <class V>
+std::vector<std::unique_ptr<DeviceSpread>> make_spreads(const std::vector<const SpreadLayout<V> *> &lays, const std::vector<int> &kinds,
+                                                        int value_bytes, const yb_gpu *gpu, cudaStream_t s) {
+  using M = typename DeviceValue<V>::type;
   if constexpr (std::is_same_v<V, double>)
     value_bytes == 8 ? allow_smem<double, false>(gpu) : (allow_smem<float, false>(gpu), allow_smem<pair2<float>, false>(gpu));
   else
     value_bytes == 16 ? allow_smem<cplx<double>, true>(gpu) : allow_smem<cplx<float>, true>(gpu);
-  auto d = std::make_unique<DeviceSpread>();
-  d->n = lay.n, d->tasks = lay.tasks, d->top = lay.top, d->slots = lay.slots, d->partials = lay.partials;
-  d->domains = lay.domains, d->blob_bytes = (int64_t)lay.blob.size();
-  d->blob.upload(lay.blob, s);
-  d->task_row.upload(lay.task_row, s);
-  d->fwd_page.upload(lay.fwd_page, s), d->bwd_page.upload(lay.bwd_page, s);
-  d->in_pos.upload(lay.in_pos, s), d->out_pos.upload(lay.out_pos, s);
-  d->part_ptr.upload(lay.part_ptr, s);
-  d->host_out_pos = lay.out_pos;
-  const int32_t t = lay.top;
-  if (t > 0) {
-    const size_t blocks = (size_t)(t + kSpreadTopRows - 1) / kSpreadTopRows;
-    const size_t m_values = blocks * t * kSpreadTopRows;
-    DeviceArray<int32_t> lp, lc, up, uc;
-    DeviceArray<M> lv, ld, uv, ud, scratch((size_t)((t + 31) / 32) * t * 32);
-    DeviceArray<unsigned long long> norm(2);
-    lp.upload(lay.l_ptr, s), lc.upload(some(lay.l_col), s), up.upload(lay.u_ptr, s), uc.upload(some(lay.u_col), s);
-    lv.upload(device_values(lay.l_val), s), ld.upload(device_values(lay.l_dinv), s);
-    uv.upload(device_values(lay.u_val), s), ud.upload(device_values(lay.u_dinv), s);
-    cuda_check(cudaMemsetAsync(norm.get(), 0, 2 * sizeof(unsigned long long), s), "clear the norms");
-    auto map = [&](auto kernel, DeviceArray<uint8_t> &to, int at) {
-      to.resize(m_values * sizeof(M));
-      M *m = reinterpret_cast<M *>(to.get());
-      cuda_check(cudaMemsetAsync(m, 0, m_values * sizeof(M), s), "clear a map");
-      kernel<<<(unsigned)((t + 31) / 32), 32, 0, s>>>(t, lp.get(), lc.get(), lv.get(), ld.get(), up.get(), uc.get(), uv.get(),
-                                                      ud.get(), scratch.get(), m);
-      cuda_check(cudaGetLastError(), "spread_map_kernel launch");
-      spread_norm_kernel<M><<<(unsigned)((t + 255) / 256), 256, 0, s>>>(t, m, norm.get() + at);
-      cuda_check(cudaGetLastError(), "spread_norm_kernel launch");
-    };
-    d->split = kind == YB_LU;
-    if (d->split)
-      map(spread_map_kernel<M, true, false>, d->m, 0), map(spread_map_kernel<M, false, true>, d->m2, 1);
-    else
-      map(spread_map_kernel<M, true, true>, d->m, 0);
-    unsigned long long bits[2] = {};
-    cuda_check(cudaMemcpyAsync(bits, norm.get(), sizeof bits, cudaMemcpyDeviceToHost, s), "download the norms");
-    cuda_check(cudaStreamSynchronize(s), "the top's maps");
-    double norms[2];
-    std::memcpy(norms, bits, sizeof norms);
-    d->top_condition = d->split ? std::max(norms[0] * lay.l_norm, norms[1] * lay.u_norm) : norms[0] * lay.s_norm;
-    if (!(d->top_condition <= kSpreadTopCondition)) return nullptr;
+  static std::atomic<int64_t> serial{0};
+  const size_t k = lays.size();
+  std::vector<std::unique_ptr<DeviceSpread>> out(k);
+  std::vector<Packer> kept(k);
+  struct Top {
+    const int32_t *lp, *lc, *up, *uc;
+    const M *lv, *ld, *uv, *ud, *sv = nullptr;
+    M *scratch[2], *m[2];
+  };
+  std::vector<Top> tops(k);
+  Packer temp;
+  const SpreadMap<M> *d_maps = nullptr;
+  unsigned long long *norms = nullptr;
+  std::vector<SpreadMap<M>> maps(2 * k);
+  temp.put(maps, d_maps);
+  temp.put(std::vector<unsigned long long>(2 * k), norms);
+  for (size_t i = 0; i < k; ++i) {
+    if (!lays[i]) continue;
+    const SpreadLayout<V> &lay = *lays[i];
+    out[i] = std::make_unique<DeviceSpread>();
+    DeviceSpread *d = out[i].get();
+    Top &t = tops[i];
+    d->serial = ++serial;
+    d->n = lay.n, d->tasks = lay.tasks, d->top = lay.top, d->slots = lay.slots, d->partials = lay.partials, d->domains = lay.domains;
+    d->blob_bytes = (int64_t)lay.blob.size();
+    d->refine = d->top > 0 && std::is_same_v<V, host::c128>;
+    d->split = d->top > 0 && kinds[i] == YB_LU && !d->refine;
+    d->host_out_pos = lay.out_pos;
+    Packer &p = kept[i];
+    p.put(lay.task_row, d->task_row), p.put(lay.fwd_page, d->fwd_page), p.put(lay.bwd_page, d->bwd_page);
+    p.put(lay.in_pos, d->in_pos), p.put(lay.out_pos, d->out_pos), p.put(lay.part_ptr, d->part_ptr);
+    if (lay.top == 0) continue;
+    if (d->refine) p.put(lay.s_ptr, d->s_ptr), p.put(lay.s_col, d->s_col), p.put(device_values(lay.s_val), t.sv);
+    temp.put(lay.l_ptr, t.lp), temp.put(lay.l_col, t.lc);
+    temp.put(device_values(lay.l_val), t.lv), temp.put(device_values(lay.l_dinv), t.ld);
+    std::vector<int32_t> u_ptr{0}, u_col;  // the rows from the last to the first
+    std::vector<V> u_val, u_dinv(lay.u_dinv.rbegin(), lay.u_dinv.rend());
+    u_col.reserve(lay.u_col.size()), u_val.reserve(lay.u_val.size());
+    for (int32_t r = lay.top - 1; r >= 0; --r) {
+      u_col.insert(u_col.end(), lay.u_col.begin() + lay.u_ptr[r], lay.u_col.begin() + lay.u_ptr[r + 1]);
+      u_val.insert(u_val.end(), lay.u_val.begin() + lay.u_ptr[r], lay.u_val.begin() + lay.u_ptr[r + 1]);
+      u_ptr.push_back((int32_t)u_col.size());
+    }
+    temp.put(u_ptr, t.up), temp.put(u_col, t.uc), temp.put(device_values(u_val), t.uv), temp.put(device_values(u_dinv), t.ud);
+  }
+  const auto blocks = [](int64_t rows, int64_t of) { return (rows + of - 1) / of; };
+  int32_t most = 0;
+  for (size_t i = 0; i < k; ++i) {
+    DeviceSpread *d = out[i].get();
+    if (!d) continue;
+    const int64_t t = d->top, count = t == 0 ? 0 : d->split ? 2 : 1;
+    most = std::max(most, d->top);
+    for (int64_t j = 0; j < count; ++j) {
+      kept[i].place((size_t)(blocks(t, kSpreadTopRows) * t * kSpreadTopRows), tops[i].m[j]);
+      temp.place((size_t)(blocks(t, 32) * t * 32), tops[i].scratch[j]);
+    }
+    kept[i].place(lays[i]->blob.size(), d->blob);
+    kept[i].upload(d->store, s);
+    cuda_check(cudaMemcpyAsync(const_cast<uint8_t *>(d->blob), lays[i]->blob.data(), lays[i]->blob.size(), cudaMemcpyHostToDevice, s),
+               "spread packet upload");
+    d->s_val = tops[i].sv;
+    if (count) d->m = tops[i].m[0];
+    if (count == 2) d->m2 = tops[i].m[1];
+    if (count)  // the rows past the last of a block of rows
+      cuda_check(cudaMemsetAsync(d->m, 0, (size_t)(d->blob - (uint8_t *)d->m), s), "clear the maps");
+  }
+  if (most > 0) {
+    DeviceArray<uint8_t> temporary;
+    // the maps' descriptors need the addresses: made first, then uploaded
+    temporary.resize(temp.size);
+    for (auto &[at, tell] : temp.places) tell(temporary.get() + at);
+    for (size_t i = 0; i < k; ++i) {
+      const DeviceSpread *d = out[i].get();
+      if (!d || d->top == 0) continue;
+      const Top &t = tops[i];
+      const SpreadMap<M> both{d->top, (int32_t)blocks(d->top, 32), t.lp, t.lc, t.lv, t.ld, t.up, t.uc, t.uv, t.ud,
+                              t.scratch[0], t.m[0], norms + 2 * i};
+      maps[2 * i] = both;
+      if (d->split) {
+        maps[2 * i + 1] = both;
+        maps[2 * i].u_ptr = nullptr, maps[2 * i + 1].l_ptr = nullptr;
+        maps[2 * i + 1].scratch = t.scratch[1], maps[2 * i + 1].m = t.m[1], maps[2 * i + 1].norm = norms + 2 * i + 1;
+      }
+    }
+    std::memcpy(temp.bytes.data() + temp.places[0].first, maps.data(), maps.size() * sizeof maps[0]);
+    cuda_check(cudaMemcpyAsync(temporary.get(), temp.bytes.data(), temp.bytes.size(), cudaMemcpyHostToDevice, s), "upload the tops");
+    spread_map_kernel<M><<<dim3((unsigned)blocks(most, 32), (unsigned)(2 * k)), 32, 0, s>>>(d_maps);
+    cuda_check(cudaGetLastError(), "spread_map_kernel launch");
+    spread_norm_kernel<M><<<dim3((unsigned)blocks(most, 256), (unsigned)(2 * k)), 256, 0, s>>>(d_maps);
+    cuda_check(cudaGetLastError(), "spread_norm_kernel launch");
+    std::vector<unsigned long long> bits(2 * k);
+    cuda_check(cudaMemcpyAsync(bits.data(), norms, bits.size() * sizeof bits[0], cudaMemcpyDeviceToHost, s), "download the norms");
+    cuda_check(cudaStreamSynchronize(s), "the tops' maps");
+    for (size_t i = 0; i < k; ++i) {
+      DeviceSpread *d = out[i].get();
+      if (!d || d->top == 0) continue;
+      double norm[2];
+      std::memcpy(norm, &bits[2 * i], sizeof norm);
+      d->top_condition = d->split ? std::max(norm[0] * lays[i]->l_norm, norm[1] * lays[i]->u_norm) : norm[0] * lays[i]->s_norm;
+      if (!(d->top_condition <= kSpreadTopCondition)) out[i] = nullptr;
+    }
   }
   cuda_check(cudaStreamSynchronize(s), "spread layout upload");
-  return d;
+  return out;
 }
 
 SpreadNet net_of(const DeviceSpread *d, int64_t groups, int64_t count) {
   SpreadNet net{};
   net.n = d->n, net.tasks = d->tasks, net.top = d->top, net.partials = d->partials;
-  net.blob = d->blob.get(), net.fwd_page = d->fwd_page.get(), net.bwd_page = d->bwd_page.get();
-  net.task_row = d->task_row.get(), net.part_ptr = d->part_ptr.get();
-  net.in_pos = d->in_pos.get(), net.out_pos = d->out_pos.get(), net.m = d->m.get(), net.m2 = d->m2.get();
+  net.blob = d->blob, net.fwd_page = d->fwd_page, net.bwd_page = d->bwd_page;
+  net.task_row = d->task_row, net.part_ptr = d->part_ptr;
+  net.in_pos = d->in_pos, net.out_pos = d->out_pos, net.m = d->m, net.m2 = d->m2;
+  net.s_ptr = d->s_ptr, net.s_col = d->s_col, net.s_val = d->s_val;
   net.groups = groups, net.count = count;
   return net;
 }
@@ -190,7 +284,7 @@ template <class T> void one_sweeps(const DeviceSpread *d, const SpreadArgs &a, c
 // The partial array of `groups` groups: the partials and the top's solutions in T, then the top's
 // right-hand sides (and, with two maps, what is between them) in full precision (every part a multiple of 128 bytes); at least one line.
 template <class T> size_t partial_bytes(const DeviceSpread *d, int64_t groups) {
-  return (size_t)groups * 32 * ((size_t)(d->partials + d->top) * sizeof(T) + (size_t)d->top * (d->split ? 2 : 1) * sizeof(typename SpreadLane<T>::Math)) + 128;
+  return (size_t)groups * 32 * ((size_t)(d->partials + d->top) * sizeof(T) + (size_t)d->top * (d->split || d->refine ? 2 : 1) * sizeof(typename SpreadLane<T>::Math)) + 128;
 }
 template <class T> void set_partial(SpreadNet &net, uint8_t *p) {
   net.partial = p;
@@ -200,34 +294,105 @@ template <class T> void set_partial(SpreadNet &net, uint8_t *p) {
 
 }  // namespace
 
+namespace {
+
+int64_t group_class(int64_t groups) {  // a layout serves the groups up to a number of three significant bits
+  int64_t most = groups;
+  for (int64_t unit = 1; most > 8 * unit || most % unit; unit *= 2) most = (most + 2 * unit - 1) / (2 * unit) * (2 * unit);
+  return most;
+}
+
+template <class V> const Plan<V> &plan_of(const yb_factor *f) {
+  if constexpr (std::is_same_v<V, double>) return f->plan;
+  else return f->cplan;
+}
+
+// A layout or, where the factor admits none, nothing.
+template <class V> std::unique_ptr<SpreadLayout<V>> try_layout(const yb_factor *f, int value_bytes, int64_t groups) {
+  try {
+    auto lay = std::make_unique<SpreadLayout<V>>(host_spread(plan_of<V>(f), value_bytes, groups, f->gpu));
+    const int32_t limit = f->is_complex ? kSpreadAutoSlotsComplex : kSpreadAutoSlots;
+    return lay->slots <= limit ? std::move(lay) : nullptr;
+  } catch (const host::Error &e) {
+    if (e.status != host::kInvalidArgument && e.status != host::kTooLarge) throw;
+    return nullptr;
+  }
+}
+
+}  // namespace
+
 DeviceSpread *spread_for(yb_factor *f, int value_bytes, int64_t groups, cudaStream_t stream) {
   const std::lock_guard<std::mutex> lock(f->spread_mutex);
-  int64_t most = groups;  // a layout for groups up to each number of three significant bits
-  for (int64_t unit = 1; most > 8 * unit || most % unit; unit *= 2) most = (most + 2 * unit - 1) / (2 * unit) * (2 * unit);
-  const auto key = std::make_pair(value_bytes, most);
+  const auto key = std::make_pair(value_bytes, group_class(groups));
   auto it = f->spreads.find(key);
   if (it != f->spreads.end()) return it->second.get();
   if (capturing(stream)) {  // nothing may be made now: the nearest layout there is, if any
     auto near = f->spreads.end();
     for (auto i = f->spreads.begin(); i != f->spreads.end(); ++i)
       if (i->first.first == value_bytes && i->second &&
-          (near == f->spreads.end() || std::abs(i->first.second - most) < std::abs(near->first.second - most)))
+          (near == f->spreads.end() || std::abs(i->first.second - key.second) < std::abs(near->first.second - key.second)))
         near = i;
     return near == f->spreads.end() ? nullptr : near->second.get();
   }
-  std::unique_ptr<DeviceSpread> d;
-  try {
-    d = f->is_complex ? make_spread(f->cplan, f->kind, value_bytes, most, f->gpu, stream)
-                      : make_spread(f->plan, f->kind, value_bytes, most, f->gpu, stream);
-    const int32_t limit = f->is_complex ? kSpreadAutoSlotsComplex : kSpreadAutoSlots;
-    if (d && d->slots > limit) d.reset();
-  } catch (const host::Error &e) {
-    if (e.status != host::kInvalidArgument && e.status != host::kTooLarge) throw;
-    d.reset();
-  }
+  const auto lay = try_layout<double>(f, value_bytes, key.second);
+  auto d = std::move(make_spreads<double>({lay.get()}, {f->kind}, value_bytes, f->gpu, stream)[0]);
   auto *out = d.get();
   f->spreads.emplace(key, std::move(d));
   return out;
+}
+
+void spread_for_batch(const std::vector<yb_factor *> &factors, int value_bytes, const std::vector<int64_t> &counts,
+                      std::vector<DeviceSpread *> &out, cudaStream_t stream) {
+  const size_t k = factors.size();
+  // each network's share of the batch in groups of its own: the cut weighs the whole batch's load
+  double load = 0;
+  for (size_t i = 0; i < k; ++i) load += (double)factors[i]->n * (double)((counts[i] + 31) / 32);
+  std::vector<std::unique_ptr<SpreadLayout<host::c128>>> made(k);
+  std::vector<std::pair<int, int64_t>> keys(k);
+  std::vector<size_t> missing;
+  std::set<std::pair<yb_factor *, int64_t>> seen;
+  for (size_t i = 0; i < k; ++i) {
+    keys[i] = {value_bytes, group_class(std::max<int64_t>(1, (int64_t)std::ceil(load / (double)factors[i]->n)))};
+    const std::lock_guard<std::mutex> lock(factors[i]->spread_mutex);
+    if (counts[i] > 0 && !factors[i]->spreads.count(keys[i]) && seen.insert({factors[i], keys[i].second}).second) missing.push_back(i);
+  }
+  // the layouts not made yet, on the host's threads, largest networks first
+  std::sort(missing.begin(), missing.end(), [&](size_t a, size_t b) { return factors[a]->n > factors[b]->n; });
+  std::atomic<size_t> next{0};
+  std::vector<std::exception_ptr> errors(missing.size());
+  auto work = [&] {
+    for (size_t m = next++; m < missing.size(); m = next++)
+      try {
+        made[missing[m]] = try_layout<host::c128>(factors[missing[m]], value_bytes, keys[missing[m]].second);
+      } catch (...) {
+        errors[m] = std::current_exception();
+      }
+  };
+  std::vector<std::thread> threads;
+  const size_t most = std::min<size_t>(missing.size(), std::max(1u, std::thread::hardware_concurrency()));
+  try {
+    for (size_t t = 1; t < most; ++t) threads.emplace_back(work);
+  } catch (const std::system_error &) {  // no more threads: those there are do
+  }
+  work();
+  for (auto &t : threads) t.join();
+  for (auto &e : errors)
+    if (e) std::rethrow_exception(e);
+  if (!missing.empty()) {
+    std::vector<const SpreadLayout<host::c128> *> lays;
+    for (size_t i : missing) lays.push_back(made[i].get());
+    auto d = make_spreads<host::c128>(lays, std::vector<int>(missing.size(), YB_LU), value_bytes, factors[0]->gpu, stream);
+    for (size_t m = 0; m < missing.size(); ++m) {
+      const std::lock_guard<std::mutex> lock(factors[missing[m]]->spread_mutex);
+      factors[missing[m]]->spreads.emplace(keys[missing[m]], std::move(d[m]));
+    }
+  }
+  out.assign(k, nullptr);
+  for (size_t i = 0; i < k; ++i) {
+    const std::lock_guard<std::mutex> lock(factors[i]->spread_mutex);
+    auto it = factors[i]->spreads.find(keys[i]);
+    if (it != factors[i]->spreads.end()) out[i] = it->second.get();
+  }
 }
 
 template <class T>
@@ -341,50 +506,54 @@ void spread_batch(const std::vector<SpreadSystem> &systems, bool add, SpreadBatc
   w.work.reserve(work_values * sizeof(T)), w.partial.reserve(part_bytes);
   const int split = split_top<T>(top_total, gpu);
   const int warps = sweep_warps<T>(slots, most_groups, gpu);
-  // the blocks' items: the gather's and scatter's, the sweeps' (each network's tasks are longest
-  // first; the networks' tasks by rank, so every network's long tasks start early), the top's
-  std::vector<SpreadItem> io, sweep, sum, top;
   T *work = reinterpret_cast<T *>(w.work.get());
   uint8_t *partial = w.partial.get();
-  int32_t most_tasks = 0;
+  std::vector<int64_t> key{(int64_t)sizeof(T), warps, split};
   for (size_t i = 0; i < k; ++i) {
     const SpreadSystem &sys = systems[i];
-    const DeviceSpread *d = sys.layout;
     const int64_t groups = (sys.count + 31) / 32;
     SpreadNet &net = nets[i];
-    net = net_of(d, groups, sys.count);
+    net = net_of(sys.layout, groups, sys.count);
     net.work = net.xout = work + kSpreadPad * 32;
     set_partial<T>(net, partial);
-    net.b = sys.b, net.ldb = d->n, net.x = sys.x, net.ldx = d->n;
-    work += (size_t)groups * d->n * 32 + 2 * kSpreadPad * 32;
-    partial += partial_bytes<T>(d, groups);
-    most_tasks = std::max(most_tasks, d->tasks);
-    const int32_t row_blocks = (int32_t)((d->n + 32 * kSpreadIoWarps - 1) / (32 * kSpreadIoWarps));
-    for (int64_t g = 0; g < groups; ++g) {
-      for (int32_t c = 0; c < row_blocks; ++c) io.push_back({(int32_t)i, c, (int32_t)g, 0});
-      for (int32_t c = 0; c < (d->top + 7) / 8; ++c) sum.push_back({(int32_t)i, c, (int32_t)g, 0});
-      for (int32_t c = 0; c < top_blocks<T>(d, split); ++c) top.push_back({(int32_t)i, c, (int32_t)g, 0});
-    }
+    net.b = sys.b, net.ldb = sys.layout->n, net.x = sys.x, net.ldx = sys.layout->n;
+    work += (size_t)groups * sys.layout->n * 32 + 2 * kSpreadPad * 32;
+    partial += partial_bytes<T>(sys.layout, groups);
+    key.push_back(sys.layout->serial), key.push_back(groups);
   }
-  for (int32_t t = 0; t < most_tasks; ++t)
-    for (size_t i = 0; i < k; ++i)
-      if (t < systems[i].layout->tasks)
-        for (int64_t g = 0; g < nets[i].groups; g += warps) sweep.push_back({(int32_t)i, t, (int32_t)g, 0});
-  const size_t n_io = io.size(), n_sweep = sweep.size(), n_sum = sum.size(), n_top = top.size();
-  if (n_io == 0) return;
-  std::vector<uint8_t> all(sizeof(SpreadNet) * k + sizeof(SpreadItem) * (n_io + n_sweep + n_sum + n_top));
-  const size_t net_bytes = sizeof(SpreadNet) * k;
-  std::memcpy(all.data(), nets.data(), net_bytes);
-  auto *items = reinterpret_cast<SpreadItem *>(all.data() + net_bytes);
-  std::copy(io.begin(), io.end(), items);
-  std::copy(sweep.begin(), sweep.end(), items + n_io);
-  std::copy(sum.begin(), sum.end(), items + n_io + n_sweep);
-  std::copy(top.begin(), top.end(), items + n_io + n_sweep + n_sum);
-  w.args.reserve(all.size());
-  cuda_check(cudaMemcpyAsync(w.args.get(), all.data(), all.size(), cudaMemcpyHostToDevice, stream), "upload the batch");
-  const auto *d_items = reinterpret_cast<const SpreadItem *>(w.args.get() + net_bytes);
+  w.nets.reserve(sizeof(SpreadNet) * k);
+  cuda_check(cudaMemcpyAsync(w.nets.get(), nets.data(), sizeof(SpreadNet) * k, cudaMemcpyHostToDevice, stream), "upload the batch");
+  if (key != w.key) {
+    // the blocks' items: the gather's and scatter's, the sweeps' (each network's tasks are longest
+    // first; the networks' tasks by rank, so every network's long tasks start early), the top's
+    std::vector<SpreadItem> io, sweep, sum, top;
+    int32_t most_tasks = 0;
+    for (size_t i = 0; i < k; ++i) {
+      const DeviceSpread *d = systems[i].layout;
+      most_tasks = std::max(most_tasks, d->tasks);
+      const int32_t row_blocks = (int32_t)((d->n + 32 * kSpreadIoWarps - 1) / (32 * kSpreadIoWarps));
+      for (int64_t g = 0; g < nets[i].groups; ++g) {
+        for (int32_t c = 0; c < row_blocks; ++c) io.push_back({(int32_t)i, c, (int32_t)g, 0});
+        for (int32_t c = 0; c < (d->top + 7) / 8; ++c) sum.push_back({(int32_t)i, c, (int32_t)g, 0});
+        for (int32_t c = 0; c < top_blocks<T>(d, split); ++c) top.push_back({(int32_t)i, c, (int32_t)g, 0});
+      }
+    }
+    for (int32_t t = 0; t < most_tasks; ++t)
+      for (size_t i = 0; i < k; ++i)
+        if (t < systems[i].layout->tasks)
+          for (int64_t g = 0; g < nets[i].groups; g += warps) sweep.push_back({(int32_t)i, t, (int32_t)g, 0});
+    w.key.clear();
+    w.n_io = io.size(), w.n_sweep = sweep.size(), w.n_sum = sum.size(), w.n_top = top.size();
+    for (auto *more : {&sweep, &sum, &top}) io.insert(io.end(), more->begin(), more->end());
+    w.items.reserve(sizeof(SpreadItem) * io.size());
+    cuda_check(cudaMemcpyAsync(w.items.get(), io.data(), sizeof(SpreadItem) * io.size(), cudaMemcpyHostToDevice, stream),
+               "upload the batch's blocks");
+    w.key = std::move(key);
+  }
+  const size_t n_io = w.n_io, n_sweep = w.n_sweep, n_sum = w.n_sum, n_top = w.n_top;
+  const auto *d_items = reinterpret_cast<const SpreadItem *>(w.items.get());
   SpreadArgs a{};
-  a.nets = reinterpret_cast<const SpreadNet *>(w.args.get());
+  a.nets = reinterpret_cast<const SpreadNet *>(w.nets.get());
   a.slots = slots;
   const size_t smem = spread_smem<T>(slots, warps);
   a.items = d_items;
@@ -394,15 +563,18 @@ void spread_batch(const std::vector<SpreadSystem> &systems, bool add, SpreadBatc
   if (n_top) {
     a.items = d_items + n_io + n_sweep;
     launch(spread_sum_kernel<T, true>, (unsigned)n_sum, 256, 0, stream, true, a);
-    a.items = d_items + n_io + n_sweep + n_sum;
-    auto phase = [&](auto one) {  // complex factors are LU factors: two maps
+    auto phase = [&](auto one) {
+      a.items = d_items + n_io + n_sweep + n_sum;
       constexpr int PHASE = decltype(one)::value;
       if (split > 1)
         launch(spread_top_kernel<T, true, spread_split<T>(), PHASE>, (unsigned)n_top, spread_top_warps<T, spread_split<T>()>() * 32, 0, stream, true, a);
       else
         launch(spread_top_kernel<T, true, 1, PHASE>, (unsigned)n_top, spread_top_warps<T, 1>() * 32, 0, stream, true, a);
     };
-    phase(std::integral_constant<int, 1>()), phase(std::integral_constant<int, 2>());
+    phase(std::integral_constant<int, 3>());
+    a.items = d_items + n_io + n_sweep;
+    launch(spread_correct_kernel<T, true>, (unsigned)n_sum, 256, 0, stream, true, a);
+    phase(std::integral_constant<int, 4>());
   }
   a.items = d_items + n_io;
   launch(spread_sweep_kernel<T, true, true>, (unsigned)n_sweep, warps * 32, smem, stream, true, a);

@@ -10,7 +10,7 @@ namespace yb {
 
 // The automatic choice takes the spread solve up to this many live values per lane: with more, too
 // few warps fit an SM to cover their shared-memory latency.
-constexpr int32_t kSpreadAutoSlots = 64, kSpreadAutoSlotsComplex = 400;
+constexpr int32_t kSpreadAutoSlots = 64, kSpreadAutoSlotsComplex = 96;
 
 // The spread layout for `groups` groups of 32 right-hand sides with values of `value_bytes`, made and
 // uploaded at its first use; null if the factor admits none.
@@ -28,6 +28,11 @@ bool spread_solve(yb_factor *f, const double *b, int64_t ldb, double *x, int64_t
 template <class T>
 void spread_sweeps(yb_factor *f, DeviceSpread *d, T *work, T *xout, int64_t groups, const uint8_t *group_active,
                    cudaStream_t stream);
+
+// The spread layouts of a batch of complex factors with these counts of right-hand sides (null: none), the
+// missing ones made on several threads of the host.
+void spread_for_batch(const std::vector<yb_factor *> &factors, int value_bytes, const std::vector<int64_t> &counts,
+                      std::vector<DeviceSpread *> &out, cudaStream_t stream);
 
 // One factor's part of a complex batch: right-hand sides and solutions complex128, column-major.
 struct SpreadSystem {

@@ -6,7 +6,7 @@
 //   spread_sweep  every task forward: z over b in the work array, updates of top rows into the
 //                 partial array
 //   spread_sum    the top's right-hand sides r_T: b_T plus the partials
-//   spread_top    x_T as a dense product of r_T, or two
+//   spread_top    x_T as a dense product of r_T, or two (complex: spread_correct between them)
 //   spread_sweep  every task backward, from the top solutions
 //   spread_out    the work array into x
 //
@@ -21,7 +21,8 @@
 // sizes before: 2,000-bus B' with one right-hand side 71 to 29 us; 10,000-bus B' with 64, 87 to 42 us,
 // with 999, 330 to 138 us, with 13,499, 1,684 to 1,494 us (the gather 0.36 and the scatter 0.35 ms at
 // 6.1 TB/s, the sweeps and the top 0.82 ms: 5.3 TB/s over their 4.3 GB); the 10,000-bus Jacobian's LU
-// with 4,096, 1,336 to 1,036 us. What bounds it: for large blocks HBM in the gather and scatter and
+// with 4,096, 1,336 to 1,036 us; 16 complex networks of 500 to 46,293 buses with 128 each, complex128 7.5 to
+// 0.91 ms, complex64 with refinement 21.1 to 5.6 ms. What bounds it: for large blocks HBM in the gather and scatter and
 // the shared-memory pipe (about 18 wavefronts a row and sweep) near HBM in the sweeps; for small ones
 // the six launches and the longest task's chain (about 290 cycles a row where a warp is alone).
 #pragma once
@@ -47,9 +48,11 @@ struct SpreadNet {
   const int32_t *__restrict__ fwd_page, *__restrict__ bwd_page, *__restrict__ task_row, *__restrict__ part_ptr;
   const int32_t *__restrict__ in_pos, *__restrict__ out_pos;
   const void *__restrict__ m, *__restrict__ m2;  // the top's maps in blocks of kSpreadTopRows rows (m2: null with one)
+  const int32_t *__restrict__ s_ptr, *__restrict__ s_col;  // S by rows (complex)
+  const void *__restrict__ s_val;
   int64_t groups, count;       // groups of a warp's columns (32, or 64 with two per lane), and columns
   void *work, *xout, *partial; // xout: where the backward sweep writes (work, or an array of its layout)
-  void *r, *r2;                // the top's right-hand sides [group][top row][32 lanes], full precision; L_TT^-1 r_T
+  void *r, *r2;                // the top's right-hand sides [group][top row][32 lanes], full precision; what is between two products
   const uint8_t *group_active; // [groups] 0: skipped; null: all run
   const void *b;               // the caller's right-hand sides and solutions
   int64_t ldb;
@@ -499,6 +502,45 @@ template <class T, bool BATCH> __global__ void __launch_bounds__(256) spread_sum
   sp_stg(static_cast<M *>(net.r) + ((size_t)g * net.top + k) * 32 + lane, s);
 }
 
+// r_T -= S r2, each row in place: the residual of the first product, for its correction.
+template <class T, bool BATCH> __global__ void __launch_bounds__(256) spread_correct_kernel(const __grid_constant__ SpreadArgs a) {
+  using M = typename SpreadLane<T>::Math;
+  using MS = typename SpreadLane<T>::MathS;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int64_t g;
+  int k;
+  const SpreadNet *np = &a.one;
+  if constexpr (BATCH) {
+    const SpreadItem it = a.items[blockIdx.x];
+    np = a.nets + it.net;
+    g = it.b, k = it.a * 8 + warp;
+  } else {
+    const int blocks = (a.one.top + 7) / 8;
+    g = blockIdx.x / blocks, k = (int)(blockIdx.x % blocks) * 8 + warp;
+  }
+  const SpreadNet &net = *np;
+  sp_ready();
+  if (k >= net.top || (net.group_active && !net.group_active[g])) return;
+  M *r = static_cast<M *>(net.r) + ((size_t)g * net.top + k) * 32 + lane;
+  const M *x = static_cast<const M *>(net.r2) + (size_t)g * net.top * 32 + lane;
+  const MS *val = static_cast<const MS *>(net.s_val);
+  const int q1 = __ldg(net.s_ptr + k + 1);
+  M s = sp_ldg(r);
+  for (int q = __ldg(net.s_ptr + k); q < q1; q += 4) {
+    M v[4];
+    MS c[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int at = min(q + i, q1 - 1);
+      c[i] = val[at], v[i] = sp_ldg(x + (size_t)__ldg(net.s_col + at) * 32);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (q + i < q1) s = sp_fnma(c[i], v[i], s);
+  }
+  sp_stg(r, s);
+}
+
 // D += A B on the FP64 tensor cores: A 8 x 4 (lane: row lane / 4, column lane % 4), B 4 x 8 (row lane % 4,
 // column lane / 4), D 8 x 8 (row lane / 4, columns 2 (lane % 4) and the next).
 __device__ __forceinline__ void sp_mma(double (&d)[2], double a, double b) {
@@ -520,7 +562,8 @@ __device__ __forceinline__ void sp_store2(cplx<float> *p, cplx<double> a, cplx<d
 
 // The top's product on the FP64 tensor cores, 16 rows by 32 columns a warp, fragments straight from L2
 // (the map and a group's columns are read by many warps; four steps of loads in flight). PHASE 0: x_T =
-// M r_T; 1: r2 = L_TT^-1 r_T; 2: x_T = U_TT^-1 r2, a triangle's zeros passed over. KS > 1: a block's KS
+// M r_T; 1: r2 = L_TT^-1 r_T; 2: x_T = U_TT^-1 r2, a triangle's zeros passed over; 3: r2 = M r_T;
+// 4: x_T = r2 + M r_T. KS > 1: a block's KS
 // warps split the map's columns and add up in order at the end: with few groups there are too few
 // tiles to fill the SMs, and a tile's chain of steps sets the time. x_T goes to its own rows after the
 // partials (the work array's top rows stay b_T) and to the separate output array if there is one.
@@ -580,10 +623,12 @@ __global__ void __launch_bounds__(spread_top_warps<T, KS>() * 32) spread_top_ker
   V *r2 = static_cast<V *>(net.r2) + (size_t)g * t * COLS + tile * 32;
   auto store = [&](int row, int col, V v0, V v1) {
     if (row >= t) return;
-    if constexpr (PHASE == 1) {
-      sp_store2(r2 + (size_t)row * COLS + col, v0, v1);
+    V *between = r2 + (size_t)row * COLS + col;
+    if constexpr (PHASE == 1 || PHASE == 3) {
+      sp_store2(between, v0, v1);
       return;
     }
+    if constexpr (PHASE == 4) v0 = sp_add(v0, between[0]), v1 = sp_add(v1, between[1]);
     sp_store2(xt + (size_t)row * COLS + col, v0, v1);
     if (xo) sp_store2(xo + (size_t)row * COLS + col, v0, v1);
   };
@@ -611,55 +656,92 @@ __global__ void __launch_bounds__(spread_top_warps<T, KS>() * 32) spread_top_ker
   }
 }
 
-// The top's map: its substitutions (LOWER, UPPER, or both) applied to the identity, 32 columns per
-// warp, in the factor's full precision. `scratch` holds [column chunk][row][32].
-template <class M, bool LOWER, bool UPPER>
-__global__ void __launch_bounds__(32) spread_map_kernel(int32_t t, const int32_t *__restrict__ l_ptr, const int32_t *__restrict__ l_col,
-                                                        const M *__restrict__ l_val, const M *__restrict__ l_dinv,
-                                                        const int32_t *__restrict__ u_ptr, const int32_t *__restrict__ u_col,
-                                                        const M *__restrict__ u_val, const M *__restrict__ u_dinv, M *scratch, M *m) {
-  const int lane = threadIdx.x, e = blockIdx.x * 32 + lane;
-  M *z = scratch + (size_t)blockIdx.x * t * 32 + lane;
-  auto row = [&](M s, const int32_t *ptr, const int32_t *col, const M *val, int p) {
-    const int q1 = __ldg(ptr + p + 1);
-    int q = __ldg(ptr + p);
-    for (; q + 4 <= q1; q += 4) {
-      M v[4], x[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) v[i] = val[q + i], x[i] = z[(size_t)__ldg(col + q + i) * 32];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) s = sp_fnma(v[i], x[i], s);
-    }
-    for (; q < q1; ++q) s = sp_fnma(val[q], z[(size_t)__ldg(col + q) * 32], s);
-    return s;
-  };
+// A top's map to make: the substitutions with its triangles (a null pointer: without that one) applied
+// to the identity, in the factor's full precision. The upper triangle's rows (pointers, entries and
+// diagonals) run from the last to the first, as they are solved. `scratch` holds [column chunk][row][32].
+template <class M> struct SpreadMap {
+  int32_t t, chunks;  // chunks of 32 columns
+  const int32_t *l_ptr, *l_col;
+  const M *l_val, *l_dinv;
+  const int32_t *u_ptr, *u_col;
+  const M *u_val, *u_dinv;
+  M *scratch, *m;
+  unsigned long long *norm;
+};
+
+// One warp makes 32 columns of map blockIdx.y; the maps of all of a batch's networks in one launch. A
+// chain of rows, each of a few entries: what bounds it is the latency from one row's solution to the
+// next row's loads of it, so the entries come 32 at a time through registers into shared memory, one
+// chunk ahead, and the rows' bounds and diagonals one row ahead.
+template <class M> __global__ void __launch_bounds__(32) spread_map_kernel(const SpreadMap<M> *__restrict__ maps) {
+  const SpreadMap<M> map = maps[blockIdx.y];
+  if ((int)blockIdx.x >= map.chunks) return;
+  __shared__ M sv[32];
+  __shared__ int32_t sc[32];
+  const int t = map.t, lane = threadIdx.x, e = blockIdx.x * 32 + lane;
+  M *z = map.scratch + (size_t)blockIdx.x * t * 32 + lane;
+  M *m = map.m;
   auto out = [&](int p, M x) {
     if (e < t) m[((size_t)(p / kSpreadTopRows) * t + e) * kSpreadTopRows + p % kSpreadTopRows] = x;
   };
-  for (int p = 0; p < t; ++p) {
-    M x = M(p == e ? 1 : 0);
-    if constexpr (LOWER) x = row(x, l_ptr, l_col, l_val, p) * l_dinv[p];
-    z[(size_t)p * 32] = x;
-    if constexpr (!UPPER) out(p, x);
-  }
-  if constexpr (UPPER)
-    for (int p = t - 1; p >= 0; --p) {
-      const M x = row(z[(size_t)p * 32], u_ptr, u_col, u_val, p) * u_dinv[p];
-      z[(size_t)p * 32] = x;
-      out(p, x);
+  // Row i of the arrays is row i of the map, or (`down`) row t - 1 - i.
+  auto sweep = [&](bool down, bool first, bool last, const int32_t *__restrict__ ptr, const int32_t *__restrict__ col,
+                   const M *__restrict__ val, const M *__restrict__ dinv) {
+    const int total = __ldg(ptr + t);
+    M v_next(0);
+    int c_next = 0;
+    auto fetch = [&](int k) {
+      if (k < total) v_next = val[k], c_next = __ldg(col + k);
+    };
+    fetch(lane);
+    int k = 0, end = __ldg(ptr + 1);
+    M d = dinv[0];
+    for (int i = 0; i < t; ++i) {
+      const int p = down ? t - 1 - i : i, end_now = end;
+      const M d_now = d;
+      if (i + 1 < t) end = __ldg(ptr + i + 2), d = dinv[i + 1];
+      M s = first ? M(p == e ? 1 : 0) : z[(size_t)p * 32];
+      while (k < end_now) {
+        if (k % 32 == 0) {
+          __syncwarp();
+          sv[lane] = v_next, sc[lane] = c_next;
+          __syncwarp();
+          fetch(k + 32 + lane);
+        }
+        const int run = min(end_now, (k / 32 + 1) * 32) - k, at = k % 32;
+        int q = 0;
+        for (; q + 4 <= run; q += 4) {
+          M x[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) x[j] = z[(size_t)sc[at + q + j] * 32];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) s = sp_fnma(sv[at + q + j], x[j], s);
+        }
+        for (; q < run; ++q) s = sp_fnma(sv[at + q], z[(size_t)sc[at + q] * 32], s);
+        k += run;
+      }
+      s = s * d_now;
+      z[(size_t)p * 32] = s;
+      if (last) out(p, s);
     }
+  };
+  if (map.l_ptr) sweep(false, true, !map.u_ptr, map.l_ptr, map.l_col, map.l_val, map.l_dinv);
+  if (map.u_ptr) sweep(true, !map.l_ptr, true, map.u_ptr, map.u_col, map.u_val, map.u_dinv);
 }
 
 __device__ __forceinline__ double spread_abs(double v) { return fabs(v); }
 __device__ __forceinline__ double spread_abs(const cplx<double> &v) { return hypot(v.re, v.im); }
 
 // ||M||inf as a bit pattern (positive doubles order as theirs; a NaN lies above them all).
-template <class M> __global__ void spread_norm_kernel(int32_t t, const M *__restrict__ m, unsigned long long *norm) {
+template <class M> __global__ void spread_norm_kernel(const SpreadMap<M> *__restrict__ maps) {
+  const SpreadMap<M> map = maps[blockIdx.y];
+  const int t = map.t;
+  const M *m = map.m;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= t) return;
   double s = 0;
   for (int k = 0; k < t; ++k) s += spread_abs(m[((size_t)(i / kSpreadTopRows) * t + k) * kSpreadTopRows + i % kSpreadTopRows]);
-  atomicMax(norm, (unsigned long long)__double_as_longlong(fabs(s)));
+  atomicMax(map.norm, (unsigned long long)__double_as_longlong(fabs(s)));
 }
 
 // A lane's row of the work array in 32-byte pieces: COLS columns from column c, as reals.
