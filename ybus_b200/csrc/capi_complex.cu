@@ -109,7 +109,9 @@ void launch_batch(const std::vector<yb_factor *> &fs, const std::vector<const cp
 // The batch's device workspace, kept between calls (one set per GPU of the first factor)
 struct BatchWork {
   DeviceArray<uint8_t> nets, rnets;
-  DeviceArray<BatchItem> items, columns;
+  DeviceArray<BatchItem> items;
+  DeviceArray<ResidualItem> pieces;
+  DeviceArray<unsigned long long> norms;
   DeviceArray<cplx<double>> scratch128, residual;
   DeviceArray<cplx<float>> scratch64;
   DeviceArray<double> ratio;
@@ -210,9 +212,9 @@ extern "C" int32_t yb_solve_batch_complex(int64_t networks, yb_factor *const *fa
     cudaStream_t s = stream ? (cudaStream_t)stream : gpu->stream;
     if (!gpu->zwork) gpu->zwork = std::make_shared<BatchWork>();
     BatchWork &w = *static_cast<BatchWork *>(gpu->zwork.get());
-    // the residual's per-network descriptors and the (network, column) list
+    // the residual's per-network descriptors and the list of its blocks
     std::vector<ResidualNet> rn(networks);
-    std::vector<BatchItem> cols;
+    std::vector<ResidualItem> pieces;
     int64_t total = 0, max_total = 0;
     for (int64_t i = 0; i < networks; ++i) total += cnt[i] * fs[i]->n;
     if (need_residual) {
@@ -221,29 +223,34 @@ extern "C" int32_t yb_solve_batch_complex(int64_t networks, yb_factor *const *fa
       int64_t all_cols = 0;
       for (int64_t i = 0; i < networks; ++i) all_cols += cnt[i];
       w.ratio.reserve((size_t)std::max<int64_t>(all_cols, 1));
+      w.norms.reserve((size_t)std::max<int64_t>(2 * all_cols, 1));
       for (int64_t i = 0; i < networks; ++i) {
         yb_factor *f = fs[i];
         rn[i] = ResidualNet{(int32_t)f->n, f->za_ptr.get(), f->za_idx.get(), f->za_val.get(), b[i], f->n, x[i], f->n,
-                            w.residual.get() + off, f->n, w.ratio.get() + ratio_off};
-        for (int64_t c = 0; c < cnt[i]; ++c) cols.push_back(BatchItem{(int32_t)i, (int32_t)c});
+                            w.residual.get() + off, f->n, w.norms.get() + 2 * ratio_off};
+        for (int64_t row = 0; row < f->n; row += kResidualRows)
+          for (int64_t c = 0; c < cnt[i]; c += kResidualColumns)
+            pieces.push_back({(int32_t)i, (int32_t)row, (int32_t)c, (int32_t)std::min<int64_t>(kResidualColumns, cnt[i] - c)});
         off += cnt[i] * f->n;
         ratio_off += cnt[i];
       }
       max_total = all_cols;
       w.rnets.reserve(sizeof(ResidualNet) * networks);
-      w.columns.reserve(std::max<size_t>(cols.size(), 1));
+      w.pieces.reserve(std::max<size_t>(pieces.size(), 1));
       cuda_check(cudaMemcpyAsync(w.rnets.get(), rn.data(), sizeof(ResidualNet) * networks, cudaMemcpyHostToDevice, s),
                  "upload residual descriptors");
-      if (!cols.empty())
-        cuda_check(cudaMemcpyAsync(w.columns.get(), cols.data(), sizeof(BatchItem) * cols.size(), cudaMemcpyHostToDevice, s),
-                   "upload columns");
+      if (!pieces.empty())
+        cuda_check(cudaMemcpyAsync(w.pieces.get(), pieces.data(), sizeof(ResidualItem) * pieces.size(), cudaMemcpyHostToDevice, s),
+                   "upload the residual's blocks");
     }
     auto residual = [&]() -> std::vector<double> {
       std::vector<double> ratios(max_total);
       if (max_total == 0) return ratios;
-      batch_residual_kernel<<<(unsigned)max_total, 256, 0, s>>>(reinterpret_cast<const ResidualNet *>(w.rnets.get()),
-                                                                w.columns.get());
+      cuda_check(cudaMemsetAsync(w.norms.get(), 0, sizeof(unsigned long long) * 2 * max_total, s), "clear the norms");
+      batch_residual_kernel<<<(unsigned)pieces.size(), 256, 0, s>>>(reinterpret_cast<const ResidualNet *>(w.rnets.get()), w.pieces.get());
       cuda_check(cudaGetLastError(), "batch_residual_kernel launch");
+      batch_ratio_kernel<<<(unsigned)((max_total + 255) / 256), 256, 0, s>>>(max_total, w.norms.get(), w.ratio.get());
+      cuda_check(cudaGetLastError(), "batch_ratio_kernel launch");
       cuda_check(cudaMemcpyAsync(ratios.data(), w.ratio.get(), sizeof(double) * max_total, cudaMemcpyDeviceToHost, s),
                  "download ratios");
       cuda_check(cudaStreamSynchronize(s), "residual");
