@@ -178,3 +178,41 @@ def test_a_complex_batch_matches_the_cpu(gpu, counts, prec, bar):
             if len(b):
                 sol = x[off:off + 2 * b.size].view(np.complex128).reshape(b.shape)
                 assert worst_relative_difference(sol, orc.solve_many_lu(lu, b)) < bar
+
+
+DOMAIN = 4
+
+
+@pytest.mark.parametrize("kind", [None, DOMAIN], ids=["spread", "domain"])
+@pytest.mark.parametrize("count", [1, 31, 33, 300])
+@pytest.mark.parametrize("name", ["grid", "lu"])
+def test_refined_solve(gpu, name, count, kind):
+    """Leading dimensions, and x in b's place (the automatic choice leaves that to the domain solve)."""
+    import torch
+    if name == "grid":
+        a = configs.bprime(grids.make_grid(1500, 520, 11))
+    else:
+        a = random_square(120, 3, 3)
+    f = host.cholesky(a) if name == "grid" else host.lu(a)
+    factor = upload(gpu, f)
+    factor.attach_matrix(a)
+    if kind is not None:
+        factor.set_tile_kind(FP32, kind)
+    n = f.n
+    rhs = right_hand_sides(n, count, 11)
+    cpu = orc.solve_many(f, rhs, threads=8)
+    p, i, v = a.to_csr().arrays()
+    for inplace in (False, True):
+        b = torch.full((count, n + 3), 3.0, dtype=torch.float64, device="cuda")
+        b[:, :n] = torch.from_numpy(rhs).cuda()
+        x = b if inplace else torch.full((count, n + 5), 7.0, dtype=torch.float64, device="cuda")
+        ratio = torch.empty(count, dtype=torch.float64, device="cuda")
+        torch.cuda.synchronize()
+        factor.solve_many_refined_device(b.data_ptr(), x.data_ptr(), count, 4, 1e-10, ratio.data_ptr(),
+                                         ldb=n + 3, ldx=x.shape[1])
+        gpu.synchronize()
+        xs = x.cpu().numpy()
+        assert np.all(xs[:, n:] == (3.0 if inplace else 7.0)), "rows past n are not written"
+        assert worst_relative_difference(xs[:, :n], cpu) < 1e-8
+        assert max(orc.relative_residual(p, i, v, xs[k, :n], rhs[k]) for k in range(0, count, 7)) <= 1.05e-10
+        assert ratio.cpu().numpy().max() <= 1e-10

@@ -2,7 +2,9 @@
 // block solves, mirroring ybus_cuda (ybus_cuda/src/lib.rs:168-219, ybus_cuda/src/factor.rs).
 #include <chrono>
 #include <cstring>
+#include <functional>
 #include <memory>
+#include <mutex>
 #include <vector>
 
 #include "../../include/ybgpu.h"
@@ -1386,7 +1388,7 @@ extern "C" int32_t yb_factor_set_refine_lane_min_count(yb_factor *f, int64_t min
   return guard([&] {
     require(f != nullptr, "null factor");
     require(min_count >= 0, "negative count");
-    f->tile32.refine_lane_min_count = min_count;
+    f->tile32.refine_lane_min_count = min_count, f->tile32.refine_shaped = true;
     return YB_OK;
   });
 }
@@ -1460,10 +1462,11 @@ extern "C" int32_t yb_factor_attach_matrix(yb_factor *f, const int64_t *a_ptr, c
 }
 
 namespace yb {
-// The refined solve's copy of A for a lane layout (LaneRefineArgs' res_*): rows in natural order,
+// The refined solve's copy of A for a layout (LaneRefineArgs' res_*): rows in natural order,
 // 32 to a slice, entry q of row 32 s + l at ptr[s] + 32 q + l, each column as the work row that
 // holds its unknown (out_pos).
-void lane_residual_matrix(yb_factor *f, DeviceLane *d, cudaStream_t stream) {
+void residual_matrix(yb_factor *f, ResidualMatrix *d, const std::vector<int32_t> &out_pos, cudaStream_t stream) {
+  const std::lock_guard<std::mutex> lock(f->spread_mutex);
   if (d->res_matrix == f->a_attached) return;
   const int64_t n = f->n, slices = (n + 31) / 32;
   std::vector<int32_t> ptr(slices + 1, 0), len(n), col;
@@ -1480,7 +1483,7 @@ void lane_residual_matrix(yb_factor *f, DeviceLane *d, cudaStream_t stream) {
       len[r] = (int32_t)(f->a_host_ptr[r + 1] - f->a_host_ptr[r]);
       for (int64_t k = f->a_host_ptr[r]; k < f->a_host_ptr[r + 1]; ++k) {
         const size_t at = o + 32 * (size_t)(k - f->a_host_ptr[r]) + (size_t)(r - 32 * s);
-        col[at] = d->host_out_pos[f->a_host_idx[k]];
+        col[at] = out_pos[f->a_host_idx[k]];
         val[at] = f->a_host_val[k];
       }
     }
@@ -1494,31 +1497,36 @@ void lane_residual_matrix(yb_factor *f, DeviceLane *d, cudaStream_t stream) {
   d->res_matrix = f->a_attached;
 }
 
-// The refined solve through the lane solve (lane_refine.cuh), per launch's run of groups: b
-// gathered once into the FP32 work array; per pass the FP32 lane solve (its correction into its
-// own array), the FP64 residual of the iterate it completes (which also writes that iterate into
-// the caller's x for the columns still refining), each column's decision, the restore of the best
-// iterate where a pass made it no better, and, while another pass may follow, the iterate carried
-// in FP64. Every kernel of a pass skips the groups that have stopped.
-void launch_lane_refined(yb_factor *f, DeviceLane *d, const double *b, int64_t ldb, double *x, int64_t ldx, int64_t count,
-                         int32_t max_steps, double tolerance, double *ratio_out, int32_t *steps_out, cudaStream_t stream) {
+// What the refined solve takes of the lane or the spread solve: positions, A for the residual, and the
+// sweeps of groups from `work` into `out`, those with a zero in `active` left out.
+struct RefineSweeps {
+  const int32_t *in_pos, *out_pos;
+  const ResidualMatrix *matrix;
+  std::function<void(float *work, float *out, int64_t groups, const uint8_t *active)> run;
+};
+
+// The refined solve (lane_refine.cuh), per launch's run of groups: b gathered once into the FP32 work
+// array; per pass the FP32 sweeps (their correction into its own array), the FP64 residual of the
+// iterate it completes (which also writes that iterate into the caller's x for the columns still
+// refining, and whose last block of a group decides for its columns), and, where there is something to
+// do, the restore of the best iterate where a pass made it no better and the iterate carried in FP64
+// while another pass may follow. Every kernel of a pass skips the groups that have stopped.
+void launch_refined(yb_factor *f, const RefineSweeps &sweeps, const double *b, int64_t ldb, double *x, int64_t ldx, int64_t count,
+                    int32_t max_steps, double tolerance, double *ratio_out, int32_t *steps_out, cudaStream_t stream) {
   using T = float;
   const int64_t n = f->n;
   const size_t group_vals = (size_t)n * 32;
   const int64_t groups_all = (count + 31) / 32;
   const int64_t per_launch = std::max<int64_t>(1, std::min<int64_t>(groups_all, (int64_t)(kLaneWorkBytes / (group_vals * sizeof(T)))));
   const int64_t cols_most = per_launch * 32;
-  lane_residual_matrix(f, d, stream);
-  f->lane_work.reserve((size_t)per_launch * group_vals * sizeof(T));
-  f->lane_partial.reserve((size_t)per_launch * std::max(d->partials, 1) * 32 * sizeof(T));
+  f->lane_work.reserve(((size_t)per_launch * group_vals + 2 * kSpreadPad * 32) * sizeof(T));
   f->refine_parts.reserve(2 * (size_t)per_launch * group_vals);
   if (max_steps >= 2) f->refine_scratch.reserve((size_t)per_launch * group_vals);
   // per column: rmax, bmax, cur, best (8 bytes each), best_steps (4); per group: col_active,
-  // write_mask, restore_mask (4 each), active (1)
-  const size_t state_bytes = (size_t)cols_most * 36 + (size_t)per_launch * 13 + 64;
+  // write_mask, restore_mask, done (4 each), active (1)
+  const size_t state_bytes = (size_t)cols_most * 36 + (size_t)per_launch * 17 + 64;
   f->refine_state.reserve(state_bytes);
-  T *work = reinterpret_cast<T *>(f->lane_work.get());
-  T *partial = reinterpret_cast<T *>(f->lane_partial.get());
+  T *work = reinterpret_cast<T *>(f->lane_work.get()) + kSpreadPad * 32;
   T *dA = f->refine_parts.get(), *dB = dA + (size_t)per_launch * group_vals;
   double *X = f->refine_scratch.get();
   uint8_t *st = f->refine_state.get();
@@ -1532,22 +1540,13 @@ void launch_lane_refined(yb_factor *f, DeviceLane *d, const double *b, int64_t l
   r.col_active = reinterpret_cast<uint32_t *>(r.best_steps + cols_most);
   r.write_mask = r.col_active + per_launch;
   r.restore_mask = r.write_mask + per_launch;
-  r.active = reinterpret_cast<uint8_t *>(r.restore_mask + per_launch);
-  r.in_pos = d->in_pos.get(), r.out_pos = d->out_pos.get();
-  r.res_ptr = d->res_ptr.get(), r.res_len = d->res_len.get(), r.res_col = d->res_col.get(), r.res_val = d->res_val.get();
+  r.done = reinterpret_cast<int32_t *>(r.restore_mask + per_launch);
+  r.active = reinterpret_cast<uint8_t *>(r.done + per_launch);
+  r.in_pos = sweeps.in_pos, r.out_pos = sweeps.out_pos;
+  const ResidualMatrix *m = sweeps.matrix;
+  r.res_ptr = m->res_ptr.get(), r.res_len = m->res_len.get(), r.res_col = m->res_col.get(), r.res_val = m->res_val.get();
   r.work = work;
   r.ldb = ldb, r.ldx = ldx;
-  const size_t smem = lane_smem<T>(d);
-  if (smem > (size_t)f->gpu->smem_optin) throw host::Error(host::kInvalidArgument, "the lane solve's block does not fit in shared memory");
-  const auto kernel = lane_kernel<T, 1>(d, smem);
-  LaneArgs a{};
-  a.n = (int32_t)n;
-  a.slots = d->slots, a.page_bytes = d->page_bytes, a.partials = d->partials;
-  a.blob = d->blob.get();
-  a.warp_page = d->warp_page.get();
-  a.error = f->error.get();
-  a.group_active = r.active;
-  a.withhold = -1;
   auto check = [](const char *what) { cuda_check(cudaGetLastError(), what); };
   for (int64_t g0 = 0; g0 < groups_all; g0 += per_launch) {
     const int64_t groups = std::min(per_launch, groups_all - g0);
@@ -1556,46 +1555,59 @@ void launch_lane_refined(yb_factor *f, DeviceLane *d, const double *b, int64_t l
     r.b = b + g0 * 32 * ldb, r.x = x + g0 * 32 * ldx;
     r.ratio_out = ratio_out ? ratio_out + g0 * 32 : nullptr;
     r.steps_out = steps_out ? steps_out + g0 * 32 : nullptr;
-    const unsigned rows_grid = (unsigned)(groups * res_parts(n));  // blocks of kResRows rows of one group
-    const unsigned group_grid = (unsigned)((groups * 32 + 127) / 128);  // a warp per group
+    r.chunks = kResChunks;
+    while (r.chunks > 1 && groups * res_parts(n, r.chunks) < 4 * (int64_t)f->gpu->sm_count) r.chunks /= 2;
+    const unsigned rows_grid = (unsigned)(groups * res_parts(n, r.chunks));
     const int64_t init_n = std::max(r.count, groups);
     lane_refine_init_kernel<<<(unsigned)((init_n + 255) / 256), 256, 0, stream>>>(r);
     check("lane_refine_init_kernel launch");
     lane_in_kernel<T><<<(unsigned)lane_io_blocks(groups, n), kLaneIoWarps * 32, 0, stream>>>(r.b, ldb, r.count, (int32_t)n,
-                                                                                           groups, d->in_pos.get(), work,
+                                                                                           groups, sweeps.in_pos, work,
                                                                                            nullptr);
     check("lane_in_kernel launch");
-    const int64_t carry_parts = std::max<int64_t>(1, (int64_t)((group_vals + 8191) / 8192));  // 8,192 values a block
-    const unsigned carry_grid = (unsigned)(groups * carry_parts);
     for (int32_t pass = 0; pass <= max_steps; ++pass) {
       T *dk = pass == 1 ? dB : dA;  // this pass's correction
-      a.xout = dk;
-      kernel<<<(unsigned)groups, d->warps * 32, smem, stream>>>(a, work, partial);
-      check("lane_solve_kernel launch");
+      sweeps.run(work, dk, groups, r.active);
       if (pass == 0)
-        lane_residual_kernel<0><<<rows_grid, kResWarps * 32, 0, stream>>>(r, dk, nullptr, nullptr, true);
+        lane_residual_kernel<0><<<rows_grid, kResWarps * 32, 0, stream>>>(r, dk, nullptr, nullptr, pass, max_steps, tolerance);
       else if (pass == 1)
-        lane_residual_kernel<1><<<rows_grid, kResWarps * 32, 0, stream>>>(r, dk, dA, nullptr, false);
+        lane_residual_kernel<1><<<rows_grid, kResWarps * 32, 0, stream>>>(r, dk, dA, nullptr, pass, max_steps, tolerance);
       else
-        lane_residual_kernel<2><<<rows_grid, kResWarps * 32, 0, stream>>>(r, dk, nullptr, X, false);
+        lane_residual_kernel<2><<<rows_grid, kResWarps * 32, 0, stream>>>(r, dk, nullptr, X, pass, max_steps, tolerance);
       check("lane_residual_kernel launch");
-      lane_refine_decide_kernel<<<group_grid, 128, 0, stream>>>(r, pass, max_steps, tolerance);
-      check("lane_refine_decide_kernel launch");
-      // the best iterate back where this pass made no better (x_{pass-1}), or x0 where pass 0 ends
+      // the best iterate back where this pass made no better (x_{pass-1}), or x0 where pass 0 ends;
+      // x_pass in FP64 for the next pass's residual
       if (pass <= 1)
-        lane_restore_kernel<T><<<rows_grid, kResWarps * 32, 0, stream>>>(r, dA);
+        lane_settle_kernel<T><<<rows_grid, kResWarps * 32, 0, stream>>>(r, dA, dB, X, pass == 1 && pass < max_steps);
       else
-        lane_restore_kernel<double><<<rows_grid, kResWarps * 32, 0, stream>>>(r, X);
-      check("lane_restore_kernel launch");
-      if (pass >= 1 && pass < max_steps) {  // x_pass in FP64 for the next pass's residual
-        if (pass == 1)
-          lane_carry_kernel<T><<<carry_grid, 256, 0, stream>>>(r, dA, dB, X, carry_parts);
-        else
-          lane_carry_kernel<double><<<carry_grid, 256, 0, stream>>>(r, X, dA, X, carry_parts);
-        check("lane_carry_kernel launch");
-      }
+        lane_settle_kernel<double><<<rows_grid, kResWarps * 32, 0, stream>>>(r, X, dA, X, pass < max_steps);
+      check("lane_settle_kernel launch");
     }
   }
+}
+
+// The lane solve's sweeps.
+void launch_lane_refined(yb_factor *f, DeviceLane *d, const double *b, int64_t ldb, double *x, int64_t ldx, int64_t count,
+                         int32_t max_steps, double tolerance, double *ratio_out, int32_t *steps_out, cudaStream_t stream) {
+  using T = float;
+  residual_matrix(f, d, d->host_out_pos, stream);
+  const size_t smem = lane_smem<T>(d);
+  if (smem > (size_t)f->gpu->smem_optin) throw host::Error(host::kInvalidArgument, "the lane solve's block does not fit in shared memory");
+  const auto kernel = lane_kernel<T, 1>(d, smem);
+  LaneArgs a{};
+  a.n = (int32_t)f->n;
+  a.slots = d->slots, a.page_bytes = d->page_bytes, a.partials = d->partials;
+  a.blob = d->blob.get();
+  a.warp_page = d->warp_page.get();
+  a.error = f->error.get();
+  a.withhold = -1;
+  const RefineSweeps sweeps{d->in_pos.get(), d->out_pos.get(), d, [&](T *work, T *out, int64_t groups, const uint8_t *active) {
+    f->lane_partial.reserve((size_t)groups * std::max(d->partials, 1) * 32 * sizeof(T));
+    a.xout = out, a.group_active = active;
+    kernel<<<(unsigned)groups, d->warps * 32, smem, stream>>>(a, work, reinterpret_cast<T *>(f->lane_partial.get()));
+    cuda_check(cudaGetLastError(), "lane_solve_kernel launch");
+  }};
+  launch_refined(f, sweeps, b, ldb, x, ldx, count, max_steps, tolerance, ratio_out, steps_out, stream);
 }
 }  // namespace yb
 
@@ -1616,6 +1628,24 @@ extern "C" int32_t yb_solve_many_refined_device(yb_factor *f, const double *d_rh
     require(!f->single, "a single-row factor needs no refinement: use yb_solve_many_device");
     cudaStream_t s = stream ? (cudaStream_t)stream : f->gpu->stream;
     const TileConfig &t32 = f->tile32;
+    // The spread solve's sweeps, unless a shape or a threshold was set, or x overlaps b (whose columns are
+    // read again after x's are written; the domain solve keeps its own residual and needs b once). On the
+    // 10,000-bus B' with random right-hand sides 185 against 376 us with one, 309 against 429 us with 256,
+    // 508 against 911 us with 600 (the domain solve), 1,229 against 1,954 us with 2,048 and 6.5 against
+    // 6.9 ms with 13,499 (the lane solve); on the 2,000-bus B' 140 against 628 us with one; the first call
+    // of a factor 8 against 347 ms.
+    const auto bytes = [&](const double *p, int64_t ld) { return std::make_pair((uintptr_t)p, (uintptr_t)(p + (count - 1) * ld + f->n)); };
+    const auto rb = bytes(d_rhs, ldb), rx = bytes(d_out, ldx);
+    if (t32.kind == kTileAuto && !t32.shaped && !t32.refine_shaped && (rb.second <= rx.first || rx.second <= rb.first)) {
+      if (DeviceSpread *d = spread_for(f, (int)sizeof(float), (count + 31) / 32, s)) {
+        residual_matrix(f, d, d->host_out_pos, s);
+        const RefineSweeps sweeps{d->in_pos, d->out_pos, d, [&](float *work, float *out, int64_t groups, const uint8_t *active) {
+          spread_sweeps<float>(f, d, work, out, groups, active, s);
+        }};
+        launch_refined(f, sweeps, d_rhs, ldb, d_out, ldx, count, max_steps, tolerance, d_ratio, d_steps, s);
+        return YB_OK;
+      }
+    }
     if (t32.kind == kTileLane ||
         (t32.kind == kTileAuto && count >= std::max(lane_threshold<float>(f, t32), t32.refine_lane_min_count))) {
       DeviceLane *d = lane_pick<float>(f, lane_shape(f, t32, count), 1, s);  // its kernels take groups of 32 columns

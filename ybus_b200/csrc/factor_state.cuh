@@ -120,29 +120,33 @@ struct TileConfig {
   // lane_warps not set by a caller or the autotuner: a solve of no more groups of 32 than SMs then
   // takes blocks of kLaneMaxWarps (one an SM, each warp's chain of rows shorter)
   bool lane_warps_auto = true;
-  // the refined solve takes the lane solve from this many right-hand sides on (its passes cost more
+  // without the spread solve the refined one takes the lane solve from this many right-hand sides on (its passes cost more
   // launches than the plain solve's, so its crossover with the fused domain refinement lies higher:
   // 2,048 on the 10,000-bus B′ with blocks of 16 warps up to one wave)
   int64_t refine_lane_min_count = 2048;
+  bool refine_shaped = false;  // a caller set it: the refined solve chooses among the lane and domain solves
+};
+
+// The refined solve's copy of the attached A for a layout (LaneRefineArgs' res_*): natural rows in
+// slices of 32, columns as work rows; built at its first use, for the matrix attached then.
+struct ResidualMatrix {
+  int64_t res_matrix = -1;  // the attach count it was built for
+  DeviceArray<int32_t> res_ptr, res_len, res_col;
+  DeviceArray<double> res_val;
 };
 
 // A lane layout on the device (LaneLayout in plan.hpp).
-struct DeviceLane {
+struct DeviceLane : ResidualMatrix {
   int32_t warps = 0, slots = 0, page_bytes = 0, domains = 0, top = 0, partials = 0, fwd_live = 0, bwd_live = 0;
   int32_t rpl = 1;  // right-hand sides per lane the layout's offsets count
   int64_t entries = 0, pages = 0;
   DeviceArray<uint8_t> blob;
   DeviceArray<int32_t> warp_page, in_pos, out_pos;
   std::vector<int32_t> host_out_pos;
-  // the refined solve's copy of the attached A (LaneRefineArgs' res_*): natural rows in slices of
-  // 32, columns as work rows; built at its first use, for the matrix attached then
-  int64_t res_matrix = -1;  // the attach count it was built for
-  DeviceArray<int32_t> res_ptr, res_len, res_col;
-  DeviceArray<double> res_val;
 };
 
 // A spread layout on the device (SpreadLayout in plan.hpp), with the top's dense map.
-struct DeviceSpread {
+struct DeviceSpread : ResidualMatrix {
   int32_t n = 0, tasks = 0, domains = 0, top = 0, slots = 0, partials = 0;
   int64_t blob_bytes = 0;
   int64_t serial = 0;  // no two layouts of a process share one

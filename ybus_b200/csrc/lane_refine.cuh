@@ -1,9 +1,9 @@
-// Mixed-precision refinement around the lane solve, for blocks large enough to take it: the
-// substitutions in FP32 through the lane solve (masked to the groups of 32 columns still refining),
+// Mixed-precision refinement around the spread solve (the automatic choice) or the lane solve: the
+// substitutions in FP32 through either's sweeps (masked to the groups of 32 columns still refining),
 // the residual R = b - A x and the iterate x = x' + d in FP64 against the FP64 matrix, with the
 // stop rule of ybus_sparse's refine_normwise (accuracy.rs:83-122) applied to every column.
 //
-// Data. b and x are the caller's (column-major). Each pass's correction d is the lane solve's
+// Data. b and x are the caller's (column-major). Each pass's correction d is the sweeps'
 // output, FP32 in the work array's layout [group][work row][lane]; the iterate is never stored in
 // full unless a third pass needs it: pass 0's iterate is d0 itself, pass 1's is d0 + d1 (both
 // FP32, added in FP64 where they are read), and only from pass 2 on is x_k kept in FP64, in the
@@ -27,7 +27,7 @@
 
 namespace yb {
 
-// The state of one launch of the refined lane solve (a contiguous run of groups).
+// The state of one launch of the refined solve (a contiguous run of groups).
 struct LaneRefineArgs {
   int32_t n;
   int64_t groups, count;                     // this launch's groups of 32 columns, and its columns
@@ -50,6 +50,8 @@ struct LaneRefineArgs {
   // per group
   uint8_t *active;                           // the group is still refining
   uint32_t *col_active, *write_mask, *restore_mask;
+  int32_t *done;                             // blocks of the group's residual that have finished this pass
+  int32_t chunks;                            // chunks of 8 rows a warp of the residual takes (kResChunks, fewer of few groups)
 };
 
 // The largest of |v| as an unsigned bit pattern: positive doubles order as their patterns, and a
@@ -58,13 +60,14 @@ __device__ __forceinline__ unsigned long long abs_bits(double v) {
   return (unsigned long long)__double_as_longlong(fabs(v));
 }
 
-// The residual and restore kernels' lanes and blocks: a warp takes chunks of 8 consecutive rows of
+// The residual and settle kernels' lanes and blocks: a warp takes chunks of 8 consecutive rows of
 // one group, four lanes per row, each lane 8 of the group's 32 columns (lane = quarter * 8 + row, so
 // the 8 lanes of a quarter hold the chunk's 8 rows of the same 8 columns); a block of kResWarps
-// warps, each taking kResChunks chunks in turn, covers kResRows rows of one group and returns at
-// once, as a whole, when that group has stopped.
-constexpr int kResWarps = 8, kResChunks = 8, kResRows = kResWarps * kResChunks * 8;
-__host__ __device__ inline int64_t res_parts(int64_t n) { return (n + kResRows - 1) / kResRows; }
+// warps, each taking `chunks` chunks in turn (kResChunks; fewer where a few groups would leave SMs
+// without a block), covers 64 chunks' rows of one group and returns at once, as a whole, when that group
+// has stopped.
+constexpr int kResWarps = 8, kResChunks = 8;
+__host__ __device__ inline int64_t res_parts(int64_t n, int chunks) { return (n + kResWarps * 8 * chunks - 1) / (kResWarps * 8 * chunks); }
 
 // Each lane holds 8 values, one per column of its quarter, for its row. Reduces every column to its
 // maximum over the quarter's 8 rows by a transposing butterfly: at each step a lane keeps half of
@@ -101,6 +104,21 @@ __device__ __forceinline__ void load8(const double *p, double (&v)[8]) {
     asm volatile("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v[c]), "=d"(v[c + 1]), "=d"(v[c + 2]), "=d"(v[c + 3])
                  : "l"(p + c));
 }
+// ... of what the same kernel writes elsewhere, as FP64
+__device__ __forceinline__ void load8_plain(const float *p, double (&v)[8]) {
+#pragma unroll
+  for (int c = 0; c < 8; c += 4) {
+    const float4 f = *reinterpret_cast<const float4 *>(p + c);
+    v[c] = f.x, v[c + 1] = f.y, v[c + 2] = f.z, v[c + 3] = f.w;
+  }
+}
+__device__ __forceinline__ void load8_plain(const double *p, double (&v)[8]) {
+#pragma unroll
+  for (int c = 0; c < 8; c += 2) {
+    const double2 f = *reinterpret_cast<const double2 *>(p + c);
+    v[c] = f.x, v[c + 1] = f.y;
+  }
+}
 
 // The iterate's 8 values of one lane's quarter at one work row, as loaded: the correction d and,
 // when there is one, the base x_{k-1} (BASE 1: FP32 parts, BASE 2: FP64); value(c) = base + d in
@@ -131,6 +149,50 @@ template <> struct Iterate8<2> {
   __device__ __forceinline__ double value(int c) const { return b[c] + (double)d[c]; }
 };
 
+// One warp per group, one lane per column, in the group's last block of the residual: each column's relative residual after `pass`
+// corrections and the state of refine_normwise (accuracy.rs:93-118): pass 0 takes x0 as the best; a
+// later pass keeps x_k if its ratio is below the best, else x_{k-1} is put back in the caller's x
+// (restore_mask); a column stops within the tolerance, on a NaN ratio, when the ratio did not
+// halve, or after max_steps, and then gets its best ratio and correction count. write_mask becomes
+// the columns whose best is x_pass, the ones the next pass may overwrite; a column that stops at
+// pass 0 has its x0 written by the restore.
+__device__ __forceinline__ void lane_refine_decide(const LaneRefineArgs &a, int64_t g, int lane, int32_t pass, int32_t max_steps,
+                                                   double tolerance) {
+  const uint32_t act = a.col_active[g], wrote = a.write_mask[g];
+  bool stop = false, write = false, restore = false;
+  if ((act >> lane) & 1u) {
+    const int64_t col = g * 32 + lane;
+    const double rn = __longlong_as_double((long long)__ldcg(a.rmax + col)), bn = __longlong_as_double((long long)__ldcg(a.bmax + col));
+    const double ratio = bn > 0.0 ? rn / bn : (rn > 0.0 ? __longlong_as_double(0x7ff0000000000000LL) : 0.0);
+    a.rmax[col] = 0ull;
+    if (pass == 0) {
+      a.best[col] = ratio, a.best_steps[col] = 0, a.cur[col] = ratio;
+      stop = ratio <= tolerance || max_steps < 1;
+      restore = stop;
+    } else {
+      const double previous = a.cur[col];
+      a.cur[col] = ratio;
+      const bool improved = ratio < a.best[col];
+      if (improved) a.best[col] = ratio, a.best_steps[col] = pass;
+      restore = !improved && ((wrote >> lane) & 1u);
+      stop = ratio != ratio || ratio > 0.5 * previous || ratio <= tolerance || pass >= max_steps;
+    }
+    if (stop) {
+      if (a.ratio_out) a.ratio_out[col] = a.best[col];
+      if (a.steps_out) a.steps_out[col] = a.best_steps[col];
+    } else {
+      write = a.best_steps[col] == pass;
+    }
+  }
+  const uint32_t stopped = __ballot_sync(0xffffffffu, stop), writes = __ballot_sync(0xffffffffu, write),
+                 restores = __ballot_sync(0xffffffffu, restore);
+  if (lane == 0) {
+    const uint32_t left = act & ~stopped;
+    a.col_active[g] = left, a.write_mask[g] = writes, a.restore_mask[g] = restores;
+    if (!left) a.active[g] = 0;
+  }
+}
+
 // The residual R = b - A x of the groups still refining, in FP64, with x = base + d formed at every
 // row read (BASE 0: x = d, pass 0). Lanes as above: b's and x's columns are read and written 8 rows
 // (64 bytes) at a time, and each row of x a lane reads is one 32-byte load, the four lanes of a row
@@ -145,12 +207,19 @@ template <> struct Iterate8<2> {
 template <int BASE>
 __global__ void __launch_bounds__(kResWarps * 32, BASE == 0 ? 4 : 3) lane_residual_kernel(LaneRefineArgs a, const float *__restrict__ d,
                                                                         const float *__restrict__ base32,
-                                                                        const double *__restrict__ base64, bool first) {
+                                                                        const double *__restrict__ base64, int32_t pass,
+                                                                        int32_t max_steps, double tolerance) {
+  constexpr bool first = BASE == 0;
   constexpr int AT = Iterate8<BASE>::AT_ONCE;
   __shared__ unsigned long long red[2][kResWarps][32];
+  __shared__ bool last;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t parts = res_parts(a.n), g = blockIdx.x / parts, part = blockIdx.x - g * parts;
-  if (g >= a.groups || !a.active[g]) return;  // the whole block
+  const int64_t parts = res_parts(a.n, a.chunks), g = blockIdx.x / parts, part = blockIdx.x - g * parts;
+  if (g >= a.groups) return;
+  if (!a.active[g]) {  // the whole block
+    if (part == 0 && threadIdx.x == 0) a.restore_mask[g] = 0;
+    return;
+  }
   const int c0 = (lane >> 3) * 8;                             // this lane's first column in the group
   const int64_t col0 = g * 32 + c0;                           // ... in the launch
   const int64_t left = a.count - col0;
@@ -159,8 +228,8 @@ __global__ void __launch_bounds__(kResWarps * 32, BASE == 0 ? 4 : 3) lane_residu
   uint32_t write = 0;
   if constexpr (BASE != 0) write = (a.write_mask[g] >> c0) & 0xffu;
   unsigned long long rmax = 0ull, bmax = 0ull;  // column `lane`'s maxima over this warp's rows
-  for (int k = 0; k < kResChunks; ++k) {
-    const int64_t i0 = ((part * kResWarps + warp) * kResChunks + k) * 8;
+  for (int k = 0; k < a.chunks; ++k) {
+    const int64_t i0 = ((part * kResWarps + warp) * a.chunks + k) * 8;
     if (i0 >= a.n) break;  // the whole warp
     const int i = (int)i0 + (lane & 7);
     const bool row = i < a.n;
@@ -234,95 +303,54 @@ __global__ void __launch_bounds__(kResWarps * 32, BASE == 0 ? 4 : 3) lane_residu
     if (mr) atomicMax(a.rmax + g * 32 + lane, mr);
     if (first && mb) atomicMax(a.bmax + g * 32 + lane, mb);
   }
+  if (warp != 0) return;
+  // the group's last block decides for its columns
+  __threadfence();
+  __syncwarp();
+  if (lane == 0) last = atomicAdd(a.done + g, 1) == (int)parts - 1;
+  __syncwarp();
+  if (!last) return;
+  __threadfence();
+  if (lane == 0) a.done[g] = 0;
+  lane_refine_decide(a, g, lane, pass, max_steps, tolerance);
 }
 
-// One warp per group, one lane per column: each column's relative residual after `pass`
-// corrections and the state of refine_normwise (accuracy.rs:93-118): pass 0 takes x0 as the best; a
-// later pass keeps x_k if its ratio is below the best, else x_{k-1} is put back in the caller's x
-// (restore_mask); a column stops within the tolerance, on a NaN ratio, when the ratio did not
-// halve, or after max_steps, and then gets its best ratio and correction count. write_mask becomes
-// the columns whose best is x_pass, the ones the next pass may overwrite; a column that stops at
-// pass 0 has its x0 written by the restore.
-__global__ void lane_refine_decide_kernel(LaneRefineArgs a, int32_t pass, int32_t max_steps, double tolerance) {
-  const int lane = threadIdx.x & 31;
-  const int64_t g = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (g >= a.groups) return;  // the whole warp
-  if (!a.active[g]) {
-    if (lane == 0) a.restore_mask[g] = 0;
-    return;
-  }
-  const uint32_t act = a.col_active[g], wrote = a.write_mask[g];
-  bool stop = false, write = false, restore = false;
-  if ((act >> lane) & 1u) {
-    const int64_t col = g * 32 + lane;
-    const double rn = __longlong_as_double((long long)a.rmax[col]), bn = __longlong_as_double((long long)a.bmax[col]);
-    const double ratio = bn > 0.0 ? rn / bn : (rn > 0.0 ? __longlong_as_double(0x7ff0000000000000LL) : 0.0);
-    a.rmax[col] = 0ull;
-    if (pass == 0) {
-      a.best[col] = ratio, a.best_steps[col] = 0, a.cur[col] = ratio;
-      stop = ratio <= tolerance || max_steps < 1;
-      restore = stop;
-    } else {
-      const double previous = a.cur[col];
-      a.cur[col] = ratio;
-      const bool improved = ratio < a.best[col];
-      if (improved) a.best[col] = ratio, a.best_steps[col] = pass;
-      restore = !improved && ((wrote >> lane) & 1u);
-      stop = ratio != ratio || ratio > 0.5 * previous || ratio <= tolerance || pass >= max_steps;
-    }
-    if (stop) {
-      if (a.ratio_out) a.ratio_out[col] = a.best[col];
-      if (a.steps_out) a.steps_out[col] = a.best_steps[col];
-    } else {
-      write = a.best_steps[col] == pass;
-    }
-  }
-  const uint32_t stopped = __ballot_sync(0xffffffffu, stop), writes = __ballot_sync(0xffffffffu, write),
-                 restores = __ballot_sync(0xffffffffu, restore);
-  if (lane == 0) {
-    const uint32_t left = act & ~stopped;
-    a.col_active[g] = left, a.write_mask[g] = writes, a.restore_mask[g] = restores;
-    if (!left) a.active[g] = 0;
-  }
-}
-
-// The caller's x of the columns in restore_mask set to the iterate `base` holds (FP32 parts or
-// FP64, in the work array's layout): x_{pass-1} for the columns a pass made no better, x0 for the
-// columns that stopped at pass 0. Blocks and lanes as in the residual; a block whose group has
-// nothing to restore returns at once.
+// What a pass leaves to do, row by row: the caller's x of the columns in restore_mask set to the
+// iterate `base` holds (FP32 parts or FP64, in the work array's layout): x_{pass-1} for the columns a
+// pass made no better, x0 for the columns that stopped at pass 0; and, with `carry`, for the groups still
+// refining X = base + d, the iterate kept in FP64 for a further pass (base FP32 parts on pass 1, X itself
+// after, each row's read before it is written). Four lanes a row, each 8 of the group's columns; a block
+// whose group has nothing to do returns at once.
 template <class B>
-__global__ void __launch_bounds__(kResWarps * 32) lane_restore_kernel(LaneRefineArgs a, const B *__restrict__ base) {
+__global__ void __launch_bounds__(kResWarps * 32) lane_settle_kernel(LaneRefineArgs a, const B *base, const float *__restrict__ d,
+                                                                    double *X, bool carry) {  // base may be X itself
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t parts = res_parts(a.n), g = blockIdx.x / parts, part = blockIdx.x - g * parts;
+  const int64_t parts = res_parts(a.n, a.chunks), g = blockIdx.x / parts, part = blockIdx.x - g * parts;
   if (g >= a.groups) return;
   const uint32_t all = a.restore_mask[g];
-  if (!all) return;  // the whole block
+  carry = carry && a.active[g];
+  if (!all && !carry) return;  // the whole block
   const int c0 = (lane >> 3) * 8;
   const uint32_t mask = (all >> c0) & 0xffu;
-  if (!mask) return;
-  for (int k = 0; k < kResChunks; ++k) {
-    const int64_t i0 = ((part * kResWarps + warp) * kResChunks + k) * 8;
+  for (int k = 0; k < a.chunks; ++k) {
+    const int64_t i0 = ((part * kResWarps + warp) * a.chunks + k) * 8;
     const int i = (int)i0 + (lane & 7);
     if (i >= a.n) break;
-    const B *src = base + ((size_t)g * a.n + __ldg(a.out_pos + i)) * 32 + c0;
+    const size_t at = ((size_t)g * a.n + __ldg(a.out_pos + i)) * 32 + c0;
+    double was[8];
+    load8_plain(base + at, was);
     double *xc = a.x + (g * 32 + c0) * a.ldx + i;
 #pragma unroll
     for (int c = 0; c < 8; ++c)
-      if ((mask >> c) & 1u) xc[c * a.ldx] = (double)src[c];
+      if ((mask >> c) & 1u) xc[c * a.ldx] = was[c];
+    if (carry) {
+      float dk[8];
+      load8(d + at, dk);
+#pragma unroll
+      for (int c = 0; c < 8; c += 2)
+        *reinterpret_cast<double2 *>(X + at + c) = make_double2(was[c] + (double)dk[c], was[c + 1] + (double)dk[c + 1]);
+    }
   }
-}
-
-// X = base + d over the work rows of the groups still refining: the iterate kept in FP64 for a
-// further pass (base FP32 parts on pass 1, X itself after). A block takes one of `parts` slices of
-// one group's values and returns at once when the group has stopped.
-template <class B>
-__global__ void __launch_bounds__(256) lane_carry_kernel(LaneRefineArgs a, const B *base, const float *__restrict__ d,
-                                                        double *X, int64_t parts) {  // base may be X itself
-  const int64_t g = blockIdx.x / parts, part = blockIdx.x - g * parts;
-  if (g >= a.groups || !a.active[g]) return;
-  const int64_t gv = (int64_t)a.n * 32, per = (gv + parts - 1) / parts;
-  const int64_t lo = g * gv + part * per, hi = g * gv + (gv < (part + 1) * per ? gv : (part + 1) * per);
-  for (int64_t k = lo + threadIdx.x; k < hi; k += blockDim.x) X[k] = (double)base[k] + (double)d[k];
 }
 
 // Every group refining with every column below `count`, no maxima yet.
@@ -333,7 +361,7 @@ __global__ void lane_refine_init_kernel(LaneRefineArgs a) {
     const int64_t left = a.count - k * 32, cols = left < 32 ? left : 32;
     a.active[k] = 1;
     a.col_active[k] = cols >= 32 ? 0xffffffffu : ((1u << cols) - 1u);
-    a.write_mask[k] = 0, a.restore_mask[k] = 0;
+    a.write_mask[k] = 0, a.restore_mask[k] = 0, a.done[k] = 0;
   }
 }
 
