@@ -7,7 +7,8 @@ import pytest
 
 import oracle.oracle as orc
 from fixtures import random_spd, random_square, right_hand_sides, star_spd, worst_relative_difference
-from ybus_b200 import FP32, FP64, CudaError, GpuFactor, configs, grids, host, solve_batch_complex
+from ybus_b200 import FP32, FP64, CudaError, GpuFactor, Pair, PairUpdate, configs, grids, host, solve_batch_complex
+from ybus_b200.dc import DcNetwork, FlowLoss
 
 pytestmark = pytest.mark.gpu
 
@@ -216,3 +217,53 @@ def test_refined_solve(gpu, name, count, kind):
         assert worst_relative_difference(xs[:, :n], cpu) < 1e-8
         assert max(orc.relative_residual(p, i, v, xs[k, :n], rhs[k]) for k in range(0, count, 7)) <= 1.05e-10
         assert ratio.cpu().numpy().max() <= 1e-10
+
+
+@pytest.mark.parametrize("count", [1, 31, 33, 300])
+@pytest.mark.parametrize("name", ["two", "path", "star", "grid"])
+def test_pairs_and_their_updates(gpu, name, count):
+    """Pairs with one end, both or none, against the CPU, and the updates bit for bit from them."""
+    f = FACTORS[name]()
+    factor = upload(gpu, f)
+    factor.set_block_width(300)
+    rng = np.random.default_rng(count)
+    plus, minus = rng.integers(-1, f.n, count), rng.integers(-1, f.n, count)
+    minus[minus == plus] = -1
+    pairs = [Pair(None if p < 0 else int(p), None if m < 0 else int(m)) for p, m in zip(plus, minus)]
+    rhs = np.zeros((count, f.n))
+    for k in range(count):
+        if plus[k] >= 0:
+            rhs[k, plus[k]] = 1.0
+        if minus[k] >= 0:
+            rhs[k, minus[k]] = -1.0
+    ys = factor.pair_solves(pairs).solutions()
+    cpu = orc.solve_many(f, rhs, threads=8)
+    some = np.abs(cpu).max(axis=1) > 0
+    assert worst_relative_difference(ys[some], cpu[some]) < 1e-12 and not ys[~some].any()
+    base, alpha, weight = rng.standard_normal(f.n), rng.standard_normal(count), 2.0 + rng.random(count)
+    out = factor.pair_updates(base, [PairUpdate(q, a, w) for q, a, w in zip(pairs, alpha, weight)]).solutions()
+    for k in range(0, count, 7):
+        exact, _ = orc.pair_update(base, ys[k], pairs[k].plus, pairs[k].minus, alpha[k], weight[k])
+        assert np.array_equal(out[k], exact)
+
+
+@pytest.mark.parametrize("slack", [0, 7, 299])
+@pytest.mark.parametrize("count", [1, 7, 33])
+def test_adjoint_of_any_slack(gpu, slack, count):
+    g = grids.make_grid(300, 100, 3)
+    rng = np.random.default_rng(count)
+    p, limits = rng.normal(0.0, 0.1, (count, g.n_bus)), rng.uniform(0.5, 2.0, g.n_branch)
+    net = DcNetwork.from_grid(gpu, g, slack)
+    loss_fn = FlowLoss(net, count)
+    loss = loss_fn.forward(p, limits)
+    gp, gb = loss_fn.backward()
+    r, c, v = grids.bbus_triplets(g)
+    keep = np.delete(np.arange(g.n_bus), slack)
+    chol = host.cholesky(host.Matrix.from_triplets(g.n_bus, g.n_bus, r, c, v).select(keep, keep))
+    position = -np.ones(g.n_bus, np.int64)
+    position[keep] = np.arange(keep.size)
+    loss_c, gp_c, gb_c = orc.flow_loss_and_gradient(chol, g.n_bus, g.frm, g.to, 1.0 / g.x, position, p, limits)
+    assert abs(loss - loss_c) <= 1e-12 * abs(loss_c)
+    assert np.abs(gp - gp_c).max() <= 1e-10 * np.abs(gp_c).max()
+    assert np.abs(gb - gb_c).max() <= 1e-10 * np.abs(gb_c).max()
+    assert (gp[:, slack] == 0.0).all()

@@ -292,7 +292,11 @@ struct yb_factor {
 namespace yb {
 void solve_pairs_device(yb_factor *f, int64_t count, const int32_t *plus, const int32_t *minus, const double *base,
                         const double *alpha, const double *inverse_weight, int32_t *singular, double *out, int64_t ldo,
-                        cudaStream_t stream);
+                        cudaStream_t stream, bool captured = false);
+// Plain FP64 solves by the spread solve where it is the automatic choice and the factor admits one; false,
+// with nothing done, elsewhere. x may be b (with its leading dimension).
+bool admits_spread_fp64(yb_factor *f, int64_t count, cudaStream_t stream);
+bool auto_spread_fp64(yb_factor *f, const double *b, int64_t ldb, double *x, int64_t ldx, int64_t count, cudaStream_t stream);
 cudaEvent_t *lane_timing_slot(yb_factor *f);  // the events of the next timed lane or spread solve, or null
 void solve_single_row_device(yb_factor *f, const double *b, int64_t ldb, double *x, int64_t ldx, int64_t count,
                              cudaStream_t stream);
