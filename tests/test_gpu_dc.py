@@ -119,3 +119,49 @@ def test_the_captured_graph_replays_new_inputs(gpu):
     assert np.allclose(scaled[1], 2.0 * first[1], rtol=1e-12)
     other = net.outage_loadings_batch(outaged[:10], sp[:11], inj[: sp[10]], weights)  # new sizes
     assert np.array_equal(other[0], first[0][: sp[10]])
+
+
+@pytest.mark.parametrize("count", [1, 97, 700, 3300])
+def test_columns_in_any_number_of_pieces(gpu, count):
+    """PTDF and LODF columns that fit one piece of the download, several, and several blocks of solves, into
+    pageable and pinned arrays, against the product of the CPU's angles; two threads at once."""
+    import threading
+
+    import torch
+
+    from ybus_b200._lib import lib, ptr
+
+    g = grids.make_grid(2000, 700, grids.SEED_BASE + 1)
+    net = DcNetwork.from_grid(gpu, g)
+    bp, chol, position = cpu_model(g)
+    rng = np.random.default_rng(count)
+    buses, branches = rng.integers(0, g.n_bus, count), rng.integers(0, g.n_branch, count)
+    pinned = torch.full((count, g.n_branch), 7.0, dtype=torch.float64, pin_memory=True)
+    results = {}
+    work = [threading.Thread(target=lambda: results.update(h=net.ptdf_columns(buses))),
+            threading.Thread(target=lambda: results.update(d=net.lodf_columns(branches)))]
+    for t in work:
+        t.start()
+    for t in work:
+        t.join()
+    assert lib().yb_dc_ptdf_columns(net._h, count, ptr(buses), pinned.data_ptr()) == 0
+    assert np.array_equal(pinned.numpy(), results["h"])
+    bridge = net.bridges()
+    for k in np.unique(np.r_[0, count - 1, rng.integers(0, count, 12)]):
+        c = np.zeros(chol.n)
+        if position[buses[k]] >= 0:
+            c[position[buses[k]]] = 1.0
+        h = flows_of(g, orc.solve_many(chol, c[None, :])[0], position)
+        assert np.abs(results["h"][k] - h).max() <= 1e-11
+        br = branches[k]
+        if bridge[br]:
+            assert np.isnan(results["d"][k]).all()
+            continue
+        c = np.zeros(chol.n)
+        for bus, sign in ((g.frm[br], 1.0), (g.to[br], -1.0)):
+            if position[bus] >= 0:
+                c[position[bus]] += sign
+        h = flows_of(g, orc.solve_many(chol, c[None, :])[0], position)
+        d = h / (1.0 - h[br])
+        d[br] = -1.0
+        assert np.abs(results["d"][k] - d).max() <= 1e-11 * max(1.0, 1.0 / abs(1.0 - h[br])) ** 2

@@ -50,7 +50,7 @@ __global__ void product_kernel(const int32_t *__restrict__ ptr, const int32_t *_
                                double *__restrict__ out, int64_t ldo) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t k = blockIdx.y;
-  if (i < rows) out[k * ldo + i] = product_entry(ptr, idx, val, offset, theta + k * ldt, i, zero[k]);
+  if (i < rows) out[k * ldo + i] = product_entry(ptr, idx, val, offset, theta + k * ldt, i, zero ? zero[k] : -1);
 }
 
 // Keeps the larger (value, row): the larger value, the smaller row on a tie, row -1 never winning
@@ -186,6 +186,16 @@ void check_operator(const yb_block *b, const yb_operator *op) {
 }
 
 }  // namespace
+
+namespace yb {
+void product_device(const yb_operator *op, const double *theta, int64_t ldt, int64_t count, double *out, cudaStream_t stream) {
+  if (count == 0 || op->rows == 0) return;
+  require(count < 65536, "at most 65,535 columns a product");
+  product_kernel<<<dim3((unsigned)((op->rows + 255) / 256), (unsigned)count), 256, 0, stream>>>(
+      op->ptr.get(), op->idx.get(), op->val.get(), op->offset.get(), (int)op->rows, theta, ldt, nullptr, out, op->rows);
+  cuda_check(cudaGetLastError(), "product_kernel launch");
+}
+}  // namespace yb
 
 extern "C" int32_t yb_pair_solves(yb_factor *f, int64_t count, const int64_t *plus, const int64_t *minus,
                                   yb_block **out) {

@@ -57,21 +57,21 @@ class DcNetwork:
     def ptdf_columns(self, buses) -> np.ndarray:
         """(count, n_branch): each bus's PTDF column (injection there, withdrawal at the slack)."""
         buses = np.ascontiguousarray(buses, np.int64)
-        out = np.zeros((buses.size, self.n_branch))
+        out = np.empty((buses.size, self.n_branch))
         _check(lib().yb_dc_ptdf_columns(self._h, buses.size, ptr(buses), ptr(out)))
         return out
 
     def ptdf_transfers(self, from_bus, to_bus) -> np.ndarray:
         f = np.ascontiguousarray(from_bus, np.int64)
         t = np.ascontiguousarray(to_bus, np.int64)
-        out = np.zeros((f.size, self.n_branch))
+        out = np.empty((f.size, self.n_branch))
         _check(lib().yb_dc_ptdf_transfers(self._h, f.size, ptr(f), ptr(t), ptr(out)))
         return out
 
     def lodf_columns(self, branches) -> np.ndarray:
         """(count, n_branch): each outaged branch's LODF column (NaN for a bridge)."""
         br = np.ascontiguousarray(branches, np.int64)
-        out = np.zeros((br.size, self.n_branch))
+        out = np.empty((br.size, self.n_branch))
         _check(lib().yb_dc_lodf_columns(self._h, br.size, ptr(br), ptr(out)))
         return out
 
