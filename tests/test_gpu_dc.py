@@ -165,3 +165,29 @@ def test_columns_in_any_number_of_pieces(gpu, count):
         d = h / (1.0 - h[br])
         d[br] = -1.0
         assert np.abs(results["d"][k] - d).max() <= 1e-11 * max(1.0, 1.0 / abs(1.0 - h[br])) ** 2
+
+
+@pytest.mark.parametrize("slack", [0, 7, 599])
+@pytest.mark.parametrize("scenarios", [1, 33])
+def test_screening_with_any_slack_and_a_scenario_not_finite(gpu, slack, scenarios):
+    """Balanced injections: the flows do not depend on the slack. Cases without scenarios, groups of columns
+    of several cases, and one scenario that is not finite, which flags its own column alone."""
+    g, outaged, sp, inj, weights = screening_case(600, 200, grids.SEED_BASE + 5, 12, 4)
+    net = DcNetwork.from_grid(gpu, g, slack)
+    _, chol, position = cpu_model(g)
+    counts = np.array([0] * 4 + [scenarios] + [1] * 7)
+    sp = np.concatenate([[0], np.cumsum(counts)])
+    rng = np.random.default_rng(scenarios)
+    inj = rng.normal(0, 0.1, (sp[-1], g.n_bus))
+    inj[:, 0] -= inj.sum(axis=1)
+    er, ev = oracle_screening(g, chol, position, outaged, sp, inj, weights)
+    spoiled = inj.copy()
+    spoiled[sp[-1] // 2, 300] = np.inf
+    for p, wrong in ((inj, -1), (spoiled, sp[-1] // 2)):
+        rows, values, bad, sing = net.outage_loadings_batch(outaged, sp, p, weights)
+        good = np.arange(sp[-1]) != wrong
+        assert not bad[good].any() and not sing[4:].any()
+        assert np.abs(values - ev)[good].max() <= 1e-10 * np.abs(ev).max()
+        assert (rows == er)[good].sum() >= good.sum() - 1
+        if wrong >= 0:
+            assert bad[wrong] == 3

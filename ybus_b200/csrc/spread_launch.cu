@@ -401,7 +401,7 @@ void spread_sweeps(yb_factor *f, DeviceSpread *d, T *work, T *xout, int64_t grou
   f->lane_partial.reserve(partial_bytes<T>(d, groups));
   SpreadArgs a{};
   a.one = net_of(d, groups, groups * 32);
-  a.one.work = work, a.one.xout = xout;
+  a.one.work = work, a.one.xout = xout, a.one.top_out = xout != work;
   set_partial<T>(a.one, f->lane_partial.get());
   a.one.group_active = group_active;
   a.slots = d->slots;
@@ -437,7 +437,7 @@ SpreadWork *work_for(yb_factor *f, size_t work_bytes, size_t partial, cudaStream
 
 template <class L>
 bool solve_lanes(yb_factor *f, DeviceSpread *d, const double *b, int64_t ldb, double *x, int64_t ldx, int64_t count,
-                 cudaStream_t stream) {
+                 cudaStream_t stream, const SpreadFinish &finish = {}) {
   constexpr int64_t COLS = 32 * SpreadLane<L>::N;  // columns of a group
   const int64_t n = f->n, groups_all = (count + COLS - 1) / COLS;
   const size_t group_bytes = (size_t)n * 32 * sizeof(L), pad_bytes = 2 * kSpreadPad * 32 * sizeof(L);
@@ -455,8 +455,9 @@ bool solve_lanes(yb_factor *f, DeviceSpread *d, const double *b, int64_t ldb, do
     SpreadArgs a{};
     a.one = net_of(d, groups, std::min(count - g0 * COLS, groups * COLS));
     a.one.work = a.one.xout = work;
+    a.one.top_out = (bool)finish;
     set_partial<L>(a.one, w->partial.get());
-    a.one.b = b + g0 * COLS * ldb, a.one.ldb = ldb, a.one.x = x + g0 * COLS * ldx, a.one.ldx = ldx;
+    a.one.b = b + g0 * COLS * ldb, a.one.ldb = ldb, a.one.x = x ? x + g0 * COLS * ldx : nullptr, a.one.ldx = ldx;
     a.slots = d->slots;
     const unsigned io = (unsigned)((groups * ((n + 31) / 32) + kSpreadIoWarps - 1) / kSpreadIoWarps);
     cudaEvent_t *ev = lane_timing_slot(f);
@@ -465,7 +466,10 @@ bool solve_lanes(yb_factor *f, DeviceSpread *d, const double *b, int64_t ldb, do
     if (ev) cuda_check(cudaEventRecord(ev[1], stream), "cudaEventRecord");
     one_sweeps<L>(d, a, f->gpu, stream);
     if (ev) cuda_check(cudaEventRecord(ev[2], stream), "cudaEventRecord");
-    launch(spread_out_kernel<L, false, false>, io, kSpreadIoWarps * 32, 0, stream, true, a);
+    if (finish)
+      finish(reinterpret_cast<const double *>(work), d->out_pos, g0 * COLS, a.one.count);
+    else
+      launch(spread_out_kernel<L, false, false>, io, kSpreadIoWarps * 32, 0, stream, true, a);
     if (ev) cuda_check(cudaEventRecord(ev[3], stream), "cudaEventRecord");
   }
   if (!capturing(stream)) cuda_check(cudaEventRecord(w->done, stream), "cudaEventRecord");
@@ -480,6 +484,10 @@ bool spread_solve(yb_factor *f, const double *b, int64_t ldb, double *x, int64_t
   if (!d) return false;
   if (sizeof(T) == 4 && count >= kSpreadPairCount) return solve_lanes<pair2<float>>(f, d, b, ldb, x, ldx, count, stream);
   return solve_lanes<T>(f, d, b, ldb, x, ldx, count, stream);
+}
+bool spread_solve_lanes(yb_factor *f, const double *b, int64_t ldb, int64_t count, cudaStream_t stream, const SpreadFinish &finish) {
+  DeviceSpread *d = spread_for(f, (int)sizeof(double), (count + 31) / 32, stream);
+  return d && solve_lanes<double>(f, d, b, ldb, nullptr, 0, count, stream, finish);
 }
 template bool spread_solve<double>(yb_factor *, const double *, int64_t, double *, int64_t, int64_t, cudaStream_t);
 template bool spread_solve<float>(yb_factor *, const double *, int64_t, double *, int64_t, int64_t, cudaStream_t);

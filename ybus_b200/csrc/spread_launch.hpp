@@ -2,6 +2,7 @@
 #pragma once
 
 #include <cstdint>
+#include <functional>
 #include <vector>
 
 #include "factor_state.cuh"
@@ -21,6 +22,13 @@ DeviceSpread *spread_for(yb_factor *f, int value_bytes, int64_t groups, cudaStre
 // or too small a workspace yet.
 template <class T>
 bool spread_solve(yb_factor *f, const double *b, int64_t ldb, double *x, int64_t ldx, int64_t count, cudaStream_t stream);
+
+// What takes the solutions where they are, in place of the scatter: columns `first` to `first + count` in groups
+// of 32 at `work` ([group][position][32], an unknown's position in `out_pos`), by launches on the solve's stream.
+using SpreadFinish = std::function<void(const double *work, const int32_t *out_pos, int64_t first, int64_t count)>;
+
+// As spread_solve in FP64, the solutions taken by `finish`.
+bool spread_solve_lanes(yb_factor *f, const double *b, int64_t ldb, int64_t count, cudaStream_t stream, const SpreadFinish &finish);
 
 // The sweeps and the top of `groups` groups whose right-hand sides are in `work` (at positions, with
 // kSpreadPad rows before and after), the solutions into `xout` (work itself, or another array of its layout);

@@ -53,6 +53,7 @@ struct SpreadNet {
   int64_t groups, count;       // groups of a warp's columns (32, or 64 with two per lane), and columns
   void *work, *xout, *partial; // xout: where the backward sweep writes (work, or an array of its layout)
   void *r, *r2;                // the top's right-hand sides [group][top row][32 lanes], full precision; what is between two products
+  bool top_out;                // the top's solutions go to xout as well (the scatter takes them from the partial array)
   const uint8_t *group_active; // [groups] 0: skipped; null: all run
   const void *b;               // the caller's right-hand sides and solutions
   int64_t ldb;
@@ -619,7 +620,7 @@ __global__ void __launch_bounds__(spread_top_warps<T, KS>() * 32) spread_top_ker
     }
   }
   S *xt = reinterpret_cast<S *>(static_cast<T *>(net.partial) + spread_top_row(net, g)) + tile * 32;
-  S *xo = net.xout != net.work ? reinterpret_cast<S *>(static_cast<T *>(net.xout) + ((size_t)g * net.n + net.n - t) * 32) + tile * 32 : nullptr;
+  S *xo = net.top_out ? reinterpret_cast<S *>(static_cast<T *>(net.xout) + ((size_t)g * net.n + net.n - t) * 32) + tile * 32 : nullptr;
   V *r2 = static_cast<V *>(net.r2) + (size_t)g * t * COLS + tile * 32;
   auto store = [&](int row, int col, V v0, V v1) {
     if (row >= t) return;
