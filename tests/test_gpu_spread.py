@@ -267,3 +267,45 @@ def test_adjoint_of_any_slack(gpu, slack, count):
     assert np.abs(gp - gp_c).max() <= 1e-10 * np.abs(gp_c).max()
     assert np.abs(gb - gb_c).max() <= 1e-10 * np.abs(gb_c).max()
     assert (gp[:, slack] == 0.0).all()
+
+
+@pytest.mark.parametrize("name", ["cholesky", "lu", "complex"])
+@pytest.mark.parametrize("count", [1, 40, 2100])
+def test_a_value_not_finite_stays_in_its_island_and_column(gpu, name, count):
+    """Two networks without a coupling in one factor; the second's solutions and the other columns' come out
+    as without the spoiled entry."""
+    import torch
+    n = 700
+    k = np.arange(n)
+    j = (k // 2 * 2 + 37 * (1 + k % 5)) % n  # neighbours of a parity: even rows and odd rows are islands
+    j = np.where((j + k) % 2 == 0, j, (j + 1) % n)
+    r, c = np.r_[k, k, j], np.r_[k, j, k]
+    keep = r != c
+    keep[:n] = True
+    w = 1.0 + (k % 7) / 7.0
+    v = np.r_[np.full(n, 30.0), -w, -w][keep]
+    r, c = r[keep], c[keep]
+    rng = np.random.default_rng(count)
+    b = rng.standard_normal((count, n))
+    spoiled = b.copy()
+    spoiled[count // 2, 10] = np.nan
+    if name == "complex":
+        a = host.Matrix.from_triplets(n, n, r, c, v * (1 + 0.25j), by_rows=False)
+        factor = GpuFactor.from_lu_complex(gpu, host.lu(a, host.COLAMD))
+        xs = []
+        for rhs in (b, spoiled):
+            t = torch.from_numpy(rhs.astype(np.complex128).view(np.float64).copy()).cuda()
+            x = torch.empty_like(t)
+            torch.cuda.synchronize()
+            solve_batch_complex([factor], [t.data_ptr()], [x.data_ptr()], [count], FP64)
+            gpu.synchronize()
+            xs.append(x.cpu().numpy().view(np.complex128))
+    else:
+        a = host.Matrix.from_triplets(n, n, r, c, v, by_rows=name == "cholesky")
+        factor = upload(gpu, host.cholesky(a) if name == "cholesky" else host.lu(a))
+        xs = [solve(gpu, factor, rhs, FP64) for rhs in (b, spoiled)]
+    clean, x = xs
+    others = np.arange(count) != count // 2
+    assert np.array_equal(x[others], clean[others])
+    assert np.isnan(x[count // 2, 10])
+    assert worst_relative_difference(x[[count // 2], 1::2], clean[[count // 2], 1::2]) < 1e-12

@@ -561,6 +561,21 @@ __device__ __forceinline__ void sp_store2(cplx<float> *p, cplx<double> a, cplx<d
   *reinterpret_cast<float4 *>(p) = make_float4((float)a.re, (float)a.im, (float)b.re, (float)b.im);
 }
 
+__device__ __forceinline__ bool sp_finite(double v) { return isfinite(v); }
+__device__ __forceinline__ bool sp_finite(const cplx<double> &v) { return isfinite(v.re) && isfinite(v.im); }
+__device__ __forceinline__ bool sp_zero(double v) { return v == 0.0; }
+__device__ __forceinline__ bool sp_zero(const cplx<double> &v) { return v.re == 0.0 && v.im == 0.0; }
+
+// An entry of the top's product over the map's entries that are not zero: the tensor product's zeros times a
+// right-hand side that is not finite would carry it to rows that do not depend on it (another island's).
+template <class V> __device__ __forceinline__ V spread_top_entry(const V *m, const V *r, int t, int cols) {
+  V s(0);
+#pragma unroll 1
+  for (int k = 0; k < t; ++k)
+    if (!sp_zero(m[(size_t)k * kSpreadTopRows])) s = sp_fnma(m[(size_t)k * kSpreadTopRows], r[(size_t)k * cols], s);
+  return V(0) - s;
+}
+
 // The top's product on the FP64 tensor cores, 16 rows by 32 columns a warp, fragments straight from L2
 // (the map and a group's columns are read by many warps; four steps of loads in flight). PHASE 0: x_T =
 // M r_T; 1: r2 = L_TT^-1 r_T; 2: x_T = U_TT^-1 r2, a triangle's zeros passed over; 3: r2 = M r_T;
@@ -624,6 +639,12 @@ __global__ void __launch_bounds__(spread_top_warps<T, KS>() * 32) spread_top_ker
   V *r2 = static_cast<V *>(net.r2) + (size_t)g * t * COLS + tile * 32;
   auto store = [&](int row, int col, V v0, V v1) {
     if (row >= t) return;
+    if (!sp_finite(v0) || !sp_finite(v1)) {
+      const V *mr = static_cast<const V *>(PHASE == 2 ? net.m2 : net.m) + (size_t)(row / kSpreadTopRows) * t * kSpreadTopRows + row % kSpreadTopRows;
+      const V *rc = static_cast<const V *>(PHASE == 2 ? net.r2 : net.r) + (size_t)g * t * COLS + tile * 32 + col;
+      if (!sp_finite(v0)) v0 = spread_top_entry(mr, rc, t, COLS);
+      if (!sp_finite(v1)) v1 = spread_top_entry(mr, rc + 1, t, COLS);
+    }
     V *between = r2 + (size_t)row * COLS + col;
     if constexpr (PHASE == 1 || PHASE == 3) {
       sp_store2(between, v0, v1);
