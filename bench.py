@@ -153,18 +153,6 @@ def algorithmic_bytes(n: int, count: int, info: dict, mode: str, steps: float = 
     return int(count * (24 * n + steps * 48 * n) + entries * 8 + 8 * (n + 1) + a_bytes)
 
 
-# DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one lane_solve_kernel<double> launch on
-# the 10,000-bus block of 13,499 right-hand sides, from one ncu capture of this kernel (2.176 GB read,
-# 2.115 GB written); other kernels and workloads report none
-LANE_FP64_TRAFFIC = {(9999, 13499): 4.290592e9}
-
-
-def traffic_of(result: dict, count: int, n: int):
-    if result.get("kernel") == "lane_solve_kernel<double>":
-        return LANE_FP64_TRAFFIC.get((n, count))
-    return None
-
-
 def _time_oracle(chol, rhs, threads: int, passes: int, seconds: float) -> tuple[float, int]:
     """Median seconds of `passes` oracle solves of `rhs` on `threads` threads (fewer if the time
     budget runs out), after one warm-up on a slice."""
@@ -514,27 +502,17 @@ def main():
         return replicas.max_over_ranks(elapsed_ms), launch_ms, kernels
 
     # which solve each mode runs (the library's automatic choice, read back from its settings)
-    lane32 = None
-    try:
-        lane32 = factor.lane_info(FP32)
-    except Exception:
-        pass
-    refine_min = factor.refine_lane_min_count()
-    use_lane32 = lane32 is not None and count >= max(refine_min, factor.lane_min_count(FP32)) and lane32["slots"] <= 64
+    ir_launches = 2 + 6 * (IR_MAX_STEPS + 1)
 
     def solver_of(mode):
         if mode == "fp64":  # gather, forward sweep, the top's sums and product, backward sweep, scatter
             return {"solver": "spread", "kernel": "spread_sweep_kernel<double>", "launches_per_step": 6,
                     "spread": factor.spread_info(FP64, count)}
-        if mode == "fp32_ir" and use_lane32:
-            # an initialisation and the gather, per pass a solve, a residual (the update folded
-            # in), a decision and the restore of columns a pass made no better, and between passes
-            # the FP64 carry of x (kernels of groups that have stopped return at once)
-            return {"solver": "lane", "kernel": "lane_solve_kernel<float>",
-                    "launches_per_step": 2 + 4 * (IR_MAX_STEPS + 1) + max(0, IR_MAX_STEPS - 1),
-                    "lane": {k: lane32[k] for k in ("warps", "slots", "domains", "top", "pages", "smem")}}
-        return {"solver": "domain", "kernel": "domain_tile_kernel", "launches_per_step": 1,
-                "tile": factor.domain_info(FP32)["tile"]}
+        # an initialisation and the gather; per pass two sweeps, the top's sums and product, a residual (the
+        # update and the decisions folded in) and what it leaves to do (kernels of groups that have stopped
+        # return at once)
+        return {"solver": "spread", "kernel": "spread_sweep_kernel<float>", "launches_per_step": ir_launches,
+                "spread": factor.spread_info(FP32, count)}
 
     from oracle import oracle as orc  # the checker, outside the timed regions
     p, i, v = bp.arrays()
@@ -588,8 +566,8 @@ def main():
                 steps_w = max(3, min(a.steps, 10))
                 elapsed_ms, launch_ms, _ = timed(lambda: blocks(mode, width), steps=steps_w)
                 r = check(mode, {"rhs_s": total * steps_w / (elapsed_ms / 1e3), "ms_per_step": elapsed_ms / steps_w,
-                                 "launches_per_step": -(-count // width) * (6 if mode == "fp64" else 1)})
-                r["solver"] = solver_of(mode)["solver"] if mode == "fp64" or width >= refine_min else "domain"
+                                 "launches_per_step": -(-count // width) * (6 if mode == "fp64" else ir_launches)})
+                r["solver"] = solver_of(mode)["solver"]
                 by_width[str(width)][mode] = r
     clock_info = clocks.stop()
 
@@ -611,7 +589,7 @@ def main():
             "accuracy": {"max_rel_residual": best["max_rel_residual"], "max_rel_err_vs_oracle": best["max_rel_err_vs_oracle"]},
             "modes": results, "modes_by_width": by_width,
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                         "traffic": traffic_of(best, count, n), "peak_source": peak_kind, "kernel": best["kernel"],
+                         "traffic": None, "peak_source": peak_kind, "kernel": best["kernel"],
                          "algorithmic_bytes_per_launch": best["algorithmic_bytes_per_launch"],
                          "kernel_ms": best["kernel_ms"], "launch_ms": best["launch_ms"], "compulsory_gbs": compulsory,
                          "compulsory_frac": compulsory / peak},

@@ -121,7 +121,7 @@ constexpr int kResidualRows = 1024, kResidualColumns = 4;
 
 // One block per ResidualItem. A row is a chain of loads (its bounds, a column index, an entry of x), so a
 // thread takes four columns' at once, and the blocks are pieces of rows, so large and small networks
-// fill the SMs alike. 21 million complex rows (16 networks of 500 to 46,293 buses, 128
+// fill the SMs alike. 21 million complex rows (16 networks of 730 to 46,293 buses, 128
 // columns each): 654 us; a block per column, its threads striding over all rows, took 1,121 us. The
 // entries of x come from L2 in sectors half used, 32 bytes each.
 __global__ void __launch_bounds__(256) batch_residual_kernel(const ResidualNet *__restrict__ nets, const ResidualItem *__restrict__ items) {

@@ -257,9 +257,9 @@ extern "C" int32_t yb_solve_batch_complex(int64_t networks, yb_factor *const *fa
       return ratios;
     };
     // the spread solve for the networks that admit it (its gather and scatter move whole complex128
-    // values: 16-byte alignment), the level-scheduled tiles for the others. At 16 networks of 500 to
+    // values: 16-byte alignment), the level-scheduled tiles for the others. At 16 networks of 730 to
     // 46,293 buses with 128 right-hand sides each 0.91 against 7.5 ms, after a first pass of 35 ms that
-    // lays them out (eight later passes pay for it)
+    // lays them out (four later passes pay for it)
     std::vector<DeviceSpread *> layouts;
     spread_for_batch(fs, precision == YB_FP64 ? 16 : 8, cnt, layouts, s);
     auto solve = [&](auto real, const std::vector<const cplx<double> *> &rhs, bool add) {

@@ -334,7 +334,7 @@ SpreadLayout<V> spread_layout(const Plan<V> &plan, int32_t value_bytes, int64_t 
   // a top, two launches more.
   const double G = (double)std::max<int64_t>(1, groups);
   // A complex top is four products of reals for one. That its map is applied twice is not charged: with 8
-  // in place of 4 a batch of 16 networks of 500 to 3,000 buses took 873 us for 912, and refined 5,778 for 5,650.
+  // in place of 4 a batch of 16 networks of 730 to 46,293 buses took 873 us for 912, and refined 5,778 for 5,650.
   constexpr double kTop = sizeof(V) == 16 ? 4 : 1;
   auto cost_of = [&](const Cut &c) {
     const double all = c.tasks * std::ceil(G / 4), wave = (double)blocks * sms, full = std::floor(all / wave);

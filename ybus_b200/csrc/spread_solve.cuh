@@ -19,9 +19,9 @@
 //
 // Measured on a B200, FP64 with device arrays, against the domain and lane solves that took these
 // sizes before: 2,000-bus B' with one right-hand side 71 to 29 us; 10,000-bus B' with 64, 87 to 42 us,
-// with 999, 330 to 138 us, with 13,499, 1,684 to 1,494 us (the gather 0.36 and the scatter 0.35 ms at
+// with 999, 330 to 141 us, with 13,499, 1,684 to 1,494 us (the gather 0.36 and the scatter 0.35 ms at
 // 6.1 TB/s, the sweeps and the top 0.82 ms: 5.3 TB/s over their 4.3 GB); the 10,000-bus Jacobian's LU
-// with 4,096, 1,336 to 1,036 us; 16 complex networks of 500 to 46,293 buses with 128 each, complex128 7.5 to
+// with 4,096, 1,336 to 1,036 us; 16 complex networks of 730 to 46,293 buses with 128 each, complex128 7.5 to
 // 0.91 ms, complex64 with refinement 21.1 to 4.3 ms. What bounds it: for large blocks HBM in the gather and scatter and
 // the shared-memory pipe (about 18 wavefronts a row and sweep) near HBM in the sweeps; for small ones
 // the six launches and the longest task's chain (about 290 cycles a row where a warp is alone).
