@@ -309,3 +309,28 @@ def test_a_value_not_finite_stays_in_its_island_and_column(gpu, name, count):
     assert np.array_equal(x[others], clean[others])
     assert np.isnan(x[count // 2, 10])
     assert worst_relative_difference(x[[count // 2], 1::2], clean[[count // 2], 1::2]) < 1e-12
+
+
+def test_a_refined_solve_that_has_run_can_be_captured(gpu):
+    """Beside a plain FP32 layout of the captured size, which holds no matrix."""
+    import torch
+    a = configs.bprime(grids.make_grid(1500, 520, 11))
+    chol = host.cholesky(a)
+    factor = GpuFactor.from_cholesky(gpu, chol)
+    factor.attach_matrix(a)
+    stream = torch.cuda.Stream()
+    b = torch.from_numpy(right_hand_sides(chol.n, 300, 5)).cuda()
+    x = torch.zeros_like(b)
+    torch.cuda.synchronize()
+    factor.solve_many_device(b.data_ptr(), x.data_ptr(), 64, FP32, stream.cuda_stream)
+    factor.solve_many_refined_device(b.data_ptr(), x.data_ptr(), 300, 4, 1e-10, stream=stream.cuda_stream)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        factor.solve_many_refined_device(b.data_ptr(), x.data_ptr(), 64, 4, 1e-10, stream=stream.cuda_stream)
+    rhs = right_hand_sides(chol.n, 64, 6)
+    b[:64].copy_(torch.from_numpy(rhs))
+    x.zero_()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert worst_relative_difference(x[:64].cpu().numpy(), orc.solve_many(chol, rhs, threads=8)) < 1e-8

@@ -1704,7 +1704,7 @@ extern "C" int32_t yb_solve_many_refined_device(yb_factor *f, const double *d_rh
     const auto bytes = [&](const double *p, int64_t ld) { return std::make_pair((uintptr_t)p, (uintptr_t)(p + (count - 1) * ld + f->n)); };
     const auto rb = bytes(d_rhs, ldb), rx = bytes(d_out, ldx);
     if (t32.kind == kTileAuto && !t32.shaped && !t32.refine_shaped && (rb.second <= rx.first || rx.second <= rb.first)) {
-      if (DeviceSpread *d = spread_for(f, (int)sizeof(float), (count + 31) / 32, s)) {
+      if (DeviceSpread *d = spread_for(f, (int)sizeof(float), (count + 31) / 32, s, f->a_attached)) {
         residual_matrix(f, d, d->host_out_pos, s);
         const RefineSweeps sweeps{d->in_pos, d->out_pos, d, [&](float *work, float *out, int64_t groups, const uint8_t *active) {
           spread_sweeps<float>(f, d, work, out, groups, active, s);

@@ -321,15 +321,17 @@ template <class V> std::unique_ptr<SpreadLayout<V>> try_layout(const yb_factor *
 
 }  // namespace
 
-DeviceSpread *spread_for(yb_factor *f, int value_bytes, int64_t groups, cudaStream_t stream) {
+DeviceSpread *spread_for(yb_factor *f, int value_bytes, int64_t groups, cudaStream_t stream, int64_t matrix) {
   const std::lock_guard<std::mutex> lock(f->spread_mutex);
   const auto key = std::make_pair(value_bytes, group_class(groups));
   auto it = f->spreads.find(key);
-  if (it != f->spreads.end()) return it->second.get();
-  if (capturing(stream)) {  // nothing may be made now: the nearest layout there is, if any
+  const bool no_more = (it == f->spreads.end() || matrix >= 0) && capturing(stream);
+  auto ready = [&](const DeviceSpread *d) { return !no_more || matrix < 0 || (d && d->res_matrix == matrix); };
+  if (it != f->spreads.end() && ready(it->second.get())) return it->second.get();
+  if (no_more) {  // nothing may be made now: the nearest layout there is, if any
     auto near = f->spreads.end();
     for (auto i = f->spreads.begin(); i != f->spreads.end(); ++i)
-      if (i->first.first == value_bytes && i->second &&
+      if (i->first.first == value_bytes && i->second && ready(i->second.get()) &&
           (near == f->spreads.end() || std::abs(i->first.second - key.second) < std::abs(near->first.second - key.second)))
         near = i;
     return near == f->spreads.end() ? nullptr : near->second.get();

@@ -14,8 +14,9 @@ namespace yb {
 constexpr int32_t kSpreadAutoSlots = 64, kSpreadAutoSlotsComplex = 96;
 
 // The spread layout for `groups` groups of 32 right-hand sides with values of `value_bytes`, made and
-// uploaded at its first use; null if the factor admits none.
-DeviceSpread *spread_for(yb_factor *f, int value_bytes, int64_t groups, cudaStream_t stream);
+// uploaded at its first use; null if the factor admits none. Under stream capture the nearest layout there
+// is, of those that hold the refined solve's copy of the matrix attached as number `matrix` (-1: of all).
+DeviceSpread *spread_for(yb_factor *f, int value_bytes, int64_t groups, cudaStream_t stream, int64_t matrix = -1);
 
 // Solves `count` right-hand sides (device arrays, column-major) in T (double or float); false, with
 // nothing done, where the factor admits no spread layout, or under stream capture where it has none
