@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <array>
+#include <atomic>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -163,12 +164,16 @@ struct DeviceSpread : ResidualMatrix {
 };
 
 // A workspace of the plain spread solve, for one stream at a time: the event marks its last use, so a
-// stream that takes it over (or one that got a destroyed stream's handle) waits for that.
+// stream that takes it over (or one that got a destroyed stream's handle) waits for that. One that a
+// capture took belongs to that graph until the graph and its executables are gone, which `released`
+// tells: no other solve takes it and it never grows, since the graph holds its pointers.
 struct SpreadWork {
   static constexpr size_t kMost = 4;  // workspaces a factor keeps; a further stream waits for the oldest
   cudaStream_t stream = nullptr;
   cudaEvent_t done = nullptr;
-  uint64_t used = 0;  // the solve that used it last
+  uint64_t used = 0;               // the solve that used it last
+  unsigned long long capture = 0;  // the capture that took it, or 0
+  std::shared_ptr<std::atomic<bool>> released;
   DeviceArray<uint8_t> work, partial;
   SpreadWork() = default;
   SpreadWork(const SpreadWork &) = delete;

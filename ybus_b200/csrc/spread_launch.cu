@@ -413,29 +413,90 @@ template void spread_sweeps<float>(yb_factor *, DeviceSpread *, float *, float *
 
 namespace {
 
-// The workspace a solve on `stream` takes, with at least the bytes asked for; null under capture when
-// the stream has none that large. The mutex is held.
-SpreadWork *work_for(yb_factor *f, size_t work_bytes, size_t partial, cudaStream_t stream) {
-  SpreadWork *w = nullptr;
-  for (auto &i : f->spread_work)
-    if (i->stream == stream) w = i.get();
-  if (capturing(stream)) return w && w->work.size() >= work_bytes && w->partial.size() >= partial ? w : nullptr;
-  if (!w)
-    for (auto &i : f->spread_work)
-      if (!w && cudaEventQuery(i->done) == cudaSuccess) w = i.get();
-  cudaGetLastError();  // a workspace still in use is no error
-  if (!w && f->spread_work.size() < SpreadWork::kMost) {
-    f->spread_work.push_back(std::make_unique<SpreadWork>());
-    w = f->spread_work.back().get();
-    cuda_check(cudaEventCreateWithFlags(&w->done, cudaEventDisableTiming), "cudaEventCreate");
+// Lets this thread allocate while a stream of it, or of another thread, is being captured: what it
+// allocates here belongs to no graph's work.
+struct CaptureAside {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  CaptureAside() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~CaptureAside() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
+// A workspace for a solve on `stream` with at least the bytes asked for, held until the solve is
+// enqueued. Eagerly one of the factor's, ordered by its event; under capture one of that capture's own
+// (a capture's solves on one stream follow one another), which the graph keeps by a user object.
+class WorkLease {
+ public:
+  WorkLease(yb_factor *f, size_t work_bytes, size_t partial_bytes, cudaStream_t stream) : lock_(f->spread_mutex), stream_(stream) {
+    const CaptureAside aside;
+    auto &all = f->spread_work;
+    // a graph that is gone gives its workspace back (the free waits for what still runs)
+    all.erase(std::remove_if(all.begin(), all.end(), [](const auto &i) { return i->capture && i->released->load(); }), all.end());
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    unsigned long long id = 0;
+    cudaGraph_t graph = nullptr;
+    cuda_check(cudaStreamGetCaptureInfo(stream, &status, &id, &graph), "cudaStreamGetCaptureInfo");
+    if (status != cudaStreamCaptureStatusNone) {
+      for (auto &i : all)
+        if (i->capture == id && i->stream == stream && i->work.size() >= work_bytes && i->partial.size() >= partial_bytes) w_ = i.get();
+      if (w_) return;
+      auto own = std::make_unique<SpreadWork>();
+      own->work.reserve(work_bytes), own->partial.reserve(partial_bytes);
+      own->stream = stream, own->capture = id;
+      own->released = std::make_shared<std::atomic<bool>>(false);
+      keep(graph, own->released);
+      all.push_back(std::move(own));
+      w_ = all.back().get();
+      return;
+    }
+    size_t eager = 0;
+    for (auto &i : all) {
+      if (i->capture) continue;
+      ++eager;
+      if (i->stream == stream) w_ = i.get();
+    }
+    if (!w_)
+      for (auto &i : all)
+        if (!w_ && !i->capture && cudaEventQuery(i->done) == cudaSuccess) w_ = i.get();
+    cudaGetLastError();  // a workspace still in use is no error
+    if (!w_ && eager < SpreadWork::kMost) {
+      all.push_back(std::make_unique<SpreadWork>());
+      w_ = all.back().get();
+      cuda_check(cudaEventCreateWithFlags(&w_->done, cudaEventDisableTiming), "cudaEventCreate");
+    }
+    if (!w_)
+      for (auto &i : all)
+        if (!i->capture && (!w_ || i->used < w_->used)) w_ = i.get();
+    cuda_check(cudaStreamWaitEvent(stream, w_->done, 0), "cudaStreamWaitEvent");
+    w_->stream = stream;
+    w_->used = ++f->spread_solves;
+    w_->work.reserve(work_bytes), w_->partial.reserve(partial_bytes);  // a larger array: the device is idle past the old one's free
   }
-  if (!w) w = std::min_element(f->spread_work.begin(), f->spread_work.end(), [](auto &a, auto &b) { return a->used < b->used; })->get();
-  cuda_check(cudaStreamWaitEvent(stream, w->done, 0), "cudaStreamWaitEvent");
-  w->stream = stream;
-  w->used = ++f->spread_solves;
-  w->work.reserve(work_bytes), w->partial.reserve(partial);  // a larger array: the device is idle past the old one's free
-  return w;
-}
+  ~WorkLease() {  // also where a launch failed: what was enqueued before it still runs
+    if (w_ && !w_->capture) cudaEventRecord(w_->done, stream_);
+  }
+  WorkLease(const WorkLease &) = delete;
+  WorkLease &operator=(const WorkLease &) = delete;
+  SpreadWork *operator->() const { return w_; }
+
+ private:
+  // `released` becomes true when `graph`, its clones and its executables are destroyed.
+  static void keep(cudaGraph_t graph, const std::shared_ptr<std::atomic<bool>> &released) {
+    using Held = std::shared_ptr<std::atomic<bool>>;
+    auto held = std::make_unique<Held>(released);
+    cudaUserObject_t object = nullptr;
+    cuda_check(cudaUserObjectCreate(&object, held.get(), [](void *p) {
+      const std::unique_ptr<Held> last(static_cast<Held *>(p));
+      (*last)->store(true);
+    }, 1, cudaUserObjectNoDestructorSync), "cudaUserObjectCreate");
+    held.release();  // the object's
+    const cudaError_t e = cudaGraphRetainUserObject(graph, object, 1, cudaGraphUserObjectMove);
+    if (e != cudaSuccess) cudaUserObjectRelease(object, 1);
+    cuda_check(e, "cudaGraphRetainUserObject");
+  }
+  std::lock_guard<std::mutex> lock_;
+  cudaStream_t stream_;
+  SpreadWork *w_ = nullptr;
+};
 
 template <class L>
 bool solve_lanes(yb_factor *f, DeviceSpread *d, const double *b, int64_t ldb, double *x, int64_t ldx, int64_t count,
@@ -447,10 +508,8 @@ bool solve_lanes(yb_factor *f, DeviceSpread *d, const double *b, int64_t ldb, do
   // small solves keep room for 1,536 right-hand sides (64 on factors of large order), so that any of
   // them can be captured once one has run
   const int64_t room = std::max<int64_t>(per_run, ((n <= 12800 ? 1536 : 64) + COLS - 1) / COLS);
-  const std::lock_guard<std::mutex> lock(f->spread_mutex);
-  SpreadWork *w = work_for(f, (size_t)(capturing(stream) ? per_run : room) * group_bytes + pad_bytes,
-                           partial_bytes<L>(d, capturing(stream) ? per_run : room), stream);
-  if (!w) return false;
+  const WorkLease w(f, (size_t)(capturing(stream) ? per_run : room) * group_bytes + pad_bytes,
+                    partial_bytes<L>(d, capturing(stream) ? per_run : room), stream);
   L *work = reinterpret_cast<L *>(w->work.get()) + kSpreadPad * 32;
   for (int64_t g0 = 0; g0 < groups_all; g0 += per_run) {
     const int64_t groups = std::min(per_run, groups_all - g0);
@@ -474,7 +533,6 @@ bool solve_lanes(yb_factor *f, DeviceSpread *d, const double *b, int64_t ldb, do
       launch(spread_out_kernel<L, false, false>, io, kSpreadIoWarps * 32, 0, stream, true, a);
     if (ev) cuda_check(cudaEventRecord(ev[3], stream), "cudaEventRecord");
   }
-  if (!capturing(stream)) cuda_check(cudaEventRecord(w->done, stream), "cudaEventRecord");
   return true;
 }
 
