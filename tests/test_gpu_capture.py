@@ -135,3 +135,60 @@ def test_a_destroyed_graph_gives_its_arrays_back(gpu, grid):
                 break
             time.sleep(0.1)
     assert back >= 8 * 3000 * chol.n, back
+
+
+def refined(factor, b, x, count, stream, ratio=None):
+    factor.solve_many_refined_device(b.data_ptr(), x.data_ptr(), count, 4, 1e-10,
+                                     None if ratio is None else ratio.data_ptr(), stream=stream.cuda_stream)
+
+
+@pytest.mark.parametrize("kind", [None, 4, 5], ids=["spread", "domain", "lane"])
+def test_a_captured_refined_solve_outlives_larger_ones(gpu, grid, kind):
+    """More columns than the solve that ran before it, and larger ones between its replays."""
+    import torch
+    a, chol = grid
+    factor = GpuFactor.from_cholesky(gpu, chol)
+    factor.attach_matrix(a)
+    if kind is not None:
+        factor.set_tile_kind(FP32, kind)
+    stream = torch.cuda.Stream()
+    b, x = columns(chol.n, 96, 5), torch.zeros(96, chol.n, dtype=torch.float64, device="cuda")
+    many, out = columns(chol.n, 5000, 7), torch.zeros(5000, chol.n, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    refined(factor, many, out, 40, stream)
+    graph = capture(stream, lambda: refined(factor, b, x, 96, stream))
+    for seed, count in ((8, 5000), (9, 1)):
+        refined(factor, many, out, count, stream)
+        b.copy_(columns(chol.n, 96, seed))
+        x.zero_()
+        torch.cuda.synchronize()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert agrees(x, chol, b, 1e-8)
+
+
+@pytest.mark.parametrize("kind", [None, 4], ids=["spread", "domain"])
+def test_refined_solves_on_several_streams_at_once(gpu, grid, kind):
+    import torch
+    a, chol = grid
+    factor = GpuFactor.from_cholesky(gpu, chol)
+    factor.attach_matrix(a)
+    if kind is not None:
+        factor.set_tile_kind(FP32, kind)
+    streams = [torch.cuda.Stream() for _ in range(6)]
+    bs = [columns(chol.n, 700 - 60 * k, k + 1) for k in range(6)]
+    xs = [torch.zeros_like(b) for b in bs]
+    ratios = [torch.zeros(b.shape[0], dtype=torch.float64, device="cuda") for b in bs]
+    torch.cuda.synchronize()
+    alone = []
+    for b, x, r in zip(bs, xs, ratios):
+        refined(factor, b, x, b.shape[0], streams[0], r)
+        torch.cuda.synchronize()
+        alone.append((x.clone(), r.clone()))
+    torch.cuda.synchronize()
+    for _ in range(10):
+        for b, x, s, r in zip(bs, xs, streams, ratios):
+            refined(factor, b, x, b.shape[0], s, r)
+    torch.cuda.synchronize()
+    for x, r, (xa, ra) in zip(xs, ratios, alone):
+        assert torch.equal(x, xa) and torch.equal(r, ra)

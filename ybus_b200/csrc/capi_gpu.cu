@@ -1564,12 +1564,13 @@ void residual_matrix(yb_factor *f, ResidualMatrix *d, const std::vector<int32_t>
   d->res_matrix = f->a_attached;
 }
 
-// What the refined solve takes of the lane or the spread solve: positions, A for the residual, and the
-// sweeps of groups from `work` into `out`, those with a zero in `active` left out.
+// What the refined solve takes of the lane or the spread solve: positions, A for the residual, the bytes of
+// the partial array, and the sweeps of groups from `work` into `out`, those with a zero in `active` left out.
 struct RefineSweeps {
   const int32_t *in_pos, *out_pos;
   const ResidualMatrix *matrix;
-  std::function<void(float *work, float *out, int64_t groups, const uint8_t *active)> run;
+  std::function<size_t(int64_t groups)> partial_bytes;
+  std::function<void(float *work, float *out, uint8_t *partial, int64_t groups, const uint8_t *active)> run;
 };
 
 // The refined solve (lane_refine.cuh), per launch's run of groups: b gathered once into the FP32 work
@@ -1586,17 +1587,19 @@ void launch_refined(yb_factor *f, const RefineSweeps &sweeps, const double *b, i
   const int64_t groups_all = (count + 31) / 32;
   const int64_t per_launch = std::max<int64_t>(1, std::min<int64_t>(groups_all, (int64_t)(kLaneWorkBytes / (group_vals * sizeof(T)))));
   const int64_t cols_most = per_launch * 32;
-  f->lane_work.reserve(((size_t)per_launch * group_vals + 2 * kSpreadPad * 32) * sizeof(T));
-  f->refine_parts.reserve(2 * (size_t)per_launch * group_vals);
-  if (max_steps >= 2) f->refine_scratch.reserve((size_t)per_launch * group_vals);
+  SpreadBytes bytes;
+  bytes.work = ((size_t)per_launch * group_vals + 2 * kSpreadPad * 32) * sizeof(T);
+  bytes.partial = sweeps.partial_bytes(per_launch);
+  bytes.corrections = 2 * (size_t)per_launch * group_vals * sizeof(T);
+  if (max_steps >= 2) bytes.iterate = (size_t)per_launch * group_vals * sizeof(double);
   // per column: rmax, bmax, cur, best (8 bytes each), best_steps (4); per group: col_active,
   // write_mask, restore_mask, done (4 each), active (1)
-  const size_t state_bytes = (size_t)cols_most * 36 + (size_t)per_launch * 17 + 64;
-  f->refine_state.reserve(state_bytes);
-  T *work = reinterpret_cast<T *>(f->lane_work.get()) + kSpreadPad * 32;
-  T *dA = f->refine_parts.get(), *dB = dA + (size_t)per_launch * group_vals;
-  double *X = f->refine_scratch.get();
-  uint8_t *st = f->refine_state.get();
+  bytes.state = (size_t)cols_most * 36 + (size_t)per_launch * 17 + 64;
+  const WorkLease w(f, bytes, stream);
+  T *work = reinterpret_cast<T *>(w->work.get()) + kSpreadPad * 32;
+  T *dA = reinterpret_cast<T *>(w->corrections.get()), *dB = dA + (size_t)per_launch * group_vals;
+  double *X = reinterpret_cast<double *>(w->iterate.get());
+  uint8_t *st = w->state.get();
   LaneRefineArgs r{};
   r.n = (int32_t)n;
   r.rmax = reinterpret_cast<unsigned long long *>(st);
@@ -1634,7 +1637,7 @@ void launch_refined(yb_factor *f, const RefineSweeps &sweeps, const double *b, i
     check("lane_in_kernel launch");
     for (int32_t pass = 0; pass <= max_steps; ++pass) {
       T *dk = pass == 1 ? dB : dA;  // this pass's correction
-      sweeps.run(work, dk, groups, r.active);
+      sweeps.run(work, dk, w->partial.get(), groups, r.active);
       if (pass == 0)
         lane_residual_kernel<0><<<rows_grid, kResWarps * 32, 0, stream>>>(r, dk, nullptr, nullptr, pass, max_steps, tolerance);
       else if (pass == 1)
@@ -1668,12 +1671,14 @@ void launch_lane_refined(yb_factor *f, DeviceLane *d, const double *b, int64_t l
   a.warp_page = d->warp_page.get();
   a.error = f->error.get();
   a.withhold = -1;
-  const RefineSweeps sweeps{d->in_pos.get(), d->out_pos.get(), d, [&](T *work, T *out, int64_t groups, const uint8_t *active) {
-    f->lane_partial.reserve((size_t)groups * std::max(d->partials, 1) * 32 * sizeof(T));
-    a.xout = out, a.group_active = active;
-    kernel<<<(unsigned)groups, d->warps * 32, smem, stream>>>(a, work, reinterpret_cast<T *>(f->lane_partial.get()));
-    cuda_check(cudaGetLastError(), "lane_solve_kernel launch");
-  }};
+  const RefineSweeps sweeps{
+      d->in_pos.get(), d->out_pos.get(), d,
+      [&](int64_t groups) { return (size_t)groups * std::max(d->partials, 1) * 32 * sizeof(T); },
+      [&](T *work, T *out, uint8_t *partial, int64_t groups, const uint8_t *active) {
+        a.xout = out, a.group_active = active;
+        kernel<<<(unsigned)groups, d->warps * 32, smem, stream>>>(a, work, reinterpret_cast<T *>(partial));
+        cuda_check(cudaGetLastError(), "lane_solve_kernel launch");
+      }};
   launch_refined(f, sweeps, b, ldb, x, ldx, count, max_steps, tolerance, ratio_out, steps_out, stream);
 }
 }  // namespace yb
@@ -1706,9 +1711,11 @@ extern "C" int32_t yb_solve_many_refined_device(yb_factor *f, const double *d_rh
     if (t32.kind == kTileAuto && !t32.shaped && !t32.refine_shaped && (rb.second <= rx.first || rx.second <= rb.first)) {
       if (DeviceSpread *d = spread_for(f, (int)sizeof(float), (count + 31) / 32, s, f->a_attached)) {
         residual_matrix(f, d, d->host_out_pos, s);
-        const RefineSweeps sweeps{d->in_pos, d->out_pos, d, [&](float *work, float *out, int64_t groups, const uint8_t *active) {
-          spread_sweeps<float>(f, d, work, out, groups, active, s);
-        }};
+        const RefineSweeps sweeps{
+            d->in_pos, d->out_pos, d, [&](int64_t groups) { return spread_partial_bytes<float>(d, groups); },
+            [&](float *work, float *out, uint8_t *partial, int64_t groups, const uint8_t *active) {
+              spread_sweeps<float>(f, d, work, out, partial, groups, active, s);
+            }};
         launch_refined(f, sweeps, d_rhs, ldb, d_out, ldx, count, max_steps, tolerance, d_ratio, d_steps, s);
         return YB_OK;
       }
@@ -1727,9 +1734,11 @@ extern "C" int32_t yb_solve_many_refined_device(yb_factor *f, const double *d_rh
       throw host::Error(host::kInvalidArgument, "the refined solve needs the domain solve, which this factor does not admit");
     const int64_t tiles = (count + cfg.width - 1) / cfg.width;
     const int64_t grid = std::min<int64_t>(tiles, (int64_t)f->gpu->sm_count);
-    f->refine_scratch.reserve((size_t)(2 * grid * f->n * cfg.width));  // each block's R and previous x
+    SpreadBytes need;
+    need.iterate = (size_t)(2 * grid * f->n * cfg.width) * sizeof(double);  // each block's R and previous x
+    const WorkLease w(f, need, s);
     RefineIO io{};
-    io.scratch = f->refine_scratch.get();
+    io.scratch = reinterpret_cast<double *>(w->iterate.get());
     io.b = d_rhs, io.ldb = ldb, io.x = d_out, io.ldx = ldx;
     io.in_slot = f->in_slot.get(), io.out_slot = f->out_slot.get();
     io.a_ptr = f->a_ptr.get(), io.a_idx = f->a_idx.get(), io.a_val = f->a_val.get();

@@ -163,9 +163,15 @@ struct DeviceSpread : ResidualMatrix {
   std::vector<int32_t> host_out_pos;
 };
 
-// A workspace of the plain spread solve, for one stream at a time: the event marks its last use, so a
-// stream that takes it over (or one that got a destroyed stream's handle) waits for that. One that a
-// capture took belongs to that graph until the graph and its executables are gone, which `released`
+// The bytes of a workspace's arrays: the work and the partial array, and the refined solves' FP32
+// corrections, FP64 iterate (the domain solve's: its residuals) and per-column state.
+struct SpreadBytes {
+  size_t work = 0, partial = 0, corrections = 0, iterate = 0, state = 0;
+};
+
+// A workspace of the spread solve and of the refined solves, for one stream at a time: the event marks its
+// last use, so a stream that takes it over (or one that got a destroyed stream's handle) waits for that. One
+// that a capture took belongs to that graph until the graph and its executables are gone, which `released`
 // tells: no other solve takes it and it never grows, since the graph holds its pointers.
 struct SpreadWork {
   static constexpr size_t kMost = 4;  // workspaces a factor keeps; a further stream waits for the oldest
@@ -174,7 +180,15 @@ struct SpreadWork {
   uint64_t used = 0;               // the solve that used it last
   unsigned long long capture = 0;  // the capture that took it, or 0
   std::shared_ptr<std::atomic<bool>> released;
-  DeviceArray<uint8_t> work, partial;
+  DeviceArray<uint8_t> work, partial, corrections, iterate, state;
+  bool holds(const SpreadBytes &b) const {
+    return work.size() >= b.work && partial.size() >= b.partial && corrections.size() >= b.corrections &&
+           iterate.size() >= b.iterate && state.size() >= b.state;
+  }
+  void reserve(const SpreadBytes &b) {
+    work.reserve(b.work), partial.reserve(b.partial), corrections.reserve(b.corrections);
+    iterate.reserve(b.iterate), state.reserve(b.state);
+  }
   SpreadWork() = default;
   SpreadWork(const SpreadWork &) = delete;
   SpreadWork &operator=(const SpreadWork &) = delete;
@@ -241,8 +255,8 @@ struct yb_factor {
   std::map<std::tuple<int, int, int, int>, std::unique_ptr<yb::DeviceDomain>> domains;
   // lane layouts by (value bytes, warps, page bytes); a null entry: the factor admits none
   std::map<std::tuple<int, int, int, int>, std::unique_ptr<yb::DeviceLane>> lanes;
-  // spread layouts by (value bytes, groups up to; a null entry: the factor admits none) and the plain
-  // solve's workspaces, one per stream in use; the mutex guards both
+  // spread layouts by (value bytes, groups up to; a null entry: the factor admits none) and the
+  // workspaces, one per stream in use; the mutex guards both
   std::map<std::pair<int, int64_t>, std::unique_ptr<yb::DeviceSpread>> spreads;
   std::vector<std::unique_ptr<yb::SpreadWork>> spread_work;
   uint64_t spread_solves = 0;
@@ -261,10 +275,7 @@ struct yb_factor {
   yb::DeviceArray<int32_t> a_ptr, a_idx;
   yb::DeviceArray<int32_t> a_csr_ptr, a_csr_idx;  // A as attached (CSR, natural order)
   yb::DeviceArray<double> a_csr_val;
-  yb::DeviceArray<uint8_t> refine_state;  // the lane refinement's per-column and per-group state
   yb::DeviceArray<double> a_val;
-  yb::DeviceArray<double> refine_scratch;  // per block n * W residuals; the lane refinement's FP64 iterate
-  yb::DeviceArray<float> refine_parts;     // the lane refinement's FP32 corrections (two work arrays)
   std::vector<int64_t> a_host_ptr, a_host_idx;  // A as attached (CSR, natural order), on the host
   std::vector<double> a_host_val;
   int64_t a_attached = 0;                  // how many times a matrix was attached

@@ -283,7 +283,7 @@ template <class T> void one_sweeps(const DeviceSpread *d, const SpreadArgs &a, c
 
 // The partial array of `groups` groups: the partials and the top's solutions in T, then the top's
 // right-hand sides (and, with two maps, what is between them) in full precision (every part a multiple of 128 bytes); at least one line.
-template <class T> size_t partial_bytes(const DeviceSpread *d, int64_t groups) {
+template <class T> size_t partial_bytes_of(const DeviceSpread *d, int64_t groups) {
   return (size_t)groups * 32 * ((size_t)(d->partials + d->top) * sizeof(T) + (size_t)d->top * (d->split || d->refine ? 2 : 1) * sizeof(typename SpreadLane<T>::Math)) + 128;
 }
 template <class T> void set_partial(SpreadNet &net, uint8_t *p) {
@@ -293,6 +293,9 @@ template <class T> void set_partial(SpreadNet &net, uint8_t *p) {
 }
 
 }  // namespace
+
+template <class T> size_t spread_partial_bytes(const DeviceSpread *d, int64_t groups) { return partial_bytes_of<T>(d, groups); }
+template size_t spread_partial_bytes<float>(const DeviceSpread *, int64_t);
 
 namespace {
 
@@ -398,18 +401,17 @@ void spread_for_batch(const std::vector<yb_factor *> &factors, int value_bytes, 
 }
 
 template <class T>
-void spread_sweeps(yb_factor *f, DeviceSpread *d, T *work, T *xout, int64_t groups, const uint8_t *group_active,
+void spread_sweeps(yb_factor *f, DeviceSpread *d, T *work, T *xout, uint8_t *partial, int64_t groups, const uint8_t *group_active,
                    cudaStream_t stream) {
-  f->lane_partial.reserve(partial_bytes<T>(d, groups));
   SpreadArgs a{};
   a.one = net_of(d, groups, groups * 32);
   a.one.work = work, a.one.xout = xout, a.one.top_out = xout != work;
-  set_partial<T>(a.one, f->lane_partial.get());
+  set_partial<T>(a.one, partial);
   a.one.group_active = group_active;
   a.slots = d->slots;
   one_sweeps<T>(d, a, f->gpu, stream);
 }
-template void spread_sweeps<float>(yb_factor *, DeviceSpread *, float *, float *, int64_t, const uint8_t *, cudaStream_t);
+template void spread_sweeps<float>(yb_factor *, DeviceSpread *, float *, float *, uint8_t *, int64_t, const uint8_t *, cudaStream_t);
 
 namespace {
 
@@ -421,82 +423,74 @@ struct CaptureAside {
   ~CaptureAside() { cudaThreadExchangeStreamCaptureMode(&mode); }
 };
 
-// A workspace for a solve on `stream` with at least the bytes asked for, held until the solve is
-// enqueued. Eagerly one of the factor's, ordered by its event; under capture one of that capture's own
-// (a capture's solves on one stream follow one another), which the graph keeps by a user object.
-class WorkLease {
- public:
-  WorkLease(yb_factor *f, size_t work_bytes, size_t partial_bytes, cudaStream_t stream) : lock_(f->spread_mutex), stream_(stream) {
-    const CaptureAside aside;
-    auto &all = f->spread_work;
-    // a graph that is gone gives its workspace back (the free waits for what still runs)
-    all.erase(std::remove_if(all.begin(), all.end(), [](const auto &i) { return i->capture && i->released->load(); }), all.end());
-    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
-    unsigned long long id = 0;
-    cudaGraph_t graph = nullptr;
-    cuda_check(cudaStreamGetCaptureInfo(stream, &status, &id, &graph), "cudaStreamGetCaptureInfo");
-    if (status != cudaStreamCaptureStatusNone) {
-      for (auto &i : all)
-        if (i->capture == id && i->stream == stream && i->work.size() >= work_bytes && i->partial.size() >= partial_bytes) w_ = i.get();
-      if (w_) return;
-      auto own = std::make_unique<SpreadWork>();
-      own->work.reserve(work_bytes), own->partial.reserve(partial_bytes);
-      own->stream = stream, own->capture = id;
-      own->released = std::make_shared<std::atomic<bool>>(false);
-      keep(graph, own->released);
-      all.push_back(std::move(own));
-      w_ = all.back().get();
-      return;
-    }
-    size_t eager = 0;
-    for (auto &i : all) {
-      if (i->capture) continue;
-      ++eager;
-      if (i->stream == stream) w_ = i.get();
-    }
-    if (!w_)
-      for (auto &i : all)
-        if (!w_ && !i->capture && cudaEventQuery(i->done) == cudaSuccess) w_ = i.get();
-    cudaGetLastError();  // a workspace still in use is no error
-    if (!w_ && eager < SpreadWork::kMost) {
-      all.push_back(std::make_unique<SpreadWork>());
-      w_ = all.back().get();
-      cuda_check(cudaEventCreateWithFlags(&w_->done, cudaEventDisableTiming), "cudaEventCreate");
-    }
-    if (!w_)
-      for (auto &i : all)
-        if (!i->capture && (!w_ || i->used < w_->used)) w_ = i.get();
-    cuda_check(cudaStreamWaitEvent(stream, w_->done, 0), "cudaStreamWaitEvent");
-    w_->stream = stream;
-    w_->used = ++f->spread_solves;
-    w_->work.reserve(work_bytes), w_->partial.reserve(partial_bytes);  // a larger array: the device is idle past the old one's free
-  }
-  ~WorkLease() {  // also where a launch failed: what was enqueued before it still runs
-    if (w_ && !w_->capture) cudaEventRecord(w_->done, stream_);
-  }
-  WorkLease(const WorkLease &) = delete;
-  WorkLease &operator=(const WorkLease &) = delete;
-  SpreadWork *operator->() const { return w_; }
+// `released` becomes true when `graph`, its clones and its executables are destroyed.
+void keep_while(cudaGraph_t graph, const std::shared_ptr<std::atomic<bool>> &released) {
+  using Held = std::shared_ptr<std::atomic<bool>>;
+  auto held = std::make_unique<Held>(released);
+  cudaUserObject_t object = nullptr;
+  cuda_check(cudaUserObjectCreate(&object, held.get(), [](void *p) {
+    const std::unique_ptr<Held> last(static_cast<Held *>(p));
+    (*last)->store(true);
+  }, 1, cudaUserObjectNoDestructorSync), "cudaUserObjectCreate");
+  held.release();  // the object's
+  const cudaError_t e = cudaGraphRetainUserObject(graph, object, 1, cudaGraphUserObjectMove);
+  if (e != cudaSuccess) cudaUserObjectRelease(object, 1);
+  cuda_check(e, "cudaGraphRetainUserObject");
+}
 
- private:
-  // `released` becomes true when `graph`, its clones and its executables are destroyed.
-  static void keep(cudaGraph_t graph, const std::shared_ptr<std::atomic<bool>> &released) {
-    using Held = std::shared_ptr<std::atomic<bool>>;
-    auto held = std::make_unique<Held>(released);
-    cudaUserObject_t object = nullptr;
-    cuda_check(cudaUserObjectCreate(&object, held.get(), [](void *p) {
-      const std::unique_ptr<Held> last(static_cast<Held *>(p));
-      (*last)->store(true);
-    }, 1, cudaUserObjectNoDestructorSync), "cudaUserObjectCreate");
-    held.release();  // the object's
-    const cudaError_t e = cudaGraphRetainUserObject(graph, object, 1, cudaGraphUserObjectMove);
-    if (e != cudaSuccess) cudaUserObjectRelease(object, 1);
-    cuda_check(e, "cudaGraphRetainUserObject");
+}  // namespace
+
+WorkLease::WorkLease(yb_factor *f, const SpreadBytes &bytes, cudaStream_t stream) : lock_(f->spread_mutex), stream_(stream) {
+  const CaptureAside aside;
+  auto &all = f->spread_work;
+  // a graph that is gone gives its workspace back (the free waits for what still runs)
+  all.erase(std::remove_if(all.begin(), all.end(), [](const auto &i) { return i->capture && i->released->load(); }), all.end());
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  unsigned long long id = 0;
+  cudaGraph_t graph = nullptr;
+  cuda_check(cudaStreamGetCaptureInfo(stream, &status, &id, &graph), "cudaStreamGetCaptureInfo");
+  if (status != cudaStreamCaptureStatusNone) {
+    for (auto &i : all)
+      if (i->capture == id && i->stream == stream && i->holds(bytes)) w_ = i.get();
+    if (w_) return;
+    auto own = std::make_unique<SpreadWork>();
+    own->reserve(bytes);
+    own->stream = stream, own->capture = id;
+    own->released = std::make_shared<std::atomic<bool>>(false);
+    keep_while(graph, own->released);
+    all.push_back(std::move(own));
+    w_ = all.back().get();
+    return;
   }
-  std::lock_guard<std::mutex> lock_;
-  cudaStream_t stream_;
-  SpreadWork *w_ = nullptr;
-};
+  size_t eager = 0;
+  for (auto &i : all) {
+    if (i->capture) continue;
+    ++eager;
+    if (i->stream == stream) w_ = i.get();
+  }
+  if (!w_)
+    for (auto &i : all)
+      if (!w_ && !i->capture && cudaEventQuery(i->done) == cudaSuccess) w_ = i.get();
+  cudaGetLastError();  // a workspace still in use is no error
+  if (!w_ && eager < SpreadWork::kMost) {
+    all.push_back(std::make_unique<SpreadWork>());
+    w_ = all.back().get();
+    cuda_check(cudaEventCreateWithFlags(&w_->done, cudaEventDisableTiming), "cudaEventCreate");
+  }
+  if (!w_)
+    for (auto &i : all)
+      if (!i->capture && (!w_ || i->used < w_->used)) w_ = i.get();
+  cuda_check(cudaStreamWaitEvent(stream, w_->done, 0), "cudaStreamWaitEvent");
+  w_->stream = stream;
+  w_->used = ++f->spread_solves;
+  w_->reserve(bytes);  // a larger array: the device is idle past the old one's free
+}
+
+WorkLease::~WorkLease() {
+  if (w_ && !w_->capture) cudaEventRecord(w_->done, stream_);
+}
+
+namespace {
 
 template <class L>
 bool solve_lanes(yb_factor *f, DeviceSpread *d, const double *b, int64_t ldb, double *x, int64_t ldx, int64_t count,
@@ -508,8 +502,10 @@ bool solve_lanes(yb_factor *f, DeviceSpread *d, const double *b, int64_t ldb, do
   // small solves keep room for 1,536 right-hand sides (64 on factors of large order), so that any of
   // them can be captured once one has run
   const int64_t room = std::max<int64_t>(per_run, ((n <= 12800 ? 1536 : 64) + COLS - 1) / COLS);
-  const WorkLease w(f, (size_t)(capturing(stream) ? per_run : room) * group_bytes + pad_bytes,
-                    partial_bytes<L>(d, capturing(stream) ? per_run : room), stream);
+  SpreadBytes bytes;
+  bytes.work = (size_t)(capturing(stream) ? per_run : room) * group_bytes + pad_bytes;
+  bytes.partial = partial_bytes_of<L>(d, capturing(stream) ? per_run : room);
+  const WorkLease w(f, bytes, stream);
   L *work = reinterpret_cast<L *>(w->work.get()) + kSpreadPad * 32;
   for (int64_t g0 = 0; g0 < groups_all; g0 += per_run) {
     const int64_t groups = std::min(per_run, groups_all - g0);
@@ -566,7 +562,7 @@ void spread_batch(const std::vector<SpreadSystem> &systems, bool add, SpreadBatc
   for (const SpreadSystem &sys : systems) {
     const int64_t groups = (sys.count + 31) / 32;
     work_values += (size_t)groups * sys.layout->n * 32 + 2 * kSpreadPad * 32;
-    part_bytes += partial_bytes<T>(sys.layout, groups);
+    part_bytes += partial_bytes_of<T>(sys.layout, groups);
     top_total += groups * top_tiles(sys.layout);
     slots = std::max(slots, sys.layout->slots);
     most_groups = std::max(most_groups, groups);
@@ -586,7 +582,7 @@ void spread_batch(const std::vector<SpreadSystem> &systems, bool add, SpreadBatc
     set_partial<T>(net, partial);
     net.b = sys.b, net.ldb = sys.layout->n, net.x = sys.x, net.ldx = sys.layout->n;
     work += (size_t)groups * sys.layout->n * 32 + 2 * kSpreadPad * 32;
-    partial += partial_bytes<T>(sys.layout, groups);
+    partial += partial_bytes_of<T>(sys.layout, groups);
     key.push_back(sys.layout->serial), key.push_back(groups);
   }
   w.nets.reserve(sizeof(SpreadNet) * k);

@@ -3,6 +3,7 @@
 
 #include <cstdint>
 #include <functional>
+#include <mutex>
 #include <vector>
 
 #include "factor_state.cuh"
@@ -31,11 +32,30 @@ using SpreadFinish = std::function<void(const double *work, const int32_t *out_p
 // As spread_solve in FP64, the solutions taken by `finish`.
 bool spread_solve_lanes(yb_factor *f, const double *b, int64_t ldb, int64_t count, cudaStream_t stream, const SpreadFinish &finish);
 
+// A workspace for a solve on `stream` with at least the bytes asked for, held until the solve is enqueued
+// (also by a launch that failed: what was enqueued before it still runs). Eagerly one of the factor's,
+// ordered by its event; under capture one of that capture's own (a capture's solves on one stream follow one
+// another), which the graph keeps by a user object.
+class WorkLease {
+ public:
+  WorkLease(yb_factor *f, const SpreadBytes &bytes, cudaStream_t stream);
+  ~WorkLease();
+  WorkLease(const WorkLease &) = delete;
+  WorkLease &operator=(const WorkLease &) = delete;
+  SpreadWork *operator->() const { return w_; }
+
+ private:
+  std::lock_guard<std::mutex> lock_;
+  cudaStream_t stream_;
+  SpreadWork *w_ = nullptr;
+};
+
 // The sweeps and the top of `groups` groups whose right-hand sides are in `work` (at positions, with
 // kSpreadPad rows before and after), the solutions into `xout` (work itself, or another array of its layout);
-// groups with a zero in `group_active` (null: none) are skipped.
+// `partial` holds spread_partial_bytes; groups with a zero in `group_active` (null: none) are skipped.
+template <class T> size_t spread_partial_bytes(const DeviceSpread *d, int64_t groups);
 template <class T>
-void spread_sweeps(yb_factor *f, DeviceSpread *d, T *work, T *xout, int64_t groups, const uint8_t *group_active,
+void spread_sweeps(yb_factor *f, DeviceSpread *d, T *work, T *xout, uint8_t *partial, int64_t groups, const uint8_t *group_active,
                    cudaStream_t stream);
 
 // The spread layouts of a batch of complex factors with these counts of right-hand sides (null: none), the
