@@ -1,13 +1,15 @@
 """Captured solves and several streams: a graph that holds a solve keeps giving the oracle's solutions
 whatever is solved between its replays and beside them, for any count once the factor has solved
 something, and gives its working arrays back when it is destroyed."""
+import threading
 import time
 
+import numpy as np
 import pytest
 
 import oracle.oracle as orc
 from fixtures import right_hand_sides, worst_relative_difference
-from ybus_b200 import FP32, FP64, GpuFactor, configs, grids, host
+from ybus_b200 import FP32, FP64, GpuFactor, configs, grids, host, solve_batch_complex
 
 pytestmark = pytest.mark.gpu
 
@@ -192,3 +194,52 @@ def test_refined_solves_on_several_streams_at_once(gpu, grid, kind):
     torch.cuda.synchronize()
     for x, r, (xa, ra) in zip(xs, ratios, alone):
         assert torch.equal(x, xa) and torch.equal(r, ra)
+
+
+def complex_batch(gpu, sizes, counts, seed):
+    import torch
+    lus, factors, bs = [], [], []
+    rng = np.random.default_rng(seed)
+    for k, (n, count) in enumerate(zip(sizes, counts)):
+        r, c, v = grids.ybus_triplets(grids.make_complex_grid(n, grids.SEED_BASE + 70 + seed + k))
+        lus.append(host.lu(host.Matrix.from_triplets(n, n, r, c, v, by_rows=False), host.COLAMD))
+        factors.append(GpuFactor.from_lu_complex(gpu, lus[-1]))
+        bs.append(torch.from_numpy(rng.standard_normal((count, 2 * n))).cuda())
+    return lus, factors, bs
+
+
+@pytest.mark.parametrize("threads", [False, True], ids=["one thread", "threads"])
+def test_complex_batches_on_two_streams_at_once(gpu, threads):
+    """Other networks and counts on each stream, the lists of blocks among what a batch uploads."""
+    import torch
+    batches = [complex_batch(gpu, (900, 400), (70, 129), 1), complex_batch(gpu, (300, 700, 500), (64, 33, 260), 9)]
+    streams = [torch.cuda.Stream() for _ in batches]
+    xs = [[torch.zeros_like(b) for b in bs] for _, _, bs in batches]
+    torch.cuda.synchronize()
+
+    def solve(k):
+        _, factors, bs = batches[k]
+        solve_batch_complex(factors, [b.data_ptr() for b in bs], [x.data_ptr() for x in xs[k]],
+                            [b.shape[0] for b in bs], FP64, stream=streams[k].cuda_stream)
+
+    for k in range(2):
+        for _ in range(8):
+            solve(k)
+    torch.cuda.synchronize()
+    alone = [[x.clone() for x in some] for some in xs]
+    torch.cuda.synchronize()
+    if threads:
+        work = [threading.Thread(target=lambda k=k: [solve(k) for _ in range(20)]) for k in range(2)]
+        for t in work:
+            t.start()
+        for t in work:
+            t.join()
+    else:
+        for _ in range(20):
+            solve(0), solve(1)
+    torch.cuda.synchronize()
+    for some, was, (lus, _, bs) in zip(xs, alone, batches):
+        for x, a, lu, b in zip(some, was, lus, bs):
+            assert torch.equal(x, a)
+            cpu = orc.solve_many_lu(lu, b[::9].cpu().numpy().view(np.complex128))
+            assert worst_relative_difference(x[::9].cpu().numpy().view(np.complex128), cpu) < 1e-12

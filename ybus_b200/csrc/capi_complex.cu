@@ -8,6 +8,7 @@
 #include <algorithm>
 #include <cmath>
 #include <memory>
+#include <mutex>
 #include <vector>
 
 #include "../../include/ybgpu.h"
@@ -106,7 +107,8 @@ void launch_batch(const std::vector<yb_factor *> &fs, const std::vector<const cp
   cuda_check(cudaGetLastError(), "batch_solve_kernel launch");
 }
 
-// The batch's device workspace, kept between calls (one set per GPU of the first factor)
+// The batch's device workspace, kept between calls (one set per GPU of the first factor): one call
+// enqueues at a time, and its stream waits for the last call's launches, whichever stream they are on.
 struct BatchWork {
   DeviceArray<uint8_t> nets, rnets;
   DeviceArray<BatchItem> items;
@@ -116,6 +118,26 @@ struct BatchWork {
   DeviceArray<cplx<float>> scratch64;
   DeviceArray<double> ratio;
   SpreadBatchWork spread;
+  cudaEvent_t done = nullptr;  // the last call's end
+  BatchWork() = default;
+  BatchWork(const BatchWork &) = delete;
+  BatchWork &operator=(const BatchWork &) = delete;
+  ~BatchWork() {
+    if (done) cudaEventDestroy(done);
+  }
+};
+
+// The order of a call on `stream` among those that use `w`; its end is recorded also where a launch failed.
+struct BatchTurn {
+  BatchWork &w;
+  cudaStream_t stream;
+  BatchTurn(BatchWork &work, cudaStream_t s) : w(work), stream(s) {
+    if (!w.done) cuda_check(cudaEventCreateWithFlags(&w.done, cudaEventDisableTiming), "cudaEventCreate");
+    cuda_check(cudaStreamWaitEvent(stream, w.done, 0), "cudaStreamWaitEvent");
+  }
+  ~BatchTurn() { cudaEventRecord(w.done, stream); }
+  BatchTurn(const BatchTurn &) = delete;
+  BatchTurn &operator=(const BatchTurn &) = delete;
 };
 
 }  // namespace
@@ -210,8 +232,10 @@ extern "C" int32_t yb_solve_batch_complex(int64_t networks, yb_factor *const *fa
     require(!need_residual || refine_possible, "refinement and ratios need the matrices: yb_factor_attach_matrix_complex");
     cuda_check(cudaSetDevice(gpu->device), "cudaSetDevice");
     cudaStream_t s = stream ? (cudaStream_t)stream : gpu->stream;
+    const std::lock_guard<std::mutex> hold(gpu->zmutex);
     if (!gpu->zwork) gpu->zwork = std::make_shared<BatchWork>();
     BatchWork &w = *static_cast<BatchWork *>(gpu->zwork.get());
+    const BatchTurn turn(w, s);
     // the residual's per-network descriptors and the list of its blocks
     std::vector<ResidualNet> rn(networks);
     std::vector<ResidualItem> pieces;

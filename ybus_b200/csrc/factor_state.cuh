@@ -34,6 +34,7 @@ struct yb_gpu {
   int64_t smem_per_sm = 0;
   std::string name;
   std::shared_ptr<void> zwork;  // the complex batch's device workspace (capi_complex.cu), kept between calls
+  std::mutex zmutex;            // held by the call that uses it
 };
 
 namespace yb {
