@@ -197,6 +197,24 @@ int32_t yb_lane_layout_lu(int64_t n, const int64_t *l_ptr, const int64_t *l_idx,
                           const int64_t *col_perm, int32_t value_bytes, int32_t page_bytes, int32_t max_slots,
                           int32_t warps, int32_t rhs_per_lane, int64_t *info, uint8_t *blob, int32_t *warp_page,
                           int32_t *in_pos, int32_t *out_pos);
+/* No ybus counterpart: the spread solve's layout for a Cholesky factor (no GPU needed), for `groups`
+ * groups of 32 right-hand sides on `sms` SMs. info receives 8 values {tasks, domains, top rows, live
+ * values per lane, partial rows, pages of 2,048 bytes, entries below and above the top triangles'
+ * diagonals}; with a blob (pages * 2,048 bytes), every array: task_row (tasks + 1), pages (first page and
+ * page count of each task's forward stream, then of its backward one: 4 * tasks), pos (in, then out: 2 n),
+ * part_ptr (top + 1), and the top's triangles by rows: top_ptr (2 (top + 1)), top_col and top_val (the
+ * entries of both, then both inverse diagonals). */
+int32_t yb_spread_layout_cholesky(int64_t n, const int64_t *l_ptr, const int64_t *l_idx, const double *l_val,
+                                  const int64_t *perm, int32_t value_bytes, int64_t groups, int32_t sms, int64_t *info,
+                                  uint8_t *blob, int32_t *task_row, int32_t *pages, int32_t *pos, int32_t *part_ptr,
+                                  int32_t *top_ptr, int32_t *top_col, double *top_val);
+/* The same for an LU factor as yb_factor_from_lu or (is_complex: every value two doubles)
+ * yb_factor_from_lu_complex takes it. */
+int32_t yb_spread_layout_lu(int64_t n, const int64_t *l_ptr, const int64_t *l_idx, const double *l_val,
+                            const int64_t *u_ptr, const int64_t *u_idx, const double *u_val, const int64_t *row_perm,
+                            const int64_t *col_perm, int32_t is_complex, int32_t value_bytes, int64_t groups, int32_t sms,
+                            int64_t *info, uint8_t *blob, int32_t *task_row, int32_t *pages, int32_t *pos, int32_t *part_ptr,
+                            int32_t *top_ptr, int32_t *top_col, double *top_val);
 /* No ybus counterpart, diagnostics on the host (no GPU needed): the domain layout a Cholesky factor
  * given as to yb_factor_from_cholesky gets for `value_bytes` (8 or 4). info receives {cut, top
  * rows, stages, warps, pages, records, entries, page bytes}, top_condition the worse infinity-norm

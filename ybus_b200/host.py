@@ -232,3 +232,34 @@ def lane_layout(factor: "HostCholesky | HostLu", value_bytes: int = 8, page_byte
             "fwd_entries": fwd_entries, "bwd_entries": bwd_entries, "warps": w, "domains": domains, "top": top,
             "partials": partials, "blob": blob, "warp_page": warp_page, "in_pos": in_pos, "out_pos": out_pos,
             "value_bytes": value_bytes, "rpl": r}
+
+
+def spread_layout(factor: "HostCholesky | HostLu", value_bytes: int = 8, groups: int = 1, sms: int = 148) -> dict:
+    """The spread solve's layout for a Cholesky or an LU factor, built on the host (no GPU): every task's
+    pages, the positions, the partial rows and the top's triangles (diagnostics and tests)."""
+    n, info = factor.n, np.zeros(8, np.int64)
+    lu_, cplx = isinstance(factor, HostLu), isinstance(factor, HostLu) and factor.is_complex
+    dt = np.complex128 if cplx else np.float64
+    l, lv = factor.l, np.ascontiguousarray(factor.l.val, dtype=dt)
+    if lu_:
+        u, uv = factor.u, np.ascontiguousarray(factor.u.val, dtype=dt)
+        fn = _lib.lib().yb_spread_layout_lu
+        args = (n, ptr(l.ptr), ptr(l.idx), ptr(lv), ptr(u.ptr), ptr(u.idx), ptr(uv), ptr(factor.row_perm),
+                ptr(factor.col_perm), int(cplx), value_bytes, groups, sms)
+    else:
+        fn = _lib.lib().yb_spread_layout_cholesky
+        args = (n, ptr(l.ptr), ptr(l.idx), ptr(lv), ptr(factor.perm), value_bytes, groups, sms)
+    check(fn(*args, ptr(info), *[None] * 8))
+    tasks, domains, top, slots, partials, pages, low, up = (int(v) for v in info)
+    blob, task_row, page = np.zeros(pages * 2048, np.uint8), np.zeros(tasks + 1, np.int32), np.zeros(4 * tasks, np.int32)
+    pos, part_ptr, top_ptr = np.zeros(2 * n, np.int32), np.zeros(top + 1, np.int32), np.zeros(2 * top + 2, np.int32)
+    top_col, top_val = np.zeros(max(low + up, 1), np.int32), np.zeros(max(low + up + 2 * top, 1), dt)
+    check(fn(*args, ptr(info), ptr(blob), ptr(task_row), ptr(page), ptr(pos), ptr(part_ptr), ptr(top_ptr), ptr(top_col),
+             ptr(top_val)))
+    cut = [low, low + up, low + up + top, low + up + 2 * top]
+    l_val, u_val, l_dinv, u_dinv = (top_val[a:b] for a, b in zip([0] + cut, cut))
+    return {"n": n, "tasks": tasks, "domains": domains, "top": top, "slots": slots, "partials": partials, "blob": blob,
+            "task_row": task_row, "fwd_page": page[:2 * tasks], "bwd_page": page[2 * tasks:], "in_pos": pos[:n],
+            "out_pos": pos[n:], "part_ptr": part_ptr, "value_bytes": value_bytes, "dtype": dt,
+            "lower": (top_ptr[:top + 1], top_col[:low], l_val, l_dinv),
+            "upper": (top_ptr[top + 1:], top_col[low:low + up], u_val, u_dinv)}
