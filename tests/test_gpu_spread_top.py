@@ -1,0 +1,93 @@
+"""The spread solve's top: its dense map with one correction leaves the residuals that a substitution leaves,
+also where the map's condition is large, in every solve that takes it; and a right-hand side that is infinite
+gives what the substitution gives."""
+import dataclasses
+
+import numpy as np
+import pytest
+
+import oracle.oracle as orc
+from fixtures import random_square
+from ybus_b200 import FP64, GpuFactor, Pair, configs, grids, host, solve_batch_complex
+
+pytestmark = pytest.mark.gpu
+
+
+def wide_grid(n_bus, extra, seed, decades):
+    g = grids.make_grid(n_bus, extra, seed)
+    spread = np.random.default_rng(seed).random(g.x.size) - 0.5
+    return dataclasses.replace(g, x=g.x * 10.0 ** (decades * spread))
+
+
+def branch_columns(g, count, seed):
+    rng = np.random.default_rng(seed)
+    e = rng.integers(0, g.n_branch, count)
+    rhs = np.zeros((count, g.n_bus))
+    rhs[np.arange(count), g.frm[e]] += 1.0
+    rhs[np.arange(count), g.to[e]] -= 1.0
+    return rhs[:, 1:], [Pair(int(f) - 1 if f > 0 else None, int(t) - 1 if t > 0 else None) for f, t in zip(g.frm[e], g.to[e])]
+
+
+def solve(gpu, factor, rhs):
+    import torch
+    b = torch.from_numpy(np.ascontiguousarray(rhs)).cuda()
+    x = torch.zeros_like(b)
+    torch.cuda.synchronize()
+    factor.solve_many_device(b.data_ptr(), x.data_ptr(), b.shape[0], FP64)
+    gpu.synchronize()
+    return x.cpu().numpy()
+
+
+def worst_residual(a, xs, rhs):
+    p, i, v = a.to_csr().arrays()
+    return max(orc.relative_residual(p, i, v, x, b) for x, b in zip(xs, rhs))
+
+
+@pytest.mark.parametrize("count", [1, 64, 999, 2100])
+@pytest.mark.parametrize("decades", [0, 3])
+def test_residuals_on_grids_of_wide_reactances(gpu, decades, count):
+    """Twice the substitution's worst over the same columns (its scatter over orders of summation), and the
+    project's bar of 1e-12; plain solves and pair solves."""
+    g = wide_grid(2000, 700, 11, decades)
+    a = configs.bprime(g)
+    chol = host.cholesky(a)
+    factor = GpuFactor.from_cholesky(gpu, chol)
+    assert factor.spread_info(FP64, count)["top"] > 0
+    rhs, pairs = branch_columns(g, count, 5)
+    some = np.unique(np.r_[np.arange(min(count, 64)), count - 1])
+    sub = worst_residual(a, orc.solve_many(chol, rhs[some], threads=8), rhs[some])
+    assert worst_residual(a, solve(gpu, factor, rhs)[some], rhs[some]) <= min(1e-12, max(4 * sub, 1e-14))
+    factor.set_block_width(count)
+    ys = factor.pair_solves(pairs).solutions()
+    assert worst_residual(a, ys[some], rhs[some]) <= min(1e-12, max(4 * sub, 1e-14))
+
+
+@pytest.mark.parametrize("count", [1, 40, 300])
+@pytest.mark.parametrize("name", ["jacobian", "random"])
+def test_residuals_of_real_lu_factors(gpu, name, count):
+    if name == "jacobian":
+        s = configs.jacobian_system(2000, 1, 5)
+        a, lu = s.jacobian, s.lu
+    else:
+        a = random_square(800, 3, 3)
+        lu = host.lu(a)
+    factor = GpuFactor.from_lu(gpu, lu)
+    rhs = np.random.default_rng(count).standard_normal((count, lu.n))
+    some = np.arange(0, count, 5)
+    sub = worst_residual(a, orc.solve_many(lu, rhs[some], threads=8), rhs[some])
+    assert worst_residual(a, solve(gpu, factor, rhs)[some], rhs[some]) <= 2 * sub
+
+
+@pytest.mark.parametrize("count", [3, 1000])
+def test_an_infinite_right_hand_side_gives_what_substitution_gives(gpu, count):
+    g = grids.make_grid(1500, 520, 11)
+    chol = host.cholesky(configs.bprime(g))
+    factor = GpuFactor.from_cholesky(gpu, chol)
+    assert factor.spread_info(FP64, count)["top"] > 0
+    rhs = np.random.default_rng(2).standard_normal((count, chol.n))
+    rhs[1, 700] = np.inf
+    rhs[2, 3] = -np.inf
+    x = solve(gpu, factor, rhs)
+    cpu = orc.solve_many(chol, rhs[:3])
+    assert np.isinf(cpu[1:]).all() and np.array_equal(x[1:3], cpu[1:])
+    assert np.isfinite(x[0]).all() and np.isfinite(x[3:]).all()

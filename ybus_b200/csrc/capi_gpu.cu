@@ -992,10 +992,6 @@ void solve_device(yb_factor *f, const double *b, int64_t ldb, double *x, int64_t
     run(0.0f, f->tile32, f->fwd32, f->bwd32, f->scratch32, f->slices32);
 }
 
-// Solves the right-hand sides e_plus - e_minus of `count` pairs (natural rows, -1 for none) into
-// `out` (n x count, natural order), with each column's rank-one update of `base` when `base` is
-// given (then alpha, inverse_weight and singular too). The domain solve where the factor admits it,
-// else the global-scratch solve.
 // The right-hand sides e_plus - e_minus (an unknown below zero: none) over the unknowns, four rows a thread.
 __global__ void __launch_bounds__(256) pair_rhs_kernel(const int32_t *__restrict__ plus, const int32_t *__restrict__ minus, int64_t n,
                                                        int64_t row_blocks, double *__restrict__ out, int64_t ldo) {
@@ -1043,14 +1039,13 @@ bool auto_spread_fp64(yb_factor *f, const double *b, int64_t ldb, double *x, int
   return admits_spread_fp64(f, count, stream) && spread_solve<double>(f, b, ldb, x, ldx, count, stream);
 }
 
-// `captured`: the launches go into a graph that is kept, so a solve that takes its workspace from the
-// factor's is not for them.
+// Solves the right-hand sides e_plus - e_minus of `count` pairs (natural rows, -1 for none) into
+// `out` (n x count, natural order), with each column's rank-one update of `base` when `base` is
+// given (then alpha, inverse_weight and singular too). `captured`: the launches go into a graph that is
+// kept, so a solve that takes its workspace from the factor's is not for them.
 // The automatic choice for a Cholesky factor writes the right-hand sides out and takes the spread solve in
-// place; LU factors keep the domain solve's substitutions (the products
-// of the spread solve's two maps round more with off-diagonal pivots: 1.0e-12 against 0.5e-12 for pairs of a
-// random matrix of 200 unknowns). A block of 1,000
-// pairs of the 10,000-bus B': 153 us, against 325 us by the domain solve, and 12 against 300 ms for a
-// factor's first.
+// place: a block of 1,000 pairs of the 10,000-bus B' 153 us, against 325 us by the domain solve, and 12 against
+// 300 ms for a factor's first. LU factors keep the domain solve, else the global-scratch solve.
 void solve_pairs_device(yb_factor *f, int64_t count, const int32_t *plus, const int32_t *minus, const double *base,
                         const double *alpha, const double *inverse_weight, int32_t *singular, double *out, int64_t ldo,
                         cudaStream_t stream, bool captured) {

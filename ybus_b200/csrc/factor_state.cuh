@@ -152,15 +152,13 @@ struct DeviceSpread : ResidualMatrix {
   int32_t n = 0, tasks = 0, domains = 0, top = 0, slots = 0, partials = 0;
   int64_t blob_bytes = 0;
   int64_t serial = 0;  // no two layouts of a process share one
-  bool split = false;  // the top as two maps (a real LU factor), m and m2, instead of one, m
-  bool refine = false;  // ... as one with a correction by S (a complex factor)
   double top_condition = 0;
   DeviceArray<uint8_t> store;  // what the pointers below point into
   const uint8_t *blob = nullptr;
   const int32_t *task_row = nullptr, *fwd_page = nullptr, *bwd_page = nullptr, *in_pos = nullptr, *out_pos = nullptr;
-  const int32_t *part_ptr = nullptr, *s_ptr = nullptr, *s_col = nullptr;
-  const void *s_val = nullptr;
-  void *m = nullptr, *m2 = nullptr;
+  const int32_t *part_ptr = nullptr, *s_ptr = nullptr, *s_col = nullptr, *u_ptr = nullptr, *u_col = nullptr;
+  const void *s_val = nullptr, *u_val = nullptr;
+  void *m = nullptr;
   std::vector<int32_t> host_out_pos;
 };
 

@@ -269,11 +269,14 @@ LaneLayout lane_layout(const Plan<T> &plan, int32_t value_bytes, int32_t page_by
 // front to back in the forward sweep and back to front in the backward one. Each sweep of a task is
 // a stream of packets in pages of kSpreadPage bytes, read by every warp that solves the task (one
 // per group of 32 right-hand sides). The top is solved between the two sweeps densely, in the factor's
-// full precision, whatever the packets' values are: for a Cholesky factor as one map x_T = S^-1 r_T;
-// for a real LU factor as x_T = U_TT^-1 (L_TT^-1 r_T), whose residuals stay near those of a substitution
-// where S^-1's do not (4.8 against 1.6 times the oracle's on the 10,000-bus Jacobian); for a complex LU
-// factor, where two maps were not enough (1.9e-12 on a 300-bus network that the substitution solves to
-// below 1e-12), as S^-1 with one correction by S, which is sparse.
+// full precision, whatever the packets' values are: as one map x_T = M r_T, M the inverse of the top's Schur
+// complement S = L_TT U_TT, and but in real FP32 with one correction: x_T += M (r_T - S x_T).
+// Without it the map's rounding, its condition times the unit roundoff, is all in the residual, up to a
+// hundred times a substitution's: with pairs of a 2,000-bus grid 5.7e-14 against 2.3e-15, with reactances
+// over three more decades 8.3e-12 against 5.3e-14, on the 10,000-bus Jacobian 6.1e-11 against 1.6e-11. With it
+// 2.6e-15, 5.3e-14 and 1.5e-11; a second correction changes nothing. A Cholesky factor's S x is a product
+// with S, which is sparse; a pivoted LU's is L_TT (U_TT x): rounding S itself costs as much as the map where
+// |L||U| is larger than S (the error of the 10,000-bus Jacobian's transposed solve 1.5e-13 by S, 1.5e-15 by its factors).
 //
 // A packet is 16-byte aligned: a head {uint32 kind, bytes, count, 0}, then by kind
 //   kSpreadRows4 / kSpreadRows1: four (one) rows' records {value 0, value 1, 1/diagonal, uint32 slots,
@@ -330,11 +333,10 @@ template <class V> struct SpreadLayout {  // V: double or complex<double>, the p
   // the top's own triangles by rows (columns as top indices) for its dense map
   std::vector<int32_t> l_ptr, l_col, u_ptr, u_col;
   std::vector<V> l_val, u_val, l_dinv, u_dinv;
-  // the top's Schur complement S = L_TT U_TT by rows (complex factors)
-  std::vector<int32_t> s_ptr, s_col;
-  std::vector<V> s_val;
+  // what the map is corrected by, by rows (spread_correction_by_schur, _by_factors): S, or -L_TT and U_TT
+  std::vector<int32_t> s_ptr, s_col, c_ptr, c_col;
+  std::vector<V> s_val, c_val;
   double s_norm = 0;                              // a bound of the infinity norm of the top's Schur complement
-  double l_norm = 0, u_norm = 0;                  // the infinity norms of L_TT and U_TT
 };
 
 // Builds the spread layout of `plan` for packets of `value_bytes` (half of the plan's value's bytes, or all
@@ -346,5 +348,9 @@ template <class V> struct SpreadLayout {  // V: double or complex<double>, the p
 template <class V>
 SpreadLayout<V> spread_layout(const Plan<V> &plan, int32_t value_bytes, int64_t groups, int32_t sms, int32_t blocks = 6,
                               const std::function<int32_t(int32_t)> &fit = {});
+
+// Fills a layout's matrices of the top's correction: S (a Cholesky factor's), or U_TT and -L_TT.
+void spread_correction_by_schur(SpreadLayout<double> &lay);
+template <class V> void spread_correction_by_factors(SpreadLayout<V> &lay);
 
 }  // namespace yb

@@ -218,6 +218,17 @@ template <class V> struct PacketWriter {
 
 template <class V> double magnitude_of(const V &v) { return std::abs(v); }
 
+// Runs `work` on this thread and `most` - 1 others, or on as many as there are.
+template <class F> void on_threads(int32_t most, const F &work) {
+  std::vector<std::thread> threads;
+  try {
+    for (int32_t i = 1; i < std::min<int32_t>(most, (int32_t)std::thread::hardware_concurrency()); ++i) threads.emplace_back(work);
+  } catch (const std::system_error &) {  // no more threads: those there are do
+  }
+  work();
+  for (auto &t : threads) t.join();
+}
+
 }  // namespace
 
 template <class V>
@@ -331,10 +342,12 @@ SpreadLayout<V> spread_layout(const Plan<V> &plan, int32_t value_bytes, int64_t 
   // The estimate of a cut, in cycles: the sweeps' blocks (a task for four groups, `blocks` an SM) in full
   // waves and one of what is left, each as long as the longest task with that many warps on its
   // scheduler; the top's map: a tile's chain of steps, its values from L2, half the FP64 rate; and, with
-  // a top, two launches more.
+  // a top, its launches.
   const double G = (double)std::max<int64_t>(1, groups);
-  // A complex top is four products of reals for one. That its map is applied twice is not charged: with 8
-  // in place of 4 a batch of 16 networks of 730 to 46,293 buses took 873 us for 912, and refined 5,778 for 5,650.
+  // A complex top is four products of reals for one. That a map is applied twice is charged to neither: times
+  // are flat in these weights (the 10,000-bus B' with 1 to 13,499 right-hand sides, its Jacobian and 300 and
+  // 2,000 buses: within 3 % with the top's charged two and three times), but with 2 in place of 4 a batch of 16
+  // complex networks of 730 to 46,293 buses took 1,082 us for 1,001, with 8 1,531, and four other batches were within 3 %.
   constexpr double kTop = sizeof(V) == 16 ? 4 : 1;
   auto cost_of = [&](const Cut &c) {
     const double all = c.tasks * std::ceil(G / 4), wave = (double)blocks * sms, full = std::floor(all / wave);
@@ -570,17 +583,8 @@ SpreadLayout<V> spread_layout(const Plan<V> &plan, int32_t value_bytes, int64_t 
         error = std::current_exception();
       }
     };
-    {
-      // a thread for 4,096 rows, at most eight: 46,293 rows' packets took 28 ms with one
-      const int32_t most = std::min<int32_t>({8, n / 4096, lay.tasks, (int32_t)std::thread::hardware_concurrency()});
-      std::vector<std::thread> threads;
-      try {
-        for (int32_t i = 1; i < most; ++i) threads.emplace_back(write_tasks);
-      } catch (const std::system_error &) {  // no more threads: those there are do
-      }
-      write_tasks();
-      for (auto &t : threads) t.join();
-    }
+    // a thread for 4,096 rows, at most eight: 46,293 rows' packets took 28 ms with one
+    on_threads(std::min<int32_t>({8, n / 4096, lay.tasks}), write_tasks);
     if (error) std::rethrow_exception(error);
     size_t blob_bytes = 0;
     for (int32_t w = 0; w < lay.tasks; ++w) {
@@ -603,40 +607,17 @@ SpreadLayout<V> spread_layout(const Plan<V> &plan, int32_t value_bytes, int64_t 
       lay.l_ptr.push_back((int32_t)lay.l_col.size()), lay.u_ptr.push_back((int32_t)lay.u_col.size());
       lay.l_dinv.push_back(plan.fwd.dinv[fat[j]]), lay.u_dinv.push_back(plan.bwd.dinv[bat[j]]);
     }
-    // the norms; || |L_TT| |U_TT| e ||inf bounds the Schur complement's
+    // || |L_TT| |U_TT| e ||inf bounds the Schur complement's norm
     {
       std::vector<double> u(lay.top);
       for (int32_t i = 0; i < lay.top; ++i) {
         u[i] = 1.0 / magnitude_of(lay.u_dinv[i]);
         for (int32_t q = lay.u_ptr[i]; q < lay.u_ptr[i + 1]; ++q) u[i] += magnitude_of(lay.u_val[q]);
-        lay.u_norm = std::max(lay.u_norm, u[i]);
       }
       for (int32_t i = 0; i < lay.top; ++i) {
-        double l = 1.0 / magnitude_of(lay.l_dinv[i]), s = l * u[i];
-        for (int32_t q = lay.l_ptr[i]; q < lay.l_ptr[i + 1]; ++q)
-          l += magnitude_of(lay.l_val[q]), s += magnitude_of(lay.l_val[q]) * u[lay.l_col[q]];
-        lay.l_norm = std::max(lay.l_norm, l), lay.s_norm = std::max(lay.s_norm, s);
-      }
-    }
-    if (std::is_same_v<V, std::complex<double>>) {
-      lay.s_ptr.assign(1, 0);
-      std::vector<V> sum(lay.top, V(0));
-      std::vector<int32_t> seen(lay.top, -1), cols;
-      for (int32_t i = 0; i < lay.top; ++i) {
-        cols.clear();
-        auto add = [&](V l, int32_t k) {  // l times U's row k
-          auto entry = [&](int32_t c, V u) {
-            if (seen[c] != i) seen[c] = i, sum[c] = V(0), cols.push_back(c);
-            sum[c] += l * u;
-          };
-          entry(k, V(1) / lay.u_dinv[k]);
-          for (int32_t q = lay.u_ptr[k]; q < lay.u_ptr[k + 1]; ++q) entry(lay.u_col[q], lay.u_val[q]);
-        };
-        for (int32_t q = lay.l_ptr[i]; q < lay.l_ptr[i + 1]; ++q) add(lay.l_val[q], lay.l_col[q]);
-        add(V(1) / lay.l_dinv[i], i);
-        std::sort(cols.begin(), cols.end());
-        for (int32_t c : cols) lay.s_col.push_back(c), lay.s_val.push_back(sum[c]);
-        lay.s_ptr.push_back((int32_t)lay.s_col.size());
+        double s = u[i] / magnitude_of(lay.l_dinv[i]);
+        for (int32_t q = lay.l_ptr[i]; q < lay.l_ptr[i + 1]; ++q) s += magnitude_of(lay.l_val[q]) * u[lay.l_col[q]];
+        lay.s_norm = std::max(lay.s_norm, s);
       }
     }
     lay.in_pos.resize(n), lay.out_pos.resize(n);
@@ -657,5 +638,63 @@ SpreadLayout<V> spread_layout(const Plan<V> &plan, int32_t value_bytes, int64_t 
 
 template SpreadLayout<double> spread_layout(const Plan<double> &, int32_t, int64_t, int32_t, int32_t, const std::function<int32_t(int32_t)> &);
 template SpreadLayout<host::c128> spread_layout(const Plan<host::c128> &, int32_t, int64_t, int32_t, int32_t, const std::function<int32_t(int32_t)> &);
+
+// S = L_TT U_TT by rows, each with the columns in order. Dense tops by several threads, a row at a time:
+// 1,500 dense rows are a billion products.
+void spread_correction_by_schur(SpreadLayout<double> &lay) {
+  using V = double;
+  std::vector<std::vector<int32_t>> cols(lay.top);
+  std::vector<std::vector<V>> vals(lay.top);
+  std::atomic<int32_t> next{0};
+  std::exception_ptr error;
+  std::mutex error_mutex;
+  auto rows = [&] {
+    try {
+      std::vector<V> sum(lay.top);
+      std::vector<int32_t> seen(lay.top, -1);
+      for (int32_t i = next++; i < lay.top; i = next++) {
+        auto entry = [&](int32_t c, V v) {
+          if (seen[c] != i) seen[c] = i, sum[c] = V(0), cols[i].push_back(c);
+          sum[c] += v;
+        };
+        auto add = [&](V l, int32_t k) {  // l times U's row k
+          entry(k, l * (V(1) / lay.u_dinv[k]));
+          for (int32_t q = lay.u_ptr[k]; q < lay.u_ptr[k + 1]; ++q) entry(lay.u_col[q], l * lay.u_val[q]);
+        };
+        for (int32_t q = lay.l_ptr[i]; q < lay.l_ptr[i + 1]; ++q) add(lay.l_val[q], lay.l_col[q]);
+        add(V(1) / lay.l_dinv[i], i);
+        std::sort(cols[i].begin(), cols[i].end());
+        for (int32_t c : cols[i]) vals[i].push_back(sum[c]);
+      }
+    } catch (...) {
+      const std::lock_guard<std::mutex> lock(error_mutex);
+      error = std::current_exception();
+    }
+  };
+  double products = 0;
+  for (int32_t k : lay.l_col) products += lay.u_ptr[k + 1] - lay.u_ptr[k] + 1;
+  on_threads((int32_t)std::min(8.0, products / 1e6), rows);
+  if (error) std::rethrow_exception(error);
+  lay.s_ptr.assign(1, 0);
+  for (int32_t i = 0; i < lay.top; ++i) {
+    lay.s_col.insert(lay.s_col.end(), cols[i].begin(), cols[i].end());
+    lay.s_val.insert(lay.s_val.end(), vals[i].begin(), vals[i].end());
+    lay.s_ptr.push_back((int32_t)lay.s_col.size());
+  }
+}
+
+template <class V> void spread_correction_by_factors(SpreadLayout<V> &lay) {
+  lay.s_ptr.assign(1, 0), lay.c_ptr.assign(1, 0);
+  for (int32_t i = 0; i < lay.top; ++i) {
+    for (int32_t q = lay.l_ptr[i]; q < lay.l_ptr[i + 1]; ++q) lay.s_col.push_back(lay.l_col[q]), lay.s_val.push_back(-lay.l_val[q]);
+    lay.s_col.push_back(i), lay.s_val.push_back(-V(1) / lay.l_dinv[i]);
+    lay.s_ptr.push_back((int32_t)lay.s_col.size());
+    for (int32_t q = lay.u_ptr[i]; q < lay.u_ptr[i + 1]; ++q) lay.c_col.push_back(lay.u_col[q]), lay.c_val.push_back(lay.u_val[q]);
+    lay.c_col.push_back(i), lay.c_val.push_back(V(1) / lay.u_dinv[i]);
+    lay.c_ptr.push_back((int32_t)lay.c_col.size());
+  }
+}
+template void spread_correction_by_factors(SpreadLayout<double> &);
+template void spread_correction_by_factors(SpreadLayout<host::c128> &);
 
 }  // namespace yb

@@ -17,8 +17,8 @@ namespace yb {
 
 namespace {
 
-// The largest condition (the norms of what a map inverts, for the Schur complement a bound, and of the
-// map) with which the top is taken densely.
+// The largest condition (a bound of the Schur complement's norm, times its map's) with which the top is
+// taken densely: its correction then leaves 1e-7 of the map's rounding, and FP32 values round more than the map.
 constexpr double kSpreadTopCondition = 1e9;
 constexpr size_t kSpreadWorkBytes = size_t(2) << 30;  // the largest work array one run of launches fills
 // FP32 takes two right-hand sides a lane from this many on (below, more warps are worth more than
@@ -81,8 +81,8 @@ struct Packer {
 // launch: an allocation for every array, and a launch and a wait for every map, took 105 ms for the first
 // pass over 16 complex networks.
 template <class V>
-std::vector<std::unique_ptr<DeviceSpread>> make_spreads(const std::vector<const SpreadLayout<V> *> &lays, const std::vector<int> &kinds,
-                                                        int value_bytes, const yb_gpu *gpu, cudaStream_t s) {
+std::vector<std::unique_ptr<DeviceSpread>> make_spreads(const std::vector<const SpreadLayout<V> *> &lays, int value_bytes,
+                                                        const yb_gpu *gpu, cudaStream_t s) {
   using M = typename DeviceValue<V>::type;
   if constexpr (std::is_same_v<V, double>)
     value_bytes == 8 ? allow_smem<double, false>(gpu) : (allow_smem<float, false>(gpu), allow_smem<pair2<float>, false>(gpu));
@@ -94,16 +94,16 @@ std::vector<std::unique_ptr<DeviceSpread>> make_spreads(const std::vector<const 
   std::vector<Packer> kept(k);
   struct Top {
     const int32_t *lp, *lc, *up, *uc;
-    const M *lv, *ld, *uv, *ud, *sv = nullptr;
-    M *scratch[2], *m[2];
+    const M *lv, *ld, *uv, *ud, *sv = nullptr, *cv = nullptr;
+    M *scratch, *m;
   };
   std::vector<Top> tops(k);
   Packer temp;
   const SpreadMap<M> *d_maps = nullptr;
   unsigned long long *norms = nullptr;
-  std::vector<SpreadMap<M>> maps(2 * k);
+  std::vector<SpreadMap<M>> maps(k);
   temp.put(maps, d_maps);
-  temp.put(std::vector<unsigned long long>(2 * k), norms);
+  temp.put(std::vector<unsigned long long>(k), norms);
   for (size_t i = 0; i < k; ++i) {
     if (!lays[i]) continue;
     const SpreadLayout<V> &lay = *lays[i];
@@ -113,14 +113,13 @@ std::vector<std::unique_ptr<DeviceSpread>> make_spreads(const std::vector<const 
     d->serial = ++serial;
     d->n = lay.n, d->tasks = lay.tasks, d->top = lay.top, d->slots = lay.slots, d->partials = lay.partials, d->domains = lay.domains;
     d->blob_bytes = (int64_t)lay.blob.size();
-    d->refine = d->top > 0 && std::is_same_v<V, host::c128>;
-    d->split = d->top > 0 && kinds[i] == YB_LU && !d->refine;
     d->host_out_pos = lay.out_pos;
     Packer &p = kept[i];
     p.put(lay.task_row, d->task_row), p.put(lay.fwd_page, d->fwd_page), p.put(lay.bwd_page, d->bwd_page);
     p.put(lay.in_pos, d->in_pos), p.put(lay.out_pos, d->out_pos), p.put(lay.part_ptr, d->part_ptr);
     if (lay.top == 0) continue;
-    if (d->refine) p.put(lay.s_ptr, d->s_ptr), p.put(lay.s_col, d->s_col), p.put(device_values(lay.s_val), t.sv);
+    if (!lay.s_ptr.empty()) p.put(lay.s_ptr, d->s_ptr), p.put(lay.s_col, d->s_col), p.put(device_values(lay.s_val), t.sv);
+    if (!lay.c_ptr.empty()) p.put(lay.c_ptr, d->u_ptr), p.put(lay.c_col, d->u_col), p.put(device_values(lay.c_val), t.cv);
     temp.put(lay.l_ptr, t.lp), temp.put(lay.l_col, t.lc);
     temp.put(device_values(lay.l_val), t.lv), temp.put(device_values(lay.l_dinv), t.ld);
     std::vector<int32_t> u_ptr{0}, u_col;  // the rows from the last to the first
@@ -138,21 +137,20 @@ std::vector<std::unique_ptr<DeviceSpread>> make_spreads(const std::vector<const 
   for (size_t i = 0; i < k; ++i) {
     DeviceSpread *d = out[i].get();
     if (!d) continue;
-    const int64_t t = d->top, count = t == 0 ? 0 : d->split ? 2 : 1;
+    const int64_t t = d->top;
     most = std::max(most, d->top);
-    for (int64_t j = 0; j < count; ++j) {
-      kept[i].place((size_t)(blocks(t, kSpreadTopRows) * t * kSpreadTopRows), tops[i].m[j]);
-      temp.place((size_t)(blocks(t, 32) * t * 32), tops[i].scratch[j]);
+    if (t > 0) {
+      kept[i].place((size_t)(blocks(t, kSpreadTopRows) * t * kSpreadTopRows), tops[i].m);
+      temp.place((size_t)(blocks(t, 32) * t * 32), tops[i].scratch);
     }
     kept[i].place(lays[i]->blob.size(), d->blob);
     kept[i].upload(d->store, s);
     cuda_check(cudaMemcpyAsync(const_cast<uint8_t *>(d->blob), lays[i]->blob.data(), lays[i]->blob.size(), cudaMemcpyHostToDevice, s),
                "spread packet upload");
-    d->s_val = tops[i].sv;
-    if (count) d->m = tops[i].m[0];
-    if (count == 2) d->m2 = tops[i].m[1];
-    if (count)  // the rows past the last of a block of rows
-      cuda_check(cudaMemsetAsync(d->m, 0, (size_t)(d->blob - (uint8_t *)d->m), s), "clear the maps");
+    d->s_val = tops[i].sv, d->u_val = tops[i].cv;
+    if (t == 0) continue;
+    d->m = tops[i].m;  // with the rows past the last of a block of rows
+    cuda_check(cudaMemsetAsync(d->m, 0, (size_t)(d->blob - (uint8_t *)d->m), s), "clear the maps");
   }
   if (most > 0) {
     DeviceArray<uint8_t> temporary;
@@ -163,30 +161,23 @@ std::vector<std::unique_ptr<DeviceSpread>> make_spreads(const std::vector<const 
       const DeviceSpread *d = out[i].get();
       if (!d || d->top == 0) continue;
       const Top &t = tops[i];
-      const SpreadMap<M> both{d->top, (int32_t)blocks(d->top, 32), t.lp, t.lc, t.lv, t.ld, t.up, t.uc, t.uv, t.ud,
-                              t.scratch[0], t.m[0], norms + 2 * i};
-      maps[2 * i] = both;
-      if (d->split) {
-        maps[2 * i + 1] = both;
-        maps[2 * i].u_ptr = nullptr, maps[2 * i + 1].l_ptr = nullptr;
-        maps[2 * i + 1].scratch = t.scratch[1], maps[2 * i + 1].m = t.m[1], maps[2 * i + 1].norm = norms + 2 * i + 1;
-      }
+      maps[i] = {d->top, (int32_t)blocks(d->top, 32), t.lp, t.lc, t.lv, t.ld, t.up, t.uc, t.uv, t.ud, t.scratch, t.m, norms + i};
     }
     std::memcpy(temp.bytes.data() + temp.places[0].first, maps.data(), maps.size() * sizeof maps[0]);
     cuda_check(cudaMemcpyAsync(temporary.get(), temp.bytes.data(), temp.bytes.size(), cudaMemcpyHostToDevice, s), "upload the tops");
-    spread_map_kernel<M><<<dim3((unsigned)blocks(most, 32), (unsigned)(2 * k)), 32, 0, s>>>(d_maps);
+    spread_map_kernel<M><<<dim3((unsigned)blocks(most, 32), (unsigned)k), 32, 0, s>>>(d_maps);
     cuda_check(cudaGetLastError(), "spread_map_kernel launch");
-    spread_norm_kernel<M><<<dim3((unsigned)blocks(most, 256), (unsigned)(2 * k)), 256, 0, s>>>(d_maps);
+    spread_norm_kernel<M><<<dim3((unsigned)blocks(most, 256), (unsigned)k), 256, 0, s>>>(d_maps);
     cuda_check(cudaGetLastError(), "spread_norm_kernel launch");
-    std::vector<unsigned long long> bits(2 * k);
+    std::vector<unsigned long long> bits(k);
     cuda_check(cudaMemcpyAsync(bits.data(), norms, bits.size() * sizeof bits[0], cudaMemcpyDeviceToHost, s), "download the norms");
     cuda_check(cudaStreamSynchronize(s), "the tops' maps");
     for (size_t i = 0; i < k; ++i) {
       DeviceSpread *d = out[i].get();
       if (!d || d->top == 0) continue;
-      double norm[2];
-      std::memcpy(norm, &bits[2 * i], sizeof norm);
-      d->top_condition = d->split ? std::max(norm[0] * lays[i]->l_norm, norm[1] * lays[i]->u_norm) : norm[0] * lays[i]->s_norm;
+      double norm;
+      std::memcpy(&norm, &bits[i], sizeof norm);
+      d->top_condition = norm * lays[i]->s_norm;
       if (!(d->top_condition <= kSpreadTopCondition)) out[i] = nullptr;
     }
   }
@@ -199,8 +190,9 @@ SpreadNet net_of(const DeviceSpread *d, int64_t groups, int64_t count) {
   net.n = d->n, net.tasks = d->tasks, net.top = d->top, net.partials = d->partials;
   net.blob = d->blob, net.fwd_page = d->fwd_page, net.bwd_page = d->bwd_page;
   net.task_row = d->task_row, net.part_ptr = d->part_ptr;
-  net.in_pos = d->in_pos, net.out_pos = d->out_pos, net.m = d->m, net.m2 = d->m2;
+  net.in_pos = d->in_pos, net.out_pos = d->out_pos, net.m = d->m;
   net.s_ptr = d->s_ptr, net.s_col = d->s_col, net.s_val = d->s_val;
+  net.u_ptr = d->u_ptr, net.u_col = d->u_col, net.u_val = d->u_val;
   net.groups = groups, net.count = count;
   return net;
 }
@@ -262,7 +254,8 @@ template <class T> void one_sweeps(const DeviceSpread *d, const SpreadArgs &a, c
   const unsigned grid = (unsigned)(d->tasks * ((groups + warps - 1) / warps));
   launch(spread_sweep_kernel<T, false, false>, grid, warps * 32, smem, s, true, a);
   if (d->top > 0) {
-    launch(spread_sum_kernel<T, false>, (unsigned)(groups * ((d->top + 7) / 8)), 256, 0, s, true, a);
+    const unsigned rows = (unsigned)(groups * ((d->top + 7) / 8));
+    launch(spread_sum_kernel<T, false>, rows, 256, 0, s, true, a);
     const int64_t columns = groups * SpreadLane<T>::N;
     const int split = split_top<T>(columns * top_tiles(d), gpu);
     const unsigned blocks = (unsigned)(columns * top_blocks<T>(d, split));
@@ -273,23 +266,29 @@ template <class T> void one_sweeps(const DeviceSpread *d, const SpreadArgs &a, c
       else
         launch(spread_top_kernel<T, false, 1, PHASE>, blocks, spread_top_warps<T, 1>() * 32, 0, s, true, a);
     };
-    if (d->split)
-      top(std::integral_constant<int, 1>()), top(std::integral_constant<int, 2>());
-    else
+    if constexpr (SpreadLane<T>::kCorrect) {
+      top(std::integral_constant<int, 1>());
+      if (d->u_val) launch(spread_correct_kernel<T, false, true>, rows, 256, 0, s, true, a);
+      launch(spread_correct_kernel<T, false, false>, rows, 256, 0, s, true, a);
+      top(std::integral_constant<int, 2>());
+    } else {
       top(std::integral_constant<int, 0>());
+    }
   }
   launch(spread_sweep_kernel<T, true, false>, grid, warps * 32, smem, s, true, a);
 }
 
 // The partial array of `groups` groups: the partials and the top's solutions in T, then the top's
-// right-hand sides (and, with two maps, what is between them) in full precision (every part a multiple of 128 bytes); at least one line.
+// right-hand sides (and, where it is corrected, the first product and U_TT times it) in full precision (every
+// part a multiple of 128 bytes); at least one line.
 template <class T> size_t partial_bytes_of(const DeviceSpread *d, int64_t groups) {
-  return (size_t)groups * 32 * ((size_t)(d->partials + d->top) * sizeof(T) + (size_t)d->top * (d->split || d->refine ? 2 : 1) * sizeof(typename SpreadLane<T>::Math)) + 128;
+  return (size_t)groups * 32 * ((size_t)(d->partials + d->top) * sizeof(T) + (size_t)d->top * (!SpreadLane<T>::kCorrect ? 1 : d->u_val ? 3 : 2) * sizeof(typename SpreadLane<T>::Math)) + 128;
 }
 template <class T> void set_partial(SpreadNet &net, uint8_t *p) {
   net.partial = p;
   uint8_t *r = p + (size_t)net.groups * 32 * (size_t)(net.partials + net.top) * sizeof(T);
-  net.r = r, net.r2 = r + (size_t)net.groups * 32 * net.top * sizeof(typename SpreadLane<T>::Math);
+  const size_t full = (size_t)net.groups * 32 * net.top * sizeof(typename SpreadLane<T>::Math);
+  net.r = r, net.r2 = r + full, net.r3 = r + 2 * full;
 }
 
 }  // namespace
@@ -314,6 +313,10 @@ template <class V> const Plan<V> &plan_of(const yb_factor *f) {
 template <class V> std::unique_ptr<SpreadLayout<V>> try_layout(const yb_factor *f, int value_bytes, int64_t groups) {
   try {
     auto lay = std::make_unique<SpreadLayout<V>>(host_spread(plan_of<V>(f), value_bytes, groups, f->gpu));
+    if constexpr (!std::is_same_v<V, double>)
+      spread_correction_by_factors(*lay);
+    else if (value_bytes == 8)
+      f->kind == YB_LU ? spread_correction_by_factors(*lay) : spread_correction_by_schur(*lay);
     const int32_t limit = f->is_complex ? kSpreadAutoSlotsComplex : kSpreadAutoSlots;
     return lay->slots <= limit ? std::move(lay) : nullptr;
   } catch (const host::Error &e) {
@@ -340,7 +343,7 @@ DeviceSpread *spread_for(yb_factor *f, int value_bytes, int64_t groups, cudaStre
     return near == f->spreads.end() ? nullptr : near->second.get();
   }
   const auto lay = try_layout<double>(f, value_bytes, key.second);
-  auto d = std::move(make_spreads<double>({lay.get()}, {f->kind}, value_bytes, f->gpu, stream)[0]);
+  auto d = std::move(make_spreads<double>({lay.get()}, value_bytes, f->gpu, stream)[0]);
   auto *out = d.get();
   f->spreads.emplace(key, std::move(d));
   return out;
@@ -386,7 +389,7 @@ void spread_for_batch(const std::vector<yb_factor *> &factors, int value_bytes, 
   if (!missing.empty()) {
     std::vector<const SpreadLayout<host::c128> *> lays;
     for (size_t i : missing) lays.push_back(made[i].get());
-    auto d = make_spreads<host::c128>(lays, std::vector<int>(missing.size(), YB_LU), value_bytes, factors[0]->gpu, stream);
+    auto d = make_spreads<host::c128>(lays, value_bytes, factors[0]->gpu, stream);
     for (size_t m = 0; m < missing.size(); ++m) {
       const std::lock_guard<std::mutex> lock(factors[missing[m]]->spread_mutex);
       factors[missing[m]]->spreads.emplace(keys[missing[m]], std::move(d[m]));
@@ -635,10 +638,11 @@ void spread_batch(const std::vector<SpreadSystem> &systems, bool add, SpreadBatc
       else
         launch(spread_top_kernel<T, true, 1, PHASE>, (unsigned)n_top, spread_top_warps<T, 1>() * 32, 0, stream, true, a);
     };
-    phase(std::integral_constant<int, 3>());
+    phase(std::integral_constant<int, 1>());
     a.items = d_items + n_io + n_sweep;
-    launch(spread_correct_kernel<T, true>, (unsigned)n_sum, 256, 0, stream, true, a);
-    phase(std::integral_constant<int, 4>());
+    launch(spread_correct_kernel<T, true, true>, (unsigned)n_sum, 256, 0, stream, true, a);
+    launch(spread_correct_kernel<T, true, false>, (unsigned)n_sum, 256, 0, stream, true, a);
+    phase(std::integral_constant<int, 2>());
   }
   a.items = d_items + n_io;
   launch(spread_sweep_kernel<T, true, true>, (unsigned)n_sweep, warps * 32, smem, stream, true, a);

@@ -6,7 +6,7 @@
 //   spread_sweep  every task forward: z over b in the work array, updates of top rows into the
 //                 partial array
 //   spread_sum    the top's right-hand sides r_T: b_T plus the partials
-//   spread_top    x_T as a dense product of r_T, or two (complex: spread_correct between them)
+//   spread_top    x_T as a dense product of r_T; but in FP32 twice, spread_correct between them
 //   spread_sweep  every task backward, from the top solutions
 //   spread_out    the work array into x
 //
@@ -47,12 +47,13 @@ struct SpreadNet {
   const uint8_t *__restrict__ blob;
   const int32_t *__restrict__ fwd_page, *__restrict__ bwd_page, *__restrict__ task_row, *__restrict__ part_ptr;
   const int32_t *__restrict__ in_pos, *__restrict__ out_pos;
-  const void *__restrict__ m, *__restrict__ m2;  // the top's maps in blocks of kSpreadTopRows rows (m2: null with one)
-  const int32_t *__restrict__ s_ptr, *__restrict__ s_col;  // S by rows (complex)
-  const void *__restrict__ s_val;
+  const void *__restrict__ m;  // the top's map in blocks of kSpreadTopRows rows
+  // what the product is corrected by, by rows: S, or (LU) U_TT and then -L_TT
+  const int32_t *__restrict__ s_ptr, *__restrict__ s_col, *__restrict__ u_ptr, *__restrict__ u_col;
+  const void *__restrict__ s_val, *__restrict__ u_val;  // u_val: null with S
   int64_t groups, count;       // groups of a warp's columns (32, or 64 with two per lane), and columns
   void *work, *xout, *partial; // xout: where the backward sweep writes (work, or an array of its layout)
-  void *r, *r2;                // the top's right-hand sides [group][top row][32 lanes], full precision; what is between two products
+  void *r, *r2, *r3;           // the top's right-hand sides [group][top row][32 lanes], full precision; the first product; U_TT times it
   bool top_out;                // the top's solutions go to xout as well (the scatter takes them from the partial array)
   const uint8_t *group_active; // [groups] 0: skipped; null: all run
   const void *b;               // the caller's right-hand sides and solutions
@@ -79,31 +80,33 @@ template <class R> struct pair2 {
 
 // What a lane holds, L: one right-hand side, or in FP32 two (each record then serves twice the
 // arithmetic, in slots as wide as FP64's). S: the factor's values; Math: a lane's
-// values in the top's product; MathS: the top's map.
+// values in the top's product; MathS: the top's map; kCorrect: the product takes one correction (real FP32
+// values round far more than it).
 template <class L> struct SpreadLane;
 template <> struct SpreadLane<double> {
   using S = double;
   using Math = double;
   using MathS = double;
   static constexpr int N = 1;
-  static constexpr bool kComplex = false;
+  static constexpr bool kComplex = false, kCorrect = true;
 };
 template <> struct SpreadLane<float> : SpreadLane<double> {
   using S = float;
+  static constexpr bool kCorrect = false;
 };
 template <> struct SpreadLane<pair2<float>> {
   using S = float;
   using Math = pair2<double>;
   using MathS = double;
   static constexpr int N = 2;
-  static constexpr bool kComplex = false;
+  static constexpr bool kComplex = false, kCorrect = false;
 };
 template <> struct SpreadLane<cplx<double>> {
   using S = cplx<double>;
   using Math = cplx<double>;
   using MathS = cplx<double>;
   static constexpr int N = 1;
-  static constexpr bool kComplex = true;
+  static constexpr bool kComplex = true, kCorrect = true;
 };
 template <> struct SpreadLane<cplx<float>> : SpreadLane<cplx<double>> {
   using S = cplx<float>;
@@ -503,8 +506,10 @@ template <class T, bool BATCH> __global__ void __launch_bounds__(256) spread_sum
   sp_stg(static_cast<M *>(net.r) + ((size_t)g * net.top + k) * 32 + lane, s);
 }
 
-// r_T -= S r2, each row in place: the residual of the first product, for its correction.
-template <class T, bool BATCH> __global__ void __launch_bounds__(256) spread_correct_kernel(const __grid_constant__ SpreadArgs a) {
+// The residual of the first product, for its correction: r_T -= S r2, or (LU) r3 = -U_TT r2 (UPPER), then
+// r_T += L_TT r3, each row in place. A warp per row and group.
+template <class T, bool BATCH, bool UPPER>
+__global__ void __launch_bounds__(256) spread_correct_kernel(const __grid_constant__ SpreadArgs a) {
   using M = typename SpreadLane<T>::Math;
   using MS = typename SpreadLane<T>::MathS;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -522,24 +527,25 @@ template <class T, bool BATCH> __global__ void __launch_bounds__(256) spread_cor
   const SpreadNet &net = *np;
   sp_ready();
   if (k >= net.top || (net.group_active && !net.group_active[g])) return;
-  M *r = static_cast<M *>(net.r) + ((size_t)g * net.top + k) * 32 + lane;
-  const M *x = static_cast<const M *>(net.r2) + (size_t)g * net.top * 32 + lane;
-  const MS *val = static_cast<const MS *>(net.s_val);
-  const int q1 = __ldg(net.s_ptr + k + 1);
-  M s = sp_ldg(r);
-  for (int q = __ldg(net.s_ptr + k); q < q1; q += 4) {
+  const int32_t *ptr = UPPER ? net.u_ptr : net.s_ptr, *col = UPPER ? net.u_col : net.s_col;
+  const MS *val = static_cast<const MS *>(UPPER ? net.u_val : net.s_val);
+  const M *x = static_cast<const M *>(UPPER || !net.u_val ? net.r2 : net.r3) + (size_t)g * net.top * 32 + lane;
+  M *to = static_cast<M *>(UPPER ? net.r3 : net.r) + ((size_t)g * net.top + k) * 32 + lane;
+  const int q1 = __ldg(ptr + k + 1);
+  M s = UPPER ? M{} : sp_ldg(to);
+  for (int q = __ldg(ptr + k); q < q1; q += 4) {
     M v[4];
     MS c[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const int at = min(q + i, q1 - 1);
-      c[i] = val[at], v[i] = sp_ldg(x + (size_t)__ldg(net.s_col + at) * 32);
+      c[i] = val[at], v[i] = sp_ldg(x + (size_t)__ldg(col + at) * 32);
     }
 #pragma unroll
     for (int i = 0; i < 4; ++i)
       if (q + i < q1) s = sp_fnma(c[i], v[i], s);
   }
-  sp_stg(r, s);
+  sp_stg(to, s);
 }
 
 // D += A B on the FP64 tensor cores: A 8 x 4 (lane: row lane / 4, column lane % 4), B 4 x 8 (row lane % 4,
@@ -578,8 +584,8 @@ template <class V> __device__ __forceinline__ V spread_top_entry(const V *m, con
 
 // The top's product on the FP64 tensor cores, 16 rows by 32 columns a warp, fragments straight from L2
 // (the map and a group's columns are read by many warps; four steps of loads in flight). PHASE 0: x_T =
-// M r_T; 1: r2 = L_TT^-1 r_T; 2: x_T = U_TT^-1 r2, a triangle's zeros passed over; 3: r2 = M r_T;
-// 4: x_T = r2 + M r_T. KS > 1: a block's KS
+// M r_T; 1: r2 = M r_T; 2, with r_T the residual: x_T = r2 + M r_T, each entry of the correction where it is
+// finite (a right-hand side that is not leaves a residual that is NaN). KS > 1: a block's KS
 // warps split the map's columns and add up in order at the end: with few groups there are too few
 // tiles to fill the SMs, and a tile's chain of steps sets the time. x_T goes to its own rows after the
 // partials (the work array's top rows stay b_T) and to the separate output array if there is one.
@@ -609,16 +615,16 @@ __global__ void __launch_bounds__(spread_top_warps<T, KS>() * 32) spread_top_ker
   sp_ready();
   if (net.group_active && !net.group_active[g]) return;  // the whole block
   const int t = net.top, row0 = ((int)block * (WARPS / KS) + warp / KS) * 16;
-  const V *r = static_cast<const V *>(PHASE == 2 ? net.r2 : net.r) + (size_t)g * t * COLS + tile * 32 + lane / 4;
-  const V *m = static_cast<const V *>(PHASE == 2 ? net.m2 : net.m) + (size_t)(row0 / kSpreadTopRows) * t * kSpreadTopRows + row0 % kSpreadTopRows + lane / 4;
+  const V *r = static_cast<const V *>(net.r) + (size_t)g * t * COLS + tile * 32 + lane / 4;
+  const V *m = static_cast<const V *>(net.m) + (size_t)(row0 / kSpreadTopRows) * t * kSpreadTopRows + row0 % kSpreadTopRows + lane / 4;
   V acc[2][4][2];
 #pragma unroll
   for (int i = 0; i < 2; ++i)
 #pragma unroll
     for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = V(0);
-  // the steps of four columns that hold entries of these rows, and this warp's share of them
-  const int first = PHASE == 2 ? row0 / 4 : 0, steps = (PHASE == 1 ? min(t, row0 + 16) + 3 : t + 3) / 4 - first;
-  const int s0 = first + (int)((int64_t)steps * (warp % KS) / KS), s1 = first + (int)((int64_t)steps * (warp % KS + 1) / KS);
+  // this warp's share of the steps of four columns
+  const int steps = (t + 3) / 4;
+  const int s0 = (int)((int64_t)steps * (warp % KS) / KS), s1 = (int)((int64_t)steps * (warp % KS + 1) / KS);
   if (row0 < t) {
 #pragma unroll 4
     for (int s = s0; s < s1; ++s) {
@@ -640,17 +646,20 @@ __global__ void __launch_bounds__(spread_top_warps<T, KS>() * 32) spread_top_ker
   auto store = [&](int row, int col, V v0, V v1) {
     if (row >= t) return;
     if (!sp_finite(v0) || !sp_finite(v1)) {
-      const V *mr = static_cast<const V *>(PHASE == 2 ? net.m2 : net.m) + (size_t)(row / kSpreadTopRows) * t * kSpreadTopRows + row % kSpreadTopRows;
-      const V *rc = static_cast<const V *>(PHASE == 2 ? net.r2 : net.r) + (size_t)g * t * COLS + tile * 32 + col;
+      const V *mr = static_cast<const V *>(net.m) + (size_t)(row / kSpreadTopRows) * t * kSpreadTopRows + row % kSpreadTopRows;
+      const V *rc = static_cast<const V *>(net.r) + (size_t)g * t * COLS + tile * 32 + col;
       if (!sp_finite(v0)) v0 = spread_top_entry(mr, rc, t, COLS);
       if (!sp_finite(v1)) v1 = spread_top_entry(mr, rc + 1, t, COLS);
     }
     V *between = r2 + (size_t)row * COLS + col;
-    if constexpr (PHASE == 1 || PHASE == 3) {
+    if constexpr (PHASE == 1) {
       sp_store2(between, v0, v1);
       return;
     }
-    if constexpr (PHASE == 4) v0 = sp_add(v0, between[0]), v1 = sp_add(v1, between[1]);
+    if constexpr (PHASE == 2) {
+      v0 = sp_finite(v0) ? sp_add(between[0], v0) : between[0];
+      v1 = sp_finite(v1) ? sp_add(between[1], v1) : between[1];
+    }
     sp_store2(xt + (size_t)row * COLS + col, v0, v1);
     if (xo) sp_store2(xo + (size_t)row * COLS + col, v0, v1);
   };
@@ -678,8 +687,8 @@ __global__ void __launch_bounds__(spread_top_warps<T, KS>() * 32) spread_top_ker
   }
 }
 
-// A top's map to make: the substitutions with its triangles (a null pointer: without that one) applied
-// to the identity, in the factor's full precision. The upper triangle's rows (pointers, entries and
+// A top's map to make: the substitutions with its triangles applied to the identity, in the factor's full
+// precision. The upper triangle's rows (pointers, entries and
 // diagonals) run from the last to the first, as they are solved. `scratch` holds [column chunk][row][32].
 template <class M> struct SpreadMap {
   int32_t t, chunks;  // chunks of 32 columns
@@ -706,8 +715,8 @@ template <class M> __global__ void __launch_bounds__(32) spread_map_kernel(const
   auto out = [&](int p, M x) {
     if (e < t) m[((size_t)(p / kSpreadTopRows) * t + e) * kSpreadTopRows + p % kSpreadTopRows] = x;
   };
-  // Row i of the arrays is row i of the map, or (`down`) row t - 1 - i.
-  auto sweep = [&](bool down, bool first, bool last, const int32_t *__restrict__ ptr, const int32_t *__restrict__ col,
+  // Row i of the arrays is row i of the map, or (upper triangle) row t - 1 - i.
+  auto sweep = [&](auto upper, const int32_t *__restrict__ ptr, const int32_t *__restrict__ col,
                    const M *__restrict__ val, const M *__restrict__ dinv) {
     const int total = __ldg(ptr + t);
     M v_next(0);
@@ -719,10 +728,10 @@ template <class M> __global__ void __launch_bounds__(32) spread_map_kernel(const
     int k = 0, end = __ldg(ptr + 1);
     M d = dinv[0];
     for (int i = 0; i < t; ++i) {
-      const int p = down ? t - 1 - i : i, end_now = end;
+      const int p = upper ? t - 1 - i : i, end_now = end;
       const M d_now = d;
       if (i + 1 < t) end = __ldg(ptr + i + 2), d = dinv[i + 1];
-      M s = first ? M(p == e ? 1 : 0) : z[(size_t)p * 32];
+      M s = upper ? z[(size_t)p * 32] : M(p == e ? 1 : 0);
       while (k < end_now) {
         if (k % 32 == 0) {
           __syncwarp();
@@ -744,11 +753,11 @@ template <class M> __global__ void __launch_bounds__(32) spread_map_kernel(const
       }
       s = s * d_now;
       z[(size_t)p * 32] = s;
-      if (last) out(p, s);
+      if (upper) out(p, s);
     }
   };
-  if (map.l_ptr) sweep(false, true, !map.u_ptr, map.l_ptr, map.l_col, map.l_val, map.l_dinv);
-  if (map.u_ptr) sweep(true, !map.l_ptr, true, map.u_ptr, map.u_col, map.u_val, map.u_dinv);
+  sweep(std::false_type(), map.l_ptr, map.l_col, map.l_val, map.l_dinv);
+  sweep(std::true_type(), map.u_ptr, map.u_col, map.u_val, map.u_dinv);
 }
 
 __device__ __forceinline__ double spread_abs(double v) { return fabs(v); }
