@@ -8,7 +8,7 @@ import pytest
 
 import oracle.oracle as orc
 from fixtures import random_square
-from ybus_b200 import FP64, GpuFactor, Pair, configs, grids, host, solve_batch_complex
+from ybus_b200 import FP64, GpuFactor, Pair, configs, grids, host
 
 pytestmark = pytest.mark.gpu
 
@@ -46,7 +46,7 @@ def worst_residual(a, xs, rhs):
 @pytest.mark.parametrize("count", [1, 64, 999, 2100])
 @pytest.mark.parametrize("decades", [0, 3])
 def test_residuals_on_grids_of_wide_reactances(gpu, decades, count):
-    """Twice the substitution's worst over the same columns (its scatter over orders of summation), and the
+    """Four times the substitution's worst over the same columns (its scatter over orders of summation), and the
     project's bar of 1e-12; plain solves and pair solves."""
     g = wide_grid(2000, 700, 11, decades)
     a = configs.bprime(g)

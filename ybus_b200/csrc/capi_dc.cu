@@ -1018,6 +1018,9 @@ extern "C" int32_t yb_dc_outage_loadings_batch(yb_dc_network *net, int64_t cases
     if (weights) w.assign(weights, weights + nl);
     cuda_check(cudaSetDevice(net->gpu->device), "cudaSetDevice");
     cudaStream_t s = net->gpu->stream;
+    // buffers of other sizes may be other buffers: whatever runs now, a graph of the old ones is gone
+    if (net->graph && (net->graph_cases != cases || net->graph_columns != S))
+      cudaGraphExecDestroy(net->graph), net->graph = nullptr;
     net->d_case_of.upload(case_of, s), net->d_plus_u.upload(pu, s), net->d_minus_u.upload(mu, s);
     net->d_plus_slot.upload(ps, s), net->d_minus_slot.upload(ms, s), net->d_branch.upload(br, s);
     net->d_invb.upload(invb, s), net->d_weight.upload(w, s);
@@ -1096,13 +1099,12 @@ extern "C" int32_t yb_dc_outage_loadings_batch(yb_dc_network *net, int64_t cases
     if (precision == YB_FP32) require(net->slack == 0, "the FP32 screening takes the slack at bus 0");
     if (lanes) {
       run();
-    } else if (precision == YB_FP64 && net->graph && net->graph_cases == cases && net->graph_columns == S) {
+    } else if (precision == YB_FP64 && net->graph) {
       // the same sizes as the captured graph: its buffers hold this batch's inputs
       cuda_check(cudaGraphLaunch(net->graph, s), "cudaGraphLaunch");
     } else {
       run();  // makes every layout and buffer the launches need, outside any capture
       if (precision == YB_FP64) {
-        if (net->graph) cudaGraphExecDestroy(net->graph), net->graph = nullptr;
         cudaGraph_t g = nullptr;
         cuda_check(cudaStreamSynchronize(s), "before capture");
         cuda_check(cudaStreamBeginCapture(s, cudaStreamCaptureModeRelaxed), "cudaStreamBeginCapture");
