@@ -280,12 +280,12 @@ extern "C" int32_t yb_solve_batch_complex(int64_t networks, yb_factor *const *fa
       cuda_check(cudaStreamSynchronize(s), "residual");
       return ratios;
     };
-    // the spread solve for the networks that admit it (its gather and scatter move whole complex128
-    // values: 16-byte alignment), the level-scheduled tiles for the others. At 16 networks of 730 to
-    // 46,293 buses with 128 right-hand sides each 0.91 against 7.5 ms, after a first pass of 35 ms that
-    // lays them out (four later passes pay for it)
+    // the spread solve for the networks that have a layout (its gather and scatter move whole complex128
+    // values: 16-byte alignment), the level-scheduled tiles for the others: those that admit none and those
+    // solved too few times yet
     std::vector<DeviceSpread *> layouts;
-    spread_for_batch(fs, precision == YB_FP64 ? 16 : 8, cnt, layouts, s);
+    const int value_bytes = precision == YB_FP64 ? 16 : 8;
+    spread_for_batch(fs, value_bytes, cnt, layouts, s);
     auto solve = [&](auto real, const std::vector<const cplx<double> *> &rhs, bool add) {
       using R = decltype(real);
       std::vector<SpreadSystem> spread;
@@ -329,6 +329,7 @@ extern "C" int32_t yb_solve_batch_complex(int64_t networks, yb_factor *const *fa
         solve(0.0f, r, true);
       }
     }
+    spread_batch_solved(fs, value_bytes, cnt, taken + 1);
     if (d_ratio) {
       const auto ratios = residual();
       int64_t off = 0;

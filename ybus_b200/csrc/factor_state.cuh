@@ -257,6 +257,7 @@ struct yb_factor {
   // spread layouts by (value bytes, groups up to; a null entry: the factor admits none) and the
   // workspaces, one per stream in use; the mutex guards both
   std::map<std::pair<int, int64_t>, std::unique_ptr<yb::DeviceSpread>> spreads;
+  std::map<std::pair<int, int64_t>, int> spread_passes;  // a complex factor's solves without the layout of their class
   std::vector<std::unique_ptr<yb::SpreadWork>> spread_work;
   uint64_t spread_solves = 0;
   std::mutex spread_mutex;

@@ -298,7 +298,17 @@ template size_t spread_partial_bytes<float>(const DeviceSpread *, int64_t);
 
 namespace {
 
-int64_t group_class(int64_t groups) {  // a layout serves the groups up to a number of three significant bits
+// A layout serves the groups up to a power of two; from 4,096 on cuts no longer differ by the load. So a
+// factor keeps 13 at most of one value's bytes, the same one for a number of right-hand sides whatever ran before.
+int64_t group_class(int64_t groups) {
+  int64_t most = 1;
+  while (most < groups && most < 4096) most *= 2;
+  return most;
+}
+// In a batch, up to a number of three significant bits: the longest task of any network sets a sweep's time, so
+// the networks' cuts have to agree (16 networks of 730 to 46,293 buses: 929 us, by powers of two 972).
+// These layouts are made only when they have paid for themselves, and kSpreadMostBatchLayouts of them.
+int64_t batch_class(int64_t groups) {
   int64_t most = groups;
   for (int64_t unit = 1; most > 8 * unit || most % unit; unit *= 2) most = (most + 2 * unit - 1) / (2 * unit) * (2 * unit);
   return most;
@@ -349,20 +359,32 @@ DeviceSpread *spread_for(yb_factor *f, int value_bytes, int64_t groups, cudaStre
   return out;
 }
 
+// Each network's class in a batch: its share of the load in groups of its own, since the cut weighs the whole
+// batch's load.
+static std::vector<std::pair<int, int64_t>> batch_keys(const std::vector<yb_factor *> &factors, int value_bytes,
+                                                       const std::vector<int64_t> &counts) {
+  double load = 0;
+  for (size_t i = 0; i < factors.size(); ++i) load += (double)factors[i]->n * (double)((counts[i] + 31) / 32);
+  std::vector<std::pair<int, int64_t>> keys;
+  for (const yb_factor *f : factors)
+    keys.push_back({value_bytes, batch_class(std::max<int64_t>(1, (int64_t)std::ceil(load / (double)f->n)))});
+  return keys;
+}
+
 void spread_for_batch(const std::vector<yb_factor *> &factors, int value_bytes, const std::vector<int64_t> &counts,
                       std::vector<DeviceSpread *> &out, cudaStream_t stream) {
   const size_t k = factors.size();
-  // each network's share of the batch in groups of its own: the cut weighs the whole batch's load
-  double load = 0;
-  for (size_t i = 0; i < k; ++i) load += (double)factors[i]->n * (double)((counts[i] + 31) / 32);
   std::vector<std::unique_ptr<SpreadLayout<host::c128>>> made(k);
-  std::vector<std::pair<int, int64_t>> keys(k);
+  const auto keys = batch_keys(factors, value_bytes, counts);
   std::vector<size_t> missing;
   std::set<std::pair<yb_factor *, int64_t>> seen;
   for (size_t i = 0; i < k; ++i) {
-    keys[i] = {value_bytes, group_class(std::max<int64_t>(1, (int64_t)std::ceil(load / (double)factors[i]->n)))};
     const std::lock_guard<std::mutex> lock(factors[i]->spread_mutex);
-    if (counts[i] > 0 && !factors[i]->spreads.count(keys[i]) && seen.insert({factors[i], keys[i].second}).second) missing.push_back(i);
+    const auto &there = factors[i]->spreads;
+    if (counts[i] > 0 && !there.count(keys[i]) && factors[i]->spread_passes[keys[i]] >= kSpreadBatchPasses &&
+        std::count_if(there.begin(), there.end(), [&](const auto &e) { return e.first.first == value_bytes; }) < kSpreadMostBatchLayouts &&
+        seen.insert({factors[i], keys[i].second}).second)
+      missing.push_back(i);
   }
   // the layouts not made yet, on the host's threads, largest networks first
   std::sort(missing.begin(), missing.end(), [&](size_t a, size_t b) { return factors[a]->n > factors[b]->n; });
@@ -397,9 +419,25 @@ void spread_for_batch(const std::vector<yb_factor *> &factors, int value_bytes, 
   }
   out.assign(k, nullptr);
   for (size_t i = 0; i < k; ++i) {
+    const yb_factor *f = factors[i];
     const std::lock_guard<std::mutex> lock(factors[i]->spread_mutex);
-    auto it = factors[i]->spreads.find(keys[i]);
-    if (it != factors[i]->spreads.end()) out[i] = it->second.get();
+    const auto it = f->spreads.find(keys[i]);
+    if (it != f->spreads.end()) {
+      out[i] = it->second.get();
+      continue;
+    }
+    int64_t distance = INT64_MAX;  // until its class has a layout: the nearest class's, if any
+    for (const auto &[key, d] : f->spreads)
+      if (d && key.first == value_bytes && std::abs(key.second - keys[i].second) < distance)
+        out[i] = d.get(), distance = std::abs(key.second - keys[i].second);
+  }
+}
+
+void spread_batch_solved(const std::vector<yb_factor *> &factors, int value_bytes, const std::vector<int64_t> &counts, int solves) {
+  const auto keys = batch_keys(factors, value_bytes, counts);
+  for (size_t i = 0; i < factors.size(); ++i) {
+    const std::lock_guard<std::mutex> lock(factors[i]->spread_mutex);
+    if (counts[i] > 0 && !factors[i]->spreads.count(keys[i])) factors[i]->spread_passes[keys[i]] += solves;
   }
 }
 

@@ -58,10 +58,20 @@ template <class T>
 void spread_sweeps(yb_factor *f, DeviceSpread *d, T *work, T *xout, uint8_t *partial, int64_t groups, const uint8_t *group_active,
                    cudaStream_t stream);
 
-// The spread layouts of a batch of complex factors with these counts of right-hand sides (null: none), the
-// missing ones made on several threads of the host.
+// A complex factor's solves that go without a layout before one is made: making it costs about what four take
+// (16 networks of 730 to 46,293 buses with 128 right-hand sides each: 31 ms, against 7.5 ms a solve by tiles and
+// 0.93 ms with it), so a factor that is solved once or twice never pays for it, and one that is solved often
+// twice what the better choice would have cost.
+constexpr int kSpreadBatchPasses = 4;
+constexpr int kSpreadMostBatchLayouts = 8;  // a complex factor keeps of one precision; further classes take the nearest
+
+// The spread layouts of a batch of complex factors with these counts of right-hand sides: of the class the batch
+// asks for, made on several threads of the host once the factor's solves in that class have paid for it;
+// until then another class's, or null.
 void spread_for_batch(const std::vector<yb_factor *> &factors, int value_bytes, const std::vector<int64_t> &counts,
                       std::vector<DeviceSpread *> &out, cudaStream_t stream);
+// Counts a batch's solves of each factor.
+void spread_batch_solved(const std::vector<yb_factor *> &factors, int value_bytes, const std::vector<int64_t> &counts, int solves);
 
 // One factor's part of a complex batch: right-hand sides and solutions complex128, column-major.
 struct SpreadSystem {
