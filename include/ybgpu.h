@@ -88,6 +88,10 @@ int32_t yb_factor_plan_info(const yb_factor *f, int32_t *fwd_levels, int32_t *bw
  * of two; threads a multiple of 32 up to 512; resident blocks per SM 1..8). */
 int32_t yb_factor_set_tile(yb_factor *f, int32_t precision, int32_t tile_width, int32_t threads,
                            int32_t blocks_per_sm);
+/* No ybus counterpart: the largest work array that one run of the spread solve fills (2 GiB until set):
+ * plain, refined and batched solves of more right-hand sides take several runs, and a factor of whose
+ * right-hand sides 32 do not fit takes the other solves. */
+int32_t yb_gpu_set_work_bytes(yb_gpu *gpu, int64_t bytes);
 /* No ybus counterpart: which tile solve runs for a precision: 0 automatic (the spread solve when the
  * factor admits it and no shape or threshold of the solves below was set for the precision; else the
  * lane solve for solves of at least the lane threshold's right-hand sides when the factor admits it; else the

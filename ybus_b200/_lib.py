@@ -87,6 +87,7 @@ SIGNATURES: dict[str, tuple] = {
     "yb_factor_set_tail_level": (i32, [vp, i32, i32]),
     "yb_factor_set_domain": (i32, [vp, i32, i32, i32, i32, i32]),
     "yb_factor_autotune": (i32, [vp, i32, i64, vp, P_dbl]),
+    "yb_gpu_set_work_bytes": (i32, [vp, i64]),
     "yb_factor_spread_info": (i32, [vp, i32, i64, vp]),
     "yb_factor_lane_info": (i32, [vp, i32, vp]),
     "yb_factor_set_lane_rhs_per_lane": (i32, [vp, i32, i32]),

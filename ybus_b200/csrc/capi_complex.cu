@@ -293,16 +293,23 @@ extern "C" int32_t yb_solve_batch_complex(int64_t networks, yb_factor *const *fa
       std::vector<const cplx<double> *> rest_b;
       std::vector<int64_t> rest_ldb, rest_cnt;
       std::vector<cplx<double> *> rest_x;
+      auto by_tiles = [&](const SpreadSystem &sys) {
+        rest.push_back(sys.factor), rest_b.push_back(sys.b), rest_ldb.push_back(sys.factor->n);
+        rest_cnt.push_back(sys.count), rest_x.push_back(sys.x);
+      };
       for (int64_t i = 0; i < networks; ++i) {
         if (cnt[i] == 0) continue;
-        if (layouts[i] && ((uintptr_t)rhs[i] | (uintptr_t)x[i]) % 16 == 0) {
-          spread.push_back({fs[i], layouts[i], rhs[i], x[i], cnt[i]});
-        } else {
-          rest.push_back(fs[i]), rest_b.push_back(rhs[i]), rest_ldb.push_back(fs[i]->n);
-          rest_cnt.push_back(cnt[i]), rest_x.push_back(x[i]);
-        }
+        const SpreadSystem sys{fs[i], layouts[i], rhs[i], x[i], cnt[i]};
+        if (layouts[i] && ((uintptr_t)rhs[i] | (uintptr_t)x[i]) % 16 == 0 && spread_batch_fits<R>(sys))
+          spread.push_back(sys);
+        else
+          by_tiles(sys);
       }
-      spread_batch<R>(spread, add, w.spread, s);
+      try {
+        spread_batch<R>(spread, add, w.spread, s);
+      } catch (const OutOfMemory &) {
+        for (const SpreadSystem &sys : spread) by_tiles(sys);
+      }
       if (rest.empty()) return;
       if constexpr (std::is_same_v<R, double>)
         launch_batch<double>(rest, rest_b, rest_ldb, rest_x, rest_cnt, add, s, w.nets, w.items, w.scratch128, gpu->sm_count);

@@ -1077,7 +1077,7 @@ extern "C" int32_t yb_dc_outage_loadings_batch(yb_dc_network *net, int64_t cases
           outage_reduce_kernel<<<(unsigned)((count + 255) / 256), 256, 0, s>>>(a, net->d_row.get(), net->d_value.get(), net->d_bad.get());
           cuda_check(cudaGetLastError(), "outage_reduce_kernel launch");
         });
-        if (!solved) throw host::Error(host::kInternal, "the screening's solve did not run");
+        if (!solved) launch_domain_fp64(f, S, io, s);
       } else if (precision == YB_FP64) {
         launch_domain_fp64(f, S, io, s);
       } else {

@@ -338,6 +338,15 @@ extern "C" int32_t yb_factor_plan_info(const yb_factor *f, int32_t *fwd_levels, 
   });
 }
 
+extern "C" int32_t yb_gpu_set_work_bytes(yb_gpu *gpu, int64_t bytes) {
+  return guard([&] {
+    require(gpu != nullptr, "null GPU");
+    require(bytes >= 0, "negative bytes");
+    gpu->work_bytes = bytes;
+    return YB_OK;
+  });
+}
+
 extern "C" int32_t yb_factor_set_tile(yb_factor *f, int32_t precision, int32_t tile_width, int32_t threads,
                                       int32_t blocks_per_sm) {
   return guard([&] {
@@ -1580,7 +1589,7 @@ void launch_refined(yb_factor *f, const RefineSweeps &sweeps, const double *b, i
   const int64_t n = f->n;
   const size_t group_vals = (size_t)n * 32;
   const int64_t groups_all = (count + 31) / 32;
-  const int64_t per_launch = std::max<int64_t>(1, std::min<int64_t>(groups_all, (int64_t)(kLaneWorkBytes / (group_vals * sizeof(T)))));
+  const int64_t per_launch = std::max<int64_t>(1, std::min<int64_t>(groups_all, std::min<int64_t>((int64_t)kLaneWorkBytes, f->gpu->work_bytes) / (int64_t)(group_vals * sizeof(T))));
   const int64_t cols_most = per_launch * 32;
   SpreadBytes bytes;
   bytes.work = ((size_t)per_launch * group_vals + 2 * kSpreadPad * 32) * sizeof(T);
@@ -1705,14 +1714,17 @@ extern "C" int32_t yb_solve_many_refined_device(yb_factor *f, const double *d_rh
     const auto rb = bytes(d_rhs, ldb), rx = bytes(d_out, ldx);
     if (t32.kind == kTileAuto && !t32.shaped && !t32.refine_shaped && (rb.second <= rx.first || rx.second <= rb.first)) {
       if (DeviceSpread *d = spread_for(f, (int)sizeof(float), (count + 31) / 32, s, f->a_attached)) {
-        residual_matrix(f, d, d->host_out_pos, s);
-        const RefineSweeps sweeps{
-            d->in_pos, d->out_pos, d, [&](int64_t groups) { return spread_partial_bytes<float>(d, groups); },
-            [&](float *work, float *out, uint8_t *partial, int64_t groups, const uint8_t *active) {
-              spread_sweeps<float>(f, d, work, out, partial, groups, active, s);
-            }};
-        launch_refined(f, sweeps, d_rhs, ldb, d_out, ldx, count, max_steps, tolerance, d_ratio, d_steps, s);
-        return YB_OK;
+        try {
+          residual_matrix(f, d, d->host_out_pos, s);
+          const RefineSweeps sweeps{
+              d->in_pos, d->out_pos, d, [&](int64_t groups) { return spread_partial_bytes<float>(d, groups); },
+              [&](float *work, float *out, uint8_t *partial, int64_t groups, const uint8_t *active) {
+                spread_sweeps<float>(f, d, work, out, partial, groups, active, s);
+              }};
+          launch_refined(f, sweeps, d_rhs, ldb, d_out, ldx, count, max_steps, tolerance, d_ratio, d_steps, s);
+          return YB_OK;
+        } catch (const OutOfMemory &) {  // nothing is launched yet: the domain solve needs less
+        }
       }
     }
     if (t32.kind == kTileLane ||

@@ -4,6 +4,7 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <string>
 #include <utility>
 #include <vector>
@@ -17,6 +18,11 @@ inline void cuda_check(cudaError_t err, const char *what) {
   if (err != cudaSuccess)
     throw host::Error(host::kCuda, std::string(what) + ": " + cudaGetErrorString(err));
 }
+
+// A device allocation that did not fit: a solve that needs less may still run.
+struct OutOfMemory : host::Error {
+  using host::Error::Error;
+};
 
 // Owns a device allocation of `count` elements of T.
 template <class T> class DeviceArray {
@@ -38,12 +44,25 @@ template <class T> class DeviceArray {
   void resize(size_t count) {
     if (count == count_) return;
     release();
-    if (count) cuda_check(cudaMalloc(&ptr_, count * sizeof(T)), "cudaMalloc");
+    if (count) {
+      const cudaError_t e = cudaMalloc(&ptr_, count * sizeof(T));
+      if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        ptr_ = nullptr;
+        throw OutOfMemory(host::kCuda, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+      }
+      cuda_check(e, "cudaMalloc");
+    }
     count_ = count;
   }
   // Grows (never shrinks) to at least `count` elements; the contents are not kept.
   void reserve(size_t count) {
     if (count > count_) resize(count);
+  }
+  // As reserve, to twice the size where that is at most 256 MB more, so that sizes that rise little by
+  // little take few allocations.
+  void grow(size_t count) {
+    if (count > count_) resize(std::max(count, count_ + std::min<size_t>(count_, (size_t(256) << 20) / sizeof(T))));
   }
   void upload(const std::vector<T> &host, cudaStream_t stream) {
     resize(host.size());

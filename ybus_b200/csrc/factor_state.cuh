@@ -33,6 +33,7 @@ struct yb_gpu {
   int64_t smem_optin = 0;       // largest dynamic shared memory a block may opt into
   int64_t smem_per_sm = 0;
   std::string name;
+  std::atomic<int64_t> work_bytes{int64_t(2) << 30};  // the largest work array one run of the spread solve fills
   std::shared_ptr<void> zwork;  // the complex batch's device workspace (capi_complex.cu), kept between calls
   std::mutex zmutex;            // held by the call that uses it
 };
@@ -184,9 +185,9 @@ struct SpreadWork {
     return work.size() >= b.work && partial.size() >= b.partial && corrections.size() >= b.corrections &&
            iterate.size() >= b.iterate && state.size() >= b.state;
   }
-  void reserve(const SpreadBytes &b) {
-    work.reserve(b.work), partial.reserve(b.partial), corrections.reserve(b.corrections);
-    iterate.reserve(b.iterate), state.reserve(b.state);
+  void grow(const SpreadBytes &b) {
+    work.grow(b.work), partial.grow(b.partial), corrections.grow(b.corrections);
+    iterate.grow(b.iterate), state.grow(b.state);
   }
   SpreadWork() = default;
   SpreadWork(const SpreadWork &) = delete;

@@ -5,6 +5,7 @@
 #include <cmath>
 #include <cstring>
 #include <functional>
+#include <optional>
 #include <set>
 #include <system_error>
 #include <thread>
@@ -20,7 +21,6 @@ namespace {
 // The largest condition (a bound of the Schur complement's norm, times its map's) with which the top is
 // taken densely: its correction then leaves 1e-7 of the map's rounding, and FP32 values round more than the map.
 constexpr double kSpreadTopCondition = 1e9;
-constexpr size_t kSpreadWorkBytes = size_t(2) << 30;  // the largest work array one run of launches fills
 // FP32 takes two right-hand sides a lane from this many on (below, more warps are worth more than
 // fewer instructions; 10,000-bus B': 127 against 147 us at 999, 375 against 400 us at 4,096).
 constexpr int64_t kSpreadPairCount = 2048;
@@ -353,7 +353,12 @@ DeviceSpread *spread_for(yb_factor *f, int value_bytes, int64_t groups, cudaStre
     return near == f->spreads.end() ? nullptr : near->second.get();
   }
   const auto lay = try_layout<double>(f, value_bytes, key.second);
-  auto d = std::move(make_spreads<double>({lay.get()}, value_bytes, f->gpu, stream)[0]);
+  std::unique_ptr<DeviceSpread> d;
+  try {
+    d = std::move(make_spreads<double>({lay.get()}, value_bytes, f->gpu, stream)[0]);
+  } catch (const OutOfMemory &) {
+    return nullptr;  // this time
+  }
   auto *out = d.get();
   f->spreads.emplace(key, std::move(d));
   return out;
@@ -411,8 +416,12 @@ void spread_for_batch(const std::vector<yb_factor *> &factors, int value_bytes, 
   if (!missing.empty()) {
     std::vector<const SpreadLayout<host::c128> *> lays;
     for (size_t i : missing) lays.push_back(made[i].get());
-    auto d = make_spreads<host::c128>(lays, value_bytes, factors[0]->gpu, stream);
-    for (size_t m = 0; m < missing.size(); ++m) {
+    std::vector<std::unique_ptr<DeviceSpread>> d;
+    try {
+      d = make_spreads<host::c128>(lays, value_bytes, factors[0]->gpu, stream);
+    } catch (const OutOfMemory &) {  // none this time
+    }
+    for (size_t m = 0; m < d.size(); ++m) {
       const std::lock_guard<std::mutex> lock(factors[missing[m]]->spread_mutex);
       factors[missing[m]]->spreads.emplace(keys[missing[m]], std::move(d[m]));
     }
@@ -495,7 +504,7 @@ WorkLease::WorkLease(yb_factor *f, const SpreadBytes &bytes, cudaStream_t stream
       if (i->capture == id && i->stream == stream && i->holds(bytes)) w_ = i.get();
     if (w_) return;
     auto own = std::make_unique<SpreadWork>();
-    own->reserve(bytes);
+    own->grow(bytes);
     own->stream = stream, own->capture = id;
     own->released = std::make_shared<std::atomic<bool>>(false);
     keep_while(graph, own->released);
@@ -524,7 +533,7 @@ WorkLease::WorkLease(yb_factor *f, const SpreadBytes &bytes, cudaStream_t stream
   cuda_check(cudaStreamWaitEvent(stream, w_->done, 0), "cudaStreamWaitEvent");
   w_->stream = stream;
   w_->used = ++f->spread_solves;
-  w_->reserve(bytes);  // a larger array: the device is idle past the old one's free
+  w_->grow(bytes);  // a larger array: the device is idle past the old one's free
 }
 
 WorkLease::~WorkLease() {
@@ -539,14 +548,18 @@ bool solve_lanes(yb_factor *f, DeviceSpread *d, const double *b, int64_t ldb, do
   constexpr int64_t COLS = 32 * SpreadLane<L>::N;  // columns of a group
   const int64_t n = f->n, groups_all = (count + COLS - 1) / COLS;
   const size_t group_bytes = (size_t)n * 32 * sizeof(L), pad_bytes = 2 * kSpreadPad * 32 * sizeof(L);
-  const int64_t per_run = std::max<int64_t>(1, std::min<int64_t>(groups_all, (int64_t)(kSpreadWorkBytes / group_bytes)));
-  // small solves keep room for 1,536 right-hand sides (64 on factors of large order), so that any of
-  // them can be captured once one has run
-  const int64_t room = std::max<int64_t>(per_run, ((n <= 12800 ? 1536 : 64) + COLS - 1) / COLS);
+  const int64_t per_run = std::min<int64_t>(groups_all, f->gpu->work_bytes / (int64_t)group_bytes);
+  if (per_run < 1) return false;
   SpreadBytes bytes;
-  bytes.work = (size_t)(capturing(stream) ? per_run : room) * group_bytes + pad_bytes;
-  bytes.partial = partial_bytes_of<L>(d, capturing(stream) ? per_run : room);
-  const WorkLease w(f, bytes, stream);
+  bytes.work = (size_t)per_run * group_bytes + pad_bytes;
+  bytes.partial = partial_bytes_of<L>(d, per_run);
+  std::optional<WorkLease> lease;
+  try {
+    lease.emplace(f, bytes, stream);
+  } catch (const OutOfMemory &) {
+    return false;
+  }
+  const WorkLease &w = *lease;
   L *work = reinterpret_cast<L *>(w->work.get()) + kSpreadPad * 32;
   for (int64_t g0 = 0; g0 < groups_all; g0 += per_run) {
     const int64_t groups = std::min(per_run, groups_all - g0);
@@ -589,26 +602,23 @@ bool spread_solve_lanes(yb_factor *f, const double *b, int64_t ldb, int64_t coun
 template bool spread_solve<double>(yb_factor *, const double *, int64_t, double *, int64_t, int64_t, cudaStream_t);
 template bool spread_solve<float>(yb_factor *, const double *, int64_t, double *, int64_t, int64_t, cudaStream_t);
 
-template <class R>
-void spread_batch(const std::vector<SpreadSystem> &systems, bool add, SpreadBatchWork &w, cudaStream_t stream) {
+namespace {
+
+// One run of launches over what fits the batch's work arrays.
+template <class R> void batch_run(const std::vector<SpreadSystem> &systems, bool add, SpreadBatchWork &w, cudaStream_t stream) {
   using T = cplx<R>;
   const size_t k = systems.size();
-  if (k == 0) return;
   const yb_gpu *gpu = systems[0].factor->gpu;
   std::vector<SpreadNet> nets(k);
-  size_t work_values = 0, part_bytes = 0;
   int64_t top_total = 0;
   int32_t slots = 0;
   int64_t most_groups = 1;
   for (const SpreadSystem &sys : systems) {
     const int64_t groups = (sys.count + 31) / 32;
-    work_values += (size_t)groups * sys.layout->n * 32 + 2 * kSpreadPad * 32;
-    part_bytes += partial_bytes_of<T>(sys.layout, groups);
     top_total += groups * top_tiles(sys.layout);
     slots = std::max(slots, sys.layout->slots);
     most_groups = std::max(most_groups, groups);
   }
-  w.work.reserve(work_values * sizeof(T)), w.partial.reserve(part_bytes);
   const int split = split_top<T>(top_total, gpu);
   const int warps = sweep_warps<T>(slots, most_groups, gpu);
   T *work = reinterpret_cast<T *>(w.work.get());
@@ -689,6 +699,44 @@ void spread_batch(const std::vector<SpreadSystem> &systems, bool add, SpreadBatc
     launch(spread_out_kernel<T, true, true>, (unsigned)n_io, kSpreadIoWarps * 32, 0, stream, true, a);
   else
     launch(spread_out_kernel<T, true, false>, (unsigned)n_io, kSpreadIoWarps * 32, 0, stream, true, a);
+}
+
+template <class T> size_t batch_work_bytes(const DeviceSpread *d, int64_t groups) {
+  return ((size_t)groups * d->n * 32 + 2 * kSpreadPad * 32) * sizeof(T);
+}
+
+}  // namespace
+
+template <class R> bool spread_batch_fits(const SpreadSystem &sys) {
+  return (int64_t)batch_work_bytes<cplx<R>>(sys.layout, 1) <= sys.factor->gpu->work_bytes;
+}
+template bool spread_batch_fits<double>(const SpreadSystem &);
+template bool spread_batch_fits<float>(const SpreadSystem &);
+
+template <class R>
+void spread_batch(const std::vector<SpreadSystem> &systems, bool add, SpreadBatchWork &w, cudaStream_t stream) {
+  using T = cplx<R>;
+  if (systems.empty()) return;
+  const size_t limit = (size_t)systems[0].factor->gpu->work_bytes;
+  // runs of as many groups as the work array holds, a network after the other
+  std::vector<std::vector<SpreadSystem>> runs(1);
+  size_t used = 0, work_most = 0, part = 0, part_most = 0;
+  for (const SpreadSystem &sys : systems) {
+    const size_t pad = batch_work_bytes<T>(sys.layout, 0), group = batch_work_bytes<T>(sys.layout, 1) - pad;
+    for (int64_t g = 0, groups = (sys.count + 31) / 32; g < groups;) {
+      if (used + pad + group > limit && used > 0) runs.emplace_back(), used = part = 0;
+      const int64_t some = std::min<int64_t>(groups - g, std::max<int64_t>(1, ((int64_t)limit - (int64_t)(used + pad)) / (int64_t)group));
+      SpreadSystem piece = sys;
+      piece.b += g * 32 * sys.layout->n, piece.x += g * 32 * sys.layout->n;
+      piece.count = std::min<int64_t>(sys.count - g * 32, some * 32);
+      runs.back().push_back(piece);
+      used += pad + (size_t)some * group, part += partial_bytes_of<T>(sys.layout, some);
+      work_most = std::max(work_most, used), part_most = std::max(part_most, part);
+      g += some;
+    }
+  }
+  w.work.grow(work_most), w.partial.grow(part_most);  // before the first launch: the tiles can still take its place
+  for (const auto &run : runs) batch_run<R>(run, add, w, stream);
 }
 template void spread_batch<double>(const std::vector<SpreadSystem> &, bool, SpreadBatchWork &, cudaStream_t);
 template void spread_batch<float>(const std::vector<SpreadSystem> &, bool, SpreadBatchWork &, cudaStream_t);

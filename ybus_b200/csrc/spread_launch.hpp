@@ -19,9 +19,9 @@ constexpr int32_t kSpreadAutoSlots = 64, kSpreadAutoSlotsComplex = 96;
 // is, of those that hold the refined solve's copy of the matrix attached as number `matrix` (-1: of all).
 DeviceSpread *spread_for(yb_factor *f, int value_bytes, int64_t groups, cudaStream_t stream, int64_t matrix = -1);
 
-// Solves `count` right-hand sides (device arrays, column-major) in T (double or float); false, with
-// nothing done, where the factor admits no spread layout, or under stream capture where it has none
-// or too small a workspace yet.
+// Solves `count` right-hand sides (device arrays, column-major) in T (double or float), in runs of the GPU's
+// work limit; false, with nothing done, where the factor admits no spread layout (or has none yet under
+// stream capture), where the limit is below a group's work array, and where the memory is not there.
 template <class T>
 bool spread_solve(yb_factor *f, const double *b, int64_t ldb, double *x, int64_t ldx, int64_t count, cudaStream_t stream);
 
@@ -82,8 +82,12 @@ struct SpreadSystem {
   int64_t count;
 };
 
-// Solves every system's right-hand sides in complex values of R (double or float) in one run of
-// launches, into x or (add) onto it.
+// Whether the GPU's work limit holds a group of a system's right-hand sides in complex values of R.
+template <class R> bool spread_batch_fits(const SpreadSystem &system);
+
+// Solves every system's right-hand sides in complex values of R (double or float), into x or (add) onto it,
+// in as many runs of launches as the GPU's work limit asks for. Throws OutOfMemory, with nothing done, where
+// the work arrays cannot be had.
 template <class R> void spread_batch(const std::vector<SpreadSystem> &systems, bool add, SpreadBatchWork &work, cudaStream_t stream);
 
 }  // namespace yb

@@ -86,6 +86,10 @@ class Gpu:
         _check(lib().yb_gpu_properties(self._h, C.byref(sm), C.byref(major), C.byref(minor), C.byref(l2)))
         return {"sm_count": sm.value, "cc": (major.value, minor.value), "l2_bytes": l2.value}
 
+    def set_work_bytes(self, nbytes: int) -> None:
+        """The largest work array that one run of the spread solve fills (2 GiB until set)."""
+        _check(lib().yb_gpu_set_work_bytes(self._h, int(nbytes)))
+
     def synchronize(self, stream: int | None = None) -> None:
         _check(lib().yb_gpu_synchronize(self._h, stream))
 
