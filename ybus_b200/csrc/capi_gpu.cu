@@ -361,7 +361,7 @@ extern "C" int32_t yb_factor_set_tile(yb_factor *f, int32_t precision, int32_t t
     t.width = tile_width;
     t.threads = threads;
     t.blocks_per_sm = blocks_per_sm;
-    t.shaped = true;
+    t.shape();
     return YB_OK;
   });
 }
@@ -371,7 +371,8 @@ extern "C" int32_t yb_factor_set_tile_kind(yb_factor *f, int32_t precision, int3
     require(f != nullptr, "null factor");
     require(precision == YB_FP64 || precision == YB_FP32, "unknown precision");
     require(kind >= kTileAuto && kind <= kTileLane, "unknown tile kind");
-    (precision == YB_FP64 ? f->tile64 : f->tile32).kind = kind;
+    TileConfig &t = precision == YB_FP64 ? f->tile64 : f->tile32;
+    t.kind = kind, t.spread_first = false;
     return YB_OK;
   });
 }
@@ -388,7 +389,7 @@ extern "C" int32_t yb_factor_set_stream(yb_factor *f, int32_t precision, int32_t
     require(narrow_rows >= 0, "narrow rows must not be negative");
     TileConfig &t = precision == YB_FP64 ? f->tile64 : f->tile32;
     t.stream_warps = warps, t.ring = ring, t.page_bytes = page_bytes, t.narrow_rows = narrow_rows;
-    t.shaped = true;
+    t.shape();
     return YB_OK;
   });
 }
@@ -399,7 +400,7 @@ extern "C" int32_t yb_factor_set_tail_level(yb_factor *f, int32_t precision, int
     require(precision == YB_FP64 || precision == YB_FP32, "unknown precision");
     require(tail_level >= -1, "the tail level is -1 (chosen), 0 (none) or a forward level");
     TileConfig &t = precision == YB_FP64 ? f->tile64 : f->tile32;
-    t.tail_level = tail_level, t.shaped = true;
+    t.tail_level = tail_level, t.shape();
     return YB_OK;
   });
 }
@@ -960,7 +961,7 @@ void solve_device(yb_factor *f, const double *b, int64_t ldb, double *x, int64_t
   if (count <= 0 || f->n == 0) return;
   auto run = [&](auto zero, const TileConfig &configured, auto &fwd, auto &bwd, auto &scratch, auto &cache) {
     using T = decltype(zero);
-    if (configured.kind == kTileAuto && !configured.shaped && spread_solve<T>(f, b, ldb, x, ldx, count, stream)) return;
+    if (configured.takes_spread() && spread_solve<T>(f, b, ldb, x, ldx, count, stream)) return;
     if (configured.kind == kTileLane || (configured.kind == kTileAuto && count >= lane_threshold<T>(f, configured))) {
       DeviceLane *d = lane_pick<T>(f, lane_shape(f, configured, count), configured.lane_rpl, stream);
       if (d && (configured.kind == kTileLane || d->slots <= kLaneAutoSlots)) {
@@ -1041,7 +1042,7 @@ __global__ void __launch_bounds__(256) pair_update_kernel(const int32_t *__restr
 }
 
 bool admits_spread_fp64(yb_factor *f, int64_t count, cudaStream_t stream) {
-  return count > 0 && f->n > 0 && f->tile64.kind == kTileAuto && !f->tile64.shaped && !f->single &&
+  return count > 0 && f->n > 0 && f->tile64.takes_spread() && !f->single &&
          spread_for(f, (int)sizeof(double), (count + 31) / 32, stream);
 }
 bool auto_spread_fp64(yb_factor *f, const double *b, int64_t ldb, double *x, int64_t ldx, int64_t count, cudaStream_t stream) {
@@ -1356,7 +1357,7 @@ extern "C" int32_t yb_factor_set_domain(yb_factor *f, int32_t precision, int32_t
     require(cut >= -1, "the cut is -1 (chosen) or a forward level");
     TileConfig &t = precision == YB_FP64 ? f->tile64 : f->tile32;
     t.domain_warps = warps, t.domain_ring = ring, t.domain_page = page_bytes, t.domain_cut = cut;
-    t.shaped = true;
+    t.shape();
     return YB_OK;
   });
 }
@@ -1411,7 +1412,7 @@ extern "C" int32_t yb_factor_spread_info(yb_factor *f, int32_t precision, int64_
     cuda_check(cudaSetDevice(f->gpu->device), "cudaSetDevice");
     const TileConfig &t = precision == YB_FP64 ? f->tile64 : f->tile32;
     DeviceSpread *d = nullptr;
-    if (t.kind == kTileAuto && !t.shaped && !f->single && f->n > 0)
+    if (t.takes_spread() && !f->single && f->n > 0)
       d = spread_for(f, precision == YB_FP64 ? 8 : 4, (count + 31) / 32, f->gpu->stream);
     if (!d) throw host::Error(host::kInvalidArgument, "the solve this precision runs is not the spread solve");
     const int64_t v[6] = {d->tasks, d->domains, d->top, d->slots, d->partials, d->blob_bytes};
@@ -1428,7 +1429,7 @@ extern "C" int32_t yb_factor_set_lane(yb_factor *f, int32_t precision, int32_t w
     require(page_bytes == 0 || (page_bytes >= 256 && page_bytes <= 16384 && page_bytes % 16 == 0),
             "pages of 256 to 16384 bytes, a multiple of 16, or 0 for the automatic choice");
     TileConfig &t = precision == YB_FP64 ? f->tile64 : f->tile32;
-    t.lane_warps = warps, t.lane_page = page_bytes, t.lane_warps_auto = false, t.shaped = true;
+    t.lane_warps = warps, t.lane_page = page_bytes, t.lane_warps_auto = false, t.shape();
     return YB_OK;
   });
 }
@@ -1439,7 +1440,7 @@ extern "C" int32_t yb_factor_set_lane_rhs_per_lane(yb_factor *f, int32_t precisi
     require(precision == YB_FP64 || precision == YB_FP32, "unknown precision");
     require(rhs_per_lane == 1 || rhs_per_lane == 2, "1 or 2 right-hand sides per lane");
     TileConfig &t = precision == YB_FP64 ? f->tile64 : f->tile32;
-    t.lane_rpl = rhs_per_lane, t.shaped = true;
+    t.lane_rpl = rhs_per_lane, t.shape();
     return YB_OK;
   });
 }
@@ -1450,7 +1451,7 @@ extern "C" int32_t yb_factor_set_lane_min_count(yb_factor *f, int32_t precision,
     require(precision == YB_FP64 || precision == YB_FP32, "unknown precision");
     require(min_count >= -1, "a count, or -1 for the automatic threshold");
     TileConfig &t = precision == YB_FP64 ? f->tile64 : f->tile32;
-    t.lane_min_count = min_count, t.shaped = true;
+    t.lane_min_count = min_count, t.shape();
     return YB_OK;
   });
 }
@@ -1712,7 +1713,7 @@ extern "C" int32_t yb_solve_many_refined_device(yb_factor *f, const double *d_rh
     // of a factor 8 against 347 ms.
     const auto bytes = [&](const double *p, int64_t ld) { return std::make_pair((uintptr_t)p, (uintptr_t)(p + (count - 1) * ld + f->n)); };
     const auto rb = bytes(d_rhs, ldb), rx = bytes(d_out, ldx);
-    if (t32.kind == kTileAuto && !t32.shaped && !t32.refine_shaped && (rb.second <= rx.first || rx.second <= rb.first)) {
+    if (t32.takes_spread() && !t32.refine_shaped && (rb.second <= rx.first || rx.second <= rb.first)) {
       if (DeviceSpread *d = spread_for(f, (int)sizeof(float), (count + 31) / 32, s, f->a_attached)) {
         try {
           residual_matrix(f, d, d->host_out_pos, s);
@@ -1779,14 +1780,16 @@ extern "C" int32_t yb_factor_autotune(yb_factor *f, int32_t precision, int64_t c
     autotune_fill_kernel<<<(unsigned)((n * count + 255) / 256), 256, 0, s>>>(b.get(), n * count);
     cuda_check(cudaGetLastError(), "autotune_fill_kernel launch");
     TileConfig &t = precision == YB_FP64 ? f->tile64 : f->tile32;
-    const TileConfig saved = t;
+    TileConfig saved = t;
+    const bool with_spread = saved.takes_spread();  // no shape was set: the spread solve is in the choice
+    saved.spread_first = false;
     TileConfig best = saved;
-    double best_time = INFINITY;
+    double best_time = INFINITY, spread_time = INFINITY;
     cudaEvent_t e0, e1;
     cuda_check(cudaEventCreate(&e0), "cudaEventCreate");
     cuda_check(cudaEventCreate(&e1), "cudaEventCreate");
-    // times one configuration (a warm-up, then the mean of three solves) and keeps the fastest
-    auto time_config = [&](const TileConfig &run) {
+    // times one configuration: a warm-up, then the mean of three solves
+    auto time_of = [&](const TileConfig &run) {
       t = run;
       solve_device(f, b.get(), n, x.get(), n, count, precision, s);
       cuda_check(cudaEventRecord(e0, s), "cudaEventRecord");
@@ -1795,8 +1798,18 @@ extern "C" int32_t yb_factor_autotune(yb_factor *f, int32_t precision, int64_t c
       cuda_check(cudaEventSynchronize(e1), "cudaEventSynchronize");
       float ms = 0;
       cuda_check(cudaEventElapsedTime(&ms, e0, e1), "cudaEventElapsedTime");
-      if (ms / 3 < best_time) best_time = ms / 3, best = run;
+      return (double)ms / 3;
     };
+    auto time_config = [&](const TileConfig &run) {  // and keeps the fastest
+      const double ms = time_of(run);
+      if (ms < best_time) best_time = ms, best = run;
+    };
+    if (with_spread && !f->single && n > 0 &&
+        spread_for(f, precision == YB_FP64 ? (int)sizeof(double) : (int)sizeof(float), (count + 31) / 32, s)) {
+      TileConfig run = saved;
+      run.spread_first = true;
+      spread_time = time_of(run);
+    }
     const int warps_list[] = {8, 12, 16}, page_list[] = {1536, 2048}, ring_list[] = {2, 3};
     for (int warps : warps_list)
       for (int page : page_list)
@@ -1845,6 +1858,7 @@ extern "C" int32_t yb_factor_autotune(yb_factor *f, int32_t precision, int64_t c
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     t = std::isfinite(best_time) ? best : saved;
+    t.spread_first = with_spread && spread_time <= best_time;
     if (config) {
       if (t.kind == kTileGlobal) {
         config[0] = t.kind, config[1] = t.width, config[2] = t.threads / 32, config[3] = t.blocks_per_sm, config[4] = 0;
@@ -1856,7 +1870,7 @@ extern "C" int32_t yb_factor_autotune(yb_factor *f, int32_t precision, int64_t c
         config[4] = t.domain_page;
       }
     }
-    if (best_ms) *best_ms = best_time;
+    if (best_ms) *best_ms = std::min(best_time, spread_time);
     return YB_OK;
   });
 }

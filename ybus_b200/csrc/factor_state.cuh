@@ -107,6 +107,10 @@ struct TileConfig {
   // a caller set a shape or a threshold of the solves below: the automatic choice is then among them,
   // as it is for a factor that admits no spread layout
   bool shaped = false;
+  // the autotuner left the shapes below as it found them fastest, and the spread solve faster still
+  bool spread_first = false;
+  bool takes_spread() const { return spread_first || (kind == kTileAuto && !shaped); }
+  void shape() { shaped = true, spread_first = false; }
   // the streamed solve's shape: warps per block, pages in flight per warp, page bytes, and the
   // row count under which a level goes to warp 0 (0: twice the rows of a slice)
   int stream_warps = 8, ring = 4, page_bytes = 2048, narrow_rows = 0;

@@ -299,7 +299,8 @@ class GpuFactor:
         return {"gather_ms": g.value, "solve_ms": s_.value, "scatter_ms": o.value, "launches": k.value}
 
     def autotune(self, precision: int = FP64, count: int = 2048) -> dict:
-        """Times the domain and lane solves' shapes on `count` right-hand sides and keeps the fastest."""
+        """Times the spread solve and the shapes of the domain, global-scratch and lane solves on `count`
+        right-hand sides and keeps the fastest; returns the fastest shape and the kept solve's time."""
         cfg = np.zeros(5, np.int32)
         ms = C.c_double()
         _check(lib().yb_factor_autotune(self._h, precision, count, ptr(cfg), C.byref(ms)))
