@@ -7,7 +7,7 @@ import numpy as np
 import pytest
 
 import oracle.oracle as orc
-from fixtures import random_square
+from fixtures import random_spd, random_square, right_hand_sides, worst_relative_difference
 from ybus_b200 import FP64, GpuFactor, Pair, configs, grids, host
 
 pytestmark = pytest.mark.gpu
@@ -91,3 +91,45 @@ def test_an_infinite_right_hand_side_gives_what_substitution_gives(gpu, count):
     cpu = orc.solve_many(chol, rhs[:3])
     assert np.isinf(cpu[1:]).all() and np.array_equal(x[1:3], cpu[1:])
     assert np.isfinite(x[0]).all() and np.isfinite(x[3:]).all()
+
+
+def hub_grid(n_bus, extra, seed, branches):
+    """A grid with a hub: a top row of as many partial sums and entries as fill several warps."""
+    g = grids.make_grid(n_bus, extra, seed)
+    far = np.random.default_rng(seed).choice(np.arange(2, n_bus), branches, replace=False)
+    return dataclasses.replace(g, frm=np.r_[g.frm, np.full(branches, 1)], to=np.r_[g.to, far],
+                               x=np.r_[g.x, np.full(branches, 0.1)])
+
+
+@pytest.mark.parametrize("count", [1, 33, 1100])
+@pytest.mark.parametrize("name", ["hub", "dense", "dense lu", "half dense", "half dense lu"])
+def test_long_rows_and_dense_tops(gpu, name, count):
+    """Against the oracle at the bar of the other solves: the sums and the correction of a hub's rows, shared by a
+    block's warps, and corrections by dense triangles, orders around a tile's 16 rows and a block's 64."""
+    matrices = {"hub": lambda: [configs.bprime(hub_grid(1200, 400, 7, b)) for b in (70, 300)],
+                "dense": lambda: [random_spd(n, n, 7) for n in (31, 48, 65, 130)],
+                "dense lu": lambda: [random_square(n, n, 3) for n in (31, 48, 65, 130)],
+                "half dense": lambda: [random_spd(200, 3, 7)], "half dense lu": lambda: [random_square(120, 3, 3)]}[name]()
+    for a in matrices:
+        f = host.lu(a) if name.endswith("lu") else host.cholesky(a)
+        factor = GpuFactor.from_lu(gpu, f) if name.endswith("lu") else GpuFactor.from_cholesky(gpu, f)
+        assert factor.spread_info(FP64, count)["top"] > 0
+        rhs = right_hand_sides(f.n, count, 11)
+        assert worst_relative_difference(solve(gpu, factor, rhs)[::7], orc.solve_many(f, rhs[::7], threads=8)) < 1e-12
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+def test_a_value_not_finite_stays_in_its_island_of_a_dense_top(gpu, bad):
+    a = random_spd(40, 40, 7)
+    p, i, v = a.to_csr().arrays()
+    r = np.repeat(np.arange(40), np.diff(p))
+    two = host.Matrix.from_triplets(80, 80, np.r_[2 * r, 2 * r + 1], np.r_[2 * i, 2 * i + 1], np.r_[v, v])
+    factor = GpuFactor.from_cholesky(gpu, host.cholesky(two))
+    assert factor.spread_info(FP64, 40)["top"] > 0
+    b = np.random.default_rng(3).standard_normal((40, 80))
+    spoiled = b.copy()
+    spoiled[20, 10] = bad
+    clean, x = solve(gpu, factor, b), solve(gpu, factor, spoiled)
+    others = np.arange(40) != 20
+    assert np.array_equal(x[others], clean[others]) and not np.isfinite(x[20, 10])
+    assert worst_relative_difference(x[[20], 1::2], clean[[20], 1::2]) < 1e-12

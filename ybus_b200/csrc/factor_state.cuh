@@ -163,7 +163,7 @@ struct DeviceSpread : ResidualMatrix {
   const int32_t *task_row = nullptr, *fwd_page = nullptr, *bwd_page = nullptr, *in_pos = nullptr, *out_pos = nullptr;
   const int32_t *part_ptr = nullptr, *s_ptr = nullptr, *s_col = nullptr, *u_ptr = nullptr, *u_col = nullptr;
   const void *s_val = nullptr, *u_val = nullptr;
-  void *m = nullptr;
+  void *m = nullptr, *m_u = nullptr, *m_l = nullptr;
   std::vector<int32_t> host_out_pos;
 };
 

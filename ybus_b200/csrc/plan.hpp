@@ -277,6 +277,7 @@ LaneLayout lane_layout(const Plan<T> &plan, int32_t value_bytes, int32_t page_by
 // 2.6e-15, 5.3e-14 and 1.5e-11; a second correction changes nothing. A Cholesky factor's S x is a product
 // with S, which is sparse; a pivoted LU's is L_TT (U_TT x): rounding S itself costs as much as the map where
 // |L||U| is larger than S (the error of the 10,000-bus Jacobian's transposed solve 1.5e-13 by S, 1.5e-15 by its factors).
+// Triangles that are dense are multiplied as the map is.
 //
 // A packet is 16-byte aligned: a head {uint32 kind, bytes, count, 0}, then by kind
 //   kSpreadRows4 / kSpreadRows1: four (one) rows' records {value 0, value 1, 1/diagonal, uint32 slots,
@@ -336,6 +337,7 @@ template <class V> struct SpreadLayout {  // V: double or complex<double>, the p
   // what the map is corrected by, by rows (spread_correction_by_schur, _by_factors): S, or -L_TT and U_TT
   std::vector<int32_t> s_ptr, s_col, c_ptr, c_col;
   std::vector<V> s_val, c_val;
+  bool dense = false;                             // ... as dense arrays on the device
   double s_norm = 0;                              // a bound of the infinity norm of the top's Schur complement
 };
 

@@ -323,8 +323,9 @@ SpreadLayout<V> spread_layout(const Plan<V> &plan, int32_t value_bytes, int64_t 
       }
   }
   // each row's work over both sweeps, in cycles of a scheduler with warps to choose from (measured:
-  // about 80 for a row of two entries and sweep, 290 where a warp is alone), and each subtree's
-  constexpr double kRow = 110, kEntry = 12, kAlone = 3.6;
+  // about 80 for a row of two entries and sweep, 290 where a warp is alone), and each subtree's; and what
+  // a task costs before its first row, both sweeps' blocks (their first page and rows)
+  constexpr double kRow = 110, kEntry = 12, kAlone = 3.6, kStart = 900;
   std::vector<double> work(n), sub(n, 0.0);
   for (int32_t v = 0; v < n; ++v)
     work[v] = kRow + kEntry * (std::max(2, col_ptr[v + 1] - col_ptr[v]) + std::max(2, b1(v) - b0(v)));
@@ -344,17 +345,17 @@ SpreadLayout<V> spread_layout(const Plan<V> &plan, int32_t value_bytes, int64_t 
   // scheduler; the top's map: a tile's chain of steps, its values from L2, half the FP64 rate; and, with
   // a top, its launches.
   const double G = (double)std::max<int64_t>(1, groups);
-  // A complex top is four products of reals for one. That a map is applied twice is charged to neither: times
-  // are flat in these weights (the 10,000-bus B' with 1 to 13,499 right-hand sides, its Jacobian and 300 and
-  // 2,000 buses: within 3 % with the top's charged two and three times), but with 2 in place of 4 a batch of 16
-  // complex networks of 730 to 46,293 buses took 1,082 us for 1,001, with 8 1,531, and four other batches were within 3 %.
-  constexpr double kTop = sizeof(V) == 16 ? 4 : 1;
+  // A complex top is four products of reals for one, and a real FP64 one is applied twice. That a complex
+  // one is too is not charged: with 8 in place of 4 a batch of 16 networks of 730 to 46,293 buses took
+  // 1,531 us for 1,001, with 2 1,082, and four other batches were within 3 %.
+  const double kTop = sizeof(V) == 16 ? 4 : value_bytes == 8 ? 2 : 1;
+  const double kLaunches = value_bytes == (int32_t)sizeof(V) ? 14000 : 8000;  // five more, or two; without rows below the top two fewer
   auto cost_of = [&](const Cut &c) {
     const double all = c.tasks * std::ceil(G / 4), wave = (double)blocks * sms, full = std::floor(all / wave);
     const double left = std::ceil((all - full * wave) / sms);
-    const double sweeps = c.longest * (full * std::max<double>(kAlone, blocks) + (left > 0 ? std::max(kAlone, left) : 0.0));
+    const double sweeps = (c.longest + kStart) * (full * std::max<double>(kAlone, blocks) + (left > 0 ? std::max(kAlone, left) : 0.0));
     const double t = c.top;
-    return sweeps + (c.top ? 20 * t + t * t / 100 + kTop * G * t * t / sms + 8000 : 0);
+    return sweeps + (c.top ? 20 * t + t * t / 100 + kTop * G * t * t / sms + kLaunches - (c.top == n ? 6000 : 0) : 0);
   };
   constexpr int kCaps = 45;  // caps a quarter octave apart
   auto cap_of = [&](int k) { return total / std::pow(2.0, 1 + k / 4.0); };
@@ -371,11 +372,18 @@ SpreadLayout<V> spread_layout(const Plan<V> &plan, int32_t value_bytes, int64_t 
       else if (parent[v] < 0 || sub[parent[v]] > cap)
         c.roots.push_back(v), domain_work += sub[v], largest = std::max(largest, sub[v]);
     }
-    // as many tasks as keep the longest near the largest domain, no more than domains
+    // as many tasks as keep the longest near the largest domain, no more than domains; or a half, a quarter
+    // and so on of them where starting so many costs more
+    int32_t tasks = 1;
     if (!c.roots.empty())
-      c.tasks = (int32_t)std::max<double>(1, std::min<double>((double)c.roots.size(), std::ceil(domain_work / std::max(largest, 1.0))));
-    c.longest = std::max(largest, domain_work / c.tasks);
-    c.cost = c.top > kSpreadMostTop ? INFINITY : cost_of(c);
+      tasks = (int32_t)std::max<double>(1, std::min<double>((double)c.roots.size(), std::ceil(domain_work / std::max(largest, 1.0))));
+    c.cost = INFINITY;
+    for (; tasks >= 1 && c.top <= kSpreadMostTop; tasks /= 2) {
+      Cut t;
+      t.top = c.top, t.tasks = tasks, t.longest = std::max(largest, domain_work / tasks);
+      t.cost = cost_of(t);
+      if (t.cost < c.cost) c.tasks = t.tasks, c.longest = t.longest, c.cost = t.cost;
+    }
     return c;
   };
   auto choose = [&] {
@@ -630,7 +638,7 @@ SpreadLayout<V> spread_layout(const Plan<V> &plan, int32_t value_bytes, int64_t 
   if (fitting < blocks) {  // the slots let an SM hold fewer: for those, where the cut is then another
     blocks = fitting;
     const Cut again = choose();
-    if (again.cap != cut.cap) return lay_out(again);
+    if (again.cap != cut.cap || again.tasks != cut.tasks) return lay_out(again);
     lay.cost = again.cost;
   }
   return lay;
@@ -639,46 +647,25 @@ SpreadLayout<V> spread_layout(const Plan<V> &plan, int32_t value_bytes, int64_t 
 template SpreadLayout<double> spread_layout(const Plan<double> &, int32_t, int64_t, int32_t, int32_t, const std::function<int32_t(int32_t)> &);
 template SpreadLayout<host::c128> spread_layout(const Plan<host::c128> &, int32_t, int64_t, int32_t, int32_t, const std::function<int32_t(int32_t)> &);
 
-// S = L_TT U_TT by rows, each with the columns in order. Dense tops by several threads, a row at a time:
-// 1,500 dense rows are a billion products.
+// S = L_TT U_TT by rows, each with the columns in order.
 void spread_correction_by_schur(SpreadLayout<double> &lay) {
-  using V = double;
-  std::vector<std::vector<int32_t>> cols(lay.top);
-  std::vector<std::vector<V>> vals(lay.top);
-  std::atomic<int32_t> next{0};
-  std::exception_ptr error;
-  std::mutex error_mutex;
-  auto rows = [&] {
-    try {
-      std::vector<V> sum(lay.top);
-      std::vector<int32_t> seen(lay.top, -1);
-      for (int32_t i = next++; i < lay.top; i = next++) {
-        auto entry = [&](int32_t c, V v) {
-          if (seen[c] != i) seen[c] = i, sum[c] = V(0), cols[i].push_back(c);
-          sum[c] += v;
-        };
-        auto add = [&](V l, int32_t k) {  // l times U's row k
-          entry(k, l * (V(1) / lay.u_dinv[k]));
-          for (int32_t q = lay.u_ptr[k]; q < lay.u_ptr[k + 1]; ++q) entry(lay.u_col[q], l * lay.u_val[q]);
-        };
-        for (int32_t q = lay.l_ptr[i]; q < lay.l_ptr[i + 1]; ++q) add(lay.l_val[q], lay.l_col[q]);
-        add(V(1) / lay.l_dinv[i], i);
-        std::sort(cols[i].begin(), cols[i].end());
-        for (int32_t c : cols[i]) vals[i].push_back(sum[c]);
-      }
-    } catch (...) {
-      const std::lock_guard<std::mutex> lock(error_mutex);
-      error = std::current_exception();
-    }
-  };
-  double products = 0;
-  for (int32_t k : lay.l_col) products += lay.u_ptr[k + 1] - lay.u_ptr[k] + 1;
-  on_threads((int32_t)std::min(8.0, products / 1e6), rows);
-  if (error) std::rethrow_exception(error);
+  std::vector<double> sum(lay.top);
+  std::vector<int32_t> seen(lay.top, -1), cols;
   lay.s_ptr.assign(1, 0);
   for (int32_t i = 0; i < lay.top; ++i) {
-    lay.s_col.insert(lay.s_col.end(), cols[i].begin(), cols[i].end());
-    lay.s_val.insert(lay.s_val.end(), vals[i].begin(), vals[i].end());
+    cols.clear();
+    auto entry = [&](int32_t c, double v) {
+      if (seen[c] != i) seen[c] = i, sum[c] = 0, cols.push_back(c);
+      sum[c] += v;
+    };
+    auto add = [&](double l, int32_t k) {  // l times U's row k
+      entry(k, l * (1 / lay.u_dinv[k]));
+      for (int32_t q = lay.u_ptr[k]; q < lay.u_ptr[k + 1]; ++q) entry(lay.u_col[q], l * lay.u_val[q]);
+    };
+    for (int32_t q = lay.l_ptr[i]; q < lay.l_ptr[i + 1]; ++q) add(lay.l_val[q], lay.l_col[q]);
+    add(1 / lay.l_dinv[i], i);
+    std::sort(cols.begin(), cols.end());
+    for (int32_t c : cols) lay.s_col.push_back(c), lay.s_val.push_back(sum[c]);
     lay.s_ptr.push_back((int32_t)lay.s_col.size());
   }
 }

@@ -95,7 +95,7 @@ std::vector<std::unique_ptr<DeviceSpread>> make_spreads(const std::vector<const 
   struct Top {
     const int32_t *lp, *lc, *up, *uc;
     const M *lv, *ld, *uv, *ud, *sv = nullptr, *cv = nullptr;
-    M *scratch, *m;
+    M *scratch, *m, *m_u = nullptr, *m_l = nullptr;
   };
   std::vector<Top> tops(k);
   Packer temp;
@@ -118,8 +118,9 @@ std::vector<std::unique_ptr<DeviceSpread>> make_spreads(const std::vector<const 
     p.put(lay.task_row, d->task_row), p.put(lay.fwd_page, d->fwd_page), p.put(lay.bwd_page, d->bwd_page);
     p.put(lay.in_pos, d->in_pos), p.put(lay.out_pos, d->out_pos), p.put(lay.part_ptr, d->part_ptr);
     if (lay.top == 0) continue;
-    if (!lay.s_ptr.empty()) p.put(lay.s_ptr, d->s_ptr), p.put(lay.s_col, d->s_col), p.put(device_values(lay.s_val), t.sv);
-    if (!lay.c_ptr.empty()) p.put(lay.c_ptr, d->u_ptr), p.put(lay.c_col, d->u_col), p.put(device_values(lay.c_val), t.cv);
+    Packer &q = lay.dense ? temp : p;
+    if (!lay.s_ptr.empty()) q.put(lay.s_ptr, d->s_ptr), q.put(lay.s_col, d->s_col), q.put(device_values(lay.s_val), t.sv);
+    if (!lay.c_ptr.empty()) q.put(lay.c_ptr, d->u_ptr), q.put(lay.c_col, d->u_col), q.put(device_values(lay.c_val), t.cv);
     temp.put(lay.l_ptr, t.lp), temp.put(lay.l_col, t.lc);
     temp.put(device_values(lay.l_val), t.lv), temp.put(device_values(lay.l_dinv), t.ld);
     std::vector<int32_t> u_ptr{0}, u_col;  // the rows from the last to the first
@@ -140,16 +141,17 @@ std::vector<std::unique_ptr<DeviceSpread>> make_spreads(const std::vector<const 
     const int64_t t = d->top;
     most = std::max(most, d->top);
     if (t > 0) {
-      kept[i].place((size_t)(blocks(t, kSpreadTopRows) * t * kSpreadTopRows), tops[i].m);
+      const size_t full = (size_t)(blocks(t, kSpreadTopRows) * t * kSpreadTopRows);
+      kept[i].place(full, tops[i].m);
+      if (lays[i]->dense) kept[i].place(full, tops[i].m_u), kept[i].place(full, tops[i].m_l);
       temp.place((size_t)(blocks(t, 32) * t * 32), tops[i].scratch);
     }
     kept[i].place(lays[i]->blob.size(), d->blob);
     kept[i].upload(d->store, s);
     cuda_check(cudaMemcpyAsync(const_cast<uint8_t *>(d->blob), lays[i]->blob.data(), lays[i]->blob.size(), cudaMemcpyHostToDevice, s),
                "spread packet upload");
-    d->s_val = tops[i].sv, d->u_val = tops[i].cv;
     if (t == 0) continue;
-    d->m = tops[i].m;  // with the rows past the last of a block of rows
+    d->m = tops[i].m, d->m_u = tops[i].m_u, d->m_l = tops[i].m_l;  // with the rows past the last of a block of rows
     cuda_check(cudaMemsetAsync(d->m, 0, (size_t)(d->blob - (uint8_t *)d->m), s), "clear the maps");
   }
   if (most > 0) {
@@ -169,6 +171,19 @@ std::vector<std::unique_ptr<DeviceSpread>> make_spreads(const std::vector<const 
     cuda_check(cudaGetLastError(), "spread_map_kernel launch");
     spread_norm_kernel<M><<<dim3((unsigned)blocks(most, 256), (unsigned)k), 256, 0, s>>>(d_maps);
     cuda_check(cudaGetLastError(), "spread_norm_kernel launch");
+    for (size_t i = 0; i < k; ++i) {
+      DeviceSpread *d = out[i].get();
+      if (!d || d->top == 0) continue;
+      if (lays[i]->dense) {
+        const unsigned grid = (unsigned)blocks(d->top, 128);
+        spread_dense_kernel<M><<<grid, 128, 0, s>>>(d->top, d->u_ptr, d->u_col, tops[i].cv, tops[i].m_u);
+        spread_dense_kernel<M><<<grid, 128, 0, s>>>(d->top, d->s_ptr, d->s_col, tops[i].sv, tops[i].m_l);
+        cuda_check(cudaGetLastError(), "spread_dense_kernel launch");
+        d->s_ptr = d->s_col = d->u_ptr = d->u_col = nullptr;  // in the temporary array
+      } else {
+        d->s_val = tops[i].sv, d->u_val = tops[i].cv;
+      }
+    }
     std::vector<unsigned long long> bits(k);
     cuda_check(cudaMemcpyAsync(bits.data(), norms, bits.size() * sizeof bits[0], cudaMemcpyDeviceToHost, s), "download the norms");
     cuda_check(cudaStreamSynchronize(s), "the tops' maps");
@@ -193,6 +208,7 @@ SpreadNet net_of(const DeviceSpread *d, int64_t groups, int64_t count) {
   net.in_pos = d->in_pos, net.out_pos = d->out_pos, net.m = d->m;
   net.s_ptr = d->s_ptr, net.s_col = d->s_col, net.s_val = d->s_val;
   net.u_ptr = d->u_ptr, net.u_col = d->u_col, net.u_val = d->u_val;
+  net.m_u = d->m_u, net.m_l = d->m_l;
   net.groups = groups, net.count = count;
   return net;
 }
@@ -252,7 +268,8 @@ template <class T> void one_sweeps(const DeviceSpread *d, const SpreadArgs &a, c
   const int warps = sweep_warps<T>(a.slots, groups, gpu);
   const size_t smem = spread_smem<T>(a.slots, warps);
   const unsigned grid = (unsigned)(d->tasks * ((groups + warps - 1) / warps));
-  launch(spread_sweep_kernel<T, false, false>, grid, warps * 32, smem, s, true, a);
+  const bool below = d->top < d->n;  // rows below the top
+  if (below) launch(spread_sweep_kernel<T, false, false>, grid, warps * 32, smem, s, true, a);
   if (d->top > 0) {
     const unsigned rows = (unsigned)(groups * ((d->top + 7) / 8));
     launch(spread_sum_kernel<T, false>, rows, 256, 0, s, true, a);
@@ -268,21 +285,25 @@ template <class T> void one_sweeps(const DeviceSpread *d, const SpreadArgs &a, c
     };
     if constexpr (SpreadLane<T>::kCorrect) {
       top(std::integral_constant<int, 1>());
-      if (d->u_val) launch(spread_correct_kernel<T, false, true>, rows, 256, 0, s, true, a);
-      launch(spread_correct_kernel<T, false, false>, rows, 256, 0, s, true, a);
+      if (d->m_u) {
+        top(std::integral_constant<int, 3>()), top(std::integral_constant<int, 4>());
+      } else {
+        if (d->u_val) launch(spread_correct_kernel<T, false, true>, rows, 256, 0, s, true, a);
+        launch(spread_correct_kernel<T, false, false>, rows, 256, 0, s, true, a);
+      }
       top(std::integral_constant<int, 2>());
     } else {
       top(std::integral_constant<int, 0>());
     }
   }
-  launch(spread_sweep_kernel<T, true, false>, grid, warps * 32, smem, s, true, a);
+  if (below) launch(spread_sweep_kernel<T, true, false>, grid, warps * 32, smem, s, true, a);
 }
 
 // The partial array of `groups` groups: the partials and the top's solutions in T, then the top's
 // right-hand sides (and, where it is corrected, the first product and U_TT times it) in full precision (every
 // part a multiple of 128 bytes); at least one line.
 template <class T> size_t partial_bytes_of(const DeviceSpread *d, int64_t groups) {
-  return (size_t)groups * 32 * ((size_t)(d->partials + d->top) * sizeof(T) + (size_t)d->top * (!SpreadLane<T>::kCorrect ? 1 : d->u_val ? 3 : 2) * sizeof(typename SpreadLane<T>::Math)) + 128;
+  return (size_t)groups * 32 * ((size_t)(d->partials + d->top) * sizeof(T) + (size_t)d->top * (!SpreadLane<T>::kCorrect ? 1 : d->u_val || d->m_u ? 3 : 2) * sizeof(typename SpreadLane<T>::Math)) + 128;
 }
 template <class T> void set_partial(SpreadNet &net, uint8_t *p) {
   net.partial = p;
@@ -325,8 +346,10 @@ template <class V> std::unique_ptr<SpreadLayout<V>> try_layout(const yb_factor *
     auto lay = std::make_unique<SpreadLayout<V>>(host_spread(plan_of<V>(f), value_bytes, groups, f->gpu));
     if constexpr (!std::is_same_v<V, double>)
       spread_correction_by_factors(*lay);
-    else if (value_bytes == 8)
-      f->kind == YB_LU ? spread_correction_by_factors(*lay) : spread_correction_by_schur(*lay);
+    else if (value_bytes == 8) {
+      lay->dense = 8 * (lay->l_col.size() + lay->u_col.size()) > (size_t)lay->top * (size_t)lay->top;
+      lay->dense || f->kind == YB_LU ? spread_correction_by_factors(*lay) : spread_correction_by_schur(*lay);
+    }
     const int32_t limit = f->is_complex ? kSpreadAutoSlotsComplex : kSpreadAutoSlots;
     return lay->slots <= limit ? std::move(lay) : nullptr;
   } catch (const host::Error &e) {

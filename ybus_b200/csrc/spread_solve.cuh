@@ -48,9 +48,10 @@ struct SpreadNet {
   const int32_t *__restrict__ fwd_page, *__restrict__ bwd_page, *__restrict__ task_row, *__restrict__ part_ptr;
   const int32_t *__restrict__ in_pos, *__restrict__ out_pos;
   const void *__restrict__ m;  // the top's map in blocks of kSpreadTopRows rows
-  // what the product is corrected by, by rows: S, or (LU) U_TT and then -L_TT
+  // what the product is corrected by, by rows: S, or (LU) U_TT and then -L_TT; or these two dense, as m
   const int32_t *__restrict__ s_ptr, *__restrict__ s_col, *__restrict__ u_ptr, *__restrict__ u_col;
   const void *__restrict__ s_val, *__restrict__ u_val;  // u_val: null with S
+  const void *__restrict__ m_u, *__restrict__ m_l;
   int64_t groups, count;       // groups of a warp's columns (32, or 64 with two per lane), and columns
   void *work, *xout, *partial; // xout: where the backward sweep writes (work, or an array of its layout)
   void *r, *r2, *r3;           // the top's right-hand sides [group][top row][32 lanes], full precision; the first product; U_TT times it
@@ -472,80 +473,147 @@ __global__ void __launch_bounds__(kSpreadWarps * 32, spread_blocks<L>()) spread_
   asm volatile("cp.async.wait_all;" ::: "memory");  // the chunks past the task's rows
 }
 
+// Partial rows q0 to q1 of a group added to s, in order, eight loads in flight.
+template <class T, class M> __device__ __forceinline__ M spread_sum_rows(const T *part, int q0, int q1, M s) {
+  for (int q = q0; q < q1; q += 8) {
+    T p[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) p[i] = sp_ldg(part + (size_t)min(q + i, q1 - 1) * 32);
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (q + i < q1) s = sp_add(s, SpreadAs<M>::of(p[i]));
+  }
+  return s;
+}
+
+// A row of a block of eight that the block's eight warps share, an eighth each, added up in order: a hub's,
+// of more than 64 entries and most of all the block's, which would be one warp's chain (2,000 buses with a hub of
+// 300 branches: 52 us of 77 with the hub's rows to a warp each).
+__device__ __forceinline__ bool spread_long_row(int some, int of_block) { return some > 64 && 2 * some > of_block; }
+
 // The top's right-hand sides r_T: each top row's b and its partials, in order, in the factor's full
-// precision. A warp per row and group.
+// precision. A warp per row and group, long rows by all.
 template <class T, bool BATCH> __global__ void __launch_bounds__(256) spread_sum_kernel(const __grid_constant__ SpreadArgs a) {
   using M = typename SpreadLane<T>::Math;
+  __shared__ __align__(16) unsigned char shared[8 * 32 * sizeof(M)];
+  M *eighth = reinterpret_cast<M *>(shared);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   int64_t g;
-  int k;
+  int k0;
   const SpreadNet *np = &a.one;
   if constexpr (BATCH) {
     const SpreadItem it = a.items[blockIdx.x];
     np = a.nets + it.net;
-    g = it.b, k = it.a * 8 + warp;
+    g = it.b, k0 = it.a * 8;
   } else {
     const int blocks = (a.one.top + 7) / 8;
-    g = blockIdx.x / blocks, k = (int)(blockIdx.x % blocks) * 8 + warp;
+    g = blockIdx.x / blocks, k0 = (int)(blockIdx.x % blocks) * 8;
   }
   const SpreadNet &net = *np;
   sp_ready();
-  if (k >= net.top || (net.group_active && !net.group_active[g])) return;
+  if (net.group_active && !net.group_active[g]) return;  // the whole block
   const T *part = static_cast<const T *>(net.partial) + (size_t)g * net.partials * 32 + lane;
-  const int q1 = __ldg(net.part_ptr + k + 1);
-  int q = __ldg(net.part_ptr + k);
-  M s = SpreadAs<M>::of(sp_ldg(static_cast<const T *>(net.work) + ((size_t)g * net.n + net.n - net.top + k) * 32 + lane));
-  for (; q < q1; q += 4) {
-    T p[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) p[i] = sp_ldg(part + (size_t)min(q + i, q1 - 1) * 32);
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-      if (q + i < q1) s = sp_add(s, SpreadAs<M>::of(p[i]));
+  const T *b = static_cast<const T *>(net.work) + ((size_t)g * net.n + net.n - net.top) * 32 + lane;
+  M *r = static_cast<M *>(net.r) + (size_t)g * net.top * 32 + lane;
+  const int k = k0 + warp, of_block = __ldg(net.part_ptr + min(k0 + 8, net.top)) - __ldg(net.part_ptr + k0);
+  if (k < net.top) {
+    const int q0 = __ldg(net.part_ptr + k), q1 = __ldg(net.part_ptr + k + 1);
+    if (!spread_long_row(q1 - q0, of_block)) sp_stg(r + (size_t)k * 32, spread_sum_rows(part, q0, q1, SpreadAs<M>::of(sp_ldg(b + (size_t)k * 32))));
   }
-  sp_stg(static_cast<M *>(net.r) + ((size_t)g * net.top + k) * 32 + lane, s);
+  if (of_block <= 64) return;
+  for (int j = k0; j < min(k0 + 8, net.top); ++j) {  // alike in every warp
+    const int q0 = __ldg(net.part_ptr + j), some = __ldg(net.part_ptr + j + 1) - q0;
+    if (!spread_long_row(some, of_block)) continue;
+    eighth[warp * 32 + lane] = spread_sum_rows(part, q0 + some * warp / 8, q0 + some * (warp + 1) / 8, M{});
+    __syncthreads();
+    if (warp == 0) {
+      M s = SpreadAs<M>::of(sp_ldg(b + (size_t)j * 32));
+      for (int w = 0; w < 8; ++w) s = sp_add(s, eighth[w * 32 + lane]);
+      sp_stg(r + (size_t)j * 32, s);
+    }
+    __syncthreads();
+  }
+}
+
+__device__ __forceinline__ double sp_shfl(double v, int lane) { return __shfl_sync(0xffffffffu, v, lane); }
+__device__ __forceinline__ cplx<double> sp_shfl(const cplx<double> &v, int lane) {
+  return cplx<double>(__shfl_sync(0xffffffffu, v.re, lane), __shfl_sync(0xffffffffu, v.im, lane));
+}
+
+// s less the entries q0 to q1 times their rows of x: 32 entries at a time, a lane each, the next ones on their
+// way; their values of x eight in flight.
+template <class MS, class M>
+__device__ __forceinline__ M spread_row_product(const int32_t *col, const MS *val, const M *x, int q0, int q1, M s) {
+  const int lane = threadIdx.x & 31;
+  int c_next = 0;
+  MS v_next{};
+  auto fetch = [&](int at) {
+    if (at < q1) c_next = __ldg(col + at), v_next = sp_ldg(val + at);
+  };
+  fetch(q0 + lane);
+  for (int q = q0; q < q1; q += 32) {
+    const int some = min(32, q1 - q), c = c_next;
+    const MS v = v_next;
+    fetch(q + 32 + lane);
+    for (int j = 0; j < some; j += 8) {
+      M xs[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) xs[i] = sp_ldg(x + (size_t)__shfl_sync(0xffffffffu, c, min(j + i, some - 1)) * 32);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const MS vi = sp_shfl(v, min(j + i, some - 1));
+        if (j + i < some) s = sp_fnma(vi, xs[i], s);
+      }
+    }
+  }
+  return s;
 }
 
 // The residual of the first product, for its correction: r_T -= S r2, or (LU) r3 = -U_TT r2 (UPPER), then
-// r_T += L_TT r3, each row in place. A warp per row and group.
+// r_T += L_TT r3, each row in place. A warp per row and group, long rows by all.
 template <class T, bool BATCH, bool UPPER>
 __global__ void __launch_bounds__(256) spread_correct_kernel(const __grid_constant__ SpreadArgs a) {
   using M = typename SpreadLane<T>::Math;
   using MS = typename SpreadLane<T>::MathS;
+  __shared__ __align__(16) unsigned char shared[8 * 32 * sizeof(M)];
+  M *eighth = reinterpret_cast<M *>(shared);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   int64_t g;
-  int k;
+  int k0;
   const SpreadNet *np = &a.one;
   if constexpr (BATCH) {
     const SpreadItem it = a.items[blockIdx.x];
     np = a.nets + it.net;
-    g = it.b, k = it.a * 8 + warp;
+    g = it.b, k0 = it.a * 8;
   } else {
     const int blocks = (a.one.top + 7) / 8;
-    g = blockIdx.x / blocks, k = (int)(blockIdx.x % blocks) * 8 + warp;
+    g = blockIdx.x / blocks, k0 = (int)(blockIdx.x % blocks) * 8;
   }
   const SpreadNet &net = *np;
   sp_ready();
-  if (k >= net.top || (net.group_active && !net.group_active[g])) return;
+  if (net.group_active && !net.group_active[g]) return;  // the whole block
   const int32_t *ptr = UPPER ? net.u_ptr : net.s_ptr, *col = UPPER ? net.u_col : net.s_col;
   const MS *val = static_cast<const MS *>(UPPER ? net.u_val : net.s_val);
   const M *x = static_cast<const M *>(UPPER || !net.u_val ? net.r2 : net.r3) + (size_t)g * net.top * 32 + lane;
-  M *to = static_cast<M *>(UPPER ? net.r3 : net.r) + ((size_t)g * net.top + k) * 32 + lane;
-  const int q1 = __ldg(ptr + k + 1);
-  M s = UPPER ? M{} : sp_ldg(to);
-  for (int q = __ldg(ptr + k); q < q1; q += 4) {
-    M v[4];
-    MS c[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int at = min(q + i, q1 - 1);
-      c[i] = val[at], v[i] = sp_ldg(x + (size_t)__ldg(col + at) * 32);
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-      if (q + i < q1) s = sp_fnma(c[i], v[i], s);
+  M *to = static_cast<M *>(UPPER ? net.r3 : net.r) + (size_t)g * net.top * 32 + lane;
+  const int k = k0 + warp, of_block = __ldg(ptr + min(k0 + 8, net.top)) - __ldg(ptr + k0);
+  if (k < net.top) {
+    const int q0 = __ldg(ptr + k), q1 = __ldg(ptr + k + 1);
+    if (!spread_long_row(q1 - q0, of_block)) sp_stg(to + (size_t)k * 32, spread_row_product(col, val, x, q0, q1, UPPER ? M{} : sp_ldg(to + (size_t)k * 32)));
   }
-  sp_stg(to, s);
+  if (of_block <= 64) return;
+  for (int j = k0; j < min(k0 + 8, net.top); ++j) {  // alike in every warp
+    const int q0 = __ldg(ptr + j), some = __ldg(ptr + j + 1) - q0;
+    if (!spread_long_row(some, of_block)) continue;
+    eighth[warp * 32 + lane] = spread_row_product(col, val, x, q0 + some * warp / 8, q0 + some * (warp + 1) / 8, M{});
+    __syncthreads();
+    if (warp == 0) {
+      M s = UPPER ? M{} : sp_ldg(to + (size_t)j * 32);
+      for (int w = 0; w < 8; ++w) s = sp_add(s, eighth[w * 32 + lane]);
+      sp_stg(to + (size_t)j * 32, s);
+    }
+    __syncthreads();
+  }
 }
 
 // D += A B on the FP64 tensor cores: A 8 x 4 (lane: row lane / 4, column lane % 4), B 4 x 8 (row lane % 4,
@@ -585,7 +653,8 @@ template <class V> __device__ __forceinline__ V spread_top_entry(const V *m, con
 // The top's product on the FP64 tensor cores, 16 rows by 32 columns a warp, fragments straight from L2
 // (the map and a group's columns are read by many warps; four steps of loads in flight). PHASE 0: x_T =
 // M r_T; 1: r2 = M r_T; 2, with r_T the residual: x_T = r2 + M r_T, each entry of the correction where it is
-// finite (a right-hand side that is not leaves a residual that is NaN). KS > 1: a block's KS
+// finite (a right-hand side that is not leaves a residual that is NaN). The residual by dense triangles, their
+// zeros passed over: 3: r3 = U_TT r2; 4: r_T -= L_TT r3. KS > 1: a block's KS
 // warps split the map's columns and add up in order at the end: with few groups there are too few
 // tiles to fill the SMs, and a tile's chain of steps sets the time. x_T goes to its own rows after the
 // partials (the work array's top rows stay b_T) and to the separate output array if there is one.
@@ -615,16 +684,17 @@ __global__ void __launch_bounds__(spread_top_warps<T, KS>() * 32) spread_top_ker
   sp_ready();
   if (net.group_active && !net.group_active[g]) return;  // the whole block
   const int t = net.top, row0 = ((int)block * (WARPS / KS) + warp / KS) * 16;
-  const V *r = static_cast<const V *>(net.r) + (size_t)g * t * COLS + tile * 32 + lane / 4;
-  const V *m = static_cast<const V *>(net.m) + (size_t)(row0 / kSpreadTopRows) * t * kSpreadTopRows + row0 % kSpreadTopRows + lane / 4;
+  const void *from = PHASE == 3 ? net.r2 : PHASE == 4 ? net.r3 : net.r, *by = PHASE == 3 ? net.m_u : PHASE == 4 ? net.m_l : net.m;
+  const V *r = static_cast<const V *>(from) + (size_t)g * t * COLS + tile * 32 + lane / 4;
+  const V *m = static_cast<const V *>(by) + (size_t)(row0 / kSpreadTopRows) * t * kSpreadTopRows + row0 % kSpreadTopRows + lane / 4;
   V acc[2][4][2];
 #pragma unroll
   for (int i = 0; i < 2; ++i)
 #pragma unroll
     for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = V(0);
-  // this warp's share of the steps of four columns
-  const int steps = (t + 3) / 4;
-  const int s0 = (int)((int64_t)steps * (warp % KS) / KS), s1 = (int)((int64_t)steps * (warp % KS + 1) / KS);
+  // the steps of four columns that hold entries of these rows, and this warp's share of them
+  const int first = PHASE == 3 ? row0 / 4 : 0, steps = ((PHASE == 4 ? min(t, row0 + 16) : t) + 3) / 4 - first;
+  const int s0 = first + (int)((int64_t)steps * (warp % KS) / KS), s1 = first + (int)((int64_t)steps * (warp % KS + 1) / KS);
   if (row0 < t) {
 #pragma unroll 4
     for (int s = s0; s < s1; ++s) {
@@ -646,12 +716,18 @@ __global__ void __launch_bounds__(spread_top_warps<T, KS>() * 32) spread_top_ker
   auto store = [&](int row, int col, V v0, V v1) {
     if (row >= t) return;
     if (!sp_finite(v0) || !sp_finite(v1)) {
-      const V *mr = static_cast<const V *>(net.m) + (size_t)(row / kSpreadTopRows) * t * kSpreadTopRows + row % kSpreadTopRows;
-      const V *rc = static_cast<const V *>(net.r) + (size_t)g * t * COLS + tile * 32 + col;
+      const V *mr = static_cast<const V *>(by) + (size_t)(row / kSpreadTopRows) * t * kSpreadTopRows + row % kSpreadTopRows;
+      const V *rc = static_cast<const V *>(from) + (size_t)g * t * COLS + tile * 32 + col;
       if (!sp_finite(v0)) v0 = spread_top_entry(mr, rc, t, COLS);
       if (!sp_finite(v1)) v1 = spread_top_entry(mr, rc + 1, t, COLS);
     }
     V *between = r2 + (size_t)row * COLS + col;
+    if constexpr (PHASE == 3 || PHASE == 4) {
+      V *to = static_cast<V *>(PHASE == 3 ? net.r3 : net.r) + (size_t)g * t * COLS + tile * 32 + (size_t)row * COLS + col;
+      if constexpr (PHASE == 4) v0 = sp_add(to[0], v0), v1 = sp_add(to[1], v1);  // m_l is -L_TT
+      sp_store2(to, v0, v1);
+      return;
+    }
     if constexpr (PHASE == 1) {
       sp_store2(between, v0, v1);
       return;
@@ -762,6 +838,14 @@ template <class M> __global__ void __launch_bounds__(32) spread_map_kernel(const
 
 __device__ __forceinline__ double spread_abs(double v) { return fabs(v); }
 __device__ __forceinline__ double spread_abs(const cplx<double> &v) { return hypot(v.re, v.im); }
+
+// A triangle by rows into a dense array of the maps' layout, which is zero elsewhere; a thread a row.
+template <class M>
+__global__ void spread_dense_kernel(int t, const int32_t *__restrict__ ptr, const int32_t *__restrict__ col, const M *__restrict__ val, M *m) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= t) return;
+  for (int q = ptr[i]; q < ptr[i + 1]; ++q) m[((size_t)(i / kSpreadTopRows) * t + col[q]) * kSpreadTopRows + i % kSpreadTopRows] = val[q];
+}
 
 // ||M||inf as a bit pattern (positive doubles order as theirs; a NaN lies above them all).
 template <class M> __global__ void spread_norm_kernel(const SpreadMap<M> *__restrict__ maps) {
