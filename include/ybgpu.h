@@ -106,7 +106,8 @@ int32_t yb_factor_set_tile_kind(yb_factor *f, int32_t precision, int32_t kind);
  * domains and 32 right-hand sides, the top of the elimination forest as a dense map between the two
  * sweeps), which the automatic choice takes for plain solves. info receives 6 values for a solve of
  * `count` right-hand sides: {tasks (bundles), domains, top rows, live values per lane, partial values
- * per group of 32, bytes of its records}; YB_ERROR_INVALID_ARGUMENT if the solve takes another kind. */
+ * per group of 32, bytes of its records}; YB_ERROR_INVALID_ARGUMENT if a shape or threshold was set or the
+ * factor admits no such layout. Factors of at most eleven levels have one and are left to the other solves. */
 int32_t yb_factor_spread_info(yb_factor *f, int32_t precision, int64_t count, int64_t *info);
 /* No ybus counterpart: the lane solve (one right-hand side per lane, a block of warps per 32; the
  * factor's rows in an elimination-tree postorder cut into subtree domains the warps take in

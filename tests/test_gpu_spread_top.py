@@ -7,7 +7,7 @@ import numpy as np
 import pytest
 
 import oracle.oracle as orc
-from fixtures import random_spd, random_square, right_hand_sides, worst_relative_difference
+from fixtures import random_spd, random_square, right_hand_sides, star_spd, worst_relative_difference
 from ybus_b200 import FP64, GpuFactor, Pair, configs, grids, host
 
 pytestmark = pytest.mark.gpu
@@ -133,3 +133,16 @@ def test_a_value_not_finite_stays_in_its_island_of_a_dense_top(gpu, bad):
     others = np.arange(40) != 20
     assert np.array_equal(x[others], clean[others]) and not np.isfinite(x[20, 10])
     assert worst_relative_difference(x[[20], 1::2], clean[[20], 1::2]) < 1e-12
+
+
+@pytest.mark.parametrize("count", [1, 64, 300])
+def test_shallow_factors_keep_the_domain_solve(gpu, count):
+    """Its bits: a star, and the smallest factor."""
+    for a in (star_spd(200), random_spd(2, 1, 7)):
+        chol = host.cholesky(a)
+        rhs = right_hand_sides(chol.n, count, 5)
+        factor, domain = GpuFactor.from_cholesky(gpu, chol), GpuFactor.from_cholesky(gpu, chol)
+        domain.set_tile_kind(FP64, 4)
+        x = solve(gpu, factor, rhs)
+        assert np.array_equal(x, solve(gpu, domain, rhs))
+        assert worst_relative_difference(x, orc.solve_many(chol, rhs)) < 1e-12

@@ -961,7 +961,7 @@ void solve_device(yb_factor *f, const double *b, int64_t ldb, double *x, int64_t
   if (count <= 0 || f->n == 0) return;
   auto run = [&](auto zero, const TileConfig &configured, auto &fwd, auto &bwd, auto &scratch, auto &cache) {
     using T = decltype(zero);
-    if (configured.takes_spread() && spread_solve<T>(f, b, ldb, x, ldx, count, stream)) return;
+    if (takes_spread(f, configured) && spread_solve<T>(f, b, ldb, x, ldx, count, stream)) return;
     if (configured.kind == kTileLane || (configured.kind == kTileAuto && count >= lane_threshold<T>(f, configured))) {
       DeviceLane *d = lane_pick<T>(f, lane_shape(f, configured, count), configured.lane_rpl, stream);
       if (d && (configured.kind == kTileLane || d->slots <= kLaneAutoSlots)) {
@@ -1042,7 +1042,7 @@ __global__ void __launch_bounds__(256) pair_update_kernel(const int32_t *__restr
 }
 
 bool admits_spread_fp64(yb_factor *f, int64_t count, cudaStream_t stream) {
-  return count > 0 && f->n > 0 && f->tile64.takes_spread() && !f->single &&
+  return count > 0 && f->n > 0 && takes_spread(f, f->tile64) && !f->single &&
          spread_for(f, (int)sizeof(double), (count + 31) / 32, stream);
 }
 bool auto_spread_fp64(yb_factor *f, const double *b, int64_t ldb, double *x, int64_t ldx, int64_t count, cudaStream_t stream) {
@@ -1412,9 +1412,9 @@ extern "C" int32_t yb_factor_spread_info(yb_factor *f, int32_t precision, int64_
     cuda_check(cudaSetDevice(f->gpu->device), "cudaSetDevice");
     const TileConfig &t = precision == YB_FP64 ? f->tile64 : f->tile32;
     DeviceSpread *d = nullptr;
-    if (t.takes_spread() && !f->single && f->n > 0)
+    if (t.admits_spread() && !f->single && f->n > 0)
       d = spread_for(f, precision == YB_FP64 ? 8 : 4, (count + 31) / 32, f->gpu->stream);
-    if (!d) throw host::Error(host::kInvalidArgument, "the solve this precision runs is not the spread solve");
+    if (!d) throw host::Error(host::kInvalidArgument, "a shape was set or the factor admits no spread layout");
     const int64_t v[6] = {d->tasks, d->domains, d->top, d->slots, d->partials, d->blob_bytes};
     std::copy(v, v + 6, info);
     return YB_OK;
@@ -1524,6 +1524,8 @@ extern "C" int32_t yb_factor_attach_matrix(yb_factor *f, const int64_t *a_ptr, c
     f->a_csr_idx.upload(csr_idx, s);
     f->a_csr_val.upload(csr_val, s);
     cuda_check(cudaStreamSynchronize(s), "matrix upload");
+    f->a_longest = 0;
+    for (int64_t i = 0; i < n; ++i) f->a_longest = std::max(f->a_longest, a_ptr[i + 1] - a_ptr[i]);
     f->a_host_ptr.assign(a_ptr, a_ptr + n + 1);
     f->a_host_idx.assign(a_idx, a_idx + nnz);
     f->a_host_val.assign(a_val, a_val + nnz);
@@ -1713,7 +1715,7 @@ extern "C" int32_t yb_solve_many_refined_device(yb_factor *f, const double *d_rh
     // of a factor 8 against 347 ms.
     const auto bytes = [&](const double *p, int64_t ld) { return std::make_pair((uintptr_t)p, (uintptr_t)(p + (count - 1) * ld + f->n)); };
     const auto rb = bytes(d_rhs, ldb), rx = bytes(d_out, ldx);
-    if (t32.takes_spread() && !t32.refine_shaped && (rb.second <= rx.first || rx.second <= rb.first)) {
+    if (takes_spread(f, t32, kSpreadFewLevelsRefined) && !t32.refine_shaped && !has_hub(f) && (rb.second <= rx.first || rx.second <= rb.first)) {
       if (DeviceSpread *d = spread_for(f, (int)sizeof(float), (count + 31) / 32, s, f->a_attached)) {
         try {
           residual_matrix(f, d, d->host_out_pos, s);
@@ -1781,7 +1783,7 @@ extern "C" int32_t yb_factor_autotune(yb_factor *f, int32_t precision, int64_t c
     cuda_check(cudaGetLastError(), "autotune_fill_kernel launch");
     TileConfig &t = precision == YB_FP64 ? f->tile64 : f->tile32;
     TileConfig saved = t;
-    const bool with_spread = saved.takes_spread();  // no shape was set: the spread solve is in the choice
+    const bool with_spread = saved.admits_spread();  // no shape was set: the spread solve is in the choice
     saved.spread_first = false;
     TileConfig best = saved;
     double best_time = INFINITY, spread_time = INFINITY;

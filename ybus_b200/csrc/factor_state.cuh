@@ -109,7 +109,7 @@ struct TileConfig {
   bool shaped = false;
   // the autotuner left the shapes below as it found them fastest, and the spread solve faster still
   bool spread_first = false;
-  bool takes_spread() const { return spread_first || (kind == kTileAuto && !shaped); }
+  bool admits_spread() const { return spread_first || (kind == kTileAuto && !shaped); }
   void shape() { shaped = true, spread_first = false; }
   // the streamed solve's shape: warps per block, pages in flight per warp, page bytes, and the
   // row count under which a level goes to warp 0 (0: twice the rows of a slice)
@@ -284,6 +284,7 @@ struct yb_factor {
   std::vector<int64_t> a_host_ptr, a_host_idx;  // A as attached (CSR, natural order), on the host
   std::vector<double> a_host_val;
   int64_t a_attached = 0;                  // how many times a matrix was attached
+  int64_t a_longest = 0;                   // entries of its longest row
   // a complex LU factor (yb_factor_from_lu_complex): its plan, its sweeps in complex128 and
   // complex64, and the complex matrix attached for refinement (CSR, natural order)
   bool is_complex = false;
@@ -311,6 +312,21 @@ struct yb_factor {
 };
 
 namespace yb {
+// The automatic choice leaves factors whose elimination forest has few levels (stars, stars of stars, shallow
+// trees, a few rows) to the domain solve, one launch whose time goes by levels, and to the lane solve: by the
+// spread solve two rows took 11.7 against 9.3 us, a star of 200 22 to 55 against 21 to 39 us, one of 5,000 89 to
+// 359 against 59 to 121, eight to a branch over nine levels 44 and 77 against 31 and 58 with 300 and 1,024
+// right-hand sides, four to a branch over eleven 36 against 27 with 1,024; with 14 levels and more the domain solve
+// took 1.2 times as long and more. In the refined solve, whose passes are many launches either way, up to seven.
+constexpr int32_t kSpreadFewLevels = 11, kSpreadFewLevelsRefined = 7;
+inline bool takes_spread(const yb_factor *f, const TileConfig &t, int32_t few = kSpreadFewLevels) {
+  return t.spread_first || (t.admits_spread() && f->plan.fwd.levels > few);
+}
+// A refined solve also looks at the matrix: its residual takes a row by four lanes, so a hub's sets the time
+// (2,000 buses, a hub of 300 branches 295 us a solve against 543 by the domain solve; 10,000, of 1,500 1,062 against 579).
+inline bool has_hub(const yb_factor *f) {
+  return f->a_longest > 512 && f->a_longest * f->n > 16 * (int64_t)f->a_host_idx.size();
+}
 void solve_pairs_device(yb_factor *f, int64_t count, const int32_t *plus, const int32_t *minus, const double *base,
                         const double *alpha, const double *inverse_weight, int32_t *singular, double *out, int64_t ldo,
                         cudaStream_t stream, bool captured = false);
