@@ -139,3 +139,27 @@ def test_a_value_not_finite_stays_in_its_island_in_every_pass(gpu, count):
         assert np.isnan(x[count // 2, 10]) and np.isfinite(x[others]).all()
         assert worst_relative_difference(x[others], clean[others]) < 1e-12 if count > 1 else True
         assert worst_relative_difference(x[[count // 2], 1::2], clean2[[count // 2], 1::2]) < 1e-12
+
+
+@pytest.mark.parametrize("count", [1, 16, 129, 700])
+def test_residuals_of_a_network_with_a_hub(gpu, count):
+    """One column a piece while there are few, four from 513 on; the ratios told are those of the solutions."""
+    import torch
+    n = 400
+    k = np.arange(1, n)
+    r, c = np.r_[np.arange(n), np.zeros(n - 1, int), k], np.r_[np.arange(n), k, np.zeros(n - 1, int)]
+    v = np.r_[np.full(n, n + 1.0), np.full(2 * n - 2, -1.0)] * (1 + 0.3j)
+    a = host.Matrix.from_triplets(n, n, r, c, v, by_rows=False)
+    lu = host.lu(a, host.COLAMD)
+    f = GpuFactor.from_lu_complex(gpu, lu)
+    f.attach_matrix_complex(a)
+    dense = np.zeros((n, n), complex)
+    dense[r, c] = v
+    b = columns(n, count, 8)
+    ratio = [torch.zeros(count, dtype=torch.float64, device="cuda")]
+    for prec in (FP64, FP32):
+        (x,), _ = batch(gpu, [f], [b], prec, max_steps=3, ratios=ratio)
+        own = np.abs(b - x @ dense.T).max(axis=1) / np.abs(b).max(axis=1)
+        # both sums of 400 products: a bound on their rounding
+        assert np.abs(ratio[0].cpu().numpy() - own).max() <= 400 * 2.0 ** -52
+        assert worst_relative_difference(x, orc.solve_many_lu(lu, b)) < (1e-12 if prec == FP64 else 1e-8)

@@ -10,6 +10,7 @@
 
 #include <cuda_runtime.h>
 
+#include <cmath>
 #include <cstdint>
 #include <type_traits>
 
@@ -112,19 +113,27 @@ struct ResidualNet {
   int64_t ldx;
   cplx<double> *r;
   int64_t ldr;
-  unsigned long long *norms;  // ||r||inf and ||b||inf of each column, as bit patterns (of doubles >= 0 these order alike)
+  unsigned long long *norms;  // ||r||inf and ||b||inf of each column, as bit patterns (of doubles >= 0 these order alike), from the first residual on
 };
 struct ResidualItem {
   int32_t net, row, column, columns;  // kResidualRows rows from `row`, `columns` columns (at most kResidualColumns)
 };
 constexpr int kResidualRows = 1024, kResidualColumns = 4;
+// A row of more entries is a chain that four columns at once make longer, so such a network's pieces have one
+// while there are few (a star of 3,000 buses, complex64 refined with 16 and 128 right-hand sides: 1.0 and 1.1 against
+// 2.1 ms).
+constexpr int64_t kResidualLongRow = 128, kResidualFewColumns = 512;
+
+// ||r||inf / ||b||inf, 0 for a zero residual and infinity for a zero b with another
+__host__ __device__ inline double batch_ratio(double rn, double bn) { return bn > 0.0 ? rn / bn : (rn > 0.0 ? HUGE_VAL : 0.0); }
 
 // One block per ResidualItem. A row is a chain of loads (its bounds, a column index, an entry of x), so a
 // thread takes four columns' at once, and the blocks are pieces of rows, so large and small networks
 // fill the SMs alike. 21 million complex rows (16 networks of 730 to 46,293 buses, 128
 // columns each): 654 us; a block per column, its threads striding over all rows, took 1,121 us. The
 // entries of x come from L2 in sectors half used, 32 bytes each.
-__global__ void __launch_bounds__(256) batch_residual_kernel(const ResidualNet *__restrict__ nets, const ResidualItem *__restrict__ items) {
+__global__ void __launch_bounds__(256) batch_residual_kernel(const ResidualNet *__restrict__ nets, const ResidualItem *__restrict__ items,
+                                                             int64_t norms_at) {
   constexpr int C = kResidualColumns;
   __shared__ double most[8][2 * C];
   const ResidualItem it = items[blockIdx.x];
@@ -138,7 +147,8 @@ __global__ void __launch_bounds__(256) batch_residual_kernel(const ResidualNet *
     if (fabs(z.re) + fabs(z.im) > most) most = fmax(most, magnitude(z));
   };
   const int end = min(net.n, it.row + kResidualRows);
-  auto rows = [&](auto all) {
+  auto rows = [&](auto most_columns, auto all) {
+    constexpr int C = decltype(most_columns)::value;
     for (int i = it.row + (int)threadIdx.x; i < end; i += 256) {
       cplx<double> ax[C];
       const int p1 = net.a_ptr[i + 1];
@@ -159,9 +169,11 @@ __global__ void __launch_bounds__(256) batch_residual_kernel(const ResidualNet *
     }
   };
   if (it.columns == C)
-    rows(std::true_type());
+    rows(std::integral_constant<int, C>(), std::true_type());
+  else if (it.columns == 1)
+    rows(std::integral_constant<int, 1>(), std::true_type());
   else
-    rows(std::false_type());
+    rows(std::integral_constant<int, C>(), std::false_type());
 #pragma unroll
   for (int c = 0; c < 2 * C; ++c) {
 #pragma unroll
@@ -172,15 +184,14 @@ __global__ void __launch_bounds__(256) batch_residual_kernel(const ResidualNet *
   if (threadIdx.x < 2 * C && (int)threadIdx.x < 2 * it.columns) {
     double m = 0;
     for (int w = 0; w < 8; ++w) m = fmax(m, most[w][threadIdx.x]);
-    atomicMax(net.norms + 2 * it.column + threadIdx.x, (unsigned long long)__double_as_longlong(m));
+    atomicMax(net.norms + norms_at + 2 * it.column + threadIdx.x, (unsigned long long)__double_as_longlong(m));
   }
 }
 
 __global__ void __launch_bounds__(256) batch_ratio_kernel(int64_t columns, const unsigned long long *__restrict__ norms, double *__restrict__ ratio) {
   const int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (c >= columns) return;
-  const double rn = __longlong_as_double((long long)norms[2 * c]), bn = __longlong_as_double((long long)norms[2 * c + 1]);
-  ratio[c] = bn > 0.0 ? rn / bn : (rn > 0.0 ? __longlong_as_double(0x7ff0000000000000LL) : 0.0);
+  ratio[c] = batch_ratio(__longlong_as_double((long long)norms[2 * c]), __longlong_as_double((long long)norms[2 * c + 1]));
 }
 
 }  // namespace yb

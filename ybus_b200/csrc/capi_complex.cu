@@ -118,7 +118,8 @@ struct BatchWork {
   DeviceArray<cplx<float>> scratch64;
   DeviceArray<double> ratio;
   SpreadBatchWork spread;
-  cudaEvent_t done = nullptr;  // the last call's end
+  cudaEvent_t done = nullptr;     // the last call's end
+  unsigned long long stream = 0;  // ... and the number of its stream
   BatchWork() = default;
   BatchWork(const BatchWork &) = delete;
   BatchWork &operator=(const BatchWork &) = delete;
@@ -132,8 +133,11 @@ struct BatchTurn {
   BatchWork &w;
   cudaStream_t stream;
   BatchTurn(BatchWork &work, cudaStream_t s) : w(work), stream(s) {
+    unsigned long long id = 0;
+    cuda_check(cudaStreamGetId(stream, &id), "cudaStreamGetId");
     if (!w.done) cuda_check(cudaEventCreateWithFlags(&w.done, cudaEventDisableTiming), "cudaEventCreate");
-    cuda_check(cudaStreamWaitEvent(stream, w.done, 0), "cudaStreamWaitEvent");
+    if (id != w.stream) cuda_check(cudaStreamWaitEvent(stream, w.done, 0), "cudaStreamWaitEvent");
+    w.stream = id;
   }
   ~BatchTurn() { cudaEventRecord(w.done, stream); }
   BatchTurn(const BatchTurn &) = delete;
@@ -199,7 +203,8 @@ extern "C" int32_t yb_factor_attach_matrix_complex(yb_factor *f, const int64_t *
     cudaStream_t s = f->gpu->stream;
     f->za_ptr.upload(p, s), f->za_idx.upload(idx, s), f->za_val.upload(val, s);
     cuda_check(cudaStreamSynchronize(s), "matrix upload");
-    f->za_rows = n;
+    f->za_rows = n, f->za_longest = 0;
+    for (int64_t i = 0; i < n; ++i) f->za_longest = std::max(f->za_longest, a_ptr[i + 1] - a_ptr[i]);
     return YB_OK;
   });
 }
@@ -247,14 +252,15 @@ extern "C" int32_t yb_solve_batch_complex(int64_t networks, yb_factor *const *fa
       int64_t all_cols = 0;
       for (int64_t i = 0; i < networks; ++i) all_cols += cnt[i];
       w.ratio.reserve((size_t)std::max<int64_t>(all_cols, 1));
-      w.norms.reserve((size_t)std::max<int64_t>(2 * all_cols, 1));
+      w.norms.reserve((size_t)std::max<int64_t>(2 * all_cols * (max_steps + 2), 1));  // of every residual
       for (int64_t i = 0; i < networks; ++i) {
         yb_factor *f = fs[i];
         rn[i] = ResidualNet{(int32_t)f->n, f->za_ptr.get(), f->za_idx.get(), f->za_val.get(), b[i], f->n, x[i], f->n,
                             w.residual.get() + off, f->n, w.norms.get() + 2 * ratio_off};
+        const int64_t columns = f->za_longest > kResidualLongRow && cnt[i] <= kResidualFewColumns ? 1 : kResidualColumns;
         for (int64_t row = 0; row < f->n; row += kResidualRows)
-          for (int64_t c = 0; c < cnt[i]; c += kResidualColumns)
-            pieces.push_back({(int32_t)i, (int32_t)row, (int32_t)c, (int32_t)std::min<int64_t>(kResidualColumns, cnt[i] - c)});
+          for (int64_t c = 0; c < cnt[i]; c += columns)
+            pieces.push_back({(int32_t)i, (int32_t)row, (int32_t)c, (int32_t)std::min<int64_t>(columns, cnt[i] - c)});
         off += cnt[i] * f->n;
         ratio_off += cnt[i];
       }
@@ -267,17 +273,25 @@ extern "C" int32_t yb_solve_batch_complex(int64_t networks, yb_factor *const *fa
         cuda_check(cudaMemcpyAsync(w.pieces.get(), pieces.data(), sizeof(ResidualItem) * pieces.size(), cudaMemcpyHostToDevice, s),
                    "upload the residual's blocks");
     }
-    auto residual = [&]() -> std::vector<double> {
-      std::vector<double> ratios(max_total);
-      if (max_total == 0) return ratios;
-      cuda_check(cudaMemsetAsync(w.norms.get(), 0, sizeof(unsigned long long) * 2 * max_total, s), "clear the norms");
-      batch_residual_kernel<<<(unsigned)pieces.size(), 256, 0, s>>>(reinterpret_cast<const ResidualNet *>(w.rnets.get()), w.pieces.get());
+    int32_t residuals = 0;
+    if (max_total > 0)
+      cuda_check(cudaMemsetAsync(w.norms.get(), 0, sizeof(unsigned long long) * 2 * max_total * (max_steps + 2), s), "clear the norms");
+    auto residual = [&]() -> const unsigned long long * {
+      if (max_total == 0) return nullptr;
+      const int64_t at = 2 * max_total * residuals++;
+      batch_residual_kernel<<<(unsigned)pieces.size(), 256, 0, s>>>(reinterpret_cast<const ResidualNet *>(w.rnets.get()), w.pieces.get(), at);
       cuda_check(cudaGetLastError(), "batch_residual_kernel launch");
-      batch_ratio_kernel<<<(unsigned)((max_total + 255) / 256), 256, 0, s>>>(max_total, w.norms.get(), w.ratio.get());
-      cuda_check(cudaGetLastError(), "batch_ratio_kernel launch");
-      cuda_check(cudaMemcpyAsync(ratios.data(), w.ratio.get(), sizeof(double) * max_total, cudaMemcpyDeviceToHost, s),
-                 "download ratios");
+      return w.norms.get() + at;
+    };
+    // the residual and its ratios, here (the kernel's ratios are for the caller's arrays, a launch less a correction)
+    std::vector<double> norms((size_t)(2 * max_total));
+    auto ratios_now = [&] {
+      const unsigned long long *now = residual();
+      std::vector<double> ratios((size_t)max_total);
+      if (max_total == 0) return ratios;
+      cuda_check(cudaMemcpyAsync(norms.data(), now, sizeof(double) * 2 * max_total, cudaMemcpyDeviceToHost, s), "download norms");
       cuda_check(cudaStreamSynchronize(s), "residual");
+      for (int64_t c = 0; c < max_total; ++c) ratios[c] = batch_ratio(norms[2 * c], norms[2 * c + 1]);
       return ratios;
     };
     // the spread solve for the networks that have a layout (its gather and scatter move whole complex128
@@ -327,7 +341,7 @@ extern "C" int32_t yb_solve_batch_complex(int64_t networks, yb_factor *const *fa
       for (int64_t i = 0; i < networks; ++i) r[i] = rn[i].r;
       double previous = INFINITY;
       for (; taken < max_steps; ++taken) {
-        const auto ratios = residual();
+        const auto ratios = ratios_now();
         double worst = 0.0;
         bool nan = false;
         for (double v : ratios) nan = nan || std::isnan(v), worst = std::max(worst, v);
@@ -338,7 +352,11 @@ extern "C" int32_t yb_solve_batch_complex(int64_t networks, yb_factor *const *fa
     }
     spread_batch_solved(fs, value_bytes, cnt, taken + 1);
     if (d_ratio) {
-      const auto ratios = residual();
+      const unsigned long long *now = residual();
+      if (max_total > 0) {
+        batch_ratio_kernel<<<(unsigned)((max_total + 255) / 256), 256, 0, s>>>(max_total, now, w.ratio.get());
+        cuda_check(cudaGetLastError(), "batch_ratio_kernel launch");
+      }
       int64_t off = 0;
       for (int64_t i = 0; i < networks; ++i) {
         if (cnt[i] && d_ratio[i])
@@ -346,7 +364,7 @@ extern "C" int32_t yb_solve_batch_complex(int64_t networks, yb_factor *const *fa
                      "copy ratios");
         off += cnt[i];
       }
-      (void)ratios;
+      cuda_check(cudaStreamSynchronize(s), "ratios");
     }
     if (steps)
       for (int64_t i = 0; i < networks; ++i) steps[i] = taken;

@@ -291,7 +291,7 @@ struct yb_factor {
   yb::Plan<yb::host::c128> cplan;
   yb::DeviceSweep<yb::cplx<double>> fwdz, bwdz;
   yb::DeviceSweep<yb::cplx<float>> fwdc, bwdc;
-  int64_t za_rows = -1;
+  int64_t za_rows = -1, za_longest = 0;  // (its rows, and the entries of its longest)
   yb::DeviceArray<int32_t> za_ptr, za_idx;
   yb::DeviceArray<yb::cplx<double>> za_val;
   yb::PinnedBuffer staging;

@@ -409,7 +409,7 @@ void spread_for_batch(const std::vector<yb_factor *> &factors, int value_bytes, 
   for (size_t i = 0; i < k; ++i) {
     const std::lock_guard<std::mutex> lock(factors[i]->spread_mutex);
     const auto &there = factors[i]->spreads;
-    if (counts[i] > 0 && !there.count(keys[i]) && factors[i]->spread_passes[keys[i]] >= kSpreadBatchPasses &&
+    if (counts[i] > 0 && !small_for_batch(factors[i]) && !there.count(keys[i]) && factors[i]->spread_passes[keys[i]] >= kSpreadBatchPasses &&
         std::count_if(there.begin(), there.end(), [&](const auto &e) { return e.first.first == value_bytes; }) < kSpreadMostBatchLayouts &&
         seen.insert({factors[i], keys[i].second}).second)
       missing.push_back(i);
