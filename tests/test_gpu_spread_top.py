@@ -62,6 +62,29 @@ def test_residuals_on_grids_of_wide_reactances(gpu, decades, count):
     assert worst_residual(a, ys[some], rhs[some]) <= min(1e-12, max(4 * sub, 1e-14))
 
 
+@pytest.mark.parametrize("count", [64, 999])
+@pytest.mark.parametrize("n_bus,extra,seed,decades", [(2000, 700, 11, 0), (2000, 700, 12, 3), (1500, 520, 13, 3)])
+def test_errors_are_a_substitutions(gpu, n_bus, extra, seed, decades, count):
+    """The mean over 64 columns of the error against L L' x = b solved in extended precision, at most twice the
+    oracle's substitution's: rounding of the same bound, in other orders."""
+    g = wide_grid(n_bus, extra, seed, decades)
+    chol = host.cholesky(configs.bprime(g))
+    rhs, _ = branch_columns(g, count, 5)
+    x = solve(gpu, GpuFactor.from_cholesky(gpu, chol), rhs)[:64]
+    b = rhs[:64].T[chol.perm].astype(np.longdouble)
+    l, lt = chol.l, chol.lt  # the diagonal last, and first
+    for k in range(chol.n):
+        some = slice(l.ptr[k], l.ptr[k + 1] - 1)
+        b[k] = (b[k] - l.val[some].astype(np.longdouble) @ b[l.idx[some]]) / np.longdouble(l.val[l.ptr[k + 1] - 1])
+    for k in range(chol.n - 1, -1, -1):
+        some = slice(lt.ptr[k] + 1, lt.ptr[k + 1])
+        b[k] = (b[k] - lt.val[some].astype(np.longdouble) @ b[lt.idx[some]]) / np.longdouble(lt.val[lt.ptr[k]])
+    exact = np.empty_like(b)
+    exact[chol.perm] = b
+    error = lambda y: float((np.abs(y - exact.T).max(axis=1) / np.abs(exact.T).max(axis=1)).mean())  # noqa: E731
+    assert error(x) <= 2 * error(orc.solve_many(chol, rhs[:64], threads=8))
+
+
 @pytest.mark.parametrize("count", [1, 40, 300])
 @pytest.mark.parametrize("name", ["jacobian", "random"])
 def test_residuals_of_real_lu_factors(gpu, name, count):

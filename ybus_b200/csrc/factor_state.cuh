@@ -161,9 +161,9 @@ struct DeviceSpread : ResidualMatrix {
   DeviceArray<uint8_t> store;  // what the pointers below point into
   const uint8_t *blob = nullptr;
   const int32_t *task_row = nullptr, *fwd_page = nullptr, *bwd_page = nullptr, *in_pos = nullptr, *out_pos = nullptr;
-  const int32_t *part_ptr = nullptr, *s_ptr = nullptr, *s_col = nullptr, *u_ptr = nullptr, *u_col = nullptr;
-  const void *s_val = nullptr, *u_val = nullptr;
-  void *m = nullptr, *m_u = nullptr, *m_l = nullptr;
+  const int32_t *part_ptr = nullptr, *low_ptr = nullptr, *low_col = nullptr, *up_ptr = nullptr, *up_col = nullptr;
+  const void *low_val = nullptr, *up_val = nullptr;
+  void *m = nullptr, *m_up = nullptr, *m_low = nullptr;
   std::vector<int32_t> host_out_pos;
 };
 

@@ -274,10 +274,10 @@ LaneLayout lane_layout(const Plan<T> &plan, int32_t value_bytes, int32_t page_by
 // Without it the map's rounding, its condition times the unit roundoff, is all in the residual, up to a
 // hundred times a substitution's: with pairs of a 2,000-bus grid 5.7e-14 against 2.3e-15, with reactances
 // over three more decades 8.3e-12 against 5.3e-14, on the 10,000-bus Jacobian 6.1e-11 against 1.6e-11. With it
-// 2.6e-15, 5.3e-14 and 1.5e-11; a second correction changes nothing. A Cholesky factor's S x is a product
-// with S, which is sparse; a pivoted LU's is L_TT (U_TT x): rounding S itself costs as much as the map where
-// |L||U| is larger than S (the error of the 10,000-bus Jacobian's transposed solve 1.5e-13 by S, 1.5e-15 by its factors).
-// Triangles that are dense are multiplied as the map is.
+// 2.6e-15, 5.3e-14 and 1.5e-11; a second correction changes nothing. S x is L_TT (U_TT x): S itself, rounded, is
+// sparser, and its rounding costs as much as the map's (mean error of the grids' pairs 1.4e-14 and 1.4e-13 by S, 5.3e-15 and
+// 3.8e-14 by its factors, as by substitution; of the Jacobian's transposed solve 1.5e-13 and 1.5e-15). Triangles that
+// are dense are multiplied as the map is.
 //
 // A packet is 16-byte aligned: a head {uint32 kind, bytes, count, 0}, then by kind
 //   kSpreadRows4 / kSpreadRows1: four (one) rows' records {value 0, value 1, 1/diagonal, uint32 slots,
@@ -334,9 +334,9 @@ template <class V> struct SpreadLayout {  // V: double or complex<double>, the p
   // the top's own triangles by rows (columns as top indices) for its dense map
   std::vector<int32_t> l_ptr, l_col, u_ptr, u_col;
   std::vector<V> l_val, u_val, l_dinv, u_dinv;
-  // what the map is corrected by, by rows (spread_correction_by_schur, _by_factors): S, or -L_TT and U_TT
-  std::vector<int32_t> s_ptr, s_col, c_ptr, c_col;
-  std::vector<V> s_val, c_val;
+  // what the map is corrected by, by rows (spread_correction): -L_TT and U_TT, with their diagonals
+  std::vector<int32_t> low_ptr, low_col, up_ptr, up_col;
+  std::vector<V> low_val, up_val;
   bool dense = false;                             // ... as dense arrays on the device
   double s_norm = 0;                              // a bound of the infinity norm of the top's Schur complement
 };
@@ -351,8 +351,7 @@ template <class V>
 SpreadLayout<V> spread_layout(const Plan<V> &plan, int32_t value_bytes, int64_t groups, int32_t sms, int32_t blocks = 6,
                               const std::function<int32_t(int32_t)> &fit = {});
 
-// Fills a layout's matrices of the top's correction: S (a Cholesky factor's), or U_TT and -L_TT.
-void spread_correction_by_schur(SpreadLayout<double> &lay);
-template <class V> void spread_correction_by_factors(SpreadLayout<V> &lay);
+// Fills a layout's matrices of the top's correction.
+template <class V> void spread_correction(SpreadLayout<V> &lay);
 
 }  // namespace yb

@@ -647,41 +647,18 @@ SpreadLayout<V> spread_layout(const Plan<V> &plan, int32_t value_bytes, int64_t 
 template SpreadLayout<double> spread_layout(const Plan<double> &, int32_t, int64_t, int32_t, int32_t, const std::function<int32_t(int32_t)> &);
 template SpreadLayout<host::c128> spread_layout(const Plan<host::c128> &, int32_t, int64_t, int32_t, int32_t, const std::function<int32_t(int32_t)> &);
 
-// S = L_TT U_TT by rows, each with the columns in order.
-void spread_correction_by_schur(SpreadLayout<double> &lay) {
-  std::vector<double> sum(lay.top);
-  std::vector<int32_t> seen(lay.top, -1), cols;
-  lay.s_ptr.assign(1, 0);
+template <class V> void spread_correction(SpreadLayout<V> &lay) {
+  lay.low_ptr.assign(1, 0), lay.up_ptr.assign(1, 0);
   for (int32_t i = 0; i < lay.top; ++i) {
-    cols.clear();
-    auto entry = [&](int32_t c, double v) {
-      if (seen[c] != i) seen[c] = i, sum[c] = 0, cols.push_back(c);
-      sum[c] += v;
-    };
-    auto add = [&](double l, int32_t k) {  // l times U's row k
-      entry(k, l * (1 / lay.u_dinv[k]));
-      for (int32_t q = lay.u_ptr[k]; q < lay.u_ptr[k + 1]; ++q) entry(lay.u_col[q], l * lay.u_val[q]);
-    };
-    for (int32_t q = lay.l_ptr[i]; q < lay.l_ptr[i + 1]; ++q) add(lay.l_val[q], lay.l_col[q]);
-    add(1 / lay.l_dinv[i], i);
-    std::sort(cols.begin(), cols.end());
-    for (int32_t c : cols) lay.s_col.push_back(c), lay.s_val.push_back(sum[c]);
-    lay.s_ptr.push_back((int32_t)lay.s_col.size());
+    for (int32_t q = lay.l_ptr[i]; q < lay.l_ptr[i + 1]; ++q) lay.low_col.push_back(lay.l_col[q]), lay.low_val.push_back(-lay.l_val[q]);
+    lay.low_col.push_back(i), lay.low_val.push_back(-V(1) / lay.l_dinv[i]);
+    lay.low_ptr.push_back((int32_t)lay.low_col.size());
+    for (int32_t q = lay.u_ptr[i]; q < lay.u_ptr[i + 1]; ++q) lay.up_col.push_back(lay.u_col[q]), lay.up_val.push_back(lay.u_val[q]);
+    lay.up_col.push_back(i), lay.up_val.push_back(V(1) / lay.u_dinv[i]);
+    lay.up_ptr.push_back((int32_t)lay.up_col.size());
   }
 }
-
-template <class V> void spread_correction_by_factors(SpreadLayout<V> &lay) {
-  lay.s_ptr.assign(1, 0), lay.c_ptr.assign(1, 0);
-  for (int32_t i = 0; i < lay.top; ++i) {
-    for (int32_t q = lay.l_ptr[i]; q < lay.l_ptr[i + 1]; ++q) lay.s_col.push_back(lay.l_col[q]), lay.s_val.push_back(-lay.l_val[q]);
-    lay.s_col.push_back(i), lay.s_val.push_back(-V(1) / lay.l_dinv[i]);
-    lay.s_ptr.push_back((int32_t)lay.s_col.size());
-    for (int32_t q = lay.u_ptr[i]; q < lay.u_ptr[i + 1]; ++q) lay.c_col.push_back(lay.u_col[q]), lay.c_val.push_back(lay.u_val[q]);
-    lay.c_col.push_back(i), lay.c_val.push_back(V(1) / lay.u_dinv[i]);
-    lay.c_ptr.push_back((int32_t)lay.c_col.size());
-  }
-}
-template void spread_correction_by_factors(SpreadLayout<double> &);
-template void spread_correction_by_factors(SpreadLayout<host::c128> &);
+template void spread_correction(SpreadLayout<double> &);
+template void spread_correction(SpreadLayout<host::c128> &);
 
 }  // namespace yb

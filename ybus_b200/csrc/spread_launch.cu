@@ -94,8 +94,8 @@ std::vector<std::unique_ptr<DeviceSpread>> make_spreads(const std::vector<const 
   std::vector<Packer> kept(k);
   struct Top {
     const int32_t *lp, *lc, *up, *uc;
-    const M *lv, *ld, *uv, *ud, *sv = nullptr, *cv = nullptr;
-    M *scratch, *m, *m_u = nullptr, *m_l = nullptr;
+    const M *lv, *ld, *uv, *ud, *low = nullptr, *up_v = nullptr;
+    M *scratch, *m, *m_up = nullptr, *m_low = nullptr;
   };
   std::vector<Top> tops(k);
   Packer temp;
@@ -119,8 +119,10 @@ std::vector<std::unique_ptr<DeviceSpread>> make_spreads(const std::vector<const 
     p.put(lay.in_pos, d->in_pos), p.put(lay.out_pos, d->out_pos), p.put(lay.part_ptr, d->part_ptr);
     if (lay.top == 0) continue;
     Packer &q = lay.dense ? temp : p;
-    if (!lay.s_ptr.empty()) q.put(lay.s_ptr, d->s_ptr), q.put(lay.s_col, d->s_col), q.put(device_values(lay.s_val), t.sv);
-    if (!lay.c_ptr.empty()) q.put(lay.c_ptr, d->u_ptr), q.put(lay.c_col, d->u_col), q.put(device_values(lay.c_val), t.cv);
+    if (!lay.low_ptr.empty()) {
+      q.put(lay.low_ptr, d->low_ptr), q.put(lay.low_col, d->low_col), q.put(device_values(lay.low_val), t.low);
+      q.put(lay.up_ptr, d->up_ptr), q.put(lay.up_col, d->up_col), q.put(device_values(lay.up_val), t.up_v);
+    }
     temp.put(lay.l_ptr, t.lp), temp.put(lay.l_col, t.lc);
     temp.put(device_values(lay.l_val), t.lv), temp.put(device_values(lay.l_dinv), t.ld);
     std::vector<int32_t> u_ptr{0}, u_col;  // the rows from the last to the first
@@ -143,7 +145,7 @@ std::vector<std::unique_ptr<DeviceSpread>> make_spreads(const std::vector<const 
     if (t > 0) {
       const size_t full = (size_t)(blocks(t, kSpreadTopRows) * t * kSpreadTopRows);
       kept[i].place(full, tops[i].m);
-      if (lays[i]->dense) kept[i].place(full, tops[i].m_u), kept[i].place(full, tops[i].m_l);
+      if (lays[i]->dense) kept[i].place(full, tops[i].m_up), kept[i].place(full, tops[i].m_low);
       temp.place((size_t)(blocks(t, 32) * t * 32), tops[i].scratch);
     }
     kept[i].place(lays[i]->blob.size(), d->blob);
@@ -151,7 +153,7 @@ std::vector<std::unique_ptr<DeviceSpread>> make_spreads(const std::vector<const 
     cuda_check(cudaMemcpyAsync(const_cast<uint8_t *>(d->blob), lays[i]->blob.data(), lays[i]->blob.size(), cudaMemcpyHostToDevice, s),
                "spread packet upload");
     if (t == 0) continue;
-    d->m = tops[i].m, d->m_u = tops[i].m_u, d->m_l = tops[i].m_l;  // with the rows past the last of a block of rows
+    d->m = tops[i].m, d->m_up = tops[i].m_up, d->m_low = tops[i].m_low;  // with the rows past the last of a block of rows
     cuda_check(cudaMemsetAsync(d->m, 0, (size_t)(d->blob - (uint8_t *)d->m), s), "clear the maps");
   }
   if (most > 0) {
@@ -176,12 +178,12 @@ std::vector<std::unique_ptr<DeviceSpread>> make_spreads(const std::vector<const 
       if (!d || d->top == 0) continue;
       if (lays[i]->dense) {
         const unsigned grid = (unsigned)blocks(d->top, 128);
-        spread_dense_kernel<M><<<grid, 128, 0, s>>>(d->top, d->u_ptr, d->u_col, tops[i].cv, tops[i].m_u);
-        spread_dense_kernel<M><<<grid, 128, 0, s>>>(d->top, d->s_ptr, d->s_col, tops[i].sv, tops[i].m_l);
+        spread_dense_kernel<M><<<grid, 128, 0, s>>>(d->top, d->up_ptr, d->up_col, tops[i].up_v, tops[i].m_up);
+        spread_dense_kernel<M><<<grid, 128, 0, s>>>(d->top, d->low_ptr, d->low_col, tops[i].low, tops[i].m_low);
         cuda_check(cudaGetLastError(), "spread_dense_kernel launch");
-        d->s_ptr = d->s_col = d->u_ptr = d->u_col = nullptr;  // in the temporary array
+        d->low_ptr = d->low_col = d->up_ptr = d->up_col = nullptr;  // in the temporary array
       } else {
-        d->s_val = tops[i].sv, d->u_val = tops[i].cv;
+        d->low_val = tops[i].low, d->up_val = tops[i].up_v;
       }
     }
     std::vector<unsigned long long> bits(k);
@@ -206,9 +208,9 @@ SpreadNet net_of(const DeviceSpread *d, int64_t groups, int64_t count) {
   net.blob = d->blob, net.fwd_page = d->fwd_page, net.bwd_page = d->bwd_page;
   net.task_row = d->task_row, net.part_ptr = d->part_ptr;
   net.in_pos = d->in_pos, net.out_pos = d->out_pos, net.m = d->m;
-  net.s_ptr = d->s_ptr, net.s_col = d->s_col, net.s_val = d->s_val;
-  net.u_ptr = d->u_ptr, net.u_col = d->u_col, net.u_val = d->u_val;
-  net.m_u = d->m_u, net.m_l = d->m_l;
+  net.low_ptr = d->low_ptr, net.low_col = d->low_col, net.low_val = d->low_val;
+  net.up_ptr = d->up_ptr, net.up_col = d->up_col, net.up_val = d->up_val;
+  net.m_up = d->m_up, net.m_low = d->m_low;
   net.groups = groups, net.count = count;
   return net;
 }
@@ -285,10 +287,10 @@ template <class T> void one_sweeps(const DeviceSpread *d, const SpreadArgs &a, c
     };
     if constexpr (SpreadLane<T>::kCorrect) {
       top(std::integral_constant<int, 1>());
-      if (d->m_u) {
+      if (d->m_up) {
         top(std::integral_constant<int, 3>()), top(std::integral_constant<int, 4>());
       } else {
-        if (d->u_val) launch(spread_correct_kernel<T, false, true>, rows, 256, 0, s, true, a);
+        launch(spread_correct_kernel<T, false, true>, rows, 256, 0, s, true, a);
         launch(spread_correct_kernel<T, false, false>, rows, 256, 0, s, true, a);
       }
       top(std::integral_constant<int, 2>());
@@ -303,7 +305,7 @@ template <class T> void one_sweeps(const DeviceSpread *d, const SpreadArgs &a, c
 // right-hand sides (and, where it is corrected, the first product and U_TT times it) in full precision (every
 // part a multiple of 128 bytes); at least one line.
 template <class T> size_t partial_bytes_of(const DeviceSpread *d, int64_t groups) {
-  return (size_t)groups * 32 * ((size_t)(d->partials + d->top) * sizeof(T) + (size_t)d->top * (!SpreadLane<T>::kCorrect ? 1 : d->u_val || d->m_u ? 3 : 2) * sizeof(typename SpreadLane<T>::Math)) + 128;
+  return (size_t)groups * 32 * ((size_t)(d->partials + d->top) * sizeof(T) + (size_t)d->top * (SpreadLane<T>::kCorrect ? 3 : 1) * sizeof(typename SpreadLane<T>::Math)) + 128;
 }
 template <class T> void set_partial(SpreadNet &net, uint8_t *p) {
   net.partial = p;
@@ -344,11 +346,9 @@ template <class V> const Plan<V> &plan_of(const yb_factor *f) {
 template <class V> std::unique_ptr<SpreadLayout<V>> try_layout(const yb_factor *f, int value_bytes, int64_t groups) {
   try {
     auto lay = std::make_unique<SpreadLayout<V>>(host_spread(plan_of<V>(f), value_bytes, groups, f->gpu));
-    if constexpr (!std::is_same_v<V, double>)
-      spread_correction_by_factors(*lay);
-    else if (value_bytes == 8) {
-      lay->dense = 8 * (lay->l_col.size() + lay->u_col.size()) > (size_t)lay->top * (size_t)lay->top;
-      lay->dense || f->kind == YB_LU ? spread_correction_by_factors(*lay) : spread_correction_by_schur(*lay);
+    if (!std::is_same_v<V, double> || value_bytes == 8) {  // not in real FP32
+      lay->dense = std::is_same_v<V, double> && 8 * (lay->l_col.size() + lay->u_col.size()) > (size_t)lay->top * (size_t)lay->top;
+      spread_correction(*lay);
     }
     const int32_t limit = f->is_complex ? kSpreadAutoSlotsComplex : kSpreadAutoSlots;
     return lay->slots <= limit ? std::move(lay) : nullptr;

@@ -48,10 +48,10 @@ struct SpreadNet {
   const int32_t *__restrict__ fwd_page, *__restrict__ bwd_page, *__restrict__ task_row, *__restrict__ part_ptr;
   const int32_t *__restrict__ in_pos, *__restrict__ out_pos;
   const void *__restrict__ m;  // the top's map in blocks of kSpreadTopRows rows
-  // what the product is corrected by, by rows: S, or (LU) U_TT and then -L_TT; or these two dense, as m
-  const int32_t *__restrict__ s_ptr, *__restrict__ s_col, *__restrict__ u_ptr, *__restrict__ u_col;
-  const void *__restrict__ s_val, *__restrict__ u_val;  // u_val: null with S
-  const void *__restrict__ m_u, *__restrict__ m_l;
+  // what the product is corrected by, by rows: U_TT and then -L_TT; or these two dense, as m
+  const int32_t *__restrict__ low_ptr, *__restrict__ low_col, *__restrict__ up_ptr, *__restrict__ up_col;
+  const void *__restrict__ low_val, *__restrict__ up_val;
+  const void *__restrict__ m_up, *__restrict__ m_low;
   int64_t groups, count;       // groups of a warp's columns (32, or 64 with two per lane), and columns
   void *work, *xout, *partial; // xout: where the backward sweep writes (work, or an array of its layout)
   void *r, *r2, *r3;           // the top's right-hand sides [group][top row][32 lanes], full precision; the first product; U_TT times it
@@ -569,8 +569,8 @@ __device__ __forceinline__ M spread_row_product(const int32_t *col, const MS *va
   return s;
 }
 
-// The residual of the first product, for its correction: r_T -= S r2, or (LU) r3 = -U_TT r2 (UPPER), then
-// r_T += L_TT r3, each row in place. A warp per row and group, long rows by all.
+// The residual of the first product, for its correction: r3 = -U_TT r2 (UPPER), then r_T += L_TT r3, each row in
+// place. A warp per row and group, long rows by all.
 template <class T, bool BATCH, bool UPPER>
 __global__ void __launch_bounds__(256) spread_correct_kernel(const __grid_constant__ SpreadArgs a) {
   using M = typename SpreadLane<T>::Math;
@@ -592,9 +592,9 @@ __global__ void __launch_bounds__(256) spread_correct_kernel(const __grid_consta
   const SpreadNet &net = *np;
   sp_ready();
   if (net.group_active && !net.group_active[g]) return;  // the whole block
-  const int32_t *ptr = UPPER ? net.u_ptr : net.s_ptr, *col = UPPER ? net.u_col : net.s_col;
-  const MS *val = static_cast<const MS *>(UPPER ? net.u_val : net.s_val);
-  const M *x = static_cast<const M *>(UPPER || !net.u_val ? net.r2 : net.r3) + (size_t)g * net.top * 32 + lane;
+  const int32_t *ptr = UPPER ? net.up_ptr : net.low_ptr, *col = UPPER ? net.up_col : net.low_col;
+  const MS *val = static_cast<const MS *>(UPPER ? net.up_val : net.low_val);
+  const M *x = static_cast<const M *>(UPPER ? net.r2 : net.r3) + (size_t)g * net.top * 32 + lane;
   M *to = static_cast<M *>(UPPER ? net.r3 : net.r) + (size_t)g * net.top * 32 + lane;
   const int k = k0 + warp, of_block = __ldg(ptr + min(k0 + 8, net.top)) - __ldg(ptr + k0);
   if (k < net.top) {
@@ -684,7 +684,7 @@ __global__ void __launch_bounds__(spread_top_warps<T, KS>() * 32) spread_top_ker
   sp_ready();
   if (net.group_active && !net.group_active[g]) return;  // the whole block
   const int t = net.top, row0 = ((int)block * (WARPS / KS) + warp / KS) * 16;
-  const void *from = PHASE == 3 ? net.r2 : PHASE == 4 ? net.r3 : net.r, *by = PHASE == 3 ? net.m_u : PHASE == 4 ? net.m_l : net.m;
+  const void *from = PHASE == 3 ? net.r2 : PHASE == 4 ? net.r3 : net.r, *by = PHASE == 3 ? net.m_up : PHASE == 4 ? net.m_low : net.m;
   const V *r = static_cast<const V *>(from) + (size_t)g * t * COLS + tile * 32 + lane / 4;
   const V *m = static_cast<const V *>(by) + (size_t)(row0 / kSpreadTopRows) * t * kSpreadTopRows + row0 % kSpreadTopRows + lane / 4;
   V acc[2][4][2];
@@ -724,7 +724,7 @@ __global__ void __launch_bounds__(spread_top_warps<T, KS>() * 32) spread_top_ker
     V *between = r2 + (size_t)row * COLS + col;
     if constexpr (PHASE == 3 || PHASE == 4) {
       V *to = static_cast<V *>(PHASE == 3 ? net.r3 : net.r) + (size_t)g * t * COLS + tile * 32 + (size_t)row * COLS + col;
-      if constexpr (PHASE == 4) v0 = sp_add(to[0], v0), v1 = sp_add(to[1], v1);  // m_l is -L_TT
+      if constexpr (PHASE == 4) v0 = sp_add(to[0], v0), v1 = sp_add(to[1], v1);  // m_low is -L_TT
       sp_store2(to, v0, v1);
       return;
     }
