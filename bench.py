@@ -502,12 +502,14 @@ def main():
         replicas.barrier()
         return replicas.max_over_ranks(elapsed_ms), launch_ms, kernels
 
-    # which solve each mode runs (the library's automatic choice, read back from its settings)
-    ir_launches = 2 + 6 * (IR_MAX_STEPS + 1)
+    # which solve each mode runs (the library's automatic choice, read back from its settings): in FP64 the
+    # gather, the forward sweep, the top's sums, product, residual (two) and correction, the backward sweep and
+    # the scatter; for FP32 with refinement see below
+    fp64_launches, ir_launches = 9, 2 + 6 * (IR_MAX_STEPS + 1)
 
     def solver_of(mode):
-        if mode == "fp64":  # gather, forward sweep, the top's sums and product, backward sweep, scatter
-            return {"solver": "spread", "kernel": "spread_sweep_kernel<double>", "launches_per_step": 6,
+        if mode == "fp64":
+            return {"solver": "spread", "kernel": "spread_sweep_kernel<double>", "launches_per_step": fp64_launches,
                     "spread": factor.spread_info(FP64, count)}
         # an initialisation and the gather; per pass two sweeps, the top's sums and product, a residual (the
         # update and the decisions folded in) and what it leaves to do (kernels of groups that have stopped
@@ -567,7 +569,7 @@ def main():
                 steps_w = max(3, min(a.steps, 10))
                 elapsed_ms, launch_ms, _ = timed(lambda: blocks(mode, width), steps=steps_w)
                 r = check(mode, {"rhs_s": total * steps_w / (elapsed_ms / 1e3), "ms_per_step": elapsed_ms / steps_w,
-                                 "launches_per_step": -(-count // width) * (6 if mode == "fp64" else ir_launches)})
+                                 "launches_per_step": -(-count // width) * (fp64_launches if mode == "fp64" else ir_launches)})
                 r["solver"] = solver_of(mode)["solver"]
                 by_width[str(width)][mode] = r
     clock_info = clocks.stop()
