@@ -143,7 +143,7 @@ def test_a_value_not_finite_stays_in_its_island_in_every_pass(gpu, count):
 
 @pytest.mark.parametrize("count", [1, 16, 129, 700])
 def test_residuals_of_a_network_with_a_hub(gpu, count):
-    """One column a piece while there are few, four from 513 on; the ratios told are those of the solutions."""
+    """One column a piece; the ratios told are those of the solutions."""
     import torch
     n = 400
     k = np.arange(1, n)

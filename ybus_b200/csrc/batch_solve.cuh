@@ -119,10 +119,10 @@ struct ResidualItem {
   int32_t net, row, column, columns;  // kResidualRows rows from `row`, `columns` columns (at most kResidualColumns)
 };
 constexpr int kResidualRows = 1024, kResidualColumns = 4;
-// A row of more entries is a chain that four columns at once make longer, so such a network's pieces have one
-// while there are few (a star of 3,000 buses, complex64 refined with 16 and 128 right-hand sides: 1.0 and 1.1 against
-// 2.1 ms).
-constexpr int64_t kResidualLongRow = 128, kResidualFewColumns = 512;
+// A row of more entries is a chain that four columns at once make longer, so such a network's pieces have one (a
+// star of 3,000 buses, complex64 refined with 16 and 1,024 right-hand sides: 1.0 and 2.9 against 2.1 and 3.0 ms), and so
+// have all where four would leave SMs without a block.
+constexpr int64_t kResidualLongRow = 128;
 
 // ||r||inf / ||b||inf, 0 for a zero residual and infinity for a zero b with another
 __host__ __device__ inline double batch_ratio(double rn, double bn) { return bn > 0.0 ? rn / bn : (rn > 0.0 ? HUGE_VAL : 0.0); }

@@ -253,11 +253,15 @@ extern "C" int32_t yb_solve_batch_complex(int64_t networks, yb_factor *const *fa
       for (int64_t i = 0; i < networks; ++i) all_cols += cnt[i];
       w.ratio.reserve((size_t)std::max<int64_t>(all_cols, 1));
       w.norms.reserve((size_t)std::max<int64_t>(2 * all_cols * (max_steps + 2), 1));  // of every residual
+      int64_t fours = 0;
+      for (int64_t i = 0; i < networks; ++i)
+        fours += (fs[i]->n + kResidualRows - 1) / kResidualRows * ((cnt[i] + kResidualColumns - 1) / kResidualColumns);
+      const bool few = fours < gpu->sm_count;
       for (int64_t i = 0; i < networks; ++i) {
         yb_factor *f = fs[i];
         rn[i] = ResidualNet{(int32_t)f->n, f->za_ptr.get(), f->za_idx.get(), f->za_val.get(), b[i], f->n, x[i], f->n,
                             w.residual.get() + off, f->n, w.norms.get() + 2 * ratio_off};
-        const int64_t columns = f->za_longest > kResidualLongRow && cnt[i] <= kResidualFewColumns ? 1 : kResidualColumns;
+        const int64_t columns = few || f->za_longest > kResidualLongRow ? 1 : kResidualColumns;
         for (int64_t row = 0; row < f->n; row += kResidualRows)
           for (int64_t c = 0; c < cnt[i]; c += columns)
             pieces.push_back({(int32_t)i, (int32_t)row, (int32_t)c, (int32_t)std::min<int64_t>(columns, cnt[i] - c)});

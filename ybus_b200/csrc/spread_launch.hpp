@@ -63,12 +63,10 @@ void spread_sweeps(yb_factor *f, DeviceSpread *d, T *work, T *xout, uint8_t *par
 // 0.93 ms with it), so a factor that is solved once or twice never pays for it, and one that is solved often
 // twice what the better choice would have cost.
 constexpr int kSpreadBatchPasses = 4;
-// A few rows, or some hundred under one another in few levels, are less than the launches: two rows 14 us by tiles
-// and 19 to 27 so, eight to a branch over seven levels in complex64 with refinement 128 to 147 and 142 to 180. (A star
-// of 3,000, 480 and 124 us, is not.)
-inline bool small_for_batch(const yb_factor *f) {
-  return f->n < 16 || (f->n <= 1024 && f->cplan.fwd.levels <= kSpreadFewLevelsRefined);
-}
+// A few rows, or some hundred in few levels, are less than the launches: two rows 14 us by tiles and 19 to 27 so,
+// 585 rows of eight to a branch (13 levels) in complex64 with refinement 128 to 147 and 135 to 180. (30 buses, 17
+// levels, 160 and 120 us, and a star of 3,000, 480 and 124 us, are not.)
+inline bool small_for_batch(const yb_factor *f) { return f->n < 16 || (f->n <= 1024 && f->cplan.fwd.levels <= 13); }
 constexpr int kSpreadMostBatchLayouts = 8;  // a complex factor keeps of one precision; further classes take the nearest
 
 // The spread layouts of a batch of complex factors with these counts of right-hand sides: of the class the batch
