@@ -364,7 +364,7 @@ __global__ void outage_epilogue_kernel(const double *__restrict__ theta, int64_t
 // kOutageBranches branches for a group of 32 columns, each of its warps every eighth, the branches' data in
 // shared memory, each angle of the group one line; columns of one case read the same y. Each column's
 // largest of a block's goes to the parts, which the next kernel reduces. 9,728 columns of the 10,000-bus grid:
-// 626 us after 852 us of solves, against 4.7 ms of the domain solve with the epilogue in its store, which had
+// 619 us after 912 us of solves, against 4.7 ms of the domain solve with the epilogue in its store, which had
 // one column's angles in shared memory at a time; L2's reads of angles bound it (2.2 GB).
 constexpr int kOutageBranches = 1024;
 struct OutageLanes {
@@ -1201,7 +1201,7 @@ __global__ void flow_loss_kernel(const double *__restrict__ theta, int64_t n, in
 
 // q = Bf' g over the unknowns, an unknown's branches in order: a thread takes one unknown for eight
 // scenarios, whose entries of g it has in flight together. 1,024 scenarios of the 10,000-bus grid: 114 us, and
-// the spread solve 165 us; the domain solve that built them in its load took 650 us.
+// the spread solve 191 us; the domain solve that built them in its load took 650 us.
 __global__ void __launch_bounds__(256) adjoint_rhs_kernel(const double *__restrict__ g, int64_t nl, const int32_t *__restrict__ inc_ptr,
                                                           const int32_t *__restrict__ inc_branch,
                                                           const double *__restrict__ inc_value, int64_t n, int64_t count,

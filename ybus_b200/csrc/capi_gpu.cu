@@ -961,7 +961,8 @@ void solve_device(yb_factor *f, const double *b, int64_t ldb, double *x, int64_t
   if (count <= 0 || f->n == 0) return;
   auto run = [&](auto zero, const TileConfig &configured, auto &fwd, auto &bwd, auto &scratch, auto &cache) {
     using T = decltype(zero);
-    if (takes_spread(f, configured) && spread_solve<T>(f, b, ldb, x, ldx, count, stream)) return;
+    const bool lanes = sizeof(T) == sizeof(double) && lanes_for_few_rows(f, configured, count);
+    if (takes_spread(f, configured) && !lanes && spread_solve<T>(f, b, ldb, x, ldx, count, stream)) return;
     if (configured.kind == kTileLane || (configured.kind == kTileAuto && count >= lane_threshold<T>(f, configured))) {
       DeviceLane *d = lane_pick<T>(f, lane_shape(f, configured, count), configured.lane_rpl, stream);
       if (d && (configured.kind == kTileLane || d->slots <= kLaneAutoSlots)) {
@@ -1054,7 +1055,7 @@ bool auto_spread_fp64(yb_factor *f, const double *b, int64_t ldb, double *x, int
 // given (then alpha, inverse_weight and singular too). `captured`: the launches go into a graph that is
 // kept, so a solve that takes its workspace from the factor's is not for them.
 // The automatic choice for a Cholesky factor writes the right-hand sides out and takes the spread solve in
-// place: a block of 1,000 pairs of the 10,000-bus B' 153 us, against 325 us by the domain solve, and 12 against
+// place: a block of 1,000 pairs of the 10,000-bus B' 200 us, against 325 us by the domain solve, and 12 against
 // 300 ms for a factor's first. LU factors keep the domain solve, else the global-scratch solve.
 void solve_pairs_device(yb_factor *f, int64_t count, const int32_t *plus, const int32_t *minus, const double *base,
                         const double *alpha, const double *inverse_weight, int32_t *singular, double *out, int64_t ldo,

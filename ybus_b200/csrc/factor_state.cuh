@@ -322,6 +322,12 @@ constexpr int32_t kSpreadFewLevels = 11, kSpreadFewLevelsRefined = 7;
 inline bool takes_spread(const yb_factor *f, const TileConfig &t, int32_t few = kSpreadFewLevels) {
   return t.spread_first || (t.admits_spread() && f->plan.fwd.levels > few);
 }
+// Of a few rows and thousands of right-hand sides the nine launches of an FP64 solve are more than the lane solve's
+// three (100 rows with 2,500, 7,000 and 13,499 right-hand sides 30, 35 and 50 us against 29, 29 and 37; 200 rows 34, 46 and
+// 63 against 35, 42 and 53; 300 rows 38, 48 and 87 against 41, 47 and 72 us).
+inline bool lanes_for_few_rows(const yb_factor *f, const TileConfig &t, int64_t count) {
+  return !t.spread_first && f->n <= 256 && count >= 2048;
+}
 // A refined solve also looks at the matrix: its residual takes a row by four lanes, so a hub's sets the time
 // (2,000 buses, a hub of 300 branches 295 us a solve against 543 by the domain solve; 10,000, of 1,500 1,062 against 579).
 inline bool has_hub(const yb_factor *f) {

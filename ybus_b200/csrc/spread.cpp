@@ -350,12 +350,16 @@ SpreadLayout<V> spread_layout(const Plan<V> &plan, int32_t value_bytes, int64_t 
   // 1,531 us for 1,001, with 2 1,082, and four other batches were within 3 %.
   const double kTop = sizeof(V) == 16 ? 4 : value_bytes == 8 ? 2 : 1;
   const double kLaunches = value_bytes == (int32_t)sizeof(V) ? 14000 : 8000;  // five more, or two; without rows below the top two fewer
+  // and a corrected top's rows: their sums and residual (3,000 buses with 7,000 and 13,499 right-hand sides 310 to 286
+  // and 587 to 530 us, 8,000 with 7,000 708 to 691, 10,000 with 1 to 13,499 the same within 2 %; with 150 in place of
+  // 80 one 10,000-bus grid's 13,499 took 1,657 us for 1,585)
+  const double kRows = value_bytes == (int32_t)sizeof(V) && sizeof(V) == 8 ? 80 : 0;
   auto cost_of = [&](const Cut &c) {
     const double all = c.tasks * std::ceil(G / 4), wave = (double)blocks * sms, full = std::floor(all / wave);
     const double left = std::ceil((all - full * wave) / sms);
     const double sweeps = (c.longest + kStart) * (full * std::max<double>(kAlone, blocks) + (left > 0 ? std::max(kAlone, left) : 0.0));
     const double t = c.top;
-    return sweeps + (c.top ? 20 * t + t * t / 100 + kTop * G * t * t / sms + kLaunches - (c.top == n ? 6000 : 0) : 0);
+    return sweeps + (c.top ? 20 * t + t * t / 100 + kTop * G * t * t / sms + kRows * G * t / sms + kLaunches - (c.top == n ? 6000 : 0) : 0);
   };
   constexpr int kCaps = 45;  // caps a quarter octave apart
   auto cap_of = [&](int k) { return total / std::pow(2.0, 1 + k / 4.0); };

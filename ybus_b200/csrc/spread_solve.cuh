@@ -6,7 +6,8 @@
 //   spread_sweep  every task forward: z over b in the work array, updates of top rows into the
 //                 partial array
 //   spread_sum    the top's right-hand sides r_T: b_T plus the partials
-//   spread_top    x_T as a dense product of r_T; but in FP32 twice, spread_correct between them
+//   spread_top    x_T as a dense product of r_T; but in real FP32 twice, and between them the residual, by
+//                 spread_correct or, where the top's triangles are dense, by spread_top
 //   spread_sweep  every task backward, from the top solutions
 //   spread_out    the work array into x
 //
@@ -18,13 +19,14 @@
 // (a block's cooperation on one group, as in the lane solve, allows 16 warps at most).
 //
 // Measured on a B200, FP64 with device arrays, against the domain and lane solves that took these
-// sizes before: 2,000-bus B' with one right-hand side 71 to 29 us; 10,000-bus B' with 64, 87 to 42 us,
-// with 999, 330 to 141 us, with 13,499, 1,684 to 1,494 us (the gather 0.36 and the scatter 0.35 ms at
-// 6.1 TB/s, the sweeps and the top 0.82 ms: 5.3 TB/s over their 4.3 GB); the 10,000-bus Jacobian's LU
-// with 4,096, 1,336 to 1,036 us; 16 complex networks of 730 to 46,293 buses with 128 each, complex128 7.5 to
-// 0.91 ms, complex64 with refinement 21.1 to 4.3 ms. What bounds it: for large blocks HBM in the gather and scatter and
-// the shared-memory pipe (about 18 wavefronts a row and sweep) near HBM in the sweeps; for small ones
-// the six launches and the longest task's chain (about 290 cycles a row where a warp is alone).
+// sizes before: 2,000-bus B' with one right-hand side 71 to 44 us; 10,000-bus B' with 64, 87 to 62 us,
+// with 999, 329 to 175 us, with 13,499, 1,684 to 1,585 us (the gather 0.36 and the scatter 0.34 ms at
+// 6.1 TB/s, the sweeps and the top 0.90 ms); the 10,000-bus Jacobian's LU with 4,096, 1,333 to 1,076 us; 16 complex
+// networks of 730 to 46,293 buses with 128 each, complex128 7.5 to 0.93 ms, complex64 with refinement 21.0 to
+// 4.4 ms. Of these the top's correction costs 15, 25, 34, 90, 40 and 20 us. What bounds it: for large
+// blocks HBM in the gather and scatter and the shared-memory pipe (about 18 wavefronts a row and sweep) near HBM in
+// the sweeps; for small ones the nine launches and the longest task's chain (about 290 cycles a row where a warp is
+// alone).
 #pragma once
 
 #include <cuda_runtime.h>
