@@ -99,8 +99,9 @@ int32_t yb_gpu_set_work_bytes(yb_gpu *gpu, int64_t bytes);
  * else the global-scratch solve), 1 the level-sliced shared-memory solve, 2 the global-scratch
  * solve, 3 the streamed solve, 4 the domain solve, 5 the lane solve (1, 3, 4 and 5 give
  * YB_ERROR_INVALID_ARGUMENT at launch if the tile does not fit in shared memory or the factor
- * admits no domain or lane layout). The lane solve serves yb_solve_many_device and yb_solve_many;
- * the pair, refined and batched solves take the automatic choice among the others. */
+ * admits no domain or lane layout). The lane solve serves yb_solve_many_device, yb_solve_many and the refined
+ * solve; the pair solves take the domain solve beside it. The automatic choice of the pair solves (Cholesky)
+ * and of the refined solve is the spread solve too; the complex batch chooses by itself. */
 int32_t yb_factor_set_tile_kind(yb_factor *f, int32_t precision, int32_t kind);
 /* No ybus counterpart: the spread solve (one right-hand side per lane, one warp per bundle of subtree
  * domains and 32 right-hand sides, the top of the elimination forest as a dense map between the two
@@ -380,9 +381,10 @@ int32_t yb_dc_outage_solutions(yb_dc_network *net, int64_t cases, const int64_t 
  * finite or above 1e5 in magnitude (with a singular case, the reference's reasons to distrust a
  * screened outage and solve it again on the CPU, gpu.rs:406-410); per case whether the update is
  * singular (1/b - c'y = 0: a bridge). All cases run as one pair solve and one
- * scenario solve with the update, flows and maxima fused (YB_FP64), captured in a CUDA graph that
- * later calls of the same sizes replay; or with FP32 substitution and FP64 refinement, then the
- * same epilogue (YB_FP32; the slack must be bus 0). */
+ * scenario solve followed by the update, flows and maxima (YB_FP64): by the spread solve, launched anew, or
+ * where that is not the factor's choice fused into the domain solve and captured in a CUDA graph that
+ * calls of the same sizes replay until one of other sizes comes; or with FP32 substitution and FP64
+ * refinement, then the same epilogue (YB_FP32; the slack must be bus 0). */
 int32_t yb_dc_outage_loadings_batch(yb_dc_network *net, int64_t cases, const int64_t *outaged,
                                     const int64_t *scenario_ptr, const double *injections, const double *weights,
                                     int32_t precision, int64_t *max_branch, double *max_loading, int32_t *flags,
